@@ -251,12 +251,12 @@ int choose_tile(fiu_ctx* ctx, const fiu_resident* res, const ScanWork& w, int re
             cudaError_t e = tensor3_layer(*r->t3, w, ctx->stream);
             if (e != cudaSuccess) return cuda_fail(ctx, e, "tensor work items of a distribution layer");
         } else {
-            cudaError_t e = tensor3_order_items(*r->t3, r->d, w.order);
+            cudaError_t e = tensor3_order_items(*r->t3, r->d, w.order, ctx->stream);
             if (e != cudaSuccess) return cuda_fail(ctx, e, "tensor work items");
         }
         kernel = FIU_KERNEL_TENSOR;
         // GEMM width N: order 3 uses 256 with one accumulator for both classes, 192 with one per class
-        tp = (w.order != 3 || r->t3->pack) ? 256 : 192;
+        tp = (w.order != 3 || r->t3->pair3) ? 256 : 192;
         return FIU_OK;
     }
     int rc = choose_kernel(ctx, res, (unsigned)w.order, requested_kernel, kernel);

@@ -167,14 +167,27 @@ cudaError_t launch_elided4p(const ScanWork& w, const long long* begin, long long
 // (row 2*snp+g = "genotype of snp == g" per sample, cases then controls, each
 // class padded to a multiple of 128 samples), their TMA descriptors and the
 // work-item prefix sums.
+// 4-bit operand layout of a data set (tensor_fp4.cuh, tensor3x.cu): e2m1 planes
+// for the operand that the MMA reads as it is, bit rows for the one its kernel
+// builds.
+struct F4Plan {
+    uint8_t* planes = nullptr;  // rows of wpr x 16 bytes, SNPs in groups of 8 (f4_row)
+    uint32_t* bits = nullptr;   // rows 2 snp + g of wpr words, one bit a sample
+    int pack = 0;               // log2 of the control weight W when one accumulator holds both classes (else 0)
+    int rows = 0, wpr = 0;      // plane rows; 32-sample words per row, cases then controls, each padded to 256
+    int nw_c = 0, nw_t = 0;     // 64-sample steps that hold samples, per class
+    CUtensorMap map_b;          // planes, box 128 B x 120 rows, 128-byte swizzle
+    CUtensorMap map_j, map_i;   // bit rows, boxes of 32 B x 64 and x 2 rows
+};
 struct T3Plan {
-    std::mutex items_mu;  // guards the order-3 / order-4 item tables made on first use
+    std::mutex items_mu;  // guards the planes and item tables made on the first use of an order
+    F4Plan f4;
     uint8_t* planes = nullptr;
     int pack = 0;         // log2 of the control weight W when one accumulator holds both classes (else 0)
     double item_combos = 0;  // combinations per work item, about 32 x L / 2
     int pitch = 0;        // bytes per plane row
     int k_cases = 0;      // padded case samples (= byte offset of the control region)
-    bool pair3 = false;   // order 3, packed classes: pair items (i, 64 j, 128 l) of the CTA-pair kernel
+    bool pair3 = false;   // order 3, classes that share an accumulator: items of the CTA-pair kernel (tensor3x.cu)
     struct T3Layers* layers = nullptr;  // order 3, packed: work items of Distribution layers (tensor3.cu)
     long long* item_begin = nullptr;
     long long total = 0;  // work items
@@ -213,8 +226,12 @@ double tensor_item_combos(const T3Plan& plan, const ScanWork& w);
 bool tensor_layer_ok(const T3Plan& plan, const ScanWork& w);
 cudaError_t tensor3_layer(T3Plan& plan, const ScanWork& w, cudaStream_t s);
 cudaError_t tensor3_prepare(const DevData& d, T3Plan& plan, cudaStream_t s);
-// The whole data set's work items at order 3 or 4, made on first use (thread-safe).
-cudaError_t tensor3_order_items(T3Plan& plan, const DevData& d, int order);
+// The operand planes that searches of an order read and the whole data set's
+// work items at order 3 or 4, made on first use (thread-safe).
+cudaError_t tensor3_order_items(T3Plan& plan, const DevData& d, int order, cudaStream_t s);
+// Tiled TMA map over rows of `pitch` bytes: boxes of box_bytes x box_rows, 128-byte swizzle or none.
+cudaError_t tensor_map(CUtensorMap* m, const void* base, int rows, int pitch, int box_bytes, int box_rows,
+                       bool swizzle);
 void tensor3_release(T3Plan& plan);
 cudaError_t launch_tensor3(const ScanWork& w, const T3Plan& plan, long long g0, long long g1, const CandSink& sink,
                            uint32_t* dump, const uint32_t* single, const uint4* pairs, const uint4* triples,

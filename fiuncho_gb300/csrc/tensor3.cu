@@ -56,7 +56,9 @@
 #include <tuple>
 #include <mutex>
 
-#include "tensor_common.cuh"
+#include "tensor3_eval.cuh"
+#include "tensor3x.h"
+#include "tensor_fp4.cuh"
 
 namespace fiu {
 
@@ -150,69 +152,14 @@ __device__ __forceinline__ int t3_slot(int jl, int k, int xy) {
     return ((jl * 8 + k) * 4 + xy) ^ ((jl & 3) | (((jl ^ (k >> 1)) & 3) << 2));
 }
 
-// Float view of the packed 16-bit pair cores [class][x][y].
-__device__ __forceinline__ float pcf(const uint4& v, int k) {
-    const uint32_t w = (&v.x)[k >> 1];
-    return u2f((k & 1) ? (w >> 16) : (w & 0xffffu));
-}
-
-// Full 27-cell table of one class in single precision (every value an exact
-// integer), the derivation of expand3: core[(x*2+y)*2+z], pair cores of
-// (i,j), (i,l), (j,l), singles of i, j, l, class size.
-__device__ __forceinline__ void expand3f(const float* core, const uint4& pij, const uint4& pil, const uint4& pjl,
-                                         const float* si, const float* sj, const float* sl, float ncls, int cls,
-                                         float* t) {
-    const int o = 4 * cls;
-#pragma unroll
-    for (int x = 0; x < 2; ++x)
-#pragma unroll
-        for (int y = 0; y < 2; ++y) {
-            t[(x * 3 + y) * 3 + 0] = core[(x * 2 + y) * 2 + 0];
-            t[(x * 3 + y) * 3 + 1] = core[(x * 2 + y) * 2 + 1];
-            t[(x * 3 + y) * 3 + 2] = pcf(pij, o + x * 2 + y);
-        }
-#pragma unroll
-    for (int x = 0; x < 2; ++x) {
-#pragma unroll
-        for (int z = 0; z < 2; ++z) t[(x * 3 + 2) * 3 + z] = pcf(pil, o + x * 2 + z);
-        t[(x * 3 + 2) * 3 + 2] = si[x];
-    }
-#pragma unroll
-    for (int y = 0; y < 2; ++y) {
-#pragma unroll
-        for (int z = 0; z < 2; ++z) t[(2 * 3 + y) * 3 + z] = pcf(pjl, o + y * 2 + z);
-        t[(2 * 3 + y) * 3 + 2] = sj[y];
-    }
-    t[24] = sl[0];
-    t[25] = sl[1];
-    t[26] = ncls;
-#pragma unroll
-    for (int xy = 0; xy < 9; ++xy) t[xy * 3 + 2] -= t[xy * 3 + 0] + t[xy * 3 + 1];
-#pragma unroll
-    for (int x = 0; x < 3; ++x)
-#pragma unroll
-        for (int z = 0; z < 3; ++z) t[(x * 3 + 2) * 3 + z] -= t[(x * 3 + 0) * 3 + z] + t[(x * 3 + 1) * 3 + z];
-#pragma unroll
-    for (int yz = 0; yz < 9; ++yz) t[18 + yz] -= t[yz] + t[9 + yz];
-}
-
 // Evaluates combination (i, j, l) whose 16 core counts (cases z0, z1, controls z0, z1 of each
-// (x, y)) sit in column group k of this warp's transpose buffer: exact 27-cell tables, the
-// bounded single-precision prefilter, the exact fixed-point key for survivors, and the
-// warp-aggregated append of candidates (warp-synchronous: every lane calls it).
-// When stage is given it holds the item's pair cores (i, l0 + ll) at [ll] and
-// single cores of l0 + ll at [128 + ll] (shared memory).
+// (x, y)) sit in column group k of this warp's transpose buffer (every lane calls it).
 __device__ __forceinline__ void t3_eval(const ScanWork& w, const CandSink& sink, float thr_f, uint32_t* dump,
                                         const uint32_t* __restrict__ single, const uint4* __restrict__ pairs,
                                         const uint32_t* ebuf, int jl, int k, int i, int j, int l, bool j_ok,
                                         const uint4& pij, const float (&si)[2][2], const float (&sj)[2][2],
-                                        int lane, const uint4* stage = nullptr, int l0 = 0) {
-    const DevData& d = w.d;
-    const int n = d.snps;
-    const uint32_t ncls[2] = {(uint32_t)d.n_cases, (uint32_t)d.n_ctrls};
-    const float ncf[2] = {(float)d.n_cases, (float)d.n_ctrls};
-    const float tiny = 9.5367431640625e-07f;  // 2^-20: x*lg2(x + tiny) = 0 at x = 0
-    const bool valid = j_ok && l < n && l > j;
+                                        int lane) {
+    const bool valid = j_ok && l < w.d.snps && l > j;
     float core[2][8];
 #pragma unroll
     for (int x4 = 0; x4 < 4; ++x4) {
@@ -222,102 +169,11 @@ __device__ __forceinline__ void t3_eval(const ScanWork& w, const CandSink& sink,
         core[1][2 * x4] = u2f(c2.y & 0xffffu);
         core[1][2 * x4 + 1] = u2f(c2.y >> 16);
     }
-    uint4 pil = make_uint4(0, 0, 0, 0), pjl = pil, sl4 = pil;
-    if (valid) {
-        pjl = __ldg(pairs + pair_index(j, l, n));
-        if (stage) {
-            pil = stage[l - l0];
-            sl4 = stage[128 + l - l0];
-        } else {
-            pil = __ldg(pairs + pair_index(i, l, n));
-            sl4 = __ldg(reinterpret_cast<const uint4*>(single) + l);
-        }
-    }
-    const float sl[2][2] = {{u2f(sl4.x), u2f(sl4.y)}, {u2f(sl4.z), u2f(sl4.w)}};
-    float t[2][27];
-#pragma unroll
-    for (int cls = 0; cls < 2; ++cls)
-        expand3f(core[cls], pij, pil, pjl, si[cls], sj[cls], sl[cls], ncf[cls], cls, t[cls]);
-    // single-precision estimate of sum over cells of T[a] + T[b] - T[a+b], in units of ln2 * 2^32
-    float kf = 0.f;
-#pragma unroll
-    for (int c = 0; c < 27; ++c) {
-        const float a = t[0][c], bb = t[1][c], s = a + bb;
-        kf = fmaf(a, t3_lg2(a + tiny), kf);
-        kf = fmaf(bb, t3_lg2(bb + tiny), kf);
-        kf = fmaf(-s, t3_lg2(s + tiny), kf);
-    }
-    const bool cand = valid && (dump != nullptr || sink.digest != nullptr || kf >= thr_f);
-    long long key = w.base_key;
-    bool pass = false;
-    unsigned long long dg = 0;
-    if (cand) {
-#pragma unroll
-        for (int c = 0; c < 27; ++c) {
-            const uint32_t a = min(f2u(fmaxf(t[0][c], 0.f)), ncls[0]);
-            const uint32_t bb = min(f2u(fmaxf(t[1][c], 0.f)), ncls[1]);
-            key += __ldg(d.ftab + a) + __ldg(d.ftab + bb) - __ldg(d.ftab + a + bb);
-        }
-        pass = key >= sink.thr;
-        if (dump) {
-            // owned prefix ordinal m of (i, j): rank offset + m * step
-            const size_t m = (size_t)((pair_index(i, j, n) - w.dist_offset) / w.dist_step);
-            uint32_t* o = dump + (m * n + l) * 54;
-#pragma unroll
-            for (int c = 0; c < 27; ++c) {
-                o[c] = f2u(t[0][c]);
-                o[27 + c] = f2u(t[1][c]);
-            }
-        }
-        if (sink.digest) {
-            const int cmb[3] = {i, j, l};
-            dg = dg_begin(cmb, 3, n);
-#pragma unroll
-            for (int c = 0; c < 27; ++c) dg = dg_cell(dg, f2u(t[0][c]), f2u(t[1][c]));
-        }
-    }
-    if (sink.digest) dg_warp_add(sink.digest, dg);
     if (sink.evaluated) {
         const unsigned vmask = __ballot_sync(0xffffffffu, valid);
         if (lane == 0 && vmask) atomicAdd(sink.evaluated, (unsigned long long)__popc(vmask));
     }
-    const unsigned mask = __ballot_sync(0xffffffffu, pass);
-    if (mask) {
-        const int leader = __ffs(mask) - 1;
-        unsigned base = 0;
-        if (lane == leader) base = atomicAdd(sink.count, (unsigned)__popc(mask));
-        base = __shfl_sync(0xffffffffu, base, leader);
-        if (pass) {
-            const unsigned idx = base + __popc(mask & ((1u << lane) - 1u));
-            if (idx < sink.cap) {
-                const int cmb[3] = {i, j, l};
-                sink.buf[idx] = Cand{key, pack_code(cmb, 3, w.bits)};
-            } else {
-                atomicOr(sink.overflow, 1u);
-            }
-        }
-    }
-}
-
-// Per-item constants of one j: the pair cores of (i, j) and the single cores of i and j as floats.
-__device__ __forceinline__ void t3_item_consts(const uint32_t* __restrict__ single, const uint4* __restrict__ pairs,
-                                               int i, int j, int n, bool j_ok, uint4& pij, float (&si)[2][2],
-                                               float (&sj)[2][2]) {
-    const uint4 a = __ldg(reinterpret_cast<const uint4*>(single) + i);
-    uint4 b = make_uint4(0, 0, 0, 0);
-    pij = make_uint4(0, 0, 0, 0);
-    if (j_ok) {
-        b = __ldg(reinterpret_cast<const uint4*>(single) + j);
-        pij = __ldg(pairs + pair_index(i, j, n));
-    }
-    si[0][0] = u2f(a.x);
-    si[0][1] = u2f(a.y);
-    si[1][0] = u2f(a.z);
-    si[1][1] = u2f(a.w);
-    sj[0][0] = u2f(b.x);
-    sj[0][1] = u2f(b.y);
-    sj[1][0] = u2f(b.z);
-    sj[1][1] = u2f(b.w);
+    t3_eval_core(w, sink, thr_f, dump, single, pairs, core, i, j, l, valid, pij, si, sj, lane);
 }
 
 struct T3Maps {
@@ -615,364 +471,6 @@ __global__ void __launch_bounds__(kT3Threads, 1)
     __syncthreads();
     if (tid == 0 && abort_flag) atomicOr(status, 1);
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
-}
-
-// ---------------------------------------------------------------------------
-// Packed classes.  When both classes fit one FP32 accumulator -- control
-// samples weighted by W = 4^h: the operand planes hold 2^h instead of 1.0 in
-// the control region, every control product is 2^h * 2^h = W, and an
-// accumulator holds cases + W * controls, exact while n_cases < W and
-// n_cases + W * n_ctrls < 2^24 -- an item needs one tensor-memory region of
-// N columns instead of two.  N = 256 (128 l per item; the MMA costs the same
-// for every N up to 256) and two regions alternate between items, so the next
-// item's GEMM runs while the epilogue reads the last one.  A is built in
-// shared memory (tensor memory is full) by six producer warps.
-constexpr int kPL = 128, kPN = 2 * kPL;                  // 128 l, N 256
-constexpr int kPBuildWarps = 6;                           // producer warps (the A build is on the critical path)
-constexpr int kPThreads = 32 * (2 + kPBuildWarps + kT3EpiWarps);  // 512: 128 registers fill the register file
-constexpr int kPSA = kT3M * kT3KB;                        // 16 KB  (i,j) rows, 128-byte swizzle
-static_assert(2 * kPN <= 512, "packed tensor kernel tensor memory");
-
-// ---------------------------------------------------------------------------
-// Packed-class order-3 kernel on CTA pairs.  A cluster of two CTAs (the two
-// SMs of a TPC) runs one GEMM of M 256 x N 256 per work item (i, 64 j, 128 l)
-// with tcgen05.mma.cta_group::2: CTA r builds the A tile of its 32 j
-// (j0 + 32 r ..) in its own shared memory and stages half r of the l rows
-// (64 l x 2 rows); CTA 0 issues the MMAs, which read both CTAs' shared memory
-// and leave each CTA's 128 accumulator rows -- its own (j, x, y) rows x the
-// item's 256 (l, z) columns -- in its own tensor memory.  The shared memory
-// of an SM then takes 82 instead of 114 KB per 128-sample stage (the l-row
-// TMA writes and MMA operand reads halve; the single-CTA kernel keeps the
-// SM's shared memory at its bank limit), and 4 stages of 41 KB fit.  (Split
-// into a 5-slot TMA ring and a 3-slot A ring it ran 18 % slower: the A build
-// then has too little slack.)
-// Handover: each CTA's TMA completes on its own `full_t`; its producer warps
-// build A once their rows landed and arrive on CTA 0's `full_a` (12 arrivals:
-// both CTAs' rows and A tiles are then in place); the MMA commits go to both
-// CTAs' `empty`, `acc_full` and `done`; both CTAs' epilogue warps arrive on
-// CTA 0's `acc_empty` (16 arrivals).  Every wait is bounded; both CTAs meet
-// at a cluster barrier before tensor memory is released.
-constexpr int kPxJ = 2 * kT3J;                                     // 64 j per pair item
-constexpr int kPxStages = 4;
-constexpr int kPxBRows = kPN / 2;                                  // this CTA's l rows (64 l x 2)
-constexpr int kPxSB = kPxBRows * kT3KB;                            // 16 KB
-constexpr int kPxStage = kPxSB + kPSA + kT3SJ + kT3SI;             // 41 KB, a multiple of 1 KB
-constexpr size_t kPxSmem = 1024 + (size_t)kPxStages * kPxStage + (size_t)kT3EpiWarps * kT3Ebuf + 2 * kPL * 16;
-constexpr uint32_t kPxIdesc = (1u << 4) | ((uint32_t)(kPN >> 3) << 17) | ((uint32_t)((2 * kT3M) >> 4) << 24);
-static_assert(kPxSmem <= 227 * 1024 - 256, "paired order-3 tensor kernel shared memory");
-
-// Pair items of one i: J-tile a starts at j0 = i+1+64a and has
-// ceil((n-1-j0)/128) L-tiles starting at l0 = j0+1+128b.
-__device__ __forceinline__ void t3x_decode(const long long* __restrict__ item_begin, int n, long long g, int& i,
-                                           int& j0, int& l0) {
-    int lo = 0, hi = n - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (item_begin[mid] <= g) lo = mid;
-        else hi = mid - 1;
-    }
-    i = lo;
-    long long q = g - item_begin[i];
-    for (int a = 0;; ++a) {
-        const int j = i + 1 + kPxJ * a;
-        const long long nl = (n - 1 - j + kPL - 1) / kPL;
-        if (q < nl) {
-            j0 = j;
-            l0 = j + 1 + kPL * (int)q;
-            return;
-        }
-        q -= nl;
-    }
-}
-
-// LIST: the list mode above (maps.j then covers the residue-ordered planes,
-// where the listed j of one i are consecutive rows).
-template <bool LIST>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1)
-    tensor3x_kernel(const __grid_constant__ T3Maps maps, const __grid_constant__ CUtensorMap map_lh, ScanWork w,
-                    const long long* __restrict__ item_begin, long long g0, long long g1, int k_cases, int pack,
-                    CandSink sink, float thr_f, uint32_t* dump, const uint32_t* __restrict__ single,
-                    const uint4* __restrict__ pairs, int* status, const long long* __restrict__ jl_begin,
-                    const int* __restrict__ jlist) {
-    extern __shared__ uint8_t smraw[];
-    __shared__ __align__(8) uint64_t full_t[kPxStages], full_a[kPxStages], empty[kPxStages];
-    __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2], done;
-    __shared__ uint32_t tmem_base;
-    __shared__ int abort_flag;
-    uint8_t* sm = (uint8_t*)(((uintptr_t)smraw + 1023) & ~(uintptr_t)1023);  // stages: B half | A | j | i
-    uint32_t* ebuf_all = reinterpret_cast<uint32_t*>(sm + kPxStages * kPxStage);
-    volatile int* abort = &abort_flag;
-    const DevData& d = w.d;
-    const int n = d.snps;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int ks_c = k_cases / kT3KB;
-    const int ksteps = ks_c + (d.tw + 1) / 2;
-    const uint32_t rank = cluster_rank();  // 0 issues the MMAs
-    const long long cid = cluster_id(), ncl = cluster_count();
-
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
-                     "r"(512));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
-    }
-    if (tid == 0) {
-        for (int s = 0; s < kPxStages; ++s) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&full_t[s])));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&full_a[s])),
-                         "r"(2 * kPBuildWarps));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&empty[s])));
-        }
-        for (int b = 0; b < 2; ++b) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&acc_full[b])));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&acc_empty[b])),
-                         "r"(2 * kT3EpiWarps));
-        }
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&done)));
-        asm volatile("fence.mbarrier_init.release.cluster;");
-        abort_flag = 0;
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;");
-    __syncthreads();
-    cluster_sync_all();  // both CTAs' barriers exist before either signals the other
-    asm volatile("tcgen05.fence::after_thread_sync;");
-    const uint32_t tmem = tmem_base;
-    bool ok = true;
-
-    if (warp == 0) {
-        // ---------------------------------------------------------------- TMA producer (both CTAs)
-        if (lane == 0) {
-            long long step = 0;
-            for (long long g = g0 + cid; g < g1 && ok; g += ncl) {
-                int i, j0 = 0, l0;
-                if (LIST) {
-                    long long p0;
-                    t3l_decode<kPxJ, kPL>(item_begin, jl_begin, jlist, n, g, i, p0, l0);
-                    // this CTA's 32 listed j: consecutive residue-ordered rows from its first one (rows
-                    // past the end of i's list are loaded too and ignored by the epilogue)
-                    p0 += kT3J * (int)rank;
-                    j0 = p0 < jl_begin[i + 1] ? residue_row(jlist[p0], w.dist_step, n) : 0;
-                } else {
-                    t3x_decode(item_begin, n, g, i, j0, l0);
-                    j0 += kT3J * (int)rank;
-                }
-                for (int ks = 0; ks < ksteps; ++ks) {
-                    const int s = (int)(step % kPxStages);
-                    const long long u = step / kPxStages;
-                    if (u > 0 && !t3_wait_cl(smem_u32(&empty[s]), (uint32_t)((u - 1) & 1), abort)) {
-                        ok = false;
-                        break;
-                    }
-                    const int k0 = ks < ks_c ? ks * kT3KB : k_cases + (ks - ks_c) * kT3KB;
-                    uint8_t* st = sm + s * kPxStage;
-                    const uint32_t bar = smem_u32(&full_t[s]);
-                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                                 "r"((uint32_t)(kPxSB + kT3SJ + 2 * kT3KB))
-                                 : "memory");
-                    t3_tma(smem_u32(st), &map_lh, k0, 2 * l0 + kPxBRows * (int)rank, bar);
-                    t3_tma(smem_u32(st + kPxSB + kPSA), &maps.j, k0, 2 * j0, bar);
-                    t3_tma(smem_u32(st + kPxSB + kPSA + kT3SJ), &maps.i, k0, 2 * i, bar);
-                    ++step;
-                }
-            }
-            if (lane == 0)
-                for (int s = 0; s < kPxStages; ++s) {
-                    if (step <= s) continue;
-                    const long long last = s + ((step - 1 - s) / kPxStages) * kPxStages;
-                    if (!t3_drain(smem_u32(&full_t[s]), (uint32_t)((last / kPxStages) & 1))) ok = false;
-                }
-        }
-    } else if (warp == 1) {
-        // ---------------------------------------------------------------- MMA issuer (CTA 0)
-        if (lane == 0 && rank == 0) {
-            long long step = 0, item = 0;
-            for (long long g = g0 + cid; g < g1 && ok; g += ncl, ++item) {
-                const int buf = (int)(item & 1);
-                if (item >= 2 && !t3_wait_cl(smem_u32(&acc_empty[buf]), (uint32_t)(((item >> 1) - 1) & 1), abort)) {
-                    ok = false;
-                    break;
-                }
-                const uint32_t dcol = tmem + (uint32_t)(kPN * buf);
-                // (N stays 256: with cta_group::2 each CTA supplies N / 2 of the B rows, so a
-                // narrower N would move the split point off the CTAs' l halves)
-                for (int ks = 0; ks < ksteps; ++ks, ++step) {
-                    const int s = (int)(step % kPxStages);
-                    // both CTAs' rows landed and both A tiles are built
-                    if (!t3_wait_cl(smem_u32(&full_a[s]), (uint32_t)((step / kPxStages) & 1), abort)) {
-                        ok = false;
-                        break;
-                    }
-                    asm volatile("tcgen05.fence::after_thread_sync;");
-                    const uint32_t sb = smem_u32(sm + s * kPxStage), sa = sb + kPxSB;
-#pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) {
-                        const uint64_t ad = t3_desc(sa + 32 * kk), bd = t3_desc(sb + 32 * kk);
-                        const uint32_t acc = (ks == 0 && kk == 0) ? 0u : 1u;
-                        asm volatile(
-                            "{.reg .pred p; setp.ne.b32 p, %4, 0;\n"
-                            "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;}\n" ::"r"(dcol),
-                            "l"(ad), "l"(bd), "r"(kPxIdesc), "r"(acc));
-                    }
-                    commit_pair(smem_u32(&empty[s]));
-                }
-                if (!ok) break;
-                commit_pair(smem_u32(&acc_full[buf]));
-            }
-            commit_pair(smem_u32(&done));
-        }
-        // neither CTA releases shared or tensor memory before the pair's MMAs are
-        // done (CTA 1 waits once its own work is over, below: waiting here would
-        // span its whole launch, longer than the bound on a single wait)
-        if (lane == 0 && rank == 0 && !t3_drain_cl(smem_u32(&done), 0)) ok = false;
-    } else if (warp < 2 + kPBuildWarps) {
-        // ---------------------------------------------------------------- A builders (both CTAs)
-        const int t = tid - 64;
-        const int c = t & 7;
-        uint32_t full_a0[kPxStages];
-#pragma unroll
-        for (int s = 0; s < kPxStages; ++s) full_a0[s] = cluster_addr(smem_u32(&full_a[s]), 0);
-        long long step = 0;
-        for (long long g = g0 + cid; g < g1 && ok; g += ncl) {
-            for (int ks = 0; ks < ksteps; ++ks, ++step) {
-                const int s = (int)(step % kPxStages);
-                if (!t3_wait(smem_u32(&full_t[s]), (uint32_t)((step / kPxStages) & 1), abort)) {
-                    ok = false;
-                    break;
-                }
-                uint8_t* st = sm + s * kPxStage;
-                uint8_t* sA = st + kPxSB;
-                const uint8_t* sJ = sA + kPSA;
-                const uint8_t* sI = sJ + kT3SJ;
-                const uint4 i0 = *reinterpret_cast<const uint4*>(sI + (c << 4));
-                const uint4 i1 = *reinterpret_cast<const uint4*>(sI + 128 + ((c ^ 1) << 4));
-                constexpr int kRows = (2 * kT3J + 4 * kPBuildWarps - 1) / (4 * kPBuildWarps);
-                uint4 jrow[kRows];
-#pragma unroll
-                for (int u = 0; u < kRows; ++u) {
-                    const int r = (t >> 3) + 4 * kPBuildWarps * u;
-                    if (r < 2 * kT3J) jrow[u] = *reinterpret_cast<const uint4*>(sJ + r * 128 + ((c ^ (r & 7)) << 4));
-                }
-#pragma unroll
-                for (int u = 0; u < kRows; ++u) {
-                    const int r = (t >> 3) + 4 * kPBuildWarps * u;
-                    if (r >= 2 * kT3J) break;
-                    const uint4 jv = jrow[u];
-                    const int m0 = 4 * (r >> 1) + (r & 1), m1 = m0 + 2;
-                    uint4 v;
-                    v.x = jv.x & i0.x;
-                    v.y = jv.y & i0.y;
-                    v.z = jv.z & i0.z;
-                    v.w = jv.w & i0.w;
-                    *reinterpret_cast<uint4*>(sA + m0 * 128 + ((c ^ (m0 & 7)) << 4)) = v;
-                    v.x = jv.x & i1.x;
-                    v.y = jv.y & i1.y;
-                    v.z = jv.z & i1.z;
-                    v.w = jv.w & i1.w;
-                    *reinterpret_cast<uint4*>(sA + m1 * 128 + ((c ^ (m1 & 7)) << 4)) = v;
-                }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) arrive_cl(full_a0[s]);
-            }
-        }
-    } else {
-        // ---------------------------------------------------------------- epilogue (both CTAs)
-        const int e = warp - (2 + kPBuildWarps);
-        const int q = warp & 3;
-        const int hh = e >> 2;
-        uint32_t* ebuf = ebuf_all + e * (kT3Ebuf / 4);
-        const uint32_t lane_base = tmem + ((uint32_t)(32 * q) << 16);
-        const uint32_t wmask = (1u << pack) - 1u;
-        const int jl = lane >> 2, xy = lane & 3, kp = lane & 3;
-        const int et = tid - 32 * (2 + kPBuildWarps);
-        const uint32_t acc_empty0[2] = {cluster_addr(smem_u32(&acc_empty[0]), 0),
-                                        cluster_addr(smem_u32(&acc_empty[1]), 0)};
-        uint4* stage = reinterpret_cast<uint4*>(ebuf_all + kT3EpiWarps * (kT3Ebuf / 4));
-        long long item = 0;
-        for (long long g = g0 + cid; g < g1 && ok; g += ncl, ++item) {
-            int i, j0 = 0, l0;
-            long long p0 = 0, p_end = 0;
-            if (LIST) {
-                t3l_decode<kPxJ, kPL>(item_begin, jl_begin, jlist, n, g, i, p0, l0);
-                p0 += kT3J * (int)rank;
-                p_end = jl_begin[i + 1];
-            } else {
-                t3x_decode(item_begin, n, g, i, j0, l0);
-                j0 += kT3J * (int)rank;
-            }
-            const int buf = (int)(item & 1);
-            asm volatile("bar.sync 1, %0;" ::"n"(32 * kT3EpiWarps) : "memory");
-            {
-                const int ll = et & (kPL - 1), l = l0 + ll;
-                if (l < n) {
-                    if (et < kPL) stage[ll] = __ldg(pairs + pair_index(i, l, n));
-                    else stage[kPL + ll] = __ldg(reinterpret_cast<const uint4*>(single) + l);
-                }
-            }
-            asm volatile("bar.sync 1, %0;" ::"n"(32 * kT3EpiWarps) : "memory");
-            const int j = t3x_j<LIST>(j0, p0, p_end, jlist, 8 * q + jl, n);
-            const bool j_ok = j < n;
-            uint4 pij;
-            float si[2][2], sj[2][2];
-            t3_item_consts(single, pairs, i, j, n, j_ok, pij, si, sj);
-            if (!t3_wait_cl(smem_u32(&acc_full[buf]), (uint32_t)((item >> 1) & 1), abort)) {
-                ok = false;
-                break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;");
-#pragma unroll 1
-            for (int cc = 0; cc < 8; ++cc) {
-                const int lg = l0 + 16 * cc + 8 * hh;
-                if (!__any_sync(0xffffffffu, j_ok && lg + 7 > j && lg < n)) {
-                    if (cc == 7) {
-                        asm volatile("tcgen05.fence::before_thread_sync;");
-                        __syncwarp();
-                        if (lane == 0) arrive_cl(acc_empty0[buf]);
-                    }
-                    continue;
-                }
-                {
-                    const uint32_t col = (uint32_t)(kPN * buf + 32 * cc + 16 * hh);
-                    uint32_t v[16];
-                    asm volatile(
-                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%"
-                        "15}, [%16];"
-                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-                          "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-                          "=r"(v[14]), "=r"(v[15])
-                        : "r"(lane_base + col));
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (cc == 7) {
-                        asm volatile("tcgen05.fence::before_thread_sync;");
-                        __syncwarp();
-                        if (lane == 0) arrive_cl(acc_empty0[buf]);
-                    }
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        const uint32_t u0 = __float2uint_rn(__uint_as_float(v[2 * k]));
-                        const uint32_t u1 = __float2uint_rn(__uint_as_float(v[2 * k + 1]));
-                        *reinterpret_cast<uint2*>(ebuf + 2 * t3_slot(jl, k, xy)) =
-                            make_uint2((u0 & wmask) | (u1 & wmask) << 16, (u0 >> pack) | (u1 >> pack) << 16);
-                    }
-                }
-                __syncwarp();
-#pragma unroll 1
-                for (int b = 0; b < 2; ++b)
-                    t3_eval(w, sink, thr_f, dump, single, pairs, ebuf, jl, 2 * kp + b, i, j, lg + 2 * kp + b, j_ok,
-                            pij, si, sj, lane, stage, l0);
-                __syncwarp();
-            }
-        }
-    }
-    if (!ok) *abort = 1;
-    asm volatile("tcgen05.fence::before_thread_sync;");
-    __syncthreads();
-    // CTA 1: its epilogue has read the last accumulators, so the pair's final
-    // commit to this CTA's `done` lands soon; it must land before the CTA exits
-    if (rank == 1 && warp == 1 && lane == 0 && !t3_drain_cl(smem_u32(&done), 0)) *abort = 1;
-    cluster_sync_all();  // the other CTA is done with this CTA's shared and tensor memory
-    asm volatile("tcgen05.fence::after_thread_sync;");
-    if (tid == 0 && abort_flag) atomicOr(status, 1);
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
 }
 
 // ---------------------------------------------------------------------------
@@ -1743,14 +1241,13 @@ static long long t2x_items(int n, std::vector<long long>& item_begin, int& n_iti
     return total;
 }
 
-// Items per i (host): prefix sums item_begin[0..n], item_begin[n] = total;
-// J j per item (kT3J, or kPxJ for the pair items of tensor3x_kernel).
-static long long t3_items(int n, int L, std::vector<long long>& item_begin, int J = kT3J) {
+// Items per i of tensor3_kernel (host): prefix sums item_begin[0..n], item_begin[n] = total.
+static long long t3_items(int n, int L, std::vector<long long>& item_begin) {
     item_begin.assign((size_t)n + 1, 0);
     long long total = 0;
     for (int i = 0; i < n; ++i) {
         item_begin[i] = total;
-        for (int j = i + 1; j < n - 1; j += J) total += (n - 1 - j + L - 1) / L;
+        for (int j = i + 1; j < n - 1; j += kT3J) total += (n - 1 - j + L - 1) / L;
     }
     item_begin[n] = total;
     return total;
@@ -1769,18 +1266,23 @@ static PFN_cuTensorMapEncodeTiled_v12000 t3_encoder() {
     return fn;
 }
 
-static cudaError_t t3_map(CUtensorMap* m, uint8_t* base, int rows, int pitch, int box_rows, bool swizzle) {
+cudaError_t tensor_map(CUtensorMap* m, const void* base, int rows, int pitch, int box_bytes, int box_rows,
+                       bool swizzle) {
     auto enc = t3_encoder();
     if (!enc) return cudaErrorNotSupported;
     cuuint64_t dims[2] = {(cuuint64_t)pitch, (cuuint64_t)rows};
     cuuint64_t strides[1] = {(cuuint64_t)pitch};
-    cuuint32_t box[2] = {(cuuint32_t)kT3KB, (cuuint32_t)box_rows};
+    cuuint32_t box[2] = {(cuuint32_t)box_bytes, (cuuint32_t)box_rows};
     cuuint32_t es[2] = {1, 1};
-    const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, base, dims, strides, box, es,
+    const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, es,
                            CU_TENSOR_MAP_INTERLEAVE_NONE,
                            swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+static cudaError_t t3_map(CUtensorMap* m, uint8_t* base, int rows, int pitch, int box_rows, bool swizzle) {
+    return tensor_map(m, base, rows, pitch, kT3KB, box_rows, swizzle);
 }
 
 // One accumulator for both classes when some W = 4^h (h <= 8, so 2^h is an
@@ -1794,53 +1296,71 @@ int tensor_pack(int n_cases, int n_ctrls) {
     return 0;
 }
 
-cudaError_t tensor3_prepare(const DevData& d, T3Plan& plan, cudaStream_t s) {
-    plan.pack = tensor_pack(d.n_cases, d.n_ctrls);
-    const int L = plan.pack ? kPL : kT3L;
-    // packed classes: CTA-pair items
-    plan.pair3 = plan.pack != 0;
-    const int J = plan.pair3 ? kPxJ : kT3J;
-    plan.item_combos = J * L / 2.0;
-    plan.k_cases = kT3KB * ((d.cw + 1) / 2);
-    plan.pitch = plan.k_cases + kT3KB * ((d.tw + 1) / 2);
-    (void)L;
-    cudaError_t e = cudaMalloc((void**)&plan.planes, (size_t)2 * d.snps * plan.pitch);
+// e4m3 planes (every use but the order-3 pair kernel's).
+static cudaError_t e4m3_planes(T3Plan& plan, const DevData& d, cudaStream_t s) {
+    if (plan.planes) return cudaSuccess;
+    uint8_t* planes = nullptr;
+    cudaError_t e = cudaMalloc((void**)&planes, (size_t)2 * d.snps * plan.pitch);
     if (e != cudaSuccess) return e;
     const long long total = 2ll * d.snps * (plan.pitch / 16);
     const int grid = (int)std::min<long long>((total + 255) / 256, 4096);
     const uint32_t ctrl_byte = plan.pack ? (uint32_t)((plan.pack / 2 + 7) << 3) : 0x38u;  // e4m3 2^h
-    t3_planes_kernel<<<grid, 256, 0, s>>>(d, plan.planes, plan.pitch, plan.k_cases, ctrl_byte);
+    t3_planes_kernel<<<grid, 256, 0, s>>>(d, planes, plan.pitch, plan.k_cases, ctrl_byte);
     count_launch();
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     const int rows = 2 * d.snps;
-    if ((e = t3_map(&plan.map_l, plan.planes, rows, plan.pitch, plan.pack ? kPN : kT3N, true)) != cudaSuccess)
-        return e;
-    if ((e = t3_map(&plan.map_j, plan.planes, rows, plan.pitch, 2 * kT3J, true)) != cudaSuccess) return e;
-    if ((e = t3_map(&plan.map_i, plan.planes, rows, plan.pitch, 2, true)) != cudaSuccess) return e;
+    // l rows of an item: 192 at order 3, 256 at order 4 when the classes pack
+    if (e == cudaSuccess) e = t3_map(&plan.map_l, planes, rows, plan.pitch, plan.pack ? kT2N : kT3N, true);
+    if (e == cudaSuccess) e = t3_map(&plan.map_j, planes, rows, plan.pitch, 2 * kT3J, true);
+    if (e == cudaSuccess) e = t3_map(&plan.map_i, planes, rows, plan.pitch, 2, true);
+    if (e == cudaSuccess) e = t3_map(&plan.map_a2, planes, rows, plan.pitch, kT2M, true);
+    if (e == cudaSuccess) e = t3_map(&plan.map_b2, planes, rows, plan.pitch, kT2N, true);
+    if (e != cudaSuccess) cudaFree(planes);
+    else plan.planes = planes;
+    return e;
+}
+
+cudaError_t tensor3_prepare(const DevData& d, T3Plan& plan, cudaStream_t) {
+    plan.pack = tensor_pack(d.n_cases, d.n_ctrls);
+    plan.f4.pack = f4_pack(d.n_cases, d.n_ctrls);
+    plan.pair3 = plan.f4.pack != 0;
+    plan.k_cases = kT3KB * ((d.cw + 1) / 2);
+    plan.pitch = plan.k_cases + kT3KB * ((d.tw + 1) / 2);
     // order 2: CTA-pair items when the classes pack (per class the MMA waits for the epilogue between
     // items, and the single-CTA kernel measured 2 % faster there)
     std::vector<long long> ib2;
     plan.pair2 = plan.pack != 0;
     plan.total2 = plan.pair2 ? t2x_items(d.snps, ib2, plan.n_itiles) : t2_items(d.snps, ib2, plan.n_itiles);
     plan.item2_combos = (double)d.snps * (d.snps - 1) / 2 / std::max(1ll, plan.total2);
-    e = cudaMalloc((void**)&plan.item2_begin, ib2.size() * sizeof(long long));
+    cudaError_t e = cudaMalloc((void**)&plan.item2_begin, ib2.size() * sizeof(long long));
     if (e == cudaSuccess)
         e = cudaMemcpy(plan.item2_begin, ib2.data(), ib2.size() * sizeof(long long), cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) return e;
-    if ((e = t3_map(&plan.map_a2, plan.planes, rows, plan.pitch, kT2M, true)) != cudaSuccess) return e;
-    return t3_map(&plan.map_b2, plan.planes, rows, plan.pitch, kT2N, true);
+    return e;
+}
+
+// The operand planes of an order, made on its first search (items_mu held).
+static cudaError_t order_planes(T3Plan& plan, const DevData& d, int order, cudaStream_t s) {
+    if (order != 3 || !plan.pair3) return e4m3_planes(plan, d, s);
+    if (plan.f4.bits) return cudaSuccess;
+    cudaError_t e = f4_prepare(d, plan.f4, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) f4_release(plan.f4);
+    return e;
 }
 
 // The work items of the whole data set at order 3 or 4, made on the first
 // search of that order (the host enumeration grows as n^2 / 16 at order 4:
 // about 0.1 s at 40 000 SNPs, which a search of another order need not pay).
-cudaError_t tensor3_order_items(T3Plan& plan, const DevData& d, int order) {
+cudaError_t tensor3_order_items(T3Plan& plan, const DevData& d, int order, cudaStream_t s) {
     std::lock_guard<std::mutex> g(plan.items_mu);
-    cudaError_t e = cudaSuccess;
+    cudaError_t e = order_planes(plan, d, order, s);
+    if (e != cudaSuccess) return e;
     if (order == 3 && !plan.item_begin) {
-        const int L = plan.pack ? kPL : kT3L, J = plan.pair3 ? kPxJ : kT3J;
         std::vector<long long> ib;
-        const long long total = t3_items(d.snps, L, ib, J);
+        if (plan.pair3) ib = t3x_items(d.snps);
+        else t3_items(d.snps, kT3L, ib);
+        const long long total = ib.back();
         long long* p = nullptr;
         e = cudaMalloc((void**)&p, ib.size() * sizeof(long long));
         if (e == cudaSuccess) e = cudaMemcpy(p, ib.data(), ib.size() * sizeof(long long), cudaMemcpyHostToDevice);
@@ -1849,6 +1369,8 @@ cudaError_t tensor3_order_items(T3Plan& plan, const DevData& d, int order) {
             return e;
         }
         plan.total = total;
+        const double n = d.snps;
+        plan.item_combos = n * (n - 1) * (n - 2) / 6.0 / std::max(1ll, total);
         plan.item_begin = p;
     }
     if (order == 4 && !plan.item4_begin && d.snps >= 4) {
@@ -1889,15 +1411,33 @@ struct T3Layer {
     double item_combos = 0;
     int n_tiles = 0;                  // order 2: tiles of owned i; order 4: listed pairs
     int4* pinfo = nullptr;            // order 4: (i, j, first owned k) of each listed pair
-    CUtensorMap map_jr;               // order 3: box 128 B x 64 rows over the residue-ordered planes
+    CUtensorMap map_jr;               // order 3: 64 rows of the residue-ordered planes (pair kernel: bit rows)
     CUtensorMap map_ar;               // order 2: box 128 B x 128 rows over the residue-ordered planes
     CUtensorMap map_kr;               // order 4: box 128 B x 32 rows over the residue-ordered planes
 };
 struct T3Layers {
     std::mutex mu;
     std::map<std::tuple<int, int, int>, T3Layer> by;  // (order, step, offset)
-    std::map<int, uint8_t*> by_residue;              // residue-ordered operand planes per step
+    // residue-ordered operand planes, and bit rows (order-3 pair kernel), per step
+    std::map<int, uint8_t*> by_residue, bits_by_residue;
 };
+
+// The rows of every SNP (row_bytes each, SNP-major in src) ordered by residue mod step, made on first use.
+static cudaError_t residue_copy(std::map<int, uint8_t*>& by, const uint8_t* src, size_t row_bytes, int n, int step,
+                                cudaStream_t s) {
+    if (by.count(step)) return cudaSuccess;
+    uint8_t* perm = nullptr;
+    cudaError_t e = cudaMalloc((void**)&perm, (size_t)n * row_bytes);
+    // residue class r holds SNPs r + step m, m < ceil((n - r) / step)
+    for (int r = 0; r < step && r < n && e == cudaSuccess; ++r)
+        e = cudaMemcpy2DAsync(perm + (size_t)residue_row(r, step, n) * row_bytes, row_bytes,
+                              src + (size_t)r * row_bytes, (size_t)step * row_bytes, row_bytes,
+                              (size_t)((n - r + step - 1) / step), cudaMemcpyDeviceToDevice, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) cudaFree(perm);
+    else by[step] = perm;
+    return e;
+}
 
 
 static bool is_layer(const ScanWork& w) { return w.dist_step != 1 || w.dist_offset != 0; }
@@ -1919,23 +1459,18 @@ cudaError_t tensor3_layer(T3Plan& plan, const ScanWork& w, cudaStream_t s) {
     std::lock_guard<std::mutex> g(plan.layers->mu);
     const auto key = std::make_tuple(w.order, w.dist_step, w.dist_offset);
     if (plan.layers->by.count(key)) return cudaSuccess;
-    uint8_t*& perm = plan.layers->by_residue[w.dist_step];
-    if (!perm) {
-        // residue class r holds SNPs r + step m, m < ceil((n - r) / step), each as its 2 plane rows
-        const int n = w.d.snps, step = w.dist_step;
-        const size_t row2 = (size_t)2 * plan.pitch;
-        cudaError_t e = cudaMalloc((void**)&perm, (size_t)n * row2);
-        for (int r = 0; r < step && r < n && e == cudaSuccess; ++r)
-            e = cudaMemcpy2DAsync(perm + (size_t)residue_row(r, step, n) * row2, row2, plan.planes + (size_t)r * row2,
-                                  (size_t)step * row2, row2, (size_t)((n - r + step - 1) / step),
-                                  cudaMemcpyDeviceToDevice, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) {
-            cudaFree(perm);
-            plan.layers->by_residue.erase(w.dist_step);
-            return e;
-        }
+    const bool px = w.order == 3 && plan.pair3;  // the pair kernel's j operand: bit rows
+    cudaError_t pe;
+    {
+        std::lock_guard<std::mutex> gp(plan.items_mu);
+        pe = order_planes(plan, w.d, w.order, s);
     }
+    if (pe == cudaSuccess)
+        pe = px ? residue_copy(plan.layers->bits_by_residue, (const uint8_t*)plan.f4.bits, (size_t)8 * plan.f4.wpr,
+                               w.d.snps, w.dist_step, s)
+                : residue_copy(plan.layers->by_residue, plan.planes, (size_t)2 * plan.pitch, w.d.snps, w.dist_step, s);
+    if (pe != cudaSuccess) return pe;
+    uint8_t* perm = px ? nullptr : plan.layers->by_residue[w.dist_step];
     const int n = w.d.snps;
     const long long step = w.dist_step, offset = w.dist_offset;
     if (w.order == 4) {
@@ -2010,16 +1545,18 @@ cudaError_t tensor3_layer(T3Plan& plan, const ScanWork& w, cudaStream_t s) {
             jl.push_back(i + 1 + (int)t);
             combos += n - 2 - i - t;
         }
-        // items of J listed j and L l: the pair kernel's (classes that pack) or the per-class kernel's
-        const int J = plan.pair3 ? kPxJ : kT3J, L = plan.pair3 ? kPL : kT3L;
-        for (size_t a = (size_t)jb[i]; a < jl.size(); a += J) total += (n - 1 - jl[a] + L - 1) / L;
+        // the pair kernel's items, or the per-class kernel's of 32 listed j and 96 l
+        for (size_t a = (size_t)jb[i]; a < jl.size(); a += px ? kPxJ : kT3J)
+            total += px ? t3x_tiles(n, jl[a]) : (n - 1 - jl[a] + kT3L - 1) / kT3L;
     }
     ib[n] = total;
     jb[n] = (long long)jl.size();
     T3Layer L;
     L.total = total;
     L.item_combos = (double)combos / std::max(1ll, total);
-    cudaError_t e = t3_map(&L.map_jr, perm, 2 * n, plan.pitch, 2 * kT3J, true);
+    cudaError_t e = px ? f4_bit_map(&L.map_jr, plan.f4, (const uint32_t*)plan.layers->bits_by_residue[w.dist_step],
+                                    2 * n, 2 * kT3J)
+                       : t3_map(&L.map_jr, perm, 2 * n, plan.pitch, 2 * kT3J, true);
     if (e == cudaSuccess) e = cudaMalloc((void**)&L.item_begin, ib.size() * sizeof(long long));
     if (e == cudaSuccess) e = cudaMalloc((void**)&L.jl_begin, jb.size() * sizeof(long long));
     if (e == cudaSuccess) e = cudaMalloc((void**)&L.jlist, std::max<size_t>(1, jl.size()) * sizeof(int));
@@ -2061,9 +1598,11 @@ void tensor3_release(T3Plan& plan) {
             cudaFree(kv.second.pinfo);
         }
         for (auto& kv : plan.layers->by_residue) cudaFree(kv.second);
+        for (auto& kv : plan.layers->bits_by_residue) cudaFree(kv.second);
         delete plan.layers;
         plan.layers = nullptr;
     }
+    f4_release(plan.f4);
     cudaFree(plan.planes);
     cudaFree(plan.item_begin);
     cudaFree(plan.item2_begin);
@@ -2166,29 +1705,6 @@ cudaError_t probe_lg2_error(unsigned max_c, double* max_abs_err, cudaStream_t s)
     return e;
 }
 
-// Clusters of two CTAs of a pair kernel that fit on the device at once (a TPC
-// each); 0 when the occupancy query is not available.
-template <class K>
-static int pair_clusters(K* kernel, int threads, size_t smem) {
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 2;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(2, 1, 1);
-    cfg.blockDim = dim3(threads, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int c = 0;
-    if (cudaOccupancyMaxActiveClusters(&c, kernel, &cfg) != cudaSuccess || c < 1) {
-        cudaGetLastError();
-        c = 0;
-    }
-    return c;
-}
-
 cudaError_t launch_tensor3(const ScanWork& w, const T3Plan& plan, long long g0, long long g1, const CandSink& sink,
                            uint32_t* dump, const uint32_t* single, const uint4* pairs, const uint4* triples,
                            int* status, cudaStream_t s, int sms) {
@@ -2218,10 +1734,6 @@ cudaError_t launch_tensor3(const ScanWork& w, const T3Plan& plan, long long g0, 
                                      (int)kT2xSmem);
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(tensor2x_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kT2xSmem);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(tensor3x_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPxSmem);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(tensor3x_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPxSmem);
         return e;
     }();
     if (attr != cudaSuccess) return attr;
@@ -2262,23 +1774,12 @@ cudaError_t launch_tensor3(const ScanWork& w, const T3Plan& plan, long long g0, 
     }
     T3Maps maps{plan.map_l, plan.map_j, plan.map_i};
     if (plan.pair3) {
-        static const int max_clusters = pair_clusters(tensor3x_kernel<false>, kPThreads, kPxSmem);
-        const long long clusters = std::min<long long>(items, max_clusters > 0 ? max_clusters : sms / 2);
-        const unsigned grid2 = (unsigned)(2 * std::max(1ll, clusters));
-        if (is_layer(w)) {
-            const T3Layer* L = find_layer(plan, w);
-            if (!L || !tensor_layer_ok(plan, w)) return cudaErrorInvalidValue;
-            const T3Maps lmaps{plan.map_l, L->map_jr, plan.map_i};
-            tensor3x_kernel<true><<<grid2, kPThreads, kPxSmem, s>>>(lmaps, plan.map_a2, w, L->item_begin, g0, g1,
-                                                                    plan.k_cases, plan.pack, sink, thr_f, dump, single,
-                                                                    pairs, status, L->jl_begin, L->jlist);
-        } else {
-            tensor3x_kernel<false><<<grid2, kPThreads, kPxSmem, s>>>(maps, plan.map_a2, w, plan.item_begin, g0, g1,
-                                                                     plan.k_cases, plan.pack, sink, thr_f, dump,
-                                                                     single, pairs, status, nullptr, nullptr);
-        }
-        count_launch();
-        return cudaGetLastError();
+        const T3Layer* L = is_layer(w) ? find_layer(plan, w) : nullptr;
+        if (is_layer(w) && (!L || !tensor_layer_ok(plan, w))) return cudaErrorInvalidValue;
+        const T3xRange r = L ? T3xRange{L->item_begin, &L->map_jr, L->jl_begin, L->jlist}
+                             : T3xRange{plan.item_begin, &plan.f4.map_j};
+        const float thr_q = f4_bound_threshold((double)sink.thr * scale, w.d.n_cases, w.d.n_ctrls, 27);
+        return launch_tensor3x(w, plan.f4, r, g0, g1, sink, dump, single, pairs, thr_f, thr_q, status, s, sms);
     }
     if (is_layer(w)) {
         const T3Layer* L = find_layer(plan, w);

@@ -1,0 +1,730 @@
+// Order-3 contingency tables on CTA pairs with 4-bit operands (classes that
+// share one accumulator).
+//
+// A cluster of two CTAs (the two SMs of a TPC) runs one GEMM per work item
+// (i, 64 j, up to 120 l):
+//     D[(j,x,y), (l,z)] = sum_s A[(j,x,y), s] B[(l,z), s]    (M 256, N <= 240)
+// with tcgen05.mma.cta_group::2.kind::mxf4, control samples weighted by W = 2^p
+// through the B scale, so an accumulator holds cases + W controls of one core
+// cell.  CTA r builds the A rows of its 32 j and stages half r of the l rows;
+// CTA 0 issues the MMAs; each CTA's 128 accumulator rows end up in its own
+// tensor memory.  Two regions of 240 columns alternate between items, so the
+// next item's GEMM runs while the epilogue evaluates the last one; the other 32
+// columns hold the scales.
+//
+// Operands.  B rows are the data set's e2m1 planes (TMA, 128-byte swizzle, 256
+// samples a stage).  A rows are built from bit rows (one bit a sample, a quarter
+// of the planes' bytes): eight producer warps in two alternating groups AND the
+// i and j words and spread the bits to nibbles straight into the swizzled A tile.
+//
+// Accumulator rows are ordered (j / 8, x, y, j % 8) and columns (l / 8, z, l % 8),
+// so that two 16x256b tensor-memory loads give a thread all 8 cores of the
+// combinations (j, l) and (j, l + 1), in neighbouring registers: no transpose
+// through shared memory.
+//
+// Epilogue.  The 27 cells of both combinations follow from the packed cores and
+// the packed marginals (pairs (i,j), (i,l), (j,l) and singles; every value an
+// exact integer below 2^24) in two-wide single precision.  A quadratic bound on
+// the MI (F4Bound) rejects nearly all of them; a warp with a survivor takes a
+// logarithm estimate with a proven error bound and, for what passes that, the
+// exact fixed-point key, so the kept set is the one of the exact key.
+//
+// What bounds it (2 000 SNPs x 4 000/4 000, one launch over the whole scan):
+// 26.3 ms; without the evaluation 22.7, without the A build and the MMAs too
+// 22.3 -- the copies out of L2 (17 KB a stage and SM, 9.5 TB/s); the MMAs alone
+// are 18.6 (120 cycles per M 256 N 240 K 64).  Whole searches: 28.8 ms against
+// 74.7 with e4m3 operands (128-byte rows of 128 samples: twice the shared-memory
+// and L2 traffic, 82 KB a stage with LSU and tensor wavefronts at 83 % of peak;
+// 81 logarithms a combination at 8 cycles a warp instruction and SM quarter where
+// the bound takes about 21 reciprocals and 215 arithmetic cycles; a transpose
+// through shared memory).  Tried on the way: A in tensor memory and B spread from
+// bits by warps (5 KB a stage from L2, N 192): 45 ms, bound by issue slots.
+//
+// Reference semantics: GenotypeTable::combine_and_popcnt for order 3
+// (src/base/gt_popcnt.cpp:4-35) and MutualInformation::compute
+// (src/base/mi_compute.cpp:16-41) over the combinations ThreadedSearch
+// visits (include/fiuncho/ThreadedSearch.h:157-180) with one worker.
+#include <algorithm>
+#include <cmath>
+
+#include "tensor3x.h"
+#include "tensor_fp4.cuh"
+
+namespace fiu {
+
+constexpr int kXJ = kPxJ / 2;                       // j per CTA
+constexpr int kXL = 8 * kPxG;                       // 120 l per item at most
+constexpr int kXN = 2 * kXL;                        // columns of an accumulator region
+constexpr int kXM = 4 * kXJ;                        // 128 accumulator rows per CTA
+constexpr int kXRow = kF4K / 2;                     // 128 bytes per operand row and stage
+constexpr int kXBitRow = kF4K / 8;                  // 32 bytes per bit row and stage
+constexpr int kXStages = 6;
+constexpr int kXSA = kXM * kXRow;                   // 16 KB
+constexpr int kXSB = kXN / 2 * kXRow;               // 15 KB: this CTA's half of the l rows
+constexpr int kXSJ = 2 * kXJ * kXBitRow;            //  2 KB
+constexpr int kXSI = 2 * kXBitRow;                  // 64 bytes
+constexpr int kXStage = (kXSA + kXSB + kXSJ + kXSI + 1023) / 1024 * 1024;  // 34 KB
+constexpr int kXColOne = 2 * kXN, kXColW = kXColOne + 16;
+// Builders in two groups that take alternate stages (a warp's chain of waits,
+// loads, shifts, stores and arrival is longer than a stage's MMAs).
+constexpr int kXBuildWarps = 4, kXEpiWarps = 8;     // builder warps per group
+constexpr int kXThreads = 32 * (4 + 2 * kXBuildWarps + kXEpiWarps);  // 640: warps 2 and 3 idle
+// registers a thread: 96 at launch; copies and MMAs keep 40, the builders 56,
+// the epilogue gets 160 (40 + 2 x 56 + 2 x 160 <= 5 x 96)
+constexpr int kXMeta = 16;                          // items in flight between the copies and the MMAs
+constexpr int kXTab = 9 * kXL * 4;                  // an item's (i, l) marginals, one column per l
+constexpr size_t kXSmem = 1024 + (size_t)kXStages * kXStage + 2 * kXTab;
+static_assert(kXSmem <= 227 * 1024 - 512, "order-3 pair kernel shared memory");
+static_assert(kXSA % 1024 == 0 && kXSB % 1024 == 0, "operand tiles on swizzle atoms");
+static_assert(kXColW + 16 <= 512, "tensor memory columns");
+static_assert(kXStages < kXMeta, "an item has a stage at least");
+
+// One item: (i, j0 ..), l-tile of ng groups of 8 from l0.  LIST (a Distribution
+// layer): p0 is the first listed j instead of j0.
+struct T3xItem {
+    int i, j0, l0, ng;
+    long long p0;
+};
+
+// Item g; i is the walker's position (the items of one walker ascend).
+template <bool LIST>
+__device__ __forceinline__ T3xItem t3x_item(const long long* __restrict__ item_begin,
+                                            const long long* __restrict__ jl_begin, const int* __restrict__ jlist,
+                                            int n, long long g, int& i) {
+    if (i < 0) {
+        int lo = 0, hi = n - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (__ldg(item_begin + mid) <= g) lo = mid;
+            else hi = mid - 1;
+        }
+        i = lo;
+    } else {
+        while (__ldg(item_begin + i + 1) <= g) ++i;
+    }
+    T3xItem it;
+    it.i = i;
+    int q = (int)(g - __ldg(item_begin + i));
+    long long p = LIST ? __ldg(jl_begin + i) : 0;
+    for (int j = LIST ? __ldg(jlist + p) : i + 1;;) {
+        const int nl = t3x_tiles(n, j);
+        if (q < nl) {
+            const int G = t3x_groups(n, j), a = G * q / nl, b = G * (q + 1) / nl;
+            it.j0 = j;
+            it.p0 = p;
+            it.l0 = ((j + 1) & ~7) + 8 * a;
+            it.ng = b - a;
+            return it;
+        }
+        q -= nl;
+        if (LIST) {
+            p += kPxJ;
+            j = __ldg(jlist + p);
+        } else {
+            j += kPxJ;
+        }
+    }
+}
+
+// Packed float c + W t of the counts of both classes.
+__device__ __forceinline__ float t3x_pk(uint32_t c, uint32_t t, float W) { return fmaf(W, u2f(t), u2f(c)); }
+// Entry (x, y) of the pair cores v, packed.
+__device__ __forceinline__ float t3x_pair(const uint4& v, int x, int y, float W) {
+    const uint32_t c = x ? v.y : v.x, t = x ? v.w : v.z;
+    return t3x_pk(y ? c >> 16 : c & 0xffffu, y ? t >> 16 : t & 0xffffu, W);
+}
+
+// The rare path (lanes with want): from the 27 packed cells t[(x*3+y)*3+z] of
+// combination (i, j, l), the bounded single-precision estimate of the key
+// (t3_margin), the exact fixed-point key for what passes it, and the
+// warp-aggregated append of candidates.  Warp-synchronous.
+__device__ __forceinline__ void t3x_survivor(const ScanWork& w, const CandSink& sink, float thr_f, uint32_t* dump,
+                                             const float (&t)[27], int pack, int i, int j, int l, bool want,
+                                             int lane) {
+    const uint32_t mask = (1u << pack) - 1u;
+    const int n = w.d.snps;
+    bool cand = want;
+    if (!dump && !sink.digest) {
+        const float tiny = 9.5367431640625e-07f;  // 2^-20: x*lg2(x + tiny) = 0 at x = 0
+        float kf = 0.f;
+#pragma unroll
+        for (int c = 0; c < 27; ++c) {
+            const uint32_t u = __float2uint_rn(t[c]);
+            const float a = u2f(u & mask), b = u2f(u >> pack), s = a + b;
+            kf = fmaf(a, t3_lg2(a + tiny), kf);
+            kf = fmaf(b, t3_lg2(b + tiny), kf);
+            kf = fmaf(-s, t3_lg2(s + tiny), kf);
+        }
+        cand = want && kf >= thr_f;
+    }
+    if (!__any_sync(0xffffffffu, cand)) return;
+    long long key = w.base_key;
+    unsigned long long dg = 0;
+    if (cand) {
+        const uint32_t nc = (uint32_t)w.d.n_cases, nt = (uint32_t)w.d.n_ctrls;
+        // owned prefix ordinal m of (i, j): rank offset + m * step
+        uint32_t* o =
+            dump ? dump + ((size_t)((pair_index(i, j, n) - w.dist_offset) / w.dist_step) * n + l) * 54 : nullptr;
+        if (sink.digest) {
+            const int cmb[3] = {i, j, l};
+            dg = dg_begin(cmb, 3, n);
+        }
+#pragma unroll
+        for (int c = 0; c < 27; ++c) {
+            const uint32_t u = __float2uint_rn(t[c]), a = min(u & mask, nc), b = min(u >> pack, nt);
+            key += __ldg(w.d.ftab + a) + __ldg(w.d.ftab + b) - __ldg(w.d.ftab + a + b);
+            if (o) {
+                o[c] = u & mask;
+                o[27 + c] = u >> pack;
+            }
+            if (sink.digest) dg = dg_cell(dg, u & mask, u >> pack);
+        }
+    }
+    if (sink.digest) dg_warp_add(sink.digest, dg);
+    const bool pass = cand && key >= sink.thr;
+    const unsigned pm = __ballot_sync(0xffffffffu, pass);
+    if (!pm) return;
+    const int leader = __ffs(pm) - 1;
+    unsigned base = 0;
+    if (lane == leader) base = atomicAdd(sink.count, (unsigned)__popc(pm));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    if (pass) {
+        const unsigned idx = base + __popc(pm & ((1u << lane) - 1u));
+        if (idx < sink.cap) {
+            const int cmb[3] = {i, j, l};
+            sink.buf[idx] = Cand{key, pack_code(cmb, 3, w.bits)};
+        } else {
+            atomicOr(sink.overflow, 1u);
+        }
+    }
+}
+
+// Columns the MMA of an item of ng groups multiplies (at least 64).
+__device__ __forceinline__ int t3x_n(int ng) { return 16 * max(ng, 4); }
+
+template <bool LIST>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
+    tensor3x_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_j,
+                    const __grid_constant__ CUtensorMap map_i, const __grid_constant__ ScanWork w,
+                    const __grid_constant__ CandSink sink, const long long* __restrict__ item_begin, long long g0,
+                    long long g1, int nw_c, int nw_t, int pack, float thr_f, float thr_q, uint32_t* dump,
+                    const uint32_t* __restrict__ single, const uint4* __restrict__ pairs, int* status,
+                    const long long* __restrict__ jl_begin, const int* __restrict__ jlist) {
+    extern __shared__ uint8_t smraw[];
+    __shared__ __align__(8) uint64_t full_t[kXStages], full_a[kXStages], empty[kXStages];
+    __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2], done;
+    __shared__ uint32_t tmem_base;
+    __shared__ int item_ng[kXMeta];  // groups of the items in flight, for the MMA issuer
+    __shared__ int abort_flag;
+    uint8_t* sm = (uint8_t*)(((uintptr_t)smraw + 1023) & ~(uintptr_t)1023);  // stages: A | B half | j | i
+    float* tabs = reinterpret_cast<float*>(sm + kXStages * kXStage);
+    volatile int* abort = &abort_flag;
+    const int n = w.d.snps;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // warp-uniform for the compiler too
+    const int ksteps = ((nw_c + 3) >> 2) + ((nw_t + 3) >> 2);  // stages of 256 samples
+    const uint32_t rank = cluster_rank();  // 0 issues the MMAs
+    const long long cid = cluster_id(), ncl = cluster_count();
+
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
+                     "r"(512));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+    }
+    if (tid == 0) {
+        auto init = [](uint64_t* b, int count) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(count));
+        };
+        for (int s = 0; s < kXStages; ++s) {
+            init(&full_t[s], 1);
+            init(&full_a[s], 2 * kXBuildWarps);
+            init(&empty[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            init(&acc_full[b], 1);
+            init(&acc_empty[b], 2 * kXEpiWarps);
+        }
+        init(&done, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;");
+        abort_flag = 0;
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    const uint32_t tmem = tmem_base;
+    if (warp >= 4 && warp < 8) f4_fill_scales<16>(tmem, warp & 3, kXColOne, kXColW, pack);
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    cluster_sync_all();  // both CTAs' barriers and scales exist before either signals the other
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    bool ok = true;
+
+    // (the register limits are set inside the branches: set before them, the
+    // compiler would hold every branch to the smallest)
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+        if (warp == 0) {
+            // ---------------------------------------------------------------- TMA producer (both CTAs)
+            if (g0 + cid < g1 && elect_one()) {
+                unsigned s = 0, par = 1;  // stage and the parity its last release has (first round: free)
+                unsigned step = 0, item = 0;
+                int wi = -1;
+                T3xItem it = t3x_item<LIST>(item_begin, jl_begin, jlist, n, g0 + cid, wi);
+                for (long long g = g0 + cid; g < g1 && ok; g += ncl) {
+                    int jr = it.j0 + kXJ * (int)rank;  // row (SNP position) of this CTA's first j
+                    if (LIST) {
+                        // 32 listed j are consecutive residue-ordered rows from the first one (rows past the
+                        // end of i's list are loaded too and ignored by the epilogue)
+                        const long long p = it.p0 + kXJ * (int)rank;
+                        jr = p < __ldg(jl_begin + it.i + 1) ? residue_row(__ldg(jlist + p), w.dist_step, n) : 0;
+                    }
+                    const int brow = 2 * it.l0 + t3x_n(it.ng) / 2 * (int)rank, irow = 2 * it.i;
+                    item_ng[item++ % kXMeta] = it.ng;
+                    T3xItem nx = it;
+                    for (int ks = 0; ks < ksteps; ++ks) {
+                        if (!t3_wait_cl(smem_u32(&empty[s]), par, abort)) {
+                            ok = false;
+                            break;
+                        }
+                        const uint32_t st = smem_u32(sm + s * kXStage), bar = smem_u32(&full_t[s]);
+                        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                                     "r"((uint32_t)(kXSB + kXSJ + kXSI))
+                                     : "memory");
+                        t3_tma(st + kXSA + kXSB, &map_j, kXBitRow * ks, 2 * jr, bar);
+                        t3_tma(st + kXSA + kXSB + kXSJ, &map_i, kXBitRow * ks, irow, bar);
+                        t3_tma(st + kXSA, &map_b, kXRow * ks, brow, bar);
+                        if (step < kXStages) ++step;
+                        if (++s == kXStages) {
+                            s = 0;
+                            par ^= 1;
+                        }
+                        // the next item's place is looked up while this item's copies are in flight
+                        if (ks == 0 && g + ncl < g1) nx = t3x_item<LIST>(item_begin, jl_begin, jlist, n, g + ncl, wi);
+                    }
+                    it = nx;
+                }
+                // no copy may be in flight when the CTA exits: the last use of every stage used
+                for (unsigned q = 0; q < step; ++q) {
+                    // stage q was last filled in the round before `par` names, or in this one when q < s
+                    if (!t3_drain(smem_u32(&full_t[q]), q < s ? par ^ 1 : par)) ok = false;
+                }
+            }
+            __syncwarp();
+        } else if (warp == 1) {
+            // ---------------------------------------------------------------- MMA issuer (CTA 0)
+            // (its own time per stage counts: about 230 cycles alone on an SM quarter, up to twice that beside
+            // the other warps, against 480 of MMA; so it decodes no items and its loop holds what it must)
+            if (rank == 0 && elect_one()) {
+                const uint32_t full0 = smem_u32(&full_a[0]), empty0 = smem_u32(&empty[0]);
+                const uint32_t desc_hi = (uint32_t)(t3_desc(0) >> 32), desc0 = (uint32_t)t3_desc(smem_u32(sm));
+                const uint32_t one = tmem + (uint32_t)kXColOne;
+                uint32_t bar = 0, ad = desc0, par = 0;  // stage: barrier offset, A descriptor, parity
+                unsigned item = 0;
+                for (long long g = g0 + cid; g < g1 && ok; g += ncl, ++item) {
+                    const unsigned buf = item & 1;
+                    if (item >= 2 && !t3_wait_cl(smem_u32(&acc_empty[buf]), ((item >> 1) - 1) & 1, abort)) {
+                        ok = false;
+                        break;
+                    }
+                    const uint32_t dcol = tmem + (uint32_t)(kXN * buf);
+                    uint32_t acc = 0, idesc = 0;
+                    for (int cls = 0; cls < 2 && ok; ++cls) {
+                        const uint32_t sfb = tmem + (uint32_t)(cls ? kXColW : kXColOne);
+                        for (int left = cls ? nw_t : nw_c; left > 0; left -= 4) {
+                            if (!t3_wait_cl(full0 + bar, par, abort)) {  // both CTAs' rows landed, A tiles built
+                                ok = false;
+                                break;
+                            }
+                            asm volatile("tcgen05.fence::after_thread_sync;");
+                            if (!acc) idesc = f4_idesc(2 * kXM, t3x_n(item_ng[item % kXMeta]));
+                            auto mma = [&](int k) {
+                                f4_mma<2>(dcol, (uint64_t)desc_hi << 32 | (ad + 2 * k),
+                                          (uint64_t)desc_hi << 32 | (ad + (kXSA >> 4) + 2 * k), idesc, one, sfb, acc);
+                                acc = 1;
+                            };
+                            mma(0);
+                            if (left >= 4) {
+                                mma(1);
+                                mma(2);
+                                mma(3);
+                            } else {  // the class's last steps
+                                for (int k = 1; k < left; ++k) mma(k);
+                            }
+                            commit_pair(empty0 + bar);
+                            bar += 8;
+                            ad += kXStage >> 4;
+                            if (bar == 8 * kXStages) {
+                                bar = 0;
+                                ad = desc0;
+                                par ^= 1;
+                            }
+                        }
+                    }
+                    if (!ok) break;
+                    commit_pair(smem_u32(&acc_full[buf]));
+                }
+                commit_pair(smem_u32(&done));
+                // neither CTA releases shared or tensor memory before the pair's MMAs are
+                // done (CTA 1 waits once its own work is over, below: waiting here would
+                // span its whole launch, longer than the bound on a single wait)
+                if (!t3_drain_cl(smem_u32(&done), 0)) ok = false;
+            }
+            __syncwarp();
+        }
+    } else if (warp < 12) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+        // ---------------------------------------------------------------- A builders (both CTAs)
+        // thread: 16-byte chunk c (32 samples) of the j rows rg, rg + 16, .. of every second stage
+        const int t = (tid - 128) & (32 * kXBuildWarps - 1), c = t & 7, rg = t >> 3;
+        const uint32_t full0 = cluster_addr(smem_u32(&full_a[0]), 0);
+        // A row (jj / 8, x, y, jj % 8) of staged row (jj, y) = rg + 16 u; x = 1 is 16 rows on, u + 1 32 rows
+        const int jj = rg >> 1, y = rg & 1;
+        const int dst0 = (8 * y + jj) * kXRow + ((c ^ jj) << 4);
+        unsigned s = 0, par = 0;
+        bool mine = warp < 8;
+        for (long long g = g0 + cid; g < g1 && ok; g += ncl) {
+            for (int ks = 0; ks < ksteps; ++ks, mine = !mine) {
+                if (mine) {
+                    if (!t3_wait(smem_u32(&full_t[s]), par, abort)) {
+                        ok = false;
+                        break;
+                    }
+                    uint8_t* st = sm + s * kXStage;
+                    const uint32_t* sJ = reinterpret_cast<const uint32_t*>(st + kXSA + kXSB) + rg * 8 + c;
+                    const uint32_t* sI = reinterpret_cast<const uint32_t*>(st + kXSA + kXSB + kXSJ) + c;
+                    uint32_t jw[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) jw[u] = sJ[128 * u];
+                    const uint32_t i0 = sI[0], i1 = sI[8];
+                    uint8_t* dst = st + dst0;
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        *reinterpret_cast<uint4*>(dst + 32 * u * kXRow) = f4_expand_a(i0, jw[u]);
+                        *reinterpret_cast<uint4*>(dst + (32 * u + 16) * kXRow) = f4_expand_a(i1, jw[u]);
+                    }
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) arrive_cl(full0 + 8 * s);
+                }
+                if (++s == kXStages) {
+                    s = 0;
+                    par ^= 1;
+                }
+            }
+        }
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 160;");
+        // ---------------------------------------------------------------- epilogue (both CTAs)
+        const int q = warp & 3, hh = (warp - 12) >> 2;  // lane quarter (8 j); the two warps of a quarter take alternate groups
+        const int jl = lane >> 2, lc = 2 * (lane & 3);  // this thread's j and its two l of a group
+        const int et = tid - 32 * 12;
+        const float W = (float)(1u << pack);
+        const float ntot = fmaf(W, (float)w.d.n_ctrls, (float)w.d.n_cases);
+        const bool all = dump != nullptr || sink.digest != nullptr;  // every combination takes the exact path
+        long long item = 0;
+        int wi = -1;
+        // (after an abort the warps keep going through the items, so that every one
+        // reaches the named barrier the same number of times)
+        for (long long g = g0 + cid; g < g1; g += ncl, ++item) {
+            const T3xItem it = t3x_item<LIST>(item_begin, jl_begin, jlist, n, g, wi);
+            const int i = it.i, l0 = it.l0, ng = it.ng;
+            const int buf = (int)(item & 1);
+            // marginal table of (i, l), packed, for every l of the item: entries (x, z), x and z in
+            // {0, 1, 2}; the buffer's readers of two items ago passed the barrier of the last item
+            float* tab = tabs + (kXTab / 4) * buf;
+            const uint4 s1 = __ldg(reinterpret_cast<const uint4*>(single) + i);
+            if (et < kXL) {
+                const int l = l0 + et;
+                float m[3][3];
+#pragma unroll
+                for (int k = 0; k < 9; ++k) m[k / 3][k % 3] = 0.f;
+                if (et < 8 * ng && l < n && l > i) {
+                    const uint4 p = __ldg(pairs + pair_index(i, l, n));
+                    const uint4 sl = __ldg(reinterpret_cast<const uint4*>(single) + l);
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) {
+#pragma unroll
+                        for (int z = 0; z < 2; ++z) m[x][z] = t3x_pair(p, x, z, W);
+                        m[x][2] = t3x_pk(x ? s1.y : s1.x, x ? s1.w : s1.z, W) - m[x][0] - m[x][1];
+                    }
+#pragma unroll
+                    for (int z = 0; z < 2; ++z)
+                        m[2][z] = t3x_pk(z ? sl.y : sl.x, z ? sl.w : sl.z, W) - m[0][z] - m[1][z];
+                    m[2][2] = ntot - t3x_pk(s1.x, s1.z, W) - t3x_pk(s1.y, s1.w, W) - m[2][0] - m[2][1];
+                }
+#pragma unroll
+                for (int k = 0; k < 9; ++k) tab[k * kXL + et] = m[k / 3][k % 3];
+            }
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * kXEpiWarps) : "memory");
+            if (!ok) continue;
+            int j = n;
+            if (LIST) {
+                const long long p = it.p0 + kXJ * (int)rank + 8 * q + jl;
+                if (p < __ldg(jl_begin + i + 1)) j = __ldg(jlist + p);
+            } else {
+                j = it.j0 + kXJ * (int)rank + 8 * q + jl;
+            }
+            const bool j_ok = j < n;
+            f2 ij[2][2], sj[2];
+            {
+                uint4 p = make_uint4(0, 0, 0, 0), sv = p;
+                if (j_ok) {
+                    p = __ldg(pairs + pair_index(i, j, n));
+                    sv = __ldg(reinterpret_cast<const uint4*>(single) + j);
+                }
+#pragma unroll
+                for (int x = 0; x < 2; ++x)
+#pragma unroll
+                    for (int y = 0; y < 2; ++y) ij[x][y] = f2_dup(t3x_pair(p, x, y, W));
+                sj[0] = f2_dup(t3x_pk(sv.x, sv.z, W));
+                sj[1] = f2_dup(t3x_pk(sv.y, sv.w, W));
+            }
+            const uint4* pj = j_ok ? pairs + pair_index(j, j + 1, n) - (j + 1) : pairs;  // + l: pair (j, l)
+            const uint4 zero4 = make_uint4(0, 0, 0, 0);
+            const int gi0 = (hh + (int)item) & 1;  // the odd group of an item goes to either warp in turn
+            uint4 pa = zero4, pb = zero4;
+            {
+                const int l = l0 + 8 * gi0 + lc;
+                if (j_ok && gi0 < ng && l < n && l > j) pa = __ldg(pj + l);
+                if (j_ok && gi0 < ng && l + 1 < n && l + 1 > j) pb = __ldg(pj + l + 1);
+            }
+            if (!t3_wait_cl(smem_u32(&acc_full[buf]), (uint32_t)((item >> 1) & 1), abort)) {
+                ok = false;
+                continue;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;");
+#pragma unroll 1
+            for (int gi = gi0; gi < ng; gi += 2) {
+                const int l = l0 + 8 * gi + lc;
+                const bool v0 = j_ok && l < n && l > j, v1 = j_ok && l + 1 < n && l + 1 > j;
+                const uint4 ca = pa, cb = pb;
+                {  // the next group's (j, l) pairs, ahead of their use
+                    const int ln = l + 16;
+                    pa = pb = zero4;
+                    if (j_ok && gi + 2 < ng && ln < n && ln > j) pa = __ldg(pj + ln);
+                    if (j_ok && gi + 2 < ng && ln + 1 < n && ln + 1 > j) pb = __ldg(pj + ln + 1);
+                }
+                const unsigned m0 = __ballot_sync(0xffffffffu, v0), m1 = __ballot_sync(0xffffffffu, v1);
+                if (!(m0 | m1)) continue;
+                if (sink.evaluated && lane == 0)
+                    atomicAdd(sink.evaluated, (unsigned long long)(__popc(m0) + __popc(m1)));
+                f2 c[2][2][2];  // [x][y][z], the two combinations side by side
+                {
+                    const uint32_t a0 = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(kXN * buf + 16 * gi);
+                    uint32_t r[2][8];
+#pragma unroll
+                    for (int x = 0; x < 2; ++x)
+                        asm volatile(
+                            "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                            : "=r"(r[x][0]), "=r"(r[x][1]), "=r"(r[x][2]), "=r"(r[x][3]), "=r"(r[x][4]),
+                              "=r"(r[x][5]), "=r"(r[x][6]), "=r"(r[x][7])
+                            : "r"(a0 + ((uint32_t)(16 * x) << 16)));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    // registers 4 z + 2 y (l) and + 1 (l + 1): lane block y, 8-column block z
+#pragma unroll
+                    for (int x = 0; x < 2; ++x)
+#pragma unroll
+                        for (int y = 0; y < 2; ++y)
+#pragma unroll
+                            for (int z = 0; z < 2; ++z)
+                                c[x][y][z] = f2_pack(__uint_as_float(r[x][4 * z + 2 * y]),
+                                                     __uint_as_float(r[x][4 * z + 2 * y + 1]));
+                }
+                const float* tl = tab + 8 * gi + lc;
+                auto il = [&](int x, int z) { return *reinterpret_cast<const f2*>(tl + (3 * x + z) * kXL); };
+                F4Bound bd(pack);
+                f2 a[2][2][3], y2[2][3];  // cells (x, y, z); cells (2, y, z)
+#pragma unroll
+                for (int x = 0; x < 2; ++x)
+#pragma unroll
+                    for (int y = 0; y < 2; ++y) {
+                        a[x][y][0] = c[x][y][0];
+                        a[x][y][1] = c[x][y][1];
+                        a[x][y][2] = f2_sub(f2_sub(ij[x][y], c[x][y][0]), c[x][y][1]);
+                        bd.two(a[x][y][0], a[x][y][1]);
+                    }
+                bd.two(a[0][0][2], a[0][1][2]);
+                bd.two(a[1][0][2], a[1][1][2]);
+#pragma unroll
+                for (int x = 0; x < 2; ++x)
+#pragma unroll
+                    for (int z = 0; z < 3; ++z) bd.one(f2_sub(f2_sub(il(x, z), a[x][0][z]), a[x][1][z]));
+#pragma unroll
+                for (int y = 0; y < 2; ++y) {
+                    f2 jl3[3];
+#pragma unroll
+                    for (int z = 0; z < 2; ++z) jl3[z] = f2_pack(t3x_pair(ca, y, z, W), t3x_pair(cb, y, z, W));
+                    jl3[2] = f2_sub(f2_sub(sj[y], jl3[0]), jl3[1]);
+#pragma unroll
+                    for (int z = 0; z < 3; ++z) {
+                        y2[y][z] = f2_sub(f2_sub(jl3[z], a[0][y][z]), a[1][y][z]);
+                        bd.one(y2[y][z]);
+                    }
+                }
+#pragma unroll
+                for (int z = 0; z < 3; ++z) bd.one(f2_sub(f2_sub(il(2, z), y2[0][z]), y2[1][z]));
+                float b0, b1;
+                f2_unpack(bd.acc, b0, b1);
+                const bool w0 = v0 && (all || b0 >= thr_q), w1 = v1 && (all || b1 >= thr_q);
+                if (__any_sync(0xffffffffu, w0 || w1)) {
+#pragma unroll 1
+                    for (int u = 0; u < 2; ++u) {
+                        const bool want = u ? w1 : w0;
+                        if (!__any_sync(0xffffffffu, want)) continue;
+                        // the combination's cells again, one lane of each pair
+                        auto at = [&](f2 v) {
+                            float lo, hi;
+                            f2_unpack(v, lo, hi);
+                            return u ? hi : lo;
+                        };
+                        const uint4 cj = u ? cb : ca;
+                        float t[27];
+#pragma unroll
+                        for (int x = 0; x < 2; ++x)
+#pragma unroll
+                            for (int y = 0; y < 2; ++y) {
+                                t[9 * x + 3 * y] = at(c[x][y][0]);
+                                t[9 * x + 3 * y + 1] = at(c[x][y][1]);
+                                t[9 * x + 3 * y + 2] = at(ij[x][y]) - t[9 * x + 3 * y] - t[9 * x + 3 * y + 1];
+                            }
+#pragma unroll
+                        for (int x = 0; x < 2; ++x)
+#pragma unroll
+                            for (int z = 0; z < 3; ++z)
+                                t[9 * x + 6 + z] = tl[(3 * x + z) * kXL + u] - t[9 * x + z] - t[9 * x + 3 + z];
+#pragma unroll
+                        for (int y = 0; y < 2; ++y) {
+                            const float z0 = t3x_pair(cj, y, 0, W), z1 = t3x_pair(cj, y, 1, W);
+                            t[18 + 3 * y] = z0 - t[3 * y] - t[9 + 3 * y];
+                            t[18 + 3 * y + 1] = z1 - t[3 * y + 1] - t[9 + 3 * y + 1];
+                            t[18 + 3 * y + 2] = at(sj[y]) - z0 - z1 - t[3 * y + 2] - t[9 + 3 * y + 2];
+                        }
+#pragma unroll
+                        for (int z = 0; z < 3; ++z)
+                            t[24 + z] = tl[(6 + z) * kXL + u] - t[18 + z] - t[21 + z];
+                        t3x_survivor(w, sink, thr_f, dump, t, pack, i, j, l + u, want, lane);
+                    }
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;");
+            __syncwarp();
+            if (lane == 0) arrive_cl(cluster_addr(smem_u32(&acc_empty[buf]), 0));
+        }
+    }
+    if (!ok) *abort = 1;
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    // CTA 1: its epilogue has read the last accumulators, so the pair's final
+    // commit to this CTA's `done` lands soon; it must land before the CTA exits
+    if (rank == 1 && warp == 1 && lane == 0 && !t3_drain_cl(smem_u32(&done), 0)) *abort = 1;
+    cluster_sync_all();  // the other CTA is done with this CTA's shared and tensor memory
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    if (tid == 0 && abort_flag) atomicOr(status, 1);
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
+}
+
+// ---------------------------------------------------------------------------
+// Operand layout of a data set, 32 samples of an SNP's genotype row g (0, 1) per thread: the bit
+// rows 2 snp + g hold the class's words of the reference layout, cases then controls, each class
+// padded to a multiple of 256 samples; the planes hold the same bits spread to e2m1 in rows
+// f4_row(snp, g), SNPs past the last one zero.
+__global__ void f4_layout_kernel(DevData d, uint32_t* bits, uint4* planes, int wpr, int wc, int nc32, int nt32,
+                                 int rows) {
+    const size_t per_snp = 3 * (size_t)(d.cw + d.tw);
+    const long long total = (long long)rows * wpr;
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
+         e += (long long)gridDim.x * blockDim.x) {
+        const int row = (int)(e / wpr), o = (int)(e - (long long)row * wpr);
+        const int snp = 8 * (row >> 4) + (row & 7), g = (row >> 3) & 1;
+        const bool ctrl = o >= wc;
+        const int k = ctrl ? o - wc : o;
+        uint32_t v = 0;
+        if (snp < d.snps) {
+            if (k < (ctrl ? nt32 : nc32)) {
+                const uint64_t word = __ldg(d.ref + snp * per_snp + (ctrl ? 3 * (size_t)d.cw : 0) +
+                                            (size_t)g * (ctrl ? d.tw : d.cw) + (k >> 1));
+                v = (uint32_t)(word >> (32 * (k & 1)));
+            }
+            bits[((size_t)2 * snp + g) * wpr + o] = v;
+        }
+        planes[e] = f4_expand_b(v);
+    }
+}
+
+int f4_pack(int n_cases, int n_ctrls) {
+    for (int p = 1; p < 24; ++p) {
+        const long long W = 1ll << p;
+        if (W > n_cases && n_cases + W * (long long)n_ctrls < (1ll << 24)) return p;
+    }
+    return 0;
+}
+
+cudaError_t f4_bit_map(CUtensorMap* m, const F4Plan& f, const uint32_t* bits, int rows, int box_rows) {
+    return tensor_map(m, bits, rows, 4 * f.wpr, kXBitRow, box_rows, false);
+}
+
+cudaError_t f4_prepare(const DevData& d, F4Plan& f, cudaStream_t s) {
+    f.nw_c = (d.n_cases + 63) / 64;
+    f.nw_t = (d.n_ctrls + 63) / 64;
+    const int wc = 8 * ((f.nw_c + 3) / 4), wt = 8 * ((f.nw_t + 3) / 4);
+    f.wpr = wc + wt;
+    f.rows = 16 * ((d.snps + 7) / 8);
+    const size_t plane_bytes = (size_t)f.rows * f.wpr * 16;  // one allocation: planes, then bits
+    cudaError_t e = cudaMalloc((void**)&f.planes, plane_bytes + (size_t)2 * d.snps * f.wpr * 4);
+    if (e != cudaSuccess) return e;
+    f.bits = reinterpret_cast<uint32_t*>(f.planes + plane_bytes);
+    const long long total = (long long)f.rows * f.wpr;
+    f4_layout_kernel<<<(unsigned)std::min<long long>((total + 255) / 256, 8192), 256, 0, s>>>(
+        d, f.bits, reinterpret_cast<uint4*>(f.planes), f.wpr, wc, 2 * f.nw_c, 2 * f.nw_t, f.rows);
+    count_launch();
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if ((e = tensor_map(&f.map_b, f.planes, f.rows, 16 * f.wpr, kXRow, kXN / 2, true)) != cudaSuccess) return e;
+    if ((e = f4_bit_map(&f.map_j, f, f.bits, 2 * d.snps, 2 * kXJ)) != cudaSuccess) return e;
+    return f4_bit_map(&f.map_i, f, f.bits, 2 * d.snps, 2);
+}
+
+void f4_release(F4Plan& f) {
+    cudaFree(f.planes);
+    f.planes = nullptr;
+    f.bits = nullptr;
+}
+
+std::vector<long long> t3x_items(int n) {
+    std::vector<long long> b((size_t)n + 1, 0);
+    for (int i = 0; i < n; ++i) {
+        long long c = 0;
+        for (int j = i + 1; j < n - 1; j += kPxJ) c += t3x_tiles(n, j);
+        b[i + 1] = b[i] + c;
+    }
+    return b;
+}
+
+cudaError_t launch_tensor3x(const ScanWork& w, const F4Plan& f, const T3xRange& r, long long g0, long long g1,
+                            const CandSink& sink, uint32_t* dump, const uint32_t* single, const uint4* pairs,
+                            float thr_f, float thr_q, int* status, cudaStream_t s, int sms) {
+    // set once, by whichever host thread comes first (thread-safe static initialisation)
+    static const cudaError_t attr = [] {
+        cudaError_t e = cudaFuncSetAttribute(tensor3x_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)kXSmem);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(tensor3x_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kXSmem);
+        return e;
+    }();
+    if (attr != cudaSuccess) return attr;
+    if (g1 <= g0) return cudaSuccess;
+    static const int max_clusters = pair_clusters(tensor3x_kernel<false>, kXThreads, kXSmem);
+    const long long clusters = std::min<long long>(g1 - g0, max_clusters > 0 ? max_clusters : sms / 2);
+    const unsigned grid = (unsigned)(2 * std::max(1ll, clusters));
+    if (r.jlist)
+        tensor3x_kernel<true><<<grid, kXThreads, kXSmem, s>>>(f.map_b, *r.map_j, f.map_i, w, sink, r.item_begin, g0, g1,
+                                                              f.nw_c, f.nw_t, f.pack, thr_f, thr_q, dump, single, pairs,
+                                                              status, r.jl_begin, r.jlist);
+    else
+        tensor3x_kernel<false><<<grid, kXThreads, kXSmem, s>>>(f.map_b, *r.map_j, f.map_i, w, sink, r.item_begin, g0,
+                                                               g1, f.nw_c, f.nw_t, f.pack, thr_f, thr_q, dump, single,
+                                                               pairs, status, nullptr, nullptr);
+    count_launch();
+    return cudaGetLastError();
+}
+
+}  // namespace fiu

@@ -1,0 +1,191 @@
+// Device helpers of the tcgen05 kernels on 4-bit operands (kind::mxf4).
+//
+// Operands are genotype indicators, 0 or 1 (or 0 and a power of two, with the
+// other operand's the inverse): e2m1 holds them exactly and tcgen05.mma kind::mxf4 sums their products in FP32, exactly
+// up to 2^24, at twice the samples per instruction of e4m3 (M 128 x N 256:
+// 64 samples in 128 cycles against 32; measured, every sum equal to the
+// integer one up to 1.67e7).  The block scales (ue8m0, one per 32 samples of a
+// row) are the same for every row and block of an instruction, so their layout
+// in tensor memory does not matter: a region of 8 columns filled with 2^0 and
+// one filled with 2^p, written once per launch.  The second is used as the B
+// scale of control samples when both classes share an accumulator, which then
+// holds cases + 2^p * controls.
+#pragma once
+
+#include <algorithm>
+#include <cmath>
+
+#include "tensor_common.cuh"
+
+namespace fiu {
+
+constexpr int kF4K = 256;                        // samples per 128-byte operand row and pipeline stage
+
+// Instruction descriptor: e2m1 x e2m1 (format 1 at bits 7 and 10), ue8m0 scales (bit 23), N / 8, M / 16.
+__host__ __device__ constexpr uint32_t f4_idesc(int M, int N) {
+    return (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | (1u << 23) | ((uint32_t)(M >> 4) << 24);
+}
+
+template <int CG>
+__device__ __forceinline__ void f4_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t sfa, uint32_t sfb,
+                                       uint32_t acc) {
+    if (CG == 1)
+        asm volatile(
+            "{.reg .pred p; setp.ne.b32 p, %6, 0;\n"
+            "tcgen05.mma.cta_group::1.kind::mxf4.block_scale.block32 [%0], %1, %2, %3, [%4], [%5], p;}\n" ::"r"(d),
+            "l"(a), "l"(b), "r"(idesc), "r"(sfa), "r"(sfb), "r"(acc));
+    else
+        asm volatile(
+            "{.reg .pred p; setp.ne.b32 p, %6, 0;\n"
+            "tcgen05.mma.cta_group::2.kind::mxf4.block_scale.block32 [%0], %1, %2, %3, [%4], [%5], p;}\n" ::"r"(d),
+            "l"(a), "l"(b), "r"(idesc), "r"(sfa), "r"(sfb), "r"(acc));
+}
+
+// Fills this warp's 32 tensor-memory lanes of both scale regions, `cols` (a
+// multiple of 8) columns each: 8 hold the scales of 256 rows.  Every lane
+// quarter has to be filled by one warp whose index is the quarter mod 4.
+template <int cols>
+__device__ __forceinline__ void f4_fill_scales(uint32_t tmem, int q, int col_one, int col_w, int p) {
+    const uint32_t base = tmem + ((uint32_t)(32 * q) << 16);
+    const uint32_t one = 0x7F7F7F7Fu, w = (uint32_t)(0x7F + p) * 0x01010101u;
+#pragma unroll
+    for (int c = 0; c < cols; c += 4) {
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %1, %1, %1};" ::"r"(base + col_one + c),
+                     "r"(one));
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %1, %1, %1};" ::"r"(base + col_w + c),
+                     "r"(w));
+    }
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
+// Operand bytes of 32 samples, one bit each: nibble u of word t belongs to bit
+// 4 u + t.  A bit is used where it stands or after one shift, so A has it as
+// 0.5, 1, 2 and 1 in words 0 to 3 and B as 2, 1, 0.5 and 1: the products of
+// two set bits are 1.  A is the AND of two (the shift and mask of a word are
+// then 6 operations, against 8 with 1.0 everywhere).
+__device__ __forceinline__ uint4 f4_expand_a(uint32_t i, uint32_t j) {
+    const uint32_t v = i & j;
+    return make_uint4(i & j & 0x11111111u, i & j & 0x22222222u, i & j & 0x44444444u, (v >> 2) & 0x22222222u);
+}
+__device__ __forceinline__ uint4 f4_expand_b(uint32_t w) {
+    const uint32_t v = w >> 2;
+    return make_uint4((w << 2) & 0x44444444u, w & 0x22222222u, v & 0x11111111u, v & 0x22222222u);
+}
+
+// Row of SNP l, genotype z in the operand planes: SNPs in groups of 8, the
+// eight rows of genotype 0 before the eight of genotype 1, so that a thread
+// reading 16x256b accumulator columns finds two neighbouring SNPs in a
+// register pair and the two genotypes in successive 8-column blocks.
+__host__ __device__ __forceinline__ int f4_row(int l, int z) { return 16 * (l >> 3) + 8 * z + (l & 7); }
+
+// ---- two single-precision values per operation (f32x2) -----------------------
+// Same arithmetic rate as the scalar forms (measured: 2 cycles against 1 per
+// warp instruction) at half the issue slots.
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 f2_pack(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void f2_unpack(f2 v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f2 f2_dup(float a) { return f2_pack(a, a); }
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2_sub(f2 a, f2 b) {
+    f2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f2 f2_fma_rz(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f2 f2_rcp(f2 v) {
+    float a, b;
+    f2_unpack(v, a, b);
+    asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(a));
+    asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(b));
+    return f2_pack(a, b);
+}
+
+// ---- the quadratic bound on the mutual information ----------------------------
+// With q the control fraction, D(p||q) the binary relative entropy in bits and
+// s, b the size and the controls of a cell, N MI = sum over the cells of
+// s D(b/s || q).  D(p||q) <= c (p - q)^2 on [0, 1] for
+//     c = max(1 / (2 ln2 q (1-q)), -lg(1-q) / q^2, -lg(q) / (1-q)^2):
+// f(p) = D(p||q) - c (p-q)^2 has f(q) = f'(q) = 0 and
+// f'' = 1 / (ln2 p (1-p)) - 2c, which is <= 0 on an interval around q (first
+// term of the maximum) and > 0 beyond it, so f falls from 0 up to where the
+// interval ends and lies below its chord to the end point (second and third
+// terms) after that.  As the sizes add up to N and the controls to n_ctrls,
+//     N MI <= c (sum b^2 / s - n_ctrls^2 / N)      [bits],
+// one reciprocal a cell instead of three logarithms.  For q = 1/2 the bound is
+// at most 4 / (2 / ln2) = 1.39 times the value, so nearly every combination
+// falls below a top-N threshold and its logarithms are never taken.
+//
+// Cells arrive packed, D = cases + W controls (exact in FP32): controls =
+// floor(D / W) by a fused multiply-add that rounds toward zero at 2^23.
+struct F4Bound {
+    f2 inv_w, m23, neg_m23, neg_w1, tiny, acc;
+    __device__ __forceinline__ explicit F4Bound(int p) {
+        inv_w = f2_dup(__uint_as_float((uint32_t)(127 - p) << 23));
+        m23 = f2_dup(8388608.0f);
+        neg_m23 = f2_dup(-8388608.0f);
+        neg_w1 = f2_dup(1.0f - (float)(1 << p));
+        tiny = f2_dup(9.5367431640625e-07f);  // 2^-20
+        acc = 0;
+    }
+    // controls b and size s (+ 2^-20, so that an empty cell divides by no zero) of packed cells D
+    __device__ __forceinline__ void split(f2 D, f2& b, f2& s) const {
+        b = f2_add(f2_fma_rz(D, inv_w, m23), neg_m23);
+        s = f2_add(f2_fma(neg_w1, b, D), tiny);
+    }
+    __device__ __forceinline__ void one(f2 D) {
+        f2 b, s;
+        split(D, b, s);
+        acc = f2_fma(b, f2_mul(b, f2_rcp(s)), acc);
+    }
+    // two cells with one reciprocal: (b1^2 s2 + b2^2 s1) / (s1 s2)
+    __device__ __forceinline__ void two(f2 D1, f2 D2) {
+        f2 b1, s1, b2, s2;
+        split(D1, b1, s1);
+        split(D2, b2, s2);
+        const f2 r = f2_rcp(f2_mul(s1, s2));
+        const f2 num = f2_fma(f2_mul(b1, b1), s2, f2_mul(f2_mul(b2, b2), s1));
+        acc = f2_fma(num, r, acc);
+    }
+};
+
+// The bound's constants for a threshold (host): a combination can only reach
+// thr_bits (N MI in bits) when sum b^2 / s >= the returned value.  Slack: each
+// of `cells` terms, at most b <= n_ctrls, carries at most 12 roundings or
+// approximations of 2^-22 and the sum `cells` more of 2^-24 of the total
+// n_ctrls; the 2^-20 shift lowers a term by at most 2^-20 of it.  Doubled.
+inline float f4_bound_threshold(double thr_bits, int n_cases, int n_ctrls, int cells) {
+    const double N = (double)n_cases + n_ctrls, q = n_ctrls / N;
+    if (n_cases < 1 || n_ctrls < 1) return -3.0e38f;
+    const double lg_q = std::log2(q), lg_1q = std::log2(1 - q);
+    const double c = std::max({1 / (2 * std::log(2.0) * q * (1 - q)), -lg_1q / (q * q), -lg_q / ((1 - q) * (1 - q))});
+    const double u = std::ldexp(1.0, -24);
+    const double slack = 2 * n_ctrls * (12 * 4 * u + 16 * u + cells * u) + 1e-3;
+    const double t = thr_bits / c * (1 - 1e-9) + q * n_ctrls - slack;
+    return (float)std::max(-3.0e38, std::min(3.0e38, t < 0 ? t * (1 + 1e-6) : t * (1 - 1e-7)));
+}
+
+}  // namespace fiu
