@@ -232,27 +232,28 @@ int choose_tile(fiu_ctx* ctx, const fiu_resident* res, const ScanWork& w, int re
             return fail(ctx, FIU_ERR_UNSUPPORTED,
                         "the tensor-core kernels need one-hot data, order 2, 3 or 4 and the whole data set on one "
                         "worker");
-        int rc = choose_kernel(ctx, res, (unsigned)w.order, FIU_KERNEL_ELIDED_HS, kernel);  // builds the core tables
-        if (rc) return rc;
         fiu_resident* r = const_cast<fiu_resident*>(res);
         if (!r->t3) {
             auto* plan = new (std::nothrow) T3Plan;
             if (!plan) return fail(ctx, FIU_ERR_NOMEM, "tensor plan");
             cudaError_t e = tensor3_prepare(r->d, *plan, ctx->stream);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
             if (e != cudaSuccess) {
                 tensor3_release(*plan);
                 delete plan;
-                return cuda_fail(ctx, e, "tensor operand planes");
+                return cuda_fail(ctx, e, "tensor work items");
             }
             r->t3 = plan;
         }
+        // the core tables; the order-4 pair kernel makes its triples itself
+        const unsigned cores = w.order == 4 && r->t3->pair3 ? 3u : (unsigned)w.order;
+        int rc = choose_kernel(ctx, res, cores, FIU_KERNEL_ELIDED_HS, kernel);
+        if (rc) return rc;
         if (!whole_data_set(res, w)) {
-            cudaError_t e = tensor3_layer(*r->t3, w, ctx->stream);
+            cudaError_t e = tensor3_layer(*r->t3, w, res->pairs, ctx->stream, ctx->sms);
             if (e != cudaSuccess) return cuda_fail(ctx, e, "tensor work items of a distribution layer");
         } else {
-            cudaError_t e = tensor3_order_items(*r->t3, r->d, w.order, ctx->stream);
-            if (e != cudaSuccess) return cuda_fail(ctx, e, "tensor work items");
+            cudaError_t e = tensor3_order_items(*r->t3, r->d, w.order, res->pairs, ctx->stream, ctx->sms);
+            if (e != cudaSuccess) return cuda_fail(ctx, e, "tensor operands and work items");
         }
         kernel = FIU_KERNEL_TENSOR;
         // GEMM width N: order 3 uses 256 with one accumulator for both classes, 192 with one per class
@@ -348,8 +349,10 @@ int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu
     int* t_status = (int*)(ctx->ctl + 16);
     if (tensor) CK(cudaMemsetAsync(t_status, 0, sizeof(int), ctx->stream), "status reset");
     const unsigned keep = outputs + std::max(32u, outputs / 8);
-    const size_t cap = std::max<size_t>({65536, (size_t)16 * keep, (size_t)res->d.snps + keep});
-    if ((rc = grow(ctx, ctx->cand, ctx->cand_cap, cap)) ||
+    const bool live = tensor && tensor_live(*res->t3, w);
+    const size_t cap = std::max<size_t>(
+        {live ? 262144u : 65536u, (size_t)(live ? 64 : 16) * keep, (size_t)res->d.snps + keep});
+    if ((rc = grow(ctx, ctx->cand, ctx->cand_cap, cap + 8192)) ||
         (rc = grow(ctx, ctx->tmp, ctx->tmp_cap, cap + 8192)) ||
         (rc = grow(ctx, ctx->mi64, ctx->mi64_cap, (size_t)keep)))
         return rc;
@@ -357,6 +360,8 @@ int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu
     unsigned* count = ctx->ctl;
     unsigned* overflow = ctx->ctl + 1;
     unsigned* scratch = ctx->ctl + 4;
+    unsigned* hist = ctx->ctl + 512;
+    long long* live_thr = (long long*)(ctx->ctl + 2);
     long long thr = (long long)0x8000000000000000ull;
     unsigned have = 0;
     const double per_prefix = (double)binom(w.dist_n, order) / std::max<double>(1.0, (double)binom(w.dist_n, order - 1));
@@ -376,14 +381,71 @@ int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu
     double seen = 0, sec_per_unit = 0;
     long long m = units / n_shards * shard + std::min<long long>(shard, units % n_shards);
     const long long m_end = m + units / n_shards + (shard < units % n_shards ? 1 : 0);
+    // With a live threshold (the kernel raises it as candidates come) two launches cover the request
+    // and the host waits once: the first takes enough units for a threshold to start from, and no
+    // more than a quarter of the candidate buffer holds, since every combination of it is one.  A
+    // buffer that overflows all the same leaves the request to the loop below.
+    if (live && !ctx->cancellable && m < m_end) {
+        const long long few = std::max<long long>(1, (long long)(2.0 * keep / std::max(1.0, per_unit)));
+        const long long fit = (long long)((double)cap / 4 / std::max(1.0, per_unit));
+        const long long m1 = std::min(m_end, m + std::max(few, std::min<long long>(fit, ctx->sms / 2)));
+        ctx->pinned[0] = ctx->pinned[1] = 0;
+        memcpy(ctx->pinned + 2, &thr, sizeof(thr));
+        CK(cudaMemcpyAsync(count, ctx->pinned, 4 * sizeof(unsigned), cudaMemcpyHostToDevice, s), "reset counters");
+        CK(cudaMemsetAsync(hist, 0, kLiveBins * sizeof(unsigned), s), "reset counters");
+        CandSink sink{ctx->cand, count, overflow, (unsigned)cap, thr, ctx->timing ? ctx->evaluated : nullptr};
+        sink.hist = hist;
+        sink.live = live_thr;
+        sink.keep = keep;
+        if (ctx->timing) CK(cudaEventRecord(ctx->ev0, s), "event");
+        CK(launch_tensor3(w, *res->t3, m, m1, sink, nullptr, res->single, res->pairs, res->triples, t_status, s,
+                          ctx->sms),
+           "tensor kernel launch");
+        if (m1 < m_end) {
+            CK(live_raise(sink, s), "threshold");
+            sink.thr = 0;  // (the kernel reads the live threshold; a threshold exists)
+            CK(launch_tensor3(w, *res->t3, m1, m_end, sink, nullptr, res->single, res->pairs, res->triples, t_status,
+                              s, ctx->sms),
+               "tensor kernel launch");
+        }
+        if (ctx->timing) CK(cudaEventRecord(ctx->ev1, s), "event");
+        unsigned* kept = scratch;  // [0]: candidates at or above the last threshold
+        CK(cudaMemsetAsync(kept, 0, sizeof(unsigned), s), "reset counters");
+        CK(live_compact(sink, ctx->tmp, kept, s), "candidate selection");
+        CK(cudaMemcpyAsync(ctx->pinned, count, 5 * sizeof(unsigned), cudaMemcpyDeviceToHost, s), "read counters");
+        CK(cudaStreamSynchronize(s), "count kernel");
+        if (ctx->timing) {
+            float ms = 0;
+            CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1), "event time");
+            ctx->count_ms += ms;
+            ctx->count_launches += m1 < m_end ? 2 : 1;
+        }
+        if (!ctx->pinned[1]) {
+            std::swap(ctx->cand, ctx->tmp);
+            std::swap(ctx->cand_cap, ctx->tmp_cap);
+            have = ctx->pinned[4];
+            if (have > keep) {
+                CK(select_top(ctx->cand, have, keep, ctx->tmp, scratch, s), "top-N selection");
+                have = keep;
+            }
+            m = m_end;
+        }
+    }
     while (m < m_end) {
         if (ctx->cancel.load(std::memory_order_relaxed)) return fail(ctx, FIU_ERR_CANCELLED, "search cancelled");
         const long long m1 = std::min(m_end, m + chunk);
         const auto t_chunk = std::chrono::steady_clock::now();
         ctx->pinned[0] = have;
         ctx->pinned[1] = 0;
-        CK(cudaMemcpyAsync(count, ctx->pinned, 2 * sizeof(unsigned), cudaMemcpyHostToDevice, s), "reset counters");
+        memcpy(ctx->pinned + 2, &thr, sizeof(thr));
+        CK(cudaMemcpyAsync(count, ctx->pinned, 4 * sizeof(unsigned), cudaMemcpyHostToDevice, s), "reset counters");
         CandSink sink{ctx->cand, count, overflow, (unsigned)cap, thr, ctx->timing ? ctx->evaluated : nullptr};
+        if (live) {
+            CK(cudaMemsetAsync(hist, 0, kLiveBins * sizeof(unsigned), s), "reset counters");
+            sink.hist = hist;
+            sink.live = live_thr;
+            sink.keep = keep;
+        }
         if (ctx->timing) CK(cudaEventRecord(ctx->ev0, s), "event");
         if (tensor)
             CK(launch_tensor3(w, *res->t3, m, m1, sink, nullptr, res->single, res->pairs, res->triples, t_status, s,
@@ -539,7 +601,7 @@ int fiu_create(int device, fiu_ctx** out) {
     if (cudaSetDevice(device) != cudaSuccess ||
         cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
         cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaMalloc((void**)&ctx->ctl, 512 * sizeof(unsigned)) != cudaSuccess ||
+        cudaMalloc((void**)&ctx->ctl, (512 + kLiveBins) * sizeof(unsigned)) != cudaSuccess ||
         cudaMallocHost((void**)&ctx->pinned, 16 * sizeof(unsigned)) != cudaSuccess) {
         fiu_destroy(ctx);
         return FIU_ERR_CUDA;

@@ -28,6 +28,22 @@ struct CandSink {
     unsigned long long* digest;
     uint32_t* dscratch;
     unsigned dscratch_threads;
+    // Live threshold (off when hist is null; kernels that know it start from
+    // *live instead of thr): every candidate is counted in hist by its key, and
+    // once `keep` of them have keys of a bin or above, *live rises to that bin's
+    // lower edge -- no combination below it can be among the best `keep`.
+    unsigned* hist;   // [kLiveBins]
+    long long* live;
+    unsigned keep;
+};
+
+// Bins of the live threshold: 128 per power of two of the key from 2^30
+// (a quarter nat of N * MI) to 2^48; below 2^30 all in bin 0.
+constexpr int kLiveBins = 18 * 128;
+// Conversion of a threshold key to the kernels' single-precision tests (linear; rounded down).
+struct LiveMap {
+    double est_k, est_c;      // logarithm estimate
+    double bound_k, bound_c;  // quadratic or quartic bound
 };
 
 // ---- multi-scan engine (batch.cu, engine.cu) ----------------------------------
@@ -178,6 +194,12 @@ struct F4Plan {
     int nw_c = 0, nw_t = 0;     // 64-sample steps that hold samples, per class
     CUtensorMap map_b;          // planes, box 128 B x 120 rows, 128-byte swizzle
     CUtensorMap map_j, map_i;   // bit rows, boxes of 32 B x 64 and x 2 rows
+    // order 4: the cores of all triples and pairs as packed floats, cases + W controls, of (l, l + 1)
+    // side by side; the entry of (.., k, l) is row_p[k] + l / 2, of (i, k, l) also + row_q[i]
+    float* tri = nullptr;       // 16 floats an entry: (x, z, w) of the genotypes of i, k and l
+    float* pairf = nullptr;     // 8 floats an entry: (z, w)
+    int *row_p = nullptr, *row_q = nullptr;
+    CUtensorMap map_b4, map_b4h, map_k4;  // planes, boxes 128 B x 112 and x 64 rows; bit rows, box 32 B x 32 rows
 };
 struct T3Plan {
     std::mutex items_mu;  // guards the planes and item tables made on the first use of an order
@@ -187,11 +209,11 @@ struct T3Plan {
     double item_combos = 0;  // combinations per work item, about 32 x L / 2
     int pitch = 0;        // bytes per plane row
     int k_cases = 0;      // padded case samples (= byte offset of the control region)
-    bool pair3 = false;   // order 3, classes that share an accumulator: items of the CTA-pair kernel (tensor3x.cu)
+    bool pair3 = false;   // orders 3 and 4, classes that share an accumulator: items of the CTA-pair kernels
     struct T3Layers* layers = nullptr;  // order 3, packed: work items of Distribution layers (tensor3.cu)
     long long* item_begin = nullptr;
     long long total = 0;  // work items
-    CUtensorMap map_l;    // box 128 B x 192 rows (256 when packed), 128-byte swizzle (l operand)
+    CUtensorMap map_l;    // box 128 B x 192 rows, 128-byte swizzle (l operand)
     CUtensorMap map_j;    // box 128 B x 64 rows, 128-byte swizzle (j rows of the (i,j) operand)
     CUtensorMap map_i;    // box 128 B x 2 rows, 128-byte swizzle (i rows)
     // order 2: work items (64 i, 128 j) over i-tiles, or pair items (2 x 64 i, 128 j) of the
@@ -203,8 +225,8 @@ struct T3Plan {
     double item2_combos = 0;
     CUtensorMap map_a2;   // box 128 B x 128 rows (i rows)
     CUtensorMap map_b2;   // box 128 B x 256 rows (j rows)
-    // order 4: work items (i, j, 16 k, 128 l) (64 l when the classes do not pack); item4_begin[j]
-    // = first item of the pairs with second SNP j, item4_per[j] = items per such pair
+    // order 4: work items (i, j, 32 k, up to 112 l) of the pair kernel, or (i, j, 16 k, 64 l) per class;
+    // item4_begin[j] = first item of the pairs with second SNP j, item4_per[j] = items per such pair
     long long* item4_begin = nullptr;
     long long* item4_per = nullptr;
     long long total4 = 0;
@@ -219,16 +241,19 @@ int tensor_pack(int n_cases, int n_ctrls);
 // combinations of an average unit.
 long long tensor_units(const T3Plan& plan, const ScanWork& w);
 double tensor_item_combos(const T3Plan& plan, const ScanWork& w);
+// Whether the kernel that serves w takes a live threshold (CandSink::hist).
+bool tensor_live(const T3Plan& plan, const ScanWork& w);
 // Whether the tensor kernels serve the Distribution layer of w (order 3,
 // classes that pack, the layer of all SNPs), and the layer's work items,
 // made on first use (host enumeration of the owned prefixes; the operand
 // planes ordered by SNP residue mod the layer's step, copied on stream s).
 bool tensor_layer_ok(const T3Plan& plan, const ScanWork& w);
-cudaError_t tensor3_layer(T3Plan& plan, const ScanWork& w, cudaStream_t s);
+cudaError_t tensor3_layer(T3Plan& plan, const ScanWork& w, const uint4* pairs, cudaStream_t s, int sms);
 cudaError_t tensor3_prepare(const DevData& d, T3Plan& plan, cudaStream_t s);
 // The operand planes that searches of an order read and the whole data set's
 // work items at order 3 or 4, made on first use (thread-safe).
-cudaError_t tensor3_order_items(T3Plan& plan, const DevData& d, int order, cudaStream_t s);
+cudaError_t tensor3_order_items(T3Plan& plan, const DevData& d, int order, const uint4* pairs, cudaStream_t s,
+                                int sms);
 // Tiled TMA map over rows of `pitch` bytes: boxes of box_bytes x box_rows, 128-byte swizzle or none.
 cudaError_t tensor_map(CUtensorMap* m, const void* base, int rows, int pitch, int box_bytes, int box_rows,
                        bool swizzle);
@@ -237,14 +262,15 @@ cudaError_t launch_tensor3(const ScanWork& w, const T3Plan& plan, long long g0, 
                            uint32_t* dump, const uint32_t* single, const uint4* pairs, const uint4* triples,
                            int* status, cudaStream_t s, int sms);
 // tensor4.cu -- order 4 on tcgen05 (one-hot data, the whole data set or a Distribution layer of it).
-std::vector<long long> t4_item_table(int n, bool pack, std::vector<long long>& per);
-long long t4_layer_items(int n, int step, long long offset, bool pack, std::vector<long long>& pbegin,
+// Item tables of the pair kernel (pair) or the per-class kernel.
+std::vector<long long> t4_item_table(int n, bool pair, std::vector<long long>& per);
+long long t4_layer_items(int n, int step, long long offset, bool pair, std::vector<long long>& pbegin,
                          std::vector<int4>& pinfo, long long& combos);
 // pinfo / n_pairs: a layer's pair tables (begin = their first items, per unused; map_k over the
 // residue-ordered planes), else nullptr
-cudaError_t launch_tensor4(const ScanWork& w, const CUtensorMap& map_l256, const CUtensorMap& map_l128,
-                           const CUtensorMap& map_k, const CUtensorMap& map_i, const long long* begin,
-                           const long long* per, int k_cases, int pack, long long g0, long long g1,
+cudaError_t launch_tensor4(const ScanWork& w, const CUtensorMap& map_l, const CUtensorMap& map_k,
+                           const CUtensorMap& map_i, const long long* begin, const long long* per, int k_cases,
+                           long long g0, long long g1,
                            const CandSink& sink, uint32_t* dump, const uint32_t* single, const uint4* pairs,
                            const uint4* triples, int* status, cudaStream_t s, int sms, const int4* pinfo = nullptr,
                            int n_pairs = 0);
@@ -262,6 +288,11 @@ cudaError_t launch_combine(const uint64_t* t1, int size1, const uint64_t* t2, in
 cudaError_t probe_popc_rate(int sms, cudaStream_t s, double* word_ops_per_s);
 cudaError_t launch_combine_popcnt(const uint64_t* t1, int size1, const uint64_t* t2, int cw, int tw,
                                   uint32_t* cases_out, uint32_t* ctrls_out, int ct_size, cudaStream_t s);
+
+// Raises *live from hist (one launch), and keeps the candidates of buf[0..*count) with keys of at least
+// *live after a last raise: they go to out, *count becomes their number.
+cudaError_t live_raise(const CandSink& sink, cudaStream_t s);
+cudaError_t live_compact(const CandSink& sink, Cand* out, unsigned* out_count, cudaStream_t s);
 
 // topn.cu -- top-N selection, FP64 rescoring, tables of given combinations.
 // Keeps the best `keep` of buf[0..M) (key desc, code asc) in buf[0..min(M,keep)),

@@ -1310,8 +1310,7 @@ static cudaError_t e4m3_planes(T3Plan& plan, const DevData& d, cudaStream_t s) {
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     const int rows = 2 * d.snps;
-    // l rows of an item: 192 at order 3, 256 at order 4 when the classes pack
-    if (e == cudaSuccess) e = t3_map(&plan.map_l, planes, rows, plan.pitch, plan.pack ? kT2N : kT3N, true);
+    if (e == cudaSuccess) e = t3_map(&plan.map_l, planes, rows, plan.pitch, kT3N, true);
     if (e == cudaSuccess) e = t3_map(&plan.map_j, planes, rows, plan.pitch, 2 * kT3J, true);
     if (e == cudaSuccess) e = t3_map(&plan.map_i, planes, rows, plan.pitch, 2, true);
     if (e == cudaSuccess) e = t3_map(&plan.map_a2, planes, rows, plan.pitch, kT2M, true);
@@ -1339,59 +1338,65 @@ cudaError_t tensor3_prepare(const DevData& d, T3Plan& plan, cudaStream_t) {
     return e;
 }
 
-// The operand planes of an order, made on its first search (items_mu held).
-static cudaError_t order_planes(T3Plan& plan, const DevData& d, int order, cudaStream_t s) {
-    if (order != 3 || !plan.pair3) return e4m3_planes(plan, d, s);
-    if (plan.f4.bits) return cudaSuccess;
-    cudaError_t e = f4_prepare(d, plan.f4, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) f4_release(plan.f4);
+// Copies a host item table to the device.
+static cudaError_t upload(long long*& out, const std::vector<long long>& v) {
+    long long* p = nullptr;
+    cudaError_t e = cudaMalloc((void**)&p, v.size() * sizeof(long long));
+    if (e == cudaSuccess) e = cudaMemcpy(p, v.data(), v.size() * sizeof(long long), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) cudaFree(p);
+    else out = p;
+    return e;
+}
+
+// Order-3 items of the whole data set.
+static cudaError_t order3_items(T3Plan& plan, const DevData& d) {
+    if (plan.item_begin) return cudaSuccess;
+    std::vector<long long> ib;
+    if (plan.pair3) ib = t3x_items(d.snps);
+    else t3_items(d.snps, kT3L, ib);
+    plan.total = ib.back();
+    const double n = d.snps;
+    plan.item_combos = n * (n - 1) * (n - 2) / 6.0 / std::max(1ll, plan.total);
+    return upload(plan.item_begin, ib);
+}
+
+// The operands of an order, made on its first search (items_mu held): e4m3 planes, or the 4-bit
+// layout and at order 4 the packed cores of the triples.
+static cudaError_t order_planes(T3Plan& plan, const DevData& d, int order, const uint4* pairs, cudaStream_t s,
+                                int sms) {
+    if (order == 2 || !plan.pair3) return e4m3_planes(plan, d, s);
+    cudaError_t e = cudaSuccess;
+    if (!plan.f4.bits) {
+        e = f4_prepare(d, plan.f4, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) f4_release(plan.f4);
+    }
+    if (e == cudaSuccess && order == 4 && !plan.f4.tri) {
+        e = order3_items(plan, d);
+        if (e == cudaSuccess) e = f4_order4_maps(plan.f4, d.snps);
+        if (e == cudaSuccess) e = f4_triples(d, plan.f4, plan.item_begin, plan.total, pairs, s, sms);
+    }
     return e;
 }
 
 // The work items of the whole data set at order 3 or 4, made on the first
 // search of that order (the host enumeration grows as n^2 / 16 at order 4:
 // about 0.1 s at 40 000 SNPs, which a search of another order need not pay).
-cudaError_t tensor3_order_items(T3Plan& plan, const DevData& d, int order, cudaStream_t s) {
+cudaError_t tensor3_order_items(T3Plan& plan, const DevData& d, int order, const uint4* pairs, cudaStream_t s,
+                                int sms) {
     std::lock_guard<std::mutex> g(plan.items_mu);
-    cudaError_t e = order_planes(plan, d, order, s);
-    if (e != cudaSuccess) return e;
-    if (order == 3 && !plan.item_begin) {
-        std::vector<long long> ib;
-        if (plan.pair3) ib = t3x_items(d.snps);
-        else t3_items(d.snps, kT3L, ib);
-        const long long total = ib.back();
-        long long* p = nullptr;
-        e = cudaMalloc((void**)&p, ib.size() * sizeof(long long));
-        if (e == cudaSuccess) e = cudaMemcpy(p, ib.data(), ib.size() * sizeof(long long), cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) {
-            cudaFree(p);
-            return e;
-        }
-        plan.total = total;
-        const double n = d.snps;
-        plan.item_combos = n * (n - 1) * (n - 2) / 6.0 / std::max(1ll, total);
-        plan.item_begin = p;
-    }
-    if (order == 4 && !plan.item4_begin && d.snps >= 4) {
+    cudaError_t e = order_planes(plan, d, order, pairs, s, sms);
+    if (e == cudaSuccess && order == 3) e = order3_items(plan, d);
+    if (e == cudaSuccess && order == 4 && !plan.item4_begin && d.snps >= 4) {
         std::vector<long long> per4;
-        const std::vector<long long> ib4 = t4_item_table(d.snps, plan.pack != 0, per4);
-        long long *pb = nullptr, *pp = nullptr;
-        e = t3_map(&plan.map_k4, plan.planes, 2 * d.snps, plan.pitch, 32, true);
-        if (e == cudaSuccess) e = cudaMalloc((void**)&pb, ib4.size() * sizeof(long long));
-        if (e == cudaSuccess) e = cudaMalloc((void**)&pp, per4.size() * sizeof(long long));
-        if (e == cudaSuccess) e = cudaMemcpy(pb, ib4.data(), ib4.size() * sizeof(long long), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(pp, per4.data(), per4.size() * sizeof(long long), cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) {
-            cudaFree(pb);
-            cudaFree(pp);
-            return e;
-        }
+        const std::vector<long long> ib4 = t4_item_table(d.snps, plan.pair3, per4);
+        if (!plan.pair3) e = t3_map(&plan.map_k4, plan.planes, 2 * d.snps, plan.pitch, 32, true);
+        if (e == cudaSuccess) e = upload(plan.item4_per, per4);
+        if (e != cudaSuccess) return e;
         plan.total4 = ib4.back();
         const double n = d.snps;
         plan.item4_combos = n * (n - 1) * (n - 2) * (n - 3) / 24.0 / std::max(1ll, plan.total4);
-        plan.item4_per = pp;
-        plan.item4_begin = pb;
+        e = upload(plan.item4_begin, ib4);
     }
     return e;
 }
@@ -1413,12 +1418,12 @@ struct T3Layer {
     int4* pinfo = nullptr;            // order 4: (i, j, first owned k) of each listed pair
     CUtensorMap map_jr;               // order 3: 64 rows of the residue-ordered planes (pair kernel: bit rows)
     CUtensorMap map_ar;               // order 2: box 128 B x 128 rows over the residue-ordered planes
-    CUtensorMap map_kr;               // order 4: box 128 B x 32 rows over the residue-ordered planes
+    CUtensorMap map_kr;               // order 4: 32 rows of the residue-ordered planes (pair kernel: bit rows)
 };
 struct T3Layers {
     std::mutex mu;
     std::map<std::tuple<int, int, int>, T3Layer> by;  // (order, step, offset)
-    // residue-ordered operand planes, and bit rows (order-3 pair kernel), per step
+    // residue-ordered operand planes, and bit rows (pair kernels of orders 3 and 4), per step
     std::map<int, uint8_t*> by_residue, bits_by_residue;
 };
 
@@ -1453,17 +1458,17 @@ static const T3Layer* find_layer(const T3Plan& plan, const ScanWork& w) {
     return it == plan.layers->by.end() ? nullptr : &it->second;
 }
 
-cudaError_t tensor3_layer(T3Plan& plan, const ScanWork& w, cudaStream_t s) {
+cudaError_t tensor3_layer(T3Plan& plan, const ScanWork& w, const uint4* pairs, cudaStream_t s, int sms) {
     if (!tensor_layer_ok(plan, w)) return cudaErrorInvalidValue;
     if (!plan.layers) plan.layers = new T3Layers;
     std::lock_guard<std::mutex> g(plan.layers->mu);
     const auto key = std::make_tuple(w.order, w.dist_step, w.dist_offset);
     if (plan.layers->by.count(key)) return cudaSuccess;
-    const bool px = w.order == 3 && plan.pair3;  // the pair kernel's j operand: bit rows
+    const bool px = w.order != 2 && plan.pair3;  // the pair kernels' j or k operand: bit rows
     cudaError_t pe;
     {
         std::lock_guard<std::mutex> gp(plan.items_mu);
-        pe = order_planes(plan, w.d, w.order, s);
+        pe = order_planes(plan, w.d, w.order, pairs, s, sms);
     }
     if (pe == cudaSuccess)
         pe = px ? residue_copy(plan.layers->bits_by_residue, (const uint8_t*)plan.f4.bits, (size_t)8 * plan.f4.wpr,
@@ -1477,12 +1482,14 @@ cudaError_t tensor3_layer(T3Plan& plan, const ScanWork& w, cudaStream_t s) {
         std::vector<long long> pb;
         std::vector<int4> pi;
         long long combos = 0;
-        const long long total = t4_layer_items(n, (int)step, offset, plan.pack != 0, pb, pi, combos);
+        const long long total = t4_layer_items(n, (int)step, offset, px, pb, pi, combos);
         T3Layer L;
         L.total = total;
         L.n_tiles = (int)pi.size();
         L.item_combos = (double)combos / std::max(1ll, total);
-        cudaError_t e = t3_map(&L.map_kr, perm, 2 * n, plan.pitch, 32, true);
+        cudaError_t e = px ? f4_bit_map(&L.map_kr, plan.f4,
+                                        (const uint32_t*)plan.layers->bits_by_residue[w.dist_step], 2 * n, 32)
+                           : t3_map(&L.map_kr, perm, 2 * n, plan.pitch, 32, true);
         if (e == cudaSuccess) e = cudaMalloc((void**)&L.item_begin, pb.size() * sizeof(long long));
         if (e == cudaSuccess) e = cudaMalloc((void**)&L.pinfo, std::max<size_t>(1, pi.size()) * sizeof(int4));
         if (e == cudaSuccess)
@@ -1573,6 +1580,8 @@ cudaError_t tensor3_layer(T3Plan& plan, const ScanWork& w, cudaStream_t s) {
     plan.layers->by[key] = L;
     return cudaSuccess;
 }
+
+bool tensor_live(const T3Plan& plan, const ScanWork& w) { return w.order != 2 && plan.pair3; }
 
 long long tensor_units(const T3Plan& plan, const ScanWork& w) {
     if (is_layer(w)) {
@@ -1709,15 +1718,17 @@ cudaError_t launch_tensor3(const ScanWork& w, const T3Plan& plan, long long g0, 
                            uint32_t* dump, const uint32_t* single, const uint4* pairs, const uint4* triples,
                            int* status, cudaStream_t s, int sms) {
     if (w.order == 4) {
-        if (is_layer(w)) {
-            const T3Layer* L = find_layer(plan, w);
-            if (!L || !tensor_layer_ok(plan, w)) return cudaErrorInvalidValue;
-            return launch_tensor4(w, plan.map_l, plan.map_a2, L->map_kr, plan.map_i, L->item_begin, nullptr,
-                                  plan.k_cases, plan.pack, g0, g1, sink, dump, single, pairs, triples, status, s, sms,
-                                  L->pinfo, L->n_tiles);
+        const T3Layer* L = is_layer(w) ? find_layer(plan, w) : nullptr;
+        if (is_layer(w) && (!L || !tensor_layer_ok(plan, w))) return cudaErrorInvalidValue;
+        if (plan.pair3) {
+            const T4xRange r = L ? T4xRange{L->item_begin, nullptr, &L->map_kr, L->pinfo, L->n_tiles}
+                                 : T4xRange{plan.item4_begin, plan.item4_per, &plan.f4.map_k4};
+            return launch_tensor4x(w, plan.f4, r, g0, g1, sink, dump, single, pairs, status, s, sms);
         }
-        return launch_tensor4(w, plan.map_l, plan.map_a2, plan.map_k4, plan.map_i, plan.item4_begin, plan.item4_per,
-                              plan.k_cases, plan.pack, g0, g1, sink, dump, single, pairs, triples, status, s, sms);
+        return launch_tensor4(w, plan.map_a2, L ? L->map_kr : plan.map_k4, plan.map_i,
+                              L ? L->item_begin : plan.item4_begin, L ? nullptr : plan.item4_per, plan.k_cases, g0, g1,
+                              sink, dump, single, pairs, triples, status, s, sms, L ? L->pinfo : nullptr,
+                              L ? L->n_tiles : 0);
     }
     // set once, by whichever host thread comes first (thread-safe static initialisation)
     static const cudaError_t attr = [] {
@@ -1778,8 +1789,8 @@ cudaError_t launch_tensor3(const ScanWork& w, const T3Plan& plan, long long g0, 
         if (is_layer(w) && (!L || !tensor_layer_ok(plan, w))) return cudaErrorInvalidValue;
         const T3xRange r = L ? T3xRange{L->item_begin, &L->map_jr, L->jl_begin, L->jlist}
                              : T3xRange{plan.item_begin, &plan.f4.map_j};
-        const float thr_q = f4_bound_threshold((double)sink.thr * scale, w.d.n_cases, w.d.n_ctrls, 27);
-        return launch_tensor3x(w, plan.f4, r, g0, g1, sink, dump, single, pairs, thr_f, thr_q, status, s, sms);
+        return launch_tensor3x(w, plan.f4, r, g0, g1, sink, dump, single, pairs,
+                               t3_margin(w.d.n_cases + w.d.n_ctrls), status, s, sms);
     }
     if (is_layer(w)) {
         const T3Layer* L = find_layer(plan, w);

@@ -47,6 +47,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "live.cuh"
 #include "tensor3x.h"
 #include "tensor_fp4.cuh"
 
@@ -58,22 +59,27 @@ constexpr int kXN = 2 * kXL;                        // columns of an accumulator
 constexpr int kXM = 4 * kXJ;                        // 128 accumulator rows per CTA
 constexpr int kXRow = kF4K / 2;                     // 128 bytes per operand row and stage
 constexpr int kXBitRow = kF4K / 8;                  // 32 bytes per bit row and stage
-constexpr int kXStages = 6;
+// Copies land in a ring of their own, deeper than the A ring: the copies' latency
+// (about 3 000 cycles from one's issue to its stage's release) times the bytes in
+// flight sets the pace.  (One ring of six stages, A beside what it is built from:
+// 540 cycles a stage whatever the MMAs took.)
+constexpr int kXStages = 8, kXAStages = 4;
 constexpr int kXSA = kXM * kXRow;                   // 16 KB
 constexpr int kXSB = kXN / 2 * kXRow;               // 15 KB: this CTA's half of the l rows
 constexpr int kXSJ = 2 * kXJ * kXBitRow;            //  2 KB
 constexpr int kXSI = 2 * kXBitRow;                  // 64 bytes
-constexpr int kXStage = (kXSA + kXSB + kXSJ + kXSI + 1023) / 1024 * 1024;  // 34 KB
+constexpr int kXStage = (kXSB + kXSJ + kXSI + 1023) / 1024 * 1024;  // 18 KB
 constexpr int kXColOne = 2 * kXN, kXColW = kXColOne + 16;
 // Builders in two groups that take alternate stages (a warp's chain of waits,
 // loads, shifts, stores and arrival is longer than a stage's MMAs).
 constexpr int kXBuildWarps = 4, kXEpiWarps = 8;     // builder warps per group
-constexpr int kXThreads = 32 * (4 + 2 * kXBuildWarps + kXEpiWarps);  // 640: warps 2 and 3 idle
-// registers a thread: 96 at launch; copies and MMAs keep 40, the builders 56,
-// the epilogue gets 160 (40 + 2 x 56 + 2 x 160 <= 5 x 96)
+constexpr int kXThreads = 32 * (4 + 2 * kXBuildWarps + kXEpiWarps);  // 640: copies, MMAs, 2 staging, 8, 8
+// registers a thread: 96 at launch, then 56 / 56 / 152 (3 x 56 + 2 x 152 <= 5 x 96)
 constexpr int kXMeta = 16;                          // items in flight between the copies and the MMAs
-constexpr int kXTab = 9 * kXL * 4;                  // an item's (i, l) marginals, one column per l
-constexpr size_t kXSmem = 1024 + (size_t)kXStages * kXStage + 2 * kXTab;
+// an item's staged tables: (i, l) marginals, one column per l; per j of this CTA (i, j) cores and j
+// singles, each twice (both halves of a pair), and j; the threshold (key, estimate, bound)
+constexpr int kXTabL = 9 * kXL * 4, kXTabJ = 6 * kXJ * 8, kXTabT = kXTabL + kXTabJ + 4 * kXJ, kXTab = kXTabT + 16;
+constexpr size_t kXSmem = 1024 + (size_t)kXStages * kXStage + (size_t)kXAStages * kXSA + 2 * kXTab;
 static_assert(kXSmem <= 227 * 1024 - 512, "order-3 pair kernel shared memory");
 static_assert(kXSA % 1024 == 0 && kXSB % 1024 == 0, "operand tiles on swizzle atoms");
 static_assert(kXColW + 16 <= 512, "tensor memory columns");
@@ -138,9 +144,9 @@ __device__ __forceinline__ float t3x_pair(const uint4& v, int x, int y, float W)
 // combination (i, j, l), the bounded single-precision estimate of the key
 // (t3_margin), the exact fixed-point key for what passes it, and the
 // warp-aggregated append of candidates.  Warp-synchronous.
-__device__ __forceinline__ void t3x_survivor(const ScanWork& w, const CandSink& sink, float thr_f, uint32_t* dump,
-                                             const float (&t)[27], int pack, int i, int j, int l, bool want,
-                                             int lane) {
+__device__ __forceinline__ void t3x_survivor(const ScanWork& w, const CandSink& sink, long long thr, float thr_f,
+                                             uint32_t* dump, const float (&t)[27], int pack, int i, int j, int l,
+                                             bool want, int lane) {
     const uint32_t mask = (1u << pack) - 1u;
     const int n = w.d.snps;
     bool cand = want;
@@ -181,7 +187,7 @@ __device__ __forceinline__ void t3x_survivor(const ScanWork& w, const CandSink& 
         }
     }
     if (sink.digest) dg_warp_add(sink.digest, dg);
-    const bool pass = cand && key >= sink.thr;
+    const bool pass = cand && key >= thr;
     const unsigned pm = __ballot_sync(0xffffffffu, pass);
     if (!pm) return;
     const int leader = __ffs(pm) - 1;
@@ -193,6 +199,7 @@ __device__ __forceinline__ void t3x_survivor(const ScanWork& w, const CandSink& 
         if (idx < sink.cap) {
             const int cmb[3] = {i, j, l};
             sink.buf[idx] = Cand{key, pack_code(cmb, 3, w.bits)};
+            if (sink.hist) atomicAdd(sink.hist + live_bin(key), 1u);
         } else {
             atomicOr(sink.overflow, 1u);
         }
@@ -202,22 +209,29 @@ __device__ __forceinline__ void t3x_survivor(const ScanWork& w, const CandSink& 
 // Columns the MMA of an item of ng groups multiplies (at least 64).
 __device__ __forceinline__ int t3x_n(int ng) { return 16 * max(ng, 4); }
 
-template <bool LIST>
+// What a launch does with the accumulators: search a data set or one Distribution layer of it, or
+// store the cores of every triple (F4Plan::tri).
+enum { kXScan, kXLayer, kXCores };
+
+template <int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
     tensor3x_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_j,
                     const __grid_constant__ CUtensorMap map_i, const __grid_constant__ ScanWork w,
                     const __grid_constant__ CandSink sink, const long long* __restrict__ item_begin, long long g0,
-                    long long g1, int nw_c, int nw_t, int pack, float thr_f, float thr_q, uint32_t* dump,
+                    long long g1, int nw_c, int nw_t, int pack, const __grid_constant__ LiveMap map, uint32_t* dump,
                     const uint32_t* __restrict__ single, const uint4* __restrict__ pairs, int* status,
-                    const long long* __restrict__ jl_begin, const int* __restrict__ jlist) {
+                    const long long* __restrict__ jl_begin, const int* __restrict__ jlist, float* tri,
+                    const int* __restrict__ row_p, const int* __restrict__ row_q) {
+    constexpr bool LIST = MODE == kXLayer;
     extern __shared__ uint8_t smraw[];
-    __shared__ __align__(8) uint64_t full_t[kXStages], full_a[kXStages], empty[kXStages];
-    __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2], done;
+    __shared__ __align__(8) uint64_t full_t[kXStages], empty[kXStages], full_a[kXAStages];
+    __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2], tab_full[2], tab_empty[2], done;
     __shared__ uint32_t tmem_base;
     __shared__ int item_ng[kXMeta];  // groups of the items in flight, for the MMA issuer
     __shared__ int abort_flag;
-    uint8_t* sm = (uint8_t*)(((uintptr_t)smraw + 1023) & ~(uintptr_t)1023);  // stages: A | B half | j | i
-    float* tabs = reinterpret_cast<float*>(sm + kXStages * kXStage);
+    uint8_t* sm = (uint8_t*)(((uintptr_t)smraw + 1023) & ~(uintptr_t)1023);  // stages: B half | j | i; then the A tiles
+    uint8_t* sma = sm + kXStages * kXStage;
+    uint8_t* tabs = sma + kXAStages * kXSA;
     volatile int* abort = &abort_flag;
     const int n = w.d.snps;
     const int tid = threadIdx.x, lane = tid & 31;
@@ -237,12 +251,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
         };
         for (int s = 0; s < kXStages; ++s) {
             init(&full_t[s], 1);
-            init(&full_a[s], 2 * kXBuildWarps);
             init(&empty[s], 1);
         }
+        for (int s = 0; s < kXAStages; ++s) init(&full_a[s], 2 * kXBuildWarps);
         for (int b = 0; b < 2; ++b) {
             init(&acc_full[b], 1);
             init(&acc_empty[b], 2 * kXEpiWarps);
+            init(&tab_full[b], 2);
+            init(&tab_empty[b], kXEpiWarps);
         }
         init(&done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;");
@@ -262,7 +278,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
     // (the register limits are set inside the branches: set before them, the
     // compiler would hold every branch to the smallest)
     if (warp < 4) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
         if (warp == 0) {
             // ---------------------------------------------------------------- TMA producer (both CTAs)
             if (g0 + cid < g1 && elect_one()) {
@@ -290,9 +306,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
                         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
                                      "r"((uint32_t)(kXSB + kXSJ + kXSI))
                                      : "memory");
-                        t3_tma(st + kXSA + kXSB, &map_j, kXBitRow * ks, 2 * jr, bar);
-                        t3_tma(st + kXSA + kXSB + kXSJ, &map_i, kXBitRow * ks, irow, bar);
-                        t3_tma(st + kXSA, &map_b, kXRow * ks, brow, bar);
+                        t3_tma(st + kXSB, &map_j, kXBitRow * ks, 2 * jr, bar);
+                        t3_tma(st + kXSB + kXSJ, &map_i, kXBitRow * ks, irow, bar);
+                        t3_tma(st, &map_b, kXRow * ks, brow, bar);
                         if (step < kXStages) ++step;
                         if (++s == kXStages) {
                             s = 0;
@@ -312,57 +328,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
             __syncwarp();
         } else if (warp == 1) {
             // ---------------------------------------------------------------- MMA issuer (CTA 0)
-            // (its own time per stage counts: about 230 cycles alone on an SM quarter, up to twice that beside
-            // the other warps, against 480 of MMA; so it decodes no items and its loop holds what it must)
             if (rank == 0 && elect_one()) {
-                const uint32_t full0 = smem_u32(&full_a[0]), empty0 = smem_u32(&empty[0]);
-                const uint32_t desc_hi = (uint32_t)(t3_desc(0) >> 32), desc0 = (uint32_t)t3_desc(smem_u32(sm));
-                const uint32_t one = tmem + (uint32_t)kXColOne;
-                uint32_t bar = 0, ad = desc0, par = 0;  // stage: barrier offset, A descriptor, parity
-                unsigned item = 0;
-                for (long long g = g0 + cid; g < g1 && ok; g += ncl, ++item) {
-                    const unsigned buf = item & 1;
-                    if (item >= 2 && !t3_wait_cl(smem_u32(&acc_empty[buf]), ((item >> 1) - 1) & 1, abort)) {
-                        ok = false;
-                        break;
-                    }
-                    const uint32_t dcol = tmem + (uint32_t)(kXN * buf);
-                    uint32_t acc = 0, idesc = 0;
-                    for (int cls = 0; cls < 2 && ok; ++cls) {
-                        const uint32_t sfb = tmem + (uint32_t)(cls ? kXColW : kXColOne);
-                        for (int left = cls ? nw_t : nw_c; left > 0; left -= 4) {
-                            if (!t3_wait_cl(full0 + bar, par, abort)) {  // both CTAs' rows landed, A tiles built
-                                ok = false;
-                                break;
-                            }
-                            asm volatile("tcgen05.fence::after_thread_sync;");
-                            if (!acc) idesc = f4_idesc(2 * kXM, t3x_n(item_ng[item % kXMeta]));
-                            auto mma = [&](int k) {
-                                f4_mma<2>(dcol, (uint64_t)desc_hi << 32 | (ad + 2 * k),
-                                          (uint64_t)desc_hi << 32 | (ad + (kXSA >> 4) + 2 * k), idesc, one, sfb, acc);
-                                acc = 1;
-                            };
-                            mma(0);
-                            if (left >= 4) {
-                                mma(1);
-                                mma(2);
-                                mma(3);
-                            } else {  // the class's last steps
-                                for (int k = 1; k < left; ++k) mma(k);
-                            }
-                            commit_pair(empty0 + bar);
-                            bar += 8;
-                            ad += kXStage >> 4;
-                            if (bar == 8 * kXStages) {
-                                bar = 0;
-                                ad = desc0;
-                                par ^= 1;
-                            }
-                        }
-                    }
-                    if (!ok) break;
-                    commit_pair(smem_u32(&acc_full[buf]));
-                }
+                ok = f4_pair_issue<kXAStages, kXStages, kXStage, kXN, kXColOne, kXColW>(
+                    (g1 - g0 - cid + ncl - 1) / ncl, smem_u32(sma), smem_u32(sm), smem_u32(&full_a[0]),
+                    smem_u32(&empty[0]), smem_u32(&acc_full[0]), smem_u32(&acc_empty[0]), tmem, nw_c, nw_t, abort,
+                    [&](unsigned item) { return t3x_n(item_ng[item % kXMeta]); });
                 commit_pair(smem_u32(&done));
                 // neither CTA releases shared or tensor memory before the pair's MMAs are
                 // done (CTA 1 waits once its own work is over, below: waiting here would
@@ -370,6 +340,82 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
                 if (!t3_drain_cl(smem_u32(&done), 0)) ok = false;
             }
             __syncwarp();
+        } else if (MODE != kXCores) {
+            // ---------------------------------------------------------------- table staging (both CTAs)
+            const int t = tid - 64;  // 0 .. 63
+            const float W = (float)(1u << pack);
+            const float ntot = fmaf(W, (float)w.d.n_ctrls, (float)w.d.n_cases);
+            const uint4* single4 = reinterpret_cast<const uint4*>(single);
+            unsigned item = 0;
+            int wi = -1;
+            for (long long g = g0 + cid; g < g1 && ok; g += ncl, ++item) {
+                const T3xItem it = t3x_item<LIST>(item_begin, jl_begin, jlist, n, g, wi);
+                const unsigned buf = item & 1;
+                if (item >= 2 && !t3_wait(smem_u32(&tab_empty[buf]), ((item >> 1) - 1) & 1, abort)) {
+                    ok = false;
+                    break;
+                }
+                uint8_t* tab = tabs + buf * kXTab;
+                const int i = it.i;
+                const uint4 s1 = __ldg(single4 + i);
+                // the threshold of this item (the pairs take turns at raising the live one)
+                if (sink.hist && rank == 0 && warp == 2 && item > 0 && (item < 3 || ((item + cid) & 7) == 0))
+                    live_update(sink, lane);
+                if (t == 0) {
+                    const long long thr = sink.hist ? *(volatile long long*)sink.live : sink.thr;
+                    float est, bound;
+                    live_tests(map, thr, est, bound);
+                    *reinterpret_cast<long long*>(tab + kXTabT) = thr;
+                    *reinterpret_cast<float2*>(tab + kXTabT + 8) = make_float2(est, bound);
+                }
+                float* tl = reinterpret_cast<float*>(tab);
+                for (int ll = t; ll < 8 * it.ng; ll += 64) {  // entries (x, z), x and z in {0, 1, any}
+                    const int l = it.l0 + ll;
+                    float m[3][3];
+#pragma unroll
+                    for (int k = 0; k < 9; ++k) m[k / 3][k % 3] = 0.f;
+                    if (l < n && l > i) {
+                        const uint4 p = __ldg(pairs + pair_index(i, l, n)), sl = __ldg(single4 + l);
+#pragma unroll
+                        for (int x = 0; x < 2; ++x) {
+#pragma unroll
+                            for (int z = 0; z < 2; ++z) m[x][z] = t3x_pair(p, x, z, W);
+                            m[x][2] = t3x_pk(x ? s1.y : s1.x, x ? s1.w : s1.z, W) - m[x][0] - m[x][1];
+                        }
+#pragma unroll
+                        for (int z = 0; z < 2; ++z)
+                            m[2][z] = t3x_pk(z ? sl.y : sl.x, z ? sl.w : sl.z, W) - m[0][z] - m[1][z];
+                        m[2][2] = ntot - t3x_pk(s1.x, s1.z, W) - t3x_pk(s1.y, s1.w, W) - m[2][0] - m[2][1];
+                    }
+#pragma unroll
+                    for (int k = 0; k < 9; ++k) tl[k * kXL + ll] = m[k / 3][k % 3];
+                }
+                if (t < kXJ) {
+                    int j = n;
+                    if (LIST) {
+                        const long long p = it.p0 + kXJ * (int)rank + t;
+                        if (p < __ldg(jl_begin + i + 1)) j = __ldg(jlist + p);
+                    } else {
+                        j = it.j0 + kXJ * (int)rank + t;
+                    }
+                    uint4 p = make_uint4(0, 0, 0, 0), sv = p;
+                    if (j < n) {
+                        p = __ldg(pairs + pair_index(i, j, n));
+                        sv = __ldg(single4 + j);
+                    }
+                    float2* tj = reinterpret_cast<float2*>(tab + kXTabL);
+#pragma unroll
+                    for (int k = 0; k < 6; ++k) {
+                        const float v = k < 4 ? t3x_pair(p, k >> 1, k & 1, W)
+                                              : t3x_pk(k & 1 ? sv.y : sv.x, k & 1 ? sv.w : sv.z, W);
+                        tj[k * kXJ + t] = make_float2(v, v);
+                    }
+                    reinterpret_cast<int*>(tab + kXTabL + kXTabJ)[t] = j;
+                }
+                __syncwarp();
+                if (lane == 0)
+                    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&tab_full[buf])) : "memory");
+            }
         }
     } else if (warp < 12) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
@@ -380,7 +426,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
         // A row (jj / 8, x, y, jj % 8) of staged row (jj, y) = rg + 16 u; x = 1 is 16 rows on, u + 1 32 rows
         const int jj = rg >> 1, y = rg & 1;
         const int dst0 = (8 * y + jj) * kXRow + ((c ^ jj) << 4);
-        unsigned s = 0, par = 0;
+        unsigned s = 0, par = 0, sa = 0;                  // copy stage, A stage
+        unsigned se = kXStages - kXAStages, pe = 1;       // the stage whose MMAs free this A stage
         bool mine = warp < 8;
         for (long long g = g0 + cid; g < g1 && ok; g += ncl) {
             for (int ks = 0; ks < ksteps; ++ks, mine = !mine) {
@@ -389,14 +436,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
                         ok = false;
                         break;
                     }
-                    uint8_t* st = sm + s * kXStage;
-                    const uint32_t* sJ = reinterpret_cast<const uint32_t*>(st + kXSA + kXSB) + rg * 8 + c;
-                    const uint32_t* sI = reinterpret_cast<const uint32_t*>(st + kXSA + kXSB + kXSJ) + c;
+                    const uint32_t* sJ = reinterpret_cast<const uint32_t*>(sm + s * kXStage + kXSB) + rg * 8 + c;
+                    const uint32_t* sI = reinterpret_cast<const uint32_t*>(sm + s * kXStage + kXSB + kXSJ) + c;
                     uint32_t jw[4];
 #pragma unroll
                     for (int u = 0; u < 4; ++u) jw[u] = sJ[128 * u];
                     const uint32_t i0 = sI[0], i1 = sI[8];
-                    uint8_t* dst = st + dst0;
+                    if (!t3_wait_cl(smem_u32(&empty[se]), pe, abort)) {
+                        ok = false;
+                        break;
+                    }
+                    uint8_t* dst = sma + sa * kXSA + dst0;
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
                         *reinterpret_cast<uint4*>(dst + 32 * u * kXRow) = f4_expand_a(i0, jw[u]);
@@ -404,93 +454,57 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
                     }
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     __syncwarp();
-                    if (lane == 0) arrive_cl(full0 + 8 * s);
+                    if (lane == 0) arrive_cl(full0 + 8 * sa);
                 }
                 if (++s == kXStages) {
                     s = 0;
                     par ^= 1;
                 }
+                if (++se == kXStages) {
+                    se = 0;
+                    pe ^= 1;
+                }
+                if (++sa == kXAStages) sa = 0;
             }
         }
     } else {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 160;");
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");
         // ---------------------------------------------------------------- epilogue (both CTAs)
         const int q = warp & 3, hh = (warp - 12) >> 2;  // lane quarter (8 j); the two warps of a quarter take alternate groups
         const int jl = lane >> 2, lc = 2 * (lane & 3);  // this thread's j and its two l of a group
-        const int et = tid - 32 * 12;
         const float W = (float)(1u << pack);
-        const float ntot = fmaf(W, (float)w.d.n_ctrls, (float)w.d.n_cases);
         const bool all = dump != nullptr || sink.digest != nullptr;  // every combination takes the exact path
-        long long item = 0;
+        unsigned item = 0;
         int wi = -1;
-        // (after an abort the warps keep going through the items, so that every one
-        // reaches the named barrier the same number of times)
-        for (long long g = g0 + cid; g < g1; g += ncl, ++item) {
+        for (long long g = g0 + cid; g < g1 && ok; g += ncl, ++item) {
             const T3xItem it = t3x_item<LIST>(item_begin, jl_begin, jlist, n, g, wi);
             const int i = it.i, l0 = it.l0, ng = it.ng;
-            const int buf = (int)(item & 1);
-            // marginal table of (i, l), packed, for every l of the item: entries (x, z), x and z in
-            // {0, 1, 2}; the buffer's readers of two items ago passed the barrier of the last item
-            float* tab = tabs + (kXTab / 4) * buf;
-            const uint4 s1 = __ldg(reinterpret_cast<const uint4*>(single) + i);
-            if (et < kXL) {
-                const int l = l0 + et;
-                float m[3][3];
-#pragma unroll
-                for (int k = 0; k < 9; ++k) m[k / 3][k % 3] = 0.f;
-                if (et < 8 * ng && l < n && l > i) {
-                    const uint4 p = __ldg(pairs + pair_index(i, l, n));
-                    const uint4 sl = __ldg(reinterpret_cast<const uint4*>(single) + l);
-#pragma unroll
-                    for (int x = 0; x < 2; ++x) {
-#pragma unroll
-                        for (int z = 0; z < 2; ++z) m[x][z] = t3x_pair(p, x, z, W);
-                        m[x][2] = t3x_pk(x ? s1.y : s1.x, x ? s1.w : s1.z, W) - m[x][0] - m[x][1];
-                    }
-#pragma unroll
-                    for (int z = 0; z < 2; ++z)
-                        m[2][z] = t3x_pk(z ? sl.y : sl.x, z ? sl.w : sl.z, W) - m[0][z] - m[1][z];
-                    m[2][2] = ntot - t3x_pk(s1.x, s1.z, W) - t3x_pk(s1.y, s1.w, W) - m[2][0] - m[2][1];
-                }
-#pragma unroll
-                for (int k = 0; k < 9; ++k) tab[k * kXL + et] = m[k / 3][k % 3];
+            const unsigned buf = item & 1, ph = (item >> 1) & 1;
+            const uint8_t* tab = tabs + buf * kXTab;
+            if (MODE != kXCores && !t3_wait(smem_u32(&tab_full[buf]), ph, abort)) {
+                ok = false;
+                break;
             }
-            asm volatile("bar.sync 1, %0;" ::"n"(32 * kXEpiWarps) : "memory");
-            if (!ok) continue;
-            int j = n;
-            if (LIST) {
-                const long long p = it.p0 + kXJ * (int)rank + 8 * q + jl;
-                if (p < __ldg(jl_begin + i + 1)) j = __ldg(jlist + p);
-            } else {
-                j = it.j0 + kXJ * (int)rank + 8 * q + jl;
-            }
+            const int j = MODE == kXCores ? it.j0 + kXJ * (int)rank + 8 * q + jl
+                                          : reinterpret_cast<const int*>(tab + kXTabL + kXTabJ)[8 * q + jl];
             const bool j_ok = j < n;
-            f2 ij[2][2], sj[2];
-            {
-                uint4 p = make_uint4(0, 0, 0, 0), sv = p;
-                if (j_ok) {
-                    p = __ldg(pairs + pair_index(i, j, n));
-                    sv = __ldg(reinterpret_cast<const uint4*>(single) + j);
-                }
-#pragma unroll
-                for (int x = 0; x < 2; ++x)
-#pragma unroll
-                    for (int y = 0; y < 2; ++y) ij[x][y] = f2_dup(t3x_pair(p, x, y, W));
-                sj[0] = f2_dup(t3x_pk(sv.x, sv.z, W));
-                sj[1] = f2_dup(t3x_pk(sv.y, sv.w, W));
-            }
+            const f2* tj = reinterpret_cast<const f2*>(tab + kXTabL) + 8 * q + jl;
+            const f2 ij[2][2] = {{tj[0], tj[kXJ]}, {tj[2 * kXJ], tj[3 * kXJ]}}, sj[2] = {tj[4 * kXJ], tj[5 * kXJ]};
+            const long long thr = *reinterpret_cast<const long long*>(tab + kXTabT);
+            const float thr_f = reinterpret_cast<const float*>(tab + kXTabT)[2];
+            const float thr_q = reinterpret_cast<const float*>(tab + kXTabT)[3];
             const uint4* pj = j_ok ? pairs + pair_index(j, j + 1, n) - (j + 1) : pairs;  // + l: pair (j, l)
             const uint4 zero4 = make_uint4(0, 0, 0, 0);
-            const int gi0 = (hh + (int)item) & 1;  // the odd group of an item goes to either warp in turn
+            const int gi0 = (hh + item) & 1;  // the odd group of an item goes to either warp in turn
             uint4 pa = zero4, pb = zero4;
             {
                 const int l = l0 + 8 * gi0 + lc;
-                if (j_ok && gi0 < ng && l < n && l > j) pa = __ldg(pj + l);
-                if (j_ok && gi0 < ng && l + 1 < n && l + 1 > j) pb = __ldg(pj + l + 1);
+                if (MODE != kXCores && j_ok && gi0 < ng && l < n && l > j) pa = __ldg(pj + l);
+                if (MODE != kXCores && j_ok && gi0 < ng && l + 1 < n && l + 1 > j) pb = __ldg(pj + l + 1);
             }
-            if (!t3_wait_cl(smem_u32(&acc_full[buf]), (uint32_t)((item >> 1) & 1), abort)) {
+            if (!t3_wait_cl(smem_u32(&acc_full[buf]), ph, abort)) {
                 ok = false;
-                continue;
+                break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;");
 #pragma unroll 1
@@ -501,8 +515,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
                 {  // the next group's (j, l) pairs, ahead of their use
                     const int ln = l + 16;
                     pa = pb = zero4;
-                    if (j_ok && gi + 2 < ng && ln < n && ln > j) pa = __ldg(pj + ln);
-                    if (j_ok && gi + 2 < ng && ln + 1 < n && ln + 1 > j) pb = __ldg(pj + ln + 1);
+                    if (MODE != kXCores && j_ok && gi + 2 < ng && ln < n && ln > j) pa = __ldg(pj + ln);
+                    if (MODE != kXCores && j_ok && gi + 2 < ng && ln + 1 < n && ln + 1 > j) pb = __ldg(pj + ln + 1);
                 }
                 const unsigned m0 = __ballot_sync(0xffffffffu, v0), m1 = __ballot_sync(0xffffffffu, v1);
                 if (!(m0 | m1)) continue;
@@ -530,7 +544,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
                                 c[x][y][z] = f2_pack(__uint_as_float(r[x][4 * z + 2 * y]),
                                                      __uint_as_float(r[x][4 * z + 2 * y + 1]));
                 }
-                const float* tl = tab + 8 * gi + lc;
+                if (MODE == kXCores) {  // entries (x, y, z) of l and l + 1 side by side, 64 bytes
+                    float4* o = reinterpret_cast<float4*>(tri) + 4 * (size_t)(__ldg(row_q + i) + __ldg(row_p + j) +
+                                                                               (l >> 1));
+                    if (v0 || v1) {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            float4 v;
+                            f2_unpack(c[k >> 1][k & 1][0], v.x, v.y);
+                            f2_unpack(c[k >> 1][k & 1][1], v.z, v.w);
+                            o[k] = v;
+                        }
+                    }
+                    continue;
+                }
+                const float* tl = reinterpret_cast<const float*>(tab) + 8 * gi + lc;
                 auto il = [&](int x, int z) { return *reinterpret_cast<const f2*>(tl + (3 * x + z) * kXL); };
                 F4Bound bd(pack);
                 f2 a[2][2][3], y2[2][3];  // cells (x, y, z); cells (2, y, z)
@@ -602,13 +630,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
 #pragma unroll
                         for (int z = 0; z < 3; ++z)
                             t[24 + z] = tl[(6 + z) * kXL + u] - t[18 + z] - t[21 + z];
-                        t3x_survivor(w, sink, thr_f, dump, t, pack, i, j, l + u, want, lane);
+                        t3x_survivor(w, sink, thr, thr_f, dump, t, pack, i, j, l + u, want, lane);
                     }
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;");
             __syncwarp();
-            if (lane == 0) arrive_cl(cluster_addr(smem_u32(&acc_empty[buf]), 0));
+            if (lane == 0) {
+                arrive_cl(cluster_addr(smem_u32(&acc_empty[buf]), 0));
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&tab_empty[buf])) : "memory");
+            }
         }
     }
     if (!ok) *abort = 1;
@@ -685,8 +716,12 @@ cudaError_t f4_prepare(const DevData& d, F4Plan& f, cudaStream_t s) {
 
 void f4_release(F4Plan& f) {
     cudaFree(f.planes);
+    cudaFree(f.tri);
+    cudaFree(f.row_p);
     f.planes = nullptr;
     f.bits = nullptr;
+    f.tri = f.pairf = nullptr;
+    f.row_p = f.row_q = nullptr;
 }
 
 std::vector<long long> t3x_items(int n) {
@@ -699,30 +734,103 @@ std::vector<long long> t3x_items(int n) {
     return b;
 }
 
+// Pair cores packed as floats, entries (z, w) of (k, l) for l and l + 1 side by side (32 bytes).
+__global__ void f4_pairf_kernel(const uint4* __restrict__ pairs, float2* out, const int* __restrict__ row_p, int n,
+                                int pack) {
+    const float W = (float)(1u << pack);
+    const int k = blockIdx.x;
+    for (int m = ((k + 1) >> 1) + threadIdx.x; m < (n + 1) / 2; m += blockDim.x) {
+        float2* o = out + 4 * (size_t)(row_p[k] + m);
+        float v[2][4];
+        for (int u = 0; u < 2; ++u) {
+            const int l = 2 * m + u;
+            const uint4 p = l > k && l < n ? __ldg(pairs + pair_index(k, l, n)) : make_uint4(0, 0, 0, 0);
+            for (int e = 0; e < 4; ++e) v[u][e] = t3x_pair(p, e >> 1, e & 1, W);
+        }
+        for (int e = 0; e < 4; ++e) o[e] = make_float2(v[0][e], v[1][e]);
+    }
+}
+
+cudaError_t f4_triples(const DevData& d, F4Plan& f, const long long* item_begin, long long items, const uint4* pairs,
+                       cudaStream_t s, int sms) {
+    const int n = d.snps;
+    // rows of l pairs: row k starts at l = k + 1 rounded down to even
+    std::vector<int> p((size_t)2 * n + 1);  // and the launch's status
+    long long at = 0;
+    std::vector<long long> P((size_t)n + 1);
+    for (int k = 0; k < n; ++k) {
+        P[k] = at;
+        p[k] = (int)(at - ((k + 1) >> 1));
+        at += ((n + 1) >> 1) - ((k + 1) >> 1);
+    }
+    P[n] = at;
+    long long B = 0;
+    for (int i = 0; i < n; ++i) {
+        p[n + i] = (int)(B - P[i + 1]);
+        B += P[n] - P[i + 1];
+    }
+    int* rows = nullptr;
+    char* tab = nullptr;  // triples, then pairs
+    cudaError_t e = cudaMalloc((void**)&rows, p.size() * sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc((void**)&tab, (size_t)B * 64 + (size_t)P[n] * 32);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(rows, p.data(), p.size() * sizeof(int), cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) {
+        f.row_p = rows;
+        f.row_q = rows + n;
+        f.tri = reinterpret_cast<float*>(tab);
+        f.pairf = reinterpret_cast<float*>(tab + (size_t)B * 64);
+        f4_pairf_kernel<<<n, 128, 0, s>>>(pairs, reinterpret_cast<float2*>(f.pairf), f.row_p, n, f.pack);
+        count_launch();
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) {
+        ScanWork w{};
+        w.d = d;
+        w.order = 3;
+        w.dist_n = n;
+        w.dist_step = 1;
+        const T3xRange r{item_begin, &f.map_j};
+        e = launch_tensor3x(w, f, r, 0, items, CandSink{}, nullptr, nullptr, pairs, 0, rows + 2 * n, s, sms, true);
+    }
+    int gave_up = 0;
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&gave_up, rows + 2 * n, sizeof(int), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess && gave_up) e = cudaErrorLaunchTimeout;
+    if (e != cudaSuccess) {
+        cudaFree(rows);
+        cudaFree(tab);
+        f.row_p = f.row_q = nullptr;
+        f.tri = f.pairf = nullptr;
+    }
+    return e;
+}
+
 cudaError_t launch_tensor3x(const ScanWork& w, const F4Plan& f, const T3xRange& r, long long g0, long long g1,
                             const CandSink& sink, uint32_t* dump, const uint32_t* single, const uint4* pairs,
-                            float thr_f, float thr_q, int* status, cudaStream_t s, int sms) {
+                            double est_margin, int* status, cudaStream_t s, int sms, bool cores) {
+    using Fn = decltype(&tensor3x_kernel<kXScan>);
+    static const Fn fns[3] = {tensor3x_kernel<kXScan>, tensor3x_kernel<kXLayer>, tensor3x_kernel<kXCores>};
     // set once, by whichever host thread comes first (thread-safe static initialisation)
     static const cudaError_t attr = [] {
-        cudaError_t e = cudaFuncSetAttribute(tensor3x_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)kXSmem);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(tensor3x_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kXSmem);
+        cudaError_t e = cudaSuccess;
+        for (Fn fn : fns)
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kXSmem);
         return e;
     }();
     if (attr != cudaSuccess) return attr;
     if (g1 <= g0) return cudaSuccess;
-    static const int max_clusters = pair_clusters(tensor3x_kernel<false>, kXThreads, kXSmem);
+    static const int max_clusters = pair_clusters(tensor3x_kernel<kXScan>, kXThreads, kXSmem);
     const long long clusters = std::min<long long>(g1 - g0, max_clusters > 0 ? max_clusters : sms / 2);
     const unsigned grid = (unsigned)(2 * std::max(1ll, clusters));
-    if (r.jlist)
-        tensor3x_kernel<true><<<grid, kXThreads, kXSmem, s>>>(f.map_b, *r.map_j, f.map_i, w, sink, r.item_begin, g0, g1,
-                                                              f.nw_c, f.nw_t, f.pack, thr_f, thr_q, dump, single, pairs,
-                                                              status, r.jl_begin, r.jlist);
-    else
-        tensor3x_kernel<false><<<grid, kXThreads, kXSmem, s>>>(f.map_b, *r.map_j, f.map_i, w, sink, r.item_begin, g0,
-                                                               g1, f.nw_c, f.nw_t, f.pack, thr_f, thr_q, dump, single,
-                                                               pairs, status, nullptr, nullptr);
+    const Fn fn = fns[cores ? kXCores : r.jlist ? kXLayer : kXScan];
+    const double scale = 1.0 / (std::log(2.0) * 4294967296.0);
+    LiveMap map{scale, -(double)w.base_key * scale - est_margin, 0, 0};
+    f4_quadratic(w.d.n_cases, w.d.n_ctrls, 27, map.bound_k, map.bound_c);
+    map.bound_k *= scale;
+    fn<<<grid, kXThreads, kXSmem, s>>>(f.map_b, *r.map_j, f.map_i, w, sink, r.item_begin, g0, g1, f.nw_c, f.nw_t,
+                                       f.pack, map, dump, single, pairs, status, r.jl_begin, r.jlist, f.tri,
+                                       f.row_p, f.row_q);
     count_launch();
     return cudaGetLastError();
 }

@@ -33,6 +33,27 @@ struct T3xRange {                        // where the items of a request are lis
 };
 cudaError_t launch_tensor3x(const ScanWork& w, const F4Plan& f, const T3xRange& r, long long g0, long long g1,
                             const CandSink& sink, uint32_t* dump, const uint32_t* single, const uint4* pairs,
-                            float thr_f, float thr_q, int* status, cudaStream_t s, int sms);
+                            double est_margin, int* status, cudaStream_t s, int sms, bool cores = false);
+// The packed cores of all pairs and triples (F4Plan::tri, pairf), by the pair kernel over the order-3 items;
+// waits for them.
+cudaError_t f4_triples(const DevData& d, F4Plan& f, const long long* item_begin, long long items, const uint4* pairs,
+                       cudaStream_t s, int sms);
+
+// Order-4 pair kernel (tensor4x.cu): items (i, j, 32 k, up to 112 l).
+constexpr int kP4K = 32;   // k per pair item (16 per CTA)
+constexpr int kP4G = 7;    // most groups of 16 l per item
+__host__ __device__ __forceinline__ int t4x_groups(int n, int kf) { return (n - ((kf + 1) & ~7) + 15) >> 4; }
+__host__ __device__ __forceinline__ int t4x_tiles(int n, int kf) { return (t4x_groups(n, kf) + kP4G - 1) / kP4G; }
+cudaError_t f4_order4_maps(F4Plan& f, int snps);
+struct T4xRange {                   // where the items of a request are listed
+    const long long* begin;         // first item of the pairs with second SNP j, [n + 1] (a layer: of each listed pair)
+    const long long* per;           // items of a pair with second SNP j
+    const CUtensorMap* map_k;       // bit rows of the k operand
+    const int4* pinfo = nullptr;    // a Distribution layer: (i, j, first owned k) of each listed pair
+    int n_pairs = 0;
+};
+cudaError_t launch_tensor4x(const ScanWork& w, const F4Plan& f, const T4xRange& r, long long g0, long long g1,
+                            const CandSink& sink, uint32_t* dump, const uint32_t* single, const uint4* pairs,
+                            int* status, cudaStream_t s, int sms);
 
 }  // namespace fiu

@@ -1,22 +1,19 @@
-// Order-4 contingency tables on the 5th-generation tensor cores (tcgen05).
+// Order-4 contingency tables on the 5th-generation tensor cores (tcgen05), one
+// accumulator per class (classes that share one take tensor4x.cu).
 //
 // For one-hot data the 16 core cells of a combination (i, j, k, l) --
 // genotypes x, y, z, w in {0, 1} -- are dot products over the samples:
 //     core[x][y][z][w] = sum_s a_ix(s) a_jy(s) a_kz(s) a_lw(s).
-// A work item is (i, j, 16 consecutive k, 128 consecutive l); it is one GEMM
-//     D[(k,x,y,z), (l,w)] = sum_s A[(k,x,y,z), s] B[(l,w), s]   (M 128, N 256)
-// over the e4m3 operand planes of tensor3.cu, both classes in one FP32
-// accumulator (control samples weighted by W = 4^h, exact while
-// n_cases < W and n_cases + W * n_ctrls < 2^24).  Classes that do not pack
-// take the split form: 64 l per item, the case samples accumulate into one
-// N 128 region and the control samples into another, two such pairs
-// alternating between items (measured against 128 l per item with one N 256
-// region per class and no alternation: 16.9 vs 18.4 ms at 150 SNPs x
-// 5 900/9 000 samples).  B rows are plane rows 2l+w
-// by TMA; A rows are the bytewise AND of the i, j and k plane rows, built in
-// shared memory by two producer warps from the TMA-staged rows (i AND j once
-// per stage, then AND each k row).  Two accumulator regions alternate between
-// items so the next item's GEMM overlaps the epilogue.
+// A work item is (i, j, 16 consecutive k, 64 consecutive l); per class it is one
+// GEMM
+//     D[(k,x,y,z), (l,w)] = sum_s A[(k,x,y,z), s] B[(l,w), s]   (M 128, N 128)
+// over the e4m3 operand planes of tensor3.cu.  Case samples accumulate into one
+// N 128 region and control samples into another, two such pairs alternating
+// between items (measured against 128 l per item with one N 256 region per class
+// and no alternation: 16.9 vs 18.4 ms at 150 SNPs x 5 900/9 000 samples).  B rows
+// are plane rows 2l+w by TMA; A rows are the bytewise AND of the i, j and k plane
+// rows, built in shared memory by two producer warps from the TMA-staged rows (i
+// AND j once per stage, then AND each k row).
 //
 // Epilogue.  Each thread reads the accumulators of one row (k, x, y, z); a
 // swizzled shared-memory transpose gives each lane the 16 core counts of one
@@ -36,12 +33,13 @@
 #include <cmath>
 
 #include "elided4_prefix.cuh"
+#include "tensor3x.h"
 #include "tensor_common.cuh"
 
 namespace fiu {
 
-constexpr int kT4K = 16, kT4L = 128;                // k and l SNPs per work item (64 l in the split form)
-constexpr int kT4M = 8 * kT4K, kT4N = 2 * kT4L;     // 128 x 256 GEMM tile
+constexpr int kT4K = 16, kT4L = 64;                 // k and l SNPs per work item
+constexpr int kT4M = 8 * kT4K, kT4N = 2 * kT4L;     // 128 x 128 GEMM tile, one accumulator region per class
 // Two A builders keep pace with the MMA (about 130 instructions per builder
 // thread and k-step against ~640 tensor cycles).  The epilogue warps (a
 // multiple of 4: each reads the tensor-memory lane quarter warp % 4) share an
@@ -55,13 +53,13 @@ constexpr int kT4Threads = 32 * (2 + kT4BuildWarps + kT4EpiWarps);
 static_assert(kT4EpiWarps % 4 == 0, "epilogue warps cover the four lane quarters evenly");
 constexpr int kT4BuildRows = 2 * kT4K / (4 * kT4BuildWarps);          // k rows per builder thread and stage
 static_assert(2 * kT4K % (4 * kT4BuildWarps) == 0, "builder threads split the k rows evenly");
-constexpr int kT4Stages = 3;
-constexpr int kT4SB = kT4N * kT3KB;                 // 32 KB  l rows
+constexpr int kT4Stages = 4;
+constexpr int kT4SB = kT4N * kT3KB;                 // 16 KB  l rows
 constexpr int kT4SA = kT4M * kT3KB;                 // 16 KB  A (k, x, y, z)
 constexpr int kT4SK = 2 * kT4K * kT3KB;             //  4 KB  k rows
 constexpr int kT4SI = 1024;                         // i rows (2 x 128 B) in a 1 KB slot
 constexpr int kT4SJ = 1024;                         // j rows
-constexpr int kT4Stage = kT4SB + kT4SA + kT4SK + kT4SI + kT4SJ;  // 54 KB, a multiple of 1 KB
+constexpr int kT4Stage = kT4SB + kT4SA + kT4SK + kT4SI + kT4SJ;  // 38 KB, a multiple of 1 KB
 constexpr int kT4Ebuf = 2048;                       // per epilogue warp: 32 combinations x 8 (x,y,z) x 8 B
 
 // Sources of the epilogue that depend on one of k or l only, copied into
@@ -83,7 +81,7 @@ constexpr size_t kT4Smem =
 // instruction descriptor: e4m3 x e4m3 -> FP32, M 128, N 256 (packed) or 128 (split)
 constexpr uint32_t t4_idesc(int N) { return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(kT4M >> 4) << 24); }
 static_assert(kT4Smem <= 227 * 1024 - 256, "order-4 tensor kernel shared memory");
-static_assert(2 * kT4N <= 512, "order-4 tensor kernel tensor memory");
+static_assert(4 * kT4N <= 512, "order-4 tensor kernel tensor memory");
 
 struct T4Maps {
     CUtensorMap l, k, i;  // boxes of 2 L (256 or 128), 32 and 2 plane rows
@@ -249,8 +247,8 @@ __device__ __forceinline__ void t4_stage(T4Item& it, long long g, int et, const 
             t4_cp16(&it.pjl[et], pairs + pair_index(j, l, n));
             t4_cp16(&it.sl[et], single4 + l);
         }
-    } else if (et >= kT4L && et < kT4L + kT4K) {
-        const int kk = et - kT4L, k = k0 + kstep * kk;
+    } else if (et >= 128 && et < 128 + kT4K) {
+        const int kk = et - 128, k = k0 + kstep * kk;
         if (k < n) {
             const uint4* t = triples + 2 * triple_index(i, j, k, n);
             t4_cp16(&it.tijk[0][kk], t);
@@ -259,7 +257,7 @@ __device__ __forceinline__ void t4_stage(T4Item& it, long long g, int et, const 
             t4_cp16(&it.pjk[kk], pairs + pair_index(j, k, n));
             t4_cp16(&it.sk[kk], single4 + k);
         }
-    } else if (et == kT4L + kT4K) {
+    } else if (et == 128 + kT4K) {
         t4_cp16(&it.pij, pairs + pair_index(i, j, n));
         t4_cp16(&it.si, single4 + i);
         t4_cp16(&it.sj, single4 + j);
@@ -365,10 +363,10 @@ __device__ __forceinline__ void t4_ld16(uint32_t taddr, uint32_t (&v)[16]) {
 // separately so that the search's instantiation carries none of its code.
 // LAYER: a Distribution layer (t4l_decode; maps.k then covers the residue-ordered planes, begin /
 // pinfo / n_pairs are the layer's pair tables).
-template <bool PACK, bool DIGEST, bool LAYER>
+template <bool DIGEST, bool LAYER>
 __global__ void __launch_bounds__(kT4Threads, 1)
     tensor4p_kernel(const __grid_constant__ T4Maps maps, ScanWork w, const long long* __restrict__ begin,
-                    const long long* __restrict__ per, long long g0, long long g1, int k_cases, int pack,
+                    const long long* __restrict__ per, long long g0, long long g1, int k_cases,
                     CandSink sink, long long thr_q, uint32_t* dump, const uint32_t* __restrict__ single,
                     const uint4* __restrict__ pairs, const uint4* __restrict__ triples, int* status,
                     const int4* __restrict__ pinfo, int n_pairs) {
@@ -385,7 +383,7 @@ __global__ void __launch_bounds__(kT4Threads, 1)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int ks_c = k_cases / kT3KB;
     const int ksteps = ks_c + (d.tw + 1) / 2;
-    constexpr int L = PACK ? kT4L : kT4L / 2;                     // l per item
+    constexpr int L = kT4L;                                         // l per item
     constexpr int NR = 2 * L;                                       // N of one accumulator region
     constexpr uint32_t kTx = NR * kT3KB + kT4SK + 2 * 2 * kT3KB;  // bytes the TMA brings per stage
     constexpr int NG = L / 8;                                       // column groups of 8 l per item
@@ -467,11 +465,10 @@ __global__ void __launch_bounds__(kT4Threads, 1)
                 const int vl = min(L, n - l0);
                 const uint32_t idesc = t4_idesc(min(NR, max(64, (2 * vl + 15) / 16 * 16)));
                 for (int ks = 0; ks < ksteps; ++ks, ++step) {
-                    // packed: one region of N 256 per buffer; split: cases in the
-                    // buffer's first N 128 columns, controls in its second
-                    const bool ctrl = !PACK && ks >= ks_c;
-                    const uint32_t dcol = tmem + (uint32_t)(kT4N * buf + (ctrl ? NR : 0));
-                    const bool first = ks == 0 || (!PACK && ks == ks_c);
+                    // cases in the buffer's first N 128 columns, controls in its second
+                    const bool ctrl = ks >= ks_c;
+                    const uint32_t dcol = tmem + (uint32_t)(2 * kT4N * buf + (ctrl ? NR : 0));
+                    const bool first = ks == 0 || ks == ks_c;
                     const int s = (int)(step % kT4Stages);
                     if (!t3_wait(smem_u32(&full_a[s]), (uint32_t)((step / kT4Stages) & 1), abort)) {
                         ok = false;
@@ -559,7 +556,6 @@ __global__ void __launch_bounds__(kT4Threads, 1)
         const int hh = e >> 2;                      // column groups hh, hh + H, ...: l offsets 8 gi + [0, 8)
         uint32_t* ebuf = ebuf_all + e * (kT4Ebuf / 4);
         const uint32_t lane_base = tmem + ((uint32_t)(32 * q) << 16);
-        const uint32_t wmask = PACK ? (1u << pack) - 1u : 0xffffffffu;
         const int kkw = lane >> 3, xyz = lane & 7;  // this thread's accumulator row (4 q + kkw, xyz)
         const int kkc = lane >> 3, llc = lane & 7;  // this lane's combination in a column group
         const int et = tid - 32 * (2 + kT4BuildWarps);  // 0 .. 32 kT4EpiWarps - 1
@@ -606,10 +602,10 @@ __global__ void __launch_bounds__(kT4Threads, 1)
                 T4KL kl{};
                 if (valid && !dump) kl = t4_load_kl(pairs, triples, i, j, k, l, n);
                 {
-                    const uint32_t col = (uint32_t)(kT4N * buf + 16 * gi);
+                    const uint32_t col = (uint32_t)(2 * kT4N * buf + 16 * gi);
                     uint32_t v[16], vt[16];
                     t4_ld16(lane_base + col, v);
-                    if (!PACK) t4_ld16(lane_base + col + NR, vt);  // control counts of the same rows / columns
+                    t4_ld16(lane_base + col + NR, vt);  // control counts of the same rows / columns
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                     if (last) {  // this warp's last read of the item's accumulators
                         asm volatile("tcgen05.fence::before_thread_sync;");
@@ -622,13 +618,8 @@ __global__ void __launch_bounds__(kT4Threads, 1)
                     for (int ll = 0; ll < 8; ++ll) {
                         const uint32_t u0 = __float2uint_rn(__uint_as_float(v[2 * ll]));
                         const uint32_t u1 = __float2uint_rn(__uint_as_float(v[2 * ll + 1]));
-                        uint2 c2;
-                        if (PACK) {
-                            c2 = make_uint2((u0 & wmask) | (u1 & wmask) << 16, (u0 >> pack) | (u1 >> pack) << 16);
-                        } else {
-                            c2 = make_uint2(u0 | u1 << 16, __float2uint_rn(__uint_as_float(vt[2 * ll])) |
-                                                               __float2uint_rn(__uint_as_float(vt[2 * ll + 1])) << 16);
-                        }
+                        const uint2 c2 = make_uint2(u0 | u1 << 16, __float2uint_rn(__uint_as_float(vt[2 * ll])) |
+                                                                       __float2uint_rn(__uint_as_float(vt[2 * ll + 1])) << 16);
                         *reinterpret_cast<uint2*>(ebuf + 2 * t4_slot(kkw, ll, xyz)) = c2;
                     }
                 }
@@ -675,11 +666,15 @@ double t4_margin(int n_samples) {
     return 2 * err + 1e-3;
 }
 
-std::vector<long long> t4_item_table(int n, bool pack, std::vector<long long>& per) {
+std::vector<long long> t4_item_table(int n, bool pair, std::vector<long long>& per) {
     std::vector<long long> begin((size_t)n + 1, 0);
     per.assign((size_t)std::max(n, 1), 0);
     for (int j = 0; j < n; ++j) {
-        per[j] = t4_items_per_pair(n, j, pack ? kT4L : kT4L / 2);
+        if (pair) {
+            for (int k0 = j + 1; k0 <= n - 2; k0 += kP4K) per[j] += t4x_tiles(n, k0);
+        } else {
+            per[j] = t4_items_per_pair(n, j, kT4L);
+        }
         begin[j + 1] = begin[j] + (long long)j * per[j];
     }
     return begin;
@@ -687,9 +682,9 @@ std::vector<long long> t4_item_table(int n, bool pack, std::vector<long long>& p
 
 // Pair tables of a Distribution layer of an order-4 scan (host): the listed pairs (i, j) with at
 // least one item, their first owned k and first item.  Returns the items; combos = combinations.
-long long t4_layer_items(int n, int step, long long offset, bool pack, std::vector<long long>& pbegin,
+long long t4_layer_items(int n, int step, long long offset, bool pair, std::vector<long long>& pbegin,
                          std::vector<int4>& pinfo, long long& combos) {
-    const int L = pack ? kT4L : kT4L / 2;
+    const int L = kT4L;
     pbegin.clear();
     pinfo.clear();
     combos = 0;
@@ -702,7 +697,8 @@ long long t4_layer_items(int n, int step, long long offset, bool pack, std::vect
             if (t >= cnt) continue;
             const int kf = j + 1 + (int)t;
             long long items = 0;
-            for (long long k = kf; k <= n - 2; k += (long long)kT4K * step) items += (n - 1 - k + L - 1) / L;
+            for (long long k = kf; k <= n - 2; k += (long long)(pair ? kP4K : kT4K) * step)
+                items += pair ? t4x_tiles(n, (int)k) : (n - 1 - k + L - 1) / L;
             for (long long k = kf; k < n; k += step) combos += n - 1 - k;
             if (items == 0) continue;
             pbegin.push_back(total);
@@ -713,22 +709,19 @@ long long t4_layer_items(int n, int step, long long offset, bool pack, std::vect
     return total;
 }
 
-cudaError_t launch_tensor4(const ScanWork& w, const CUtensorMap& map_l256, const CUtensorMap& map_l128,
-                           const CUtensorMap& map_k, const CUtensorMap& map_i, const long long* begin,
-                           const long long* per, int k_cases, int pack, long long g0, long long g1,
-                           const CandSink& sink, uint32_t* dump, const uint32_t* single, const uint4* pairs,
-                           const uint4* triples, int* status, cudaStream_t s, int sms, const int4* pinfo,
-                           int n_pairs) {
+cudaError_t launch_tensor4(const ScanWork& w, const CUtensorMap& map_l, const CUtensorMap& map_k,
+                           const CUtensorMap& map_i, const long long* begin, const long long* per, int k_cases,
+                           long long g0, long long g1, const CandSink& sink, uint32_t* dump, const uint32_t* single,
+                           const uint4* pairs, const uint4* triples, int* status, cudaStream_t s, int sms,
+                           const int4* pinfo, int n_pairs) {
     const bool layer = pinfo != nullptr;
     if (!triples || !pairs || !single || !begin || (!per && !layer)) return cudaErrorInvalidValue;
-    static LaunchCache cache[8];
+    static LaunchCache cache[4];
     const bool dg = sink.digest != nullptr;
-    using Fn = decltype(&tensor4p_kernel<true, true, true>);
-    static const Fn fns[8] = {tensor4p_kernel<false, false, false>, tensor4p_kernel<false, true, false>,
-                              tensor4p_kernel<true, false, false>,  tensor4p_kernel<true, true, false>,
-                              tensor4p_kernel<false, false, true>,  tensor4p_kernel<false, true, true>,
-                              tensor4p_kernel<true, false, true>,   tensor4p_kernel<true, true, true>};
-    const int v = (layer ? 4 : 0) + (pack ? 2 : 0) + (dg ? 1 : 0);
+    using Fn = decltype(&tensor4p_kernel<true, true>);
+    static const Fn fns[4] = {tensor4p_kernel<false, false>, tensor4p_kernel<true, false>, tensor4p_kernel<false, true>,
+                              tensor4p_kernel<true, true>};
+    const int v = (layer ? 2 : 0) + (dg ? 1 : 0);
     const Fn fn = fns[v];
     int per_sm = 1;
     cudaError_t e = blocks_per_sm(cache[v], fn, kT4Threads, kT4Smem, per_sm);
@@ -740,8 +733,8 @@ cudaError_t launch_tensor4(const ScanWork& w, const CUtensorMap& map_l256, const
     const double thr = ((double)sink.thr - (double)w.base_key) * scale - t4_margin(w.d.n_cases + w.d.n_ctrls) * 65536.0;
     const long long thr_q = (long long)std::floor(std::max(-9.0e18, std::min(9.0e18, thr)));
     const unsigned grid = (unsigned)(items < sms ? items : sms);
-    const T4Maps maps{pack ? map_l256 : map_l128, map_k, map_i};
-    fn<<<grid, kT4Threads, kT4Smem, s>>>(maps, w, begin, per, g0, g1, k_cases, pack, sink, thr_q, dump, single, pairs,
+    const T4Maps maps{map_l, map_k, map_i};
+    fn<<<grid, kT4Threads, kT4Smem, s>>>(maps, w, begin, per, g0, g1, k_cases, sink, thr_q, dump, single, pairs,
                                          triples, status, pinfo, n_pairs);
     count_launch();
     return cudaGetLastError();

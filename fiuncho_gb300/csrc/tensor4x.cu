@@ -1,0 +1,719 @@
+// Order-4 contingency tables on CTA pairs with 4-bit operands (classes that
+// share one accumulator).
+//
+// A cluster of two CTAs runs one GEMM per work item (i, j, 32 k, up to 112 l):
+//     D[(k,x,y,z), (l,w)] = sum_s A[(k,x,y,z), s] B[(l,w), s]    (M 256, N <= 224)
+// as the order-3 pair kernel does (tensor3x.cu: operand formats, roles,
+// handover, scales).  CTA r builds the A rows of its 16 k -- the AND of the i, j
+// and k bit rows, spread to nibbles -- and stages half r of the l rows.
+//
+// Accumulator rows are ordered (k / 4, x, y, z, k % 4).  A 16x256b load of a
+// 16-row block gives a thread the rows (x, y = 0, 1) of one z and one k; it loads
+// two column groups (16 l) and exchanges halves with the lane of the other z (16
+// shuffles): each lane then holds all 16 cores of the combinations (k, l) and
+// (k, l + 1) of one group.  The lane of z = 1 keeps its rows first, so its z
+// runs 1, 0, 2: it reads the tables that depend on k's genotype in that order.
+//
+// Epilogue.  The 81 cells of both combinations follow slice by slice (genotype of
+// l) from the packed cores and marginals in two-wide single precision: per l the
+// tables of (i,j,l), (i,l), (j,l), l and per k those of (i,j,k), (i,k), (j,k), k
+// are staged in shared memory one item ahead by two warps of their own; the
+// triples (i,k,l), (j,k,l) and the pair (k,l) come as packed floats of (l, l + 1)
+// side by side (F4Plan::tri, pairf; the triples are made by the order-3 pair
+// kernel, whose accumulators they are).  The quartic bound (F4Bound4) rejects
+// nearly all combinations (300 SNPs x 558/1 012: 5 500 of 3.3e8 pass it); the
+// others get the exact fixed-point key, so the kept set is the one of the exact
+// key.
+//
+// Measured (whole searches): 300 SNPs x 4 000/4 000 81.9 -> 37.0 ms, 300 x
+// 558/1 012 66.2 -> 31.0 ms, against e4m3 operands, one CTA a tile, 243
+// logarithms a combination (1 944 cycles a warp and SM quarter; the bound takes 81
+// reciprocals and about 930 arithmetic cycles) and triples counted by POPC.
+// Without the evaluation the two take 26 and 13 ms.
+//
+// Reference semantics: GenotypeTable::combine_and_popcnt for order 4
+// (src/base/gt_popcnt.cpp:4-35) and MutualInformation::compute
+// (src/base/mi_compute.cpp:16-41) over the combinations ThreadedSearch
+// visits (include/fiuncho/ThreadedSearch.h:157-180) with one worker.
+#include <algorithm>
+#include <cmath>
+
+#include "elided4_prefix.cuh"
+#include "exact_key.cuh"
+#include "live.cuh"
+#include "tensor3x.h"
+#include "tensor_fp4.cuh"
+
+namespace fiu {
+
+constexpr int kYK = kP4K / 2;                       // k per CTA
+constexpr int kYL = 16 * kP4G;                      // 112 l per item at most
+constexpr int kYN = 2 * kYL;                        // columns of an accumulator region
+constexpr int kYRow = kF4K / 2;                     // 128 bytes per operand row and stage
+constexpr int kYBitRow = kF4K / 8;                  // 32 bytes per bit row and stage
+constexpr int kYHalfG = 4;                          // items of at most 4 groups bring 64 l rows a CTA, others 112
+constexpr int kYStages = 8, kYAStages = 4;          // rings of the copies and of A, as in the order-3 kernel
+constexpr int kYSA = 8 * kYK * kYRow;               // 16 KB
+constexpr int kYSB = kYN / 2 * kYRow;               // 14 KB: this CTA's half of the l rows
+constexpr int kYSK = 2 * kYK * kYBitRow;            //  1 KB
+constexpr int kYSI = 2 * kYBitRow;                  // 64 bytes of i, 64 of j (on 128-byte boundaries)
+constexpr int kYStage = (kYSB + kYSK + 256 + 1023) / 1024 * 1024;  // 16 KB
+constexpr int kYColOne = 2 * kYN, kYColW = kYColOne + 16;
+// 640 threads: copies, MMAs and two staging warps; two groups of four builders
+// that take alternate stages; eight epilogue warps.  Registers a thread: 96 at
+// launch, then 56 / 56 / 152 (3 x 56 + 2 x 152 <= 5 x 96).
+constexpr int kYBuildWarps = 4, kYEpiWarps = 8;
+constexpr int kYThreads = 32 * (4 + 2 * kYBuildWarps + kYEpiWarps);
+constexpr int kYMeta = 16;                          // items in flight between the copies and the MMAs
+// staged tables of an item: per l (ijl (x,y,w), il (x,w), jl (y,w), l (w); w = 0, 1, any), per k of
+// this CTA (ijk, ik, jk, k cores, each twice: both halves of a pair)
+// and the item's threshold (key, estimate, bound)
+constexpr int kYTabL = 27 * kYL * 4, kYTabK = 18 * kYK * 8, kYTab = kYTabL + kYTabK + 16;
+constexpr size_t kYSmem = 1024 + (size_t)kYStages * kYStage + (size_t)kYAStages * kYSA + 2 * kYTab;
+static_assert(kYSmem <= 227 * 1024 - 512, "order-4 pair kernel shared memory");
+static_assert(kYSA % 1024 == 0 && kYSB % 1024 == 0, "operand tiles on swizzle atoms");
+static_assert(kYColW + 16 <= 512, "tensor memory columns");
+static_assert(kYStages < kYMeta, "an item has a stage at least");
+
+// One item: (i, j, k0 ..), l-tile of ng groups of 16 from l0.
+struct T4xItem {
+    int i, j, k0, l0, ng;
+};
+
+// Item g; at is the walker's position (the items of one walker ascend): the
+// second SNP j, or in a layer the listed pair.
+template <bool LAYER>
+__device__ __forceinline__ T4xItem t4x_item(const long long* __restrict__ begin, const long long* __restrict__ per,
+                                            const int4* __restrict__ pinfo, int n_pairs, int n, int step,
+                                            long long g, int& at) {
+    if (at < 0) {
+        int lo = 0, hi = (LAYER ? n_pairs : n) - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (__ldg(begin + mid) <= g) lo = mid;
+            else hi = mid - 1;
+        }
+        at = lo;
+    } else {
+        while (__ldg(begin + at + 1) <= g) ++at;
+    }
+    T4xItem it;
+    const unsigned rel = (unsigned)(g - __ldg(begin + at));
+    unsigned q = rel;
+    int k;
+    if (LAYER) {
+        const int4 f = __ldg(pinfo + at);
+        it.i = f.x;
+        it.j = f.y;
+        k = f.z;
+    } else {
+        const unsigned pj = (unsigned)__ldg(per + at);
+        it.j = at;
+        it.i = (int)(rel / pj);
+        q = rel - it.i * pj;
+        k = at + 1;
+    }
+    for (;; k += kP4K * (LAYER ? step : 1)) {
+        const unsigned nl = t4x_tiles(n, k);
+        if (q < nl) {
+            const int G = t4x_groups(n, k), a = G * (int)q / (int)nl, b = G * ((int)q + 1) / (int)nl;
+            it.k0 = k;
+            it.l0 = ((k + 1) & ~7) + 16 * a;
+            it.ng = b - a;
+            return it;
+        }
+        q -= nl;
+    }
+}
+
+// Columns the MMA of an item of ng groups multiplies (at least 64).
+__device__ __forceinline__ int t4x_n(int ng) { return 32 * max(ng, 2); }
+
+__device__ __forceinline__ float t4x_pk(uint32_t c, uint32_t t, float W) { return fmaf(W, u2f(t), u2f(c)); }
+__device__ __forceinline__ float t4x_pair(const uint4& v, int x, int y, float W) {
+    const uint32_t c = x ? v.y : v.x, t = x ? v.w : v.z;
+    return t4x_pk(y ? c >> 16 : c & 0xffffu, y ? t >> 16 : t & 0xffffu, W);
+}
+
+// One 27-cell slice (one genotype of l) from its 8 cores c (x, y, z) and packed
+// marginals: mij (x, y), mik (x, z), mil (x), mjk (y, z), mjl (y), mkl (z = 0, 1,
+// any).  T is one value or two side by side; use(q, cell) gets cell (x, y, z) at
+// q = (x*3+y)*3+z.
+__device__ __forceinline__ f2 t4x_less(f2 a, f2 b, f2 c) { return f2_sub(f2_sub(a, b), c); }
+__device__ __forceinline__ float t4x_less(float a, float b, float c) { return a - b - c; }
+template <class T, class Use>
+__device__ __forceinline__ void t4x_slice(const T (&c)[2][2][2], const T (&mij)[2][2], const T (&mik)[2][2],
+                                          const T (&mil)[2], const T (&mjk)[2][2], const T (&mjl)[2],
+                                          const T (&mkl)[3], Use&& use) {
+    T a[2][3][3];  // cells of x = 0, 1
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+#pragma unroll
+        for (int y = 0; y < 2; ++y) {
+            a[x][y][0] = c[x][y][0];
+            a[x][y][1] = c[x][y][1];
+            a[x][y][2] = t4x_less(mij[x][y], c[x][y][0], c[x][y][1]);
+        }
+        const T k2 = t4x_less(mil[x], mik[x][0], mik[x][1]);
+#pragma unroll
+        for (int z = 0; z < 3; ++z) a[x][2][z] = t4x_less(z < 2 ? mik[x][z] : k2, a[x][0][z], a[x][1][z]);
+#pragma unroll
+        for (int y = 0; y < 3; ++y)
+#pragma unroll
+            for (int z = 0; z < 3; ++z) use((x * 3 + y) * 3 + z, a[x][y][z]);
+    }
+    const T j0 = t4x_less(mjl[0], mjk[0][0], mjk[0][1]), j1 = t4x_less(mjl[1], mjk[1][0], mjk[1][1]);
+#pragma unroll
+    for (int z = 0; z < 3; ++z) {
+        const T m0 = z < 2 ? mjk[0][z] : j0, m1 = z < 2 ? mjk[1][z] : j1;
+        use(18 + z, t4x_less(m0, a[0][0][z], a[1][0][z]));
+        use(21 + z, t4x_less(m1, a[0][1][z], a[1][1][z]));
+        use(24 + z, t4x_less(t4x_less(mkl[z], m0, m1), a[0][2][z], a[1][2][z]));
+    }
+}
+
+// What a lane holds for its combinations: cores (x, y, z, w), the triples (i,k,l) (x, z, w) and
+// (j,k,l) (y, z, w), the pair (k,l) (z, w); z in the lane's order.
+template <class T>
+struct T4xCores {
+    T c[2][2][2][2], ik[2][2][2], jk[2][2][2], kl[2][2];
+};
+
+// The three slices of the combinations in v.  tabl(e) and tabk(e) return the
+// staged entries (kYTabL and kYTabK order, z in the lane's order).
+template <class T, class TL, class TK, class Use>
+__device__ __forceinline__ void t4x_slices(const T4xCores<T>& v, TL&& tabl, TK&& tabk, Use&& use) {
+#pragma unroll
+    for (int w = 0; w < 3; ++w) {
+        T c[2][2][2], mij[2][2], mik[2][2], mil[2], mjk[2][2], mjl[2], mkl[3];
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int y = 0; y < 2; ++y) {
+                mij[x][y] = tabl((x * 2 + y) * 3 + w);
+#pragma unroll
+                for (int z = 0; z < 2; ++z)
+                    c[x][y][z] = w < 2 ? v.c[x][y][z][w & 1]
+                                       : t4x_less(tabk((x * 2 + y) * 2 + z), v.c[x][y][z][0], v.c[x][y][z][1]);
+            }
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            mil[x] = tabl(12 + x * 3 + w);
+            mjl[x] = tabl(18 + x * 3 + w);
+#pragma unroll
+            for (int z = 0; z < 2; ++z) {
+                mik[x][z] = w < 2 ? v.ik[x][z][w & 1] : t4x_less(tabk(8 + x * 2 + z), v.ik[x][z][0], v.ik[x][z][1]);
+                mjk[x][z] = w < 2 ? v.jk[x][z][w & 1] : t4x_less(tabk(12 + x * 2 + z), v.jk[x][z][0], v.jk[x][z][1]);
+            }
+        }
+#pragma unroll
+        for (int z = 0; z < 2; ++z) mkl[z] = w < 2 ? v.kl[z][w & 1] : t4x_less(tabk(16 + z), v.kl[z][0], v.kl[z][1]);
+        mkl[2] = t4x_less(tabl(24 + w), mkl[0], mkl[1]);
+        t4x_slice<T>(c, mij, mik, mil, mjk, mjl, mkl, [&](int q, T cell) { use(w, q, cell); });
+    }
+}
+
+__device__ __forceinline__ void t4x_append(const ScanWork& w, const CandSink& sink, const int (&cmb)[4],
+                                           long long key) {
+    const unsigned idx = atomicAdd(sink.count, 1u);
+    if (idx < sink.cap) {
+        sink.buf[idx] = Cand{key, pack_code(cmb, 4, w.bits)};
+        if (sink.hist) atomicAdd(sink.hist + live_bin(key), 1u);
+    } else {
+        atomicOr(sink.overflow, 1u);
+    }
+}
+
+// ALL: every combination takes the exact path (a search's first units, before a threshold; dumps and
+// digests).  Otherwise the bound comes first and the few combinations above it are evaluated from the
+// data set (warp_exact_key): the exact path's registers beside the bound's cost 20 % of the whole.
+template <bool LAYER, bool ALL>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
+    tensor4x_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_bh,
+                    const __grid_constant__ CUtensorMap map_k,
+                    const __grid_constant__ CUtensorMap map_i, const __grid_constant__ ScanWork w,
+                    const __grid_constant__ CandSink sink, const long long* __restrict__ begin,
+                    const long long* __restrict__ per, const int4* __restrict__ pinfo, int n_pairs, long long g0,
+                    long long g1, int nw_c, int nw_t, int pack, const __grid_constant__ LiveMap map,
+                    const __grid_constant__ F4Quartic quart,
+                    uint32_t* dump, const uint32_t* __restrict__ single, const uint4* __restrict__ pairs,
+                    const float* __restrict__ tri, const float* __restrict__ pairf, const int* __restrict__ row_p,
+                    const int* __restrict__ row_q, int* status) {
+    extern __shared__ uint8_t smraw[];
+    __shared__ __align__(8) uint64_t full_t[kYStages], empty[kYStages], full_a[kYAStages];
+    __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2], tab_full[2], tab_empty[2], done;
+    __shared__ uint32_t tmem_base;
+    __shared__ int item_ng[kYMeta];  // groups of the items in flight, for the MMA issuer
+    __shared__ int abort_flag;
+    uint8_t* sm = (uint8_t*)(((uintptr_t)smraw + 1023) & ~(uintptr_t)1023);  // stages: B half | k | i | j; then the A tiles
+    uint8_t* sma = sm + kYStages * kYStage;
+    uint8_t* tabs = sma + kYAStages * kYSA;
+    volatile int* abort = &abort_flag;
+    const int n = w.d.snps, kstep = LAYER ? w.dist_step : 1;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // warp-uniform for the compiler too
+    const int ksteps = ((nw_c + 3) >> 2) + ((nw_t + 3) >> 2);  // stages of 256 samples
+    const uint32_t rank = cluster_rank();  // 0 issues the MMAs
+    const long long cid = cluster_id(), ncl = cluster_count();
+
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
+                     "r"(512));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+    }
+    if (tid == 0) {
+        auto init = [](uint64_t* b, int count) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(count));
+        };
+        for (int s = 0; s < kYStages; ++s) {
+            init(&full_t[s], 1);
+            init(&empty[s], 1);
+        }
+        for (int s = 0; s < kYAStages; ++s) init(&full_a[s], 2 * kYBuildWarps);
+        for (int b = 0; b < 2; ++b) {
+            init(&acc_full[b], 1);
+            init(&acc_empty[b], 2 * kYEpiWarps);
+            init(&tab_full[b], 2);
+            init(&tab_empty[b], kYEpiWarps);
+        }
+        init(&done, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;");
+        abort_flag = 0;
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    const uint32_t tmem = tmem_base;
+    if (warp >= 4 && warp < 8) f4_fill_scales<16>(tmem, warp & 3, kYColOne, kYColW, pack);
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    cluster_sync_all();  // both CTAs' barriers and scales exist before either signals the other
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    bool ok = true;
+
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+        if (warp == 0) {
+            // ---------------------------------------------------------------- TMA producer (both CTAs)
+            if (g0 + cid < g1 && elect_one()) {
+                unsigned s = 0, par = 1;  // stage and the parity its last release has (first round: free)
+                unsigned step = 0, item = 0;
+                int at = -1;
+                T4xItem it = t4x_item<LAYER>(begin, per, pinfo, n_pairs, n, kstep, g0 + cid, at);
+                for (long long g = g0 + cid; g < g1 && ok; g += ncl) {
+                    // this CTA's first k row (in a layer the owned k are consecutive residue-ordered rows;
+                    // rows past the last owned one are loaded too and ignored by the epilogue)
+                    const int krow = 2 * ((LAYER ? residue_row(it.k0, kstep, n) : it.k0) + kYK * (int)rank);
+                    const int brow = 2 * it.l0 + t4x_n(it.ng) / 2 * (int)rank, irow = 2 * it.i, jrow = 2 * it.j;
+                    const bool half = it.ng <= kYHalfG;
+                    item_ng[item++ % kYMeta] = it.ng;
+                    T4xItem nx = it;
+                    for (int ks = 0; ks < ksteps; ++ks) {
+                        if (!t3_wait_cl(smem_u32(&empty[s]), par, abort)) {
+                            ok = false;
+                            break;
+                        }
+                        const uint32_t st = smem_u32(sm + s * kYStage), bar = smem_u32(&full_t[s]);
+                        const uint32_t sk = st + kYSB;
+                        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                                     "r"((uint32_t)((half ? 16 * kYHalfG * kYRow : kYSB) + kYSK + 2 * kYSI))
+                                     : "memory");
+                        t3_tma(sk, &map_k, kYBitRow * ks, krow, bar);
+                        t3_tma(sk + kYSK, &map_i, kYBitRow * ks, irow, bar);
+                        t3_tma(sk + kYSK + 128, &map_i, kYBitRow * ks, jrow, bar);
+                        t3_tma(st, half ? &map_bh : &map_b, kYRow * ks, brow, bar);
+                        if (step < kYStages) ++step;
+                        if (++s == kYStages) {
+                            s = 0;
+                            par ^= 1;
+                        }
+                        // the next item's place is looked up while this item's copies are in flight
+                        if (ks == 0 && g + ncl < g1)
+                            nx = t4x_item<LAYER>(begin, per, pinfo, n_pairs, n, kstep, g + ncl, at);
+                    }
+                    it = nx;
+                }
+                // no copy may be in flight when the CTA exits: the last use of every stage used
+                for (unsigned q = 0; q < step; ++q) {
+                    // stage q was last filled in the round before `par` names, or in this one when q < s
+                    if (!t3_drain(smem_u32(&full_t[q]), q < s ? par ^ 1 : par)) ok = false;
+                }
+            }
+            __syncwarp();
+        } else if (warp == 1) {
+            // ---------------------------------------------------------------- MMA issuer (CTA 0)
+            if (rank == 0 && elect_one()) {
+                ok = f4_pair_issue<kYAStages, kYStages, kYStage, kYN, kYColOne, kYColW>(
+                    (g1 - g0 - cid + ncl - 1) / ncl, smem_u32(sma), smem_u32(sm), smem_u32(&full_a[0]),
+                    smem_u32(&empty[0]), smem_u32(&acc_full[0]), smem_u32(&acc_empty[0]), tmem, nw_c, nw_t, abort,
+                    [&](unsigned item) { return t4x_n(item_ng[item % kYMeta]); });
+                commit_pair(smem_u32(&done));
+                // neither CTA releases shared or tensor memory before the pair's MMAs are
+                // done (CTA 1 waits once its own work is over, below)
+                if (!t3_drain_cl(smem_u32(&done), 0)) ok = false;
+            }
+            __syncwarp();
+        } else {
+            // ---------------------------------------------------------------- table staging (both CTAs)
+            const int t = tid - 64;  // 0 .. 63
+            const float W = (float)(1u << pack);
+            const float ntot = fmaf(W, (float)w.d.n_ctrls, (float)w.d.n_cases);
+            const uint4* single4 = reinterpret_cast<const uint4*>(single);
+            unsigned item = 0;
+            int at = -1;
+            for (long long g = g0 + cid; g < g1 && ok; g += ncl, ++item) {
+                const T4xItem it = t4x_item<LAYER>(begin, per, pinfo, n_pairs, n, kstep, g, at);
+                const unsigned buf = item & 1;
+                if (item >= 2 && !t3_wait(smem_u32(&tab_empty[buf]), ((item >> 1) - 1) & 1, abort)) {
+                    ok = false;
+                    break;
+                }
+                // the threshold of this item (the pairs take turns at raising the live one)
+                if (sink.hist && rank == 0 && warp == 2 && item > 0 && (item < 3 || ((item + cid) & 7) == 0))
+                    live_update(sink, lane);
+                if (t == 0) {
+                    const long long thr = sink.hist ? *(volatile long long*)sink.live : sink.thr;
+                    float est, bound;
+                    live_tests(map, thr, est, bound);
+                    uint8_t* o = tabs + buf * kYTab + kYTabL + kYTabK;
+                    *reinterpret_cast<long long*>(o) = thr;
+                    *reinterpret_cast<float*>(o + 8) = bound;
+                }
+                float* tl = reinterpret_cast<float*>(tabs + buf * kYTab);
+                float2* tk = reinterpret_cast<float2*>(tabs + buf * kYTab + kYTabL);
+                const int i = it.i, j = it.j;
+                const uint4 pij4 = __ldg(pairs + pair_index(i, j, n));
+                const uint4 si = __ldg(single4 + i), sj = __ldg(single4 + j);
+                const float* tij = tri + 16ll * (__ldg(row_q + i) + __ldg(row_p + j));
+                const float ci[2] = {t4x_pk(si.x, si.z, W), t4x_pk(si.y, si.w, W)};
+                const float cj[2] = {t4x_pk(sj.x, sj.z, W), t4x_pk(sj.y, sj.w, W)};
+                for (int ll = t; ll < 16 * it.ng; ll += 64) {
+                    const int l = it.l0 + ll;
+                    float v[27];
+#pragma unroll
+                    for (int e = 0; e < 27; ++e) v[e] = 0.f;
+                    if (l < n && l > j) {
+                        const float* e3 = tij + 16ll * (l >> 1) + (l & 1);
+                        const uint4 pi = __ldg(pairs + pair_index(i, l, n)), pj = __ldg(pairs + pair_index(j, l, n));
+                        const uint4 sl = __ldg(single4 + l);
+#pragma unroll
+                        for (int xy = 0; xy < 4; ++xy) {
+                            v[3 * xy] = __ldg(e3 + 4 * xy);
+                            v[3 * xy + 1] = __ldg(e3 + 4 * xy + 2);
+                            v[3 * xy + 2] = t4x_pair(pij4, xy >> 1, xy & 1, W) - v[3 * xy] - v[3 * xy + 1];
+                        }
+#pragma unroll
+                        for (int x = 0; x < 2; ++x) {
+#pragma unroll
+                            for (int w2 = 0; w2 < 2; ++w2) {
+                                v[12 + 3 * x + w2] = t4x_pair(pi, x, w2, W);
+                                v[18 + 3 * x + w2] = t4x_pair(pj, x, w2, W);
+                            }
+                            v[14 + 3 * x] = ci[x] - v[12 + 3 * x] - v[13 + 3 * x];
+                            v[20 + 3 * x] = cj[x] - v[18 + 3 * x] - v[19 + 3 * x];
+                        }
+                        v[24] = t4x_pk(sl.x, sl.z, W);
+                        v[25] = t4x_pk(sl.y, sl.w, W);
+                        // "any" entries hold what is left after genotypes 0 and 1, so the slice of
+                        // genotype 2 reads its marginals as the other slices do
+                        v[26] = ntot - v[24] - v[25];
+                    }
+#pragma unroll
+                    for (int e = 0; e < 27; ++e) tl[e * kYL + ll] = v[e];
+                }
+                if (t < kYK) {
+                    const int k = it.k0 + kstep * (kYK * (int)rank + t);
+                    float v[18];
+#pragma unroll
+                    for (int e = 0; e < 18; ++e) v[e] = 0.f;
+                    if (k < n) {
+                        const float* e3 = tij + 16ll * (k >> 1) + (k & 1);
+                        const uint4 pi = __ldg(pairs + pair_index(i, k, n)), pj = __ldg(pairs + pair_index(j, k, n));
+                        const uint4 sk = __ldg(single4 + k);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) v[e] = __ldg(e3 + 2 * e);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            v[8 + e] = t4x_pair(pi, e >> 1, e & 1, W);
+                            v[12 + e] = t4x_pair(pj, e >> 1, e & 1, W);
+                        }
+                        v[16] = t4x_pk(sk.x, sk.z, W);
+                        v[17] = t4x_pk(sk.y, sk.w, W);
+                    }
+#pragma unroll
+                    for (int e = 0; e < 18; ++e) tk[e * kYK + t] = make_float2(v[e], v[e]);
+                }
+                __syncwarp();
+                if (lane == 0)
+                    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&tab_full[buf])) : "memory");
+            }
+        }
+    } else if (warp < 12) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+        // ---------------------------------------------------------------- A builders (both CTAs)
+        // thread: 16-byte chunk c (32 samples) of the k rows rg and rg + 16 of every second stage
+        const int t = (tid - 128) & (32 * kYBuildWarps - 1), c = t & 7, rg = t >> 3;
+        const uint32_t full0 = cluster_addr(smem_u32(&full_a[0]), 0);
+        // A row (kk / 4, x, y, z, kk % 4) of staged row (kk, z) = rg + 16 u: u + 1 is 64 rows on
+        const int kk = rg >> 1, z = rg & 1, m0 = 32 * (kk >> 2) + 4 * z + (kk & 3);
+        const int dst0 = m0 * kYRow + ((c ^ (m0 & 7)) << 4);
+        unsigned s = 0, par = 0, sa = 0;                  // copy stage, A stage
+        unsigned se = kYStages - kYAStages, pe = 1;       // the stage whose MMAs free this A stage
+        bool mine = warp < 8;
+        for (long long g = g0 + cid; g < g1 && ok; g += ncl) {
+            for (int ks = 0; ks < ksteps; ++ks, mine = !mine) {
+                if (mine) {
+                    if (!t3_wait(smem_u32(&full_t[s]), par, abort)) {
+                        ok = false;
+                        break;
+                    }
+                    const uint32_t* sK = reinterpret_cast<const uint32_t*>(sm + s * kYStage + kYSB);
+                    const uint32_t* sI = sK + kYSK / 4 + c;
+                    const uint32_t k0 = sK[rg * 8 + c], k1 = sK[(rg + 16) * 8 + c];
+                    const uint32_t i0 = sI[0], i1 = sI[8], j0 = sI[32], j1 = sI[40];
+                    if (!t3_wait_cl(smem_u32(&empty[se]), pe, abort)) {
+                        ok = false;
+                        break;
+                    }
+                    uint8_t* dst = sma + sa * kYSA + dst0;
+#pragma unroll
+                    for (int xy = 0; xy < 4; ++xy) {
+                        const uint32_t ij = (xy & 2 ? i1 : i0) & (xy & 1 ? j1 : j0);
+                        *reinterpret_cast<uint4*>(dst + 8 * xy * kYRow) = f4_expand_a(ij, k0);
+                        *reinterpret_cast<uint4*>(dst + (64 + 8 * xy) * kYRow) = f4_expand_a(ij, k1);
+                    }
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) arrive_cl(full0 + 8 * sa);
+                }
+                if (++s == kYStages) {
+                    s = 0;
+                    par ^= 1;
+                }
+                if (++se == kYStages) {
+                    se = 0;
+                    pe ^= 1;
+                }
+                if (++sa == kYAStages) sa = 0;
+            }
+        }
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");
+        // ---------------------------------------------------------------- epilogue (both CTAs)
+        const int q = warp & 3, hh = (warp - 12) >> 2;  // lane quarter (4 k); its two warps take alternate groups
+        const int zb = lane >> 4, kk = 4 * q + ((lane >> 2) & 3), lc = 2 * (lane & 3);
+        const uint32_t wmask = (1u << pack) - 1u;
+        unsigned item = 0;
+        int at = -1;
+        for (long long g = g0 + cid; g < g1 && ok; g += ncl, ++item) {
+            const T4xItem it = t4x_item<LAYER>(begin, per, pinfo, n_pairs, n, kstep, g, at);
+            const unsigned buf = item & 1, ph = (item >> 1) & 1;
+            const int k = it.k0 + kstep * (kYK * (int)rank + kk);
+            const bool k_ok = k < n;
+            // entries of the rows (i, k), (j, k) and k, in units of 16 bytes
+            const int rp = k_ok ? __ldg(row_p + k) : 0;
+            const uint4* tik = reinterpret_cast<const uint4*>(tri) + 4 * ((long long)__ldg(row_q + it.i) + rp);
+            const uint4* tjk = reinterpret_cast<const uint4*>(tri) + 4 * ((long long)__ldg(row_q + it.j) + rp);
+            const uint4* tkl = reinterpret_cast<const uint4*>(pairf) + 2 * (long long)rp;
+            if (!t3_wait(smem_u32(&tab_full[buf]), ph, abort) || !t3_wait_cl(smem_u32(&acc_full[buf]), ph, abort)) {
+                ok = false;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;");
+            const float* tabl0 = reinterpret_cast<const float*>(tabs + buf * kYTab);
+            const f2* tabk0 = reinterpret_cast<const f2*>(tabs + buf * kYTab + kYTabL) + kk;
+            const long long thr = *reinterpret_cast<const long long*>(tabs + buf * kYTab + kYTabL + kYTabK);
+            const float thr_q = *reinterpret_cast<const float*>(tabs + buf * kYTab + kYTabL + kYTabK + 8);
+            // (i,k,l), (j,k,l) and (k,l) of group gi: 16 bytes hold one (x, z) and both w
+            T4xCores<f2> v;
+            auto load = [&](int gi) {
+                const int l = it.l0 + 16 * gi + 8 * zb + lc, m = l >> 1;
+                const bool any = gi < it.ng && k_ok && l < n && l + 1 > k;
+                auto ld = [&](const uint4* p, f2 (&o)[2]) {
+                    uint4 x = make_uint4(0, 0, 0, 0);
+                    if (any) x = __ldg(p);
+                    o[0] = f2_pack(__uint_as_float(x.x), __uint_as_float(x.y));
+                    o[1] = f2_pack(__uint_as_float(x.z), __uint_as_float(x.w));
+                };
+#pragma unroll
+                for (int x = 0; x < 2; ++x)
+#pragma unroll
+                    for (int z = 0; z < 2; ++z) {
+                        ld(tik + 4 * m + 2 * x + (z ^ zb), v.ik[x][z]);
+                        ld(tjk + 4 * m + 2 * x + (z ^ zb), v.jk[x][z]);
+                    }
+#pragma unroll
+                for (int z = 0; z < 2; ++z) ld(tkl + 2 * m + (z ^ zb), v.kl[z]);
+            };
+            load(hh);
+#pragma unroll 1
+            for (int gi = hh; gi < it.ng; gi += 2) {
+                const int ll = 16 * gi + 8 * zb + lc, l = it.l0 + ll;
+                const bool v0 = k_ok && l < n && l > k, v1 = k_ok && l + 1 < n && l + 1 > k;
+                const unsigned m0 = __ballot_sync(0xffffffffu, v0), m1 = __ballot_sync(0xffffffffu, v1);
+                if (!(m0 | m1)) {
+                    load(gi + 2);
+                    continue;
+                }
+                if (sink.evaluated && lane == 0)
+                    atomicAdd(sink.evaluated, (unsigned long long)(__popc(m0) + __popc(m1)));
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    uint32_t r[16];  // 8 group + 4 w + 2 y (l) and + 1 (l + 1)
+                    asm volatile(
+                        "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
+                        "[%16];"
+                        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+                          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+                          "=r"(r[14]), "=r"(r[15])
+                        : "r"(tmem + ((uint32_t)(32 * q + 16 * x) << 16) + (uint32_t)(kYN * buf + 32 * gi)));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int y = 0; y < 2; ++y)
+#pragma unroll
+                        for (int w2 = 0; w2 < 2; ++w2) {
+                            const int e = 4 * w2 + 2 * y;
+                            const uint32_t o0 = zb ? r[8 + e] : r[e], o1 = zb ? r[9 + e] : r[1 + e];
+                            const uint32_t s0 = zb ? r[e] : r[8 + e], s1 = zb ? r[1 + e] : r[9 + e];
+                            const uint32_t p0 = __shfl_xor_sync(0xffffffffu, s0, 16);
+                            const uint32_t p1 = __shfl_xor_sync(0xffffffffu, s1, 16);
+                            v.c[x][y][0][w2] = f2_pack(__uint_as_float(o0), __uint_as_float(o1));
+                            v.c[x][y][1][w2] = f2_pack(__uint_as_float(p0), __uint_as_float(p1));
+                        }
+                }
+                const float* tl = tabl0 + ll;
+                // per-k entries: the index's last bit is z
+                auto tabk = [&](int e) { return tabk0[(e ^ zb) * kYK]; };
+                if constexpr (!ALL) {
+                    F4Bound4 bd(pack, quart);
+                    t4x_slices<f2>(
+                        v, [&](int e) { return *reinterpret_cast<const f2*>(tl + e * kYL); }, tabk,
+                        [&](int sw, int c, f2 cell) {
+                            // the last slice has read the triples: the next group's are on their way
+                            // while its cells are summed
+                            if (sw == 2 && c == 0) load(gi + 2);
+                            bd.one(cell);
+                        });
+                    float b0, b1;
+                    f2_unpack(bd.acc, b0, b1);
+                    unsigned s0 = __ballot_sync(0xffffffffu, v0 && b0 >= thr_q);
+                    unsigned s1 = __ballot_sync(0xffffffffu, v1 && b1 >= thr_q);
+                    while (s0 | s1) {
+                        const int u = s0 ? 0 : 1, src = __ffs(u ? s1 : s0) - 1;
+                        if (u) s1 &= s1 - 1;
+                        else s0 &= s0 - 1;
+                        const int cmb[4] = {it.i, it.j, __shfl_sync(0xffffffffu, k, src),
+                                            __shfl_sync(0xffffffffu, l, src) + u};
+                        const long long key = warp_exact_key<4>(&w.d, w.base_key, cmb[0], cmb[1], cmb[2], cmb[3]);
+                        if (lane == 0 && key >= thr) t4x_append(w, sink, cmb, key);
+                    }
+                } else {
+#pragma unroll 1
+                    for (int u = 0; u < 2; ++u) {
+                        const bool want = u ? v1 : v0;
+                        auto at1 = [&](f2 a) {
+                            float lo, hi;
+                            f2_unpack(a, lo, hi);
+                            return u ? hi : lo;
+                        };
+                        T4xCores<float> s;
+#pragma unroll
+                        for (int e = 0; e < 16; ++e)
+                            s.c[e >> 3][(e >> 2) & 1][(e >> 1) & 1][e & 1] = at1(v.c[e >> 3][(e >> 2) & 1][(e >> 1) & 1][e & 1]);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            s.ik[e >> 2][(e >> 1) & 1][e & 1] = at1(v.ik[e >> 2][(e >> 1) & 1][e & 1]);
+                            s.jk[e >> 2][(e >> 1) & 1][e & 1] = at1(v.jk[e >> 2][(e >> 1) & 1][e & 1]);
+                        }
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) s.kl[e >> 1][e & 1] = at1(v.kl[e >> 1][e & 1]);
+                        const int cmb[4] = {it.i, it.j, k, l + u};
+                        long long key = w.base_key;
+                        uint32_t* o = nullptr;
+                        if (want) {
+                            // owned prefix ordinal of (i, j, k): rank offset + m * step
+                            if (dump)
+                                o = dump + ((size_t)((triple_index(it.i, it.j, k, n) - w.dist_offset) / w.dist_step) * n +
+                                            cmb[3]) * 162;
+                            const unsigned gt = blockIdx.x * blockDim.x + threadIdx.x;
+                            if (sink.digest && gt < sink.dscratch_threads) o = sink.dscratch + (size_t)gt * 162;
+                            const uint32_t nc = (uint32_t)w.d.n_cases, nt = (uint32_t)w.d.n_ctrls;
+                            t4x_slices<float>(
+                                s, [&](int e) { return tl[e * kYL + u]; }, [&](int e) { return at1(tabk(e)); },
+                                [&](int sw, int c, float cell) {
+                                    const uint32_t cu = __float2uint_rn(cell);
+                                    const uint32_t a = min(cu & wmask, nc), b = min(cu >> pack, nt);
+                                    key += __ldg(w.d.ftab + a) + __ldg(w.d.ftab + b) - __ldg(w.d.ftab + a + b);
+                                    if (o) {
+                                        const int z = c % 3, zt = z < 2 ? z ^ zb : 2;
+                                        o[(c - z + zt) * 3 + sw] = a;
+                                        o[81 + (c - z + zt) * 3 + sw] = b;
+                                    }
+                                });
+                        }
+                        if (sink.digest) dg_warp_add(sink.digest, want && o ? dg_table(cmb, 4, n, o, 81) : 0ull);
+                        if (want && key >= thr) t4x_append(w, sink, cmb, key);
+                    }
+                    load(gi + 2);
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;");
+            __syncwarp();
+            if (lane == 0) {
+                arrive_cl(cluster_addr(smem_u32(&acc_empty[buf]), 0));
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&tab_empty[buf])) : "memory");
+            }
+        }
+    }
+    if (!ok) *abort = 1;
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    // CTA 1: its epilogue has read the last accumulators, so the pair's final
+    // commit to this CTA's `done` lands soon; it must land before the CTA exits
+    if (rank == 1 && warp == 1 && lane == 0 && !t3_drain_cl(smem_u32(&done), 0)) *abort = 1;
+    cluster_sync_all();  // the other CTA is done with this CTA's shared and tensor memory
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    if (tid == 0 && abort_flag) atomicOr(status, 1);
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
+}
+
+cudaError_t f4_order4_maps(F4Plan& f, int snps) {
+    cudaError_t e = tensor_map(&f.map_b4, f.planes, f.rows, 16 * f.wpr, kYRow, kYN / 2, true);
+    if (e == cudaSuccess) e = tensor_map(&f.map_b4h, f.planes, f.rows, 16 * f.wpr, kYRow, 16 * kYHalfG, true);
+    if (e == cudaSuccess) e = f4_bit_map(&f.map_k4, f, f.bits, 2 * snps, 2 * kYK);
+    return e;
+}
+
+cudaError_t launch_tensor4x(const ScanWork& w, const F4Plan& f, const T4xRange& r, long long g0, long long g1,
+                            const CandSink& sink, uint32_t* dump, const uint32_t* single, const uint4* pairs,
+                            int* status, cudaStream_t s, int sms) {
+    if (!f.tri || !pairs || !single || !r.begin || (!r.per && !r.pinfo)) return cudaErrorInvalidValue;
+    using Fn = decltype(&tensor4x_kernel<false, false>);
+    static const Fn fns[4] = {tensor4x_kernel<false, false>, tensor4x_kernel<true, false>, tensor4x_kernel<false, true>,
+                              tensor4x_kernel<true, true>};
+    // set once, by whichever host thread comes first (thread-safe static initialisation)
+    static const cudaError_t attr = [] {
+        cudaError_t e = cudaSuccess;
+        for (Fn fn : fns)
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kYSmem);
+        return e;
+    }();
+    if (attr != cudaSuccess) return attr;
+    if (g1 <= g0) return cudaSuccess;
+    static const int max_clusters = pair_clusters(tensor4x_kernel<false, false>, kYThreads, kYSmem);
+    const long long clusters = std::min<long long>(g1 - g0, max_clusters > 0 ? max_clusters : sms / 2);
+    const unsigned grid = (unsigned)(2 * std::max(1ll, clusters));
+    const double scale = 1.0 / (std::log(2.0) * 4294967296.0);
+    LiveMap map{0, 0, 0, 0};
+    const F4Quartic quart = f4_quartic(w.d.n_cases, w.d.n_ctrls, 81, map.bound_k, map.bound_c);
+    map.bound_k *= scale;
+    const bool all = dump || sink.digest || sink.thr == (long long)0x8000000000000000ull;
+    fns[2 * all + (r.pinfo != nullptr)]<<<grid, kYThreads, kYSmem, s>>>(
+        f.map_b4, f.map_b4h, *r.map_k, f.map_i, w, sink, r.begin, r.per, r.pinfo, r.n_pairs, g0, g1, f.nw_c, f.nw_t, f.pack, map,
+        quart, dump, single, pairs, f.tri, f.pairf, f.row_p, f.row_q, status);
+    count_launch();
+    return cudaGetLastError();
+}
+
+}  // namespace fiu

@@ -41,6 +41,68 @@ __device__ __forceinline__ void f4_mma(uint32_t d, uint64_t a, uint64_t b, uint3
             "l"(a), "l"(b), "r"(idesc), "r"(sfa), "r"(sfb), "r"(acc));
 }
 
+// The MMA issuer of a CTA-pair kernel (one elected thread of CTA 0): for each of
+// `items` items the GEMM of M 256 x n_of(item) columns over the class's 64-sample
+// steps.  A tiles come from a ring of kA stages of 16 KB at a0 (full0), B tiles
+// from a ring of kB stages of kBStage bytes at b0, released by empty0 (kB
+// barriers); accumulator regions of kRegion columns alternate by acc_full0 /
+// acc_empty0.  Returns false after a wait that gave up.  Its own time per stage
+// counts (about 230 cycles alone on an SM quarter, up to twice that beside other
+// warps, against 480 of MMA at N 240), so the loop holds what it must and decodes
+// no items.
+template <int kA, int kB, int kBStage, int kRegion, int kOne, int kW, class NOf>
+__device__ __forceinline__ bool f4_pair_issue(long long items, uint32_t a0, uint32_t b0, uint32_t full0,
+                                              uint32_t empty0, uint32_t acc_full0, uint32_t acc_empty0, uint32_t tmem,
+                                              int nw_c, int nw_t, volatile int* abort, NOf&& n_of) {
+    const uint32_t desc_hi = (uint32_t)(t3_desc(0) >> 32), desc_a = (uint32_t)t3_desc(a0), desc_b = (uint32_t)t3_desc(b0);
+    const uint32_t one = tmem + (uint32_t)kOne;
+    uint32_t fbar = 0, ad = desc_a, par = 0;  // A stage: barrier offset, descriptor, parity
+    uint32_t ebar = 0, bd = desc_b;           // B stage
+    for (unsigned item = 0; item < items; ++item) {
+        const unsigned buf = item & 1;
+        if (item >= 2 && !t3_wait_cl(acc_empty0 + 8 * buf, ((item >> 1) - 1) & 1, abort)) return false;
+        const uint32_t dcol = tmem + (uint32_t)(kRegion * buf);
+        uint32_t acc = 0, idesc = 0;
+        for (int cls = 0; cls < 2; ++cls) {
+            const uint32_t sfb = tmem + (uint32_t)(cls ? kW : kOne);
+            for (int left = cls ? nw_t : nw_c; left > 0; left -= 4) {
+                if (!t3_wait_cl(full0 + fbar, par, abort)) return false;  // both CTAs' A and B are in place
+                asm volatile("tcgen05.fence::after_thread_sync;");
+                if (!acc) idesc = f4_idesc(256, n_of(item));
+                auto mma = [&](int k) {
+                    f4_mma<2>(dcol, (uint64_t)desc_hi << 32 | (ad + 2 * k), (uint64_t)desc_hi << 32 | (bd + 2 * k),
+                              idesc, one, sfb, acc);
+                    acc = 1;
+                };
+                mma(0);
+                if (left >= 4) {
+                    mma(1);
+                    mma(2);
+                    mma(3);
+                } else {  // the class's last steps
+                    for (int k = 1; k < left; ++k) mma(k);
+                }
+                commit_pair(empty0 + ebar);
+                fbar += 8;
+                ad += 16384 >> 4;
+                if (fbar == 8 * kA) {
+                    fbar = 0;
+                    ad = desc_a;
+                    par ^= 1;
+                }
+                ebar += 8;
+                bd += kBStage >> 4;
+                if (ebar == 8 * kB) {
+                    ebar = 0;
+                    bd = desc_b;
+                }
+            }
+        }
+        commit_pair(acc_full0 + 8 * buf);
+    }
+    return true;
+}
+
 // Fills this warp's 32 tensor-memory lanes of both scale regions, `cols` (a
 // multiple of 8) columns each: 8 hold the scales of 256 rows.  Every lane
 // quarter has to be filled by one warp whose index is the quarter mod 4.
@@ -172,20 +234,73 @@ struct F4Bound {
     }
 };
 
-// The bound's constants for a threshold (host): a combination can only reach
-// thr_bits (N MI in bits) when sum b^2 / s >= the returned value.  Slack: each
-// of `cells` terms, at most b <= n_ctrls, carries at most 12 roundings or
-// approximations of 2^-22 and the sum `cells` more of 2^-24 of the total
-// n_ctrls; the 2^-20 shift lowers a term by at most 2^-20 of it.  Doubled.
-inline float f4_bound_threshold(double thr_bits, int n_cases, int n_ctrls, int cells) {
+// A closer bound, for tables of many cells (order 4, where the quadratic one
+// leaves a third of the warps a survivor).  g(p) = D(p||q) / (p-q)^2 is an
+// average of D''(q + u (p-q)) = 1 / (ln2 t (1-t)) over u, which is convex, so g
+// is convex in p and lies below its chord L(p) = g(0) + (g(1) - g(0)) p.  It lies
+// below Q(p) = L(p) - k p (1-p) as well, k the least (L - g) / (p (1-p)) (which
+// grows without limit towards both ends).  So D <= (p-q)^2 Q(p), exact at p = 0,
+// p = 1 and where k is taken.  Summed over the cells with p = b/s the powers
+// below the second give constants:
+//     N MI <= a0 N + a1 n_ctrls + sum b p (a2 + a3 p + a4 p^2).
+struct F4Quartic {
+    float a2, a3, a4;
+};
+struct F4Bound4 : F4Bound {
+    f2 a2, a3, a4;
+    __device__ __forceinline__ F4Bound4(int p, const F4Quartic& k) : F4Bound(p) {
+        a2 = f2_dup(k.a2);
+        a3 = f2_dup(k.a3);
+        a4 = f2_dup(k.a4);
+    }
+    __device__ __forceinline__ void one(f2 D) {
+        f2 b, s;
+        split(D, b, s);
+        const f2 pr = f2_mul(b, f2_rcp(s));
+        acc = f2_fma(f2_mul(b, pr), f2_fma(pr, f2_fma(pr, a4, a3), a2), acc);
+    }
+};
+// The quartic bound's coefficients and test (as f4_quadratic).
+// Slack: a term of magnitude at most b (|a2| + |a3| + |a4|) carries at most 12
+// roundings of 2^-24, the sum `cells` more; doubled.
+inline F4Quartic f4_quartic(int n_cases, int n_ctrls, int cells, double& bound_k, double& bound_c) {
+    const double N = (double)n_cases + n_ctrls, q = n_ctrls / N, r = 1 - q, l2 = std::log(2.0);
+    const double L0 = -std::log2(r) / (q * q), L1 = -std::log2(q) / (r * r);
+    double k = 1e300;  // the least on a grid, lowered by 0.1 %: between grid points the ratio moves less
+    for (int i = 1; i < 1024; ++i) {
+        const double p = i / 1024.0, d = p - q;
+        const double g = std::fabs(d) < 1e-4 ? 1 / (2 * l2 * q * r)
+                                             : (p * std::log2(p / q) + (1 - p) * std::log2((1 - p) / r)) / (d * d);
+        k = std::min(k, (L0 + (L1 - L0) * p - g) / (p * (1 - p)));
+    }
+    k = std::max(0.0, k * 0.999 - 1e-4);
+    const double A = L0, B = L1 - L0 - k, C = k;
+    const double a4 = C, a3 = B - 2 * q * C, a2 = A - 2 * q * B + q * q * C, a1 = q * q * B - 2 * q * A, a0 = q * q * A;
+    const double S = std::fabs(a2) + std::fabs(a3) + std::fabs(a4), u = std::ldexp(1.0, -24);
+    const double slack = 2 * n_ctrls * S * (12 + 3 + cells) * u + 1e-3;  // 3: the coefficients' own rounding
+    bound_k = 1 - 1e-9;
+    bound_c = -a0 * N - a1 * n_ctrls - slack;
+    return F4Quartic{(float)a2, (float)a3, (float)a4};
+}
+
+// The quadratic bound's test (host): a combination whose N MI reaches thr_bits has
+// sum b^2 / s >= bound_k * thr_bits + bound_c.  Slack: each of `cells` terms, at
+// most b <= n_ctrls, carries at most 12 roundings or approximations of 2^-22 and
+// the sum `cells` more of 2^-24 of the total n_ctrls; the 2^-20 shift lowers a term
+// by at most 2^-20 of it.  Doubled.
+inline void f4_quadratic(int n_cases, int n_ctrls, int cells, double& bound_k, double& bound_c) {
     const double N = (double)n_cases + n_ctrls, q = n_ctrls / N;
-    if (n_cases < 1 || n_ctrls < 1) return -3.0e38f;
     const double lg_q = std::log2(q), lg_1q = std::log2(1 - q);
     const double c = std::max({1 / (2 * std::log(2.0) * q * (1 - q)), -lg_1q / (q * q), -lg_q / ((1 - q) * (1 - q))});
     const double u = std::ldexp(1.0, -24);
-    const double slack = 2 * n_ctrls * (12 * 4 * u + 16 * u + cells * u) + 1e-3;
-    const double t = thr_bits / c * (1 - 1e-9) + q * n_ctrls - slack;
-    return (float)std::max(-3.0e38, std::min(3.0e38, t < 0 ? t * (1 + 1e-6) : t * (1 - 1e-7)));
+    bound_k = (1 - 1e-9) / c;
+    bound_c = q * n_ctrls * (1 - 1e-9) - (2 * n_ctrls * (12 * 4 * u + 16 * u + cells * u) + 1e-3);
+}
+
+// A threshold key as the kernels' tests, rounded down (device).
+__device__ __forceinline__ void live_tests(const LiveMap& m, long long thr, float& est, float& bound) {
+    est = __double2float_rd(fma((double)thr, m.est_k, m.est_c));
+    bound = __double2float_rd(fma((double)thr, m.bound_k, m.bound_c));
 }
 
 }  // namespace fiu

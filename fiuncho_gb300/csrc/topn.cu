@@ -5,6 +5,7 @@
 // ThreadedSearch::run (include/fiuncho/ThreadedSearch.h:241-245).  Here the
 // order is total -- value descending, then combination ascending -- so results
 // do not depend on how the work was split.
+#include "live.cuh"
 #include "topn_dev.cuh"
 
 namespace fiu {
@@ -128,6 +129,35 @@ cudaError_t select_top(Cand* buf, unsigned M, unsigned keep, Cand* tmp, unsigned
     if ((e = sort_small<Cand, CandBetter>(sure, total, worst, s)) != cudaSuccess) return e;
     return cudaMemcpyAsync(buf, sure, (size_t)(total < keep ? total : keep) * sizeof(Cand), cudaMemcpyDeviceToDevice,
                            s);
+}
+
+// ---- live threshold -----------------------------------------------------------
+__global__ void live_raise_kernel(CandSink sink) { live_update(sink, threadIdx.x); }
+
+__global__ void live_compact_kernel(CandSink sink, Cand* __restrict__ out, unsigned* out_count) {
+    __shared__ long long thr;
+    if (threadIdx.x < 32) {
+        const long long t = live_scan(sink.hist, sink.keep, threadIdx.x);
+        if (threadIdx.x == 0) thr = max(t, *sink.live);
+    }
+    __syncthreads();
+    const unsigned m = min(*sink.count, sink.cap);
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
+        const Cand c = sink.buf[i];
+        if (c.key >= thr) out[atomicAdd(out_count, 1u)] = c;
+    }
+}
+
+cudaError_t live_raise(const CandSink& sink, cudaStream_t s) {
+    live_raise_kernel<<<1, 32, 0, s>>>(sink);
+    count_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t live_compact(const CandSink& sink, Cand* out, unsigned* out_count, cudaStream_t s) {
+    live_compact_kernel<<<64, 256, 0, s>>>(sink, out, out_count);
+    count_launch();
+    return cudaGetLastError();
 }
 
 __global__ void rescore_kernel(DevData d, int K, int bits, const Cand* __restrict__ cands, unsigned n,

@@ -1,7 +1,8 @@
 """Tensor-core kernels at the edges of their tiles: every contingency table of a scan, as the kernel
 that serves it computes them, against the oracle's (64-bit digests of all tables), and the top-N
 against the full-table kernel's.  Sizes sit on and beside the tile edges of the kernels: 8 SNPs (column
-groups), 64 and 120 SNPs (tiles), 64 and 256 samples (steps and stages of a class)."""
+groups), 16, 32 and 64 SNPs (rows of a tile), 112 and 120 SNPs (columns), 64 and 256 samples (steps and
+stages of a class)."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -46,3 +47,52 @@ def test_order3_tile_edges(oracle, snps, cases, ctrls):
 def test_order3_layer_edges(oracle, snps, step, offset):
     from fiuncho_gb300 import Distribution
     _check(3, snps, 130, 199, oracle, Distribution(snps, 2, step, offset))
+
+
+EDGES_4 = [  # snps, cases, controls
+    (4, 1, 1), (5, 64, 65), (9, 63, 256), (17, 257, 129), (33, 65, 300), (34, 1023, 40), (36, 50, 4000),
+    (47, 2047, 2049),
+]
+
+
+@pytest.mark.parametrize("snps,cases,ctrls", EDGES_4)
+def test_order4_tile_edges(oracle, snps, cases, ctrls):
+    _check(4, snps, cases, ctrls, oracle)
+
+
+@pytest.mark.parametrize("snps,step,offset", [(20, 2, 1), (37, 3, 0), (18, 19, 5), (40, 5, 4)])
+def test_order4_layer_edges(oracle, snps, step, offset):
+    from fiuncho_gb300 import Distribution
+    _check(4, snps, 130, 199, oracle, Distribution(snps, 3, step, offset))
+
+
+@pytest.mark.parametrize("snps,order", [(130, 4), (260, 3)])
+def test_wide_tiles_against_the_reduced_work_kernel(snps, order):
+    """Full column tiles (112 and 120 SNPs): digests of two kernels that share no code path."""
+    from fiuncho_gb300 import GpuSearch, _lib
+    from fiuncho_gb300.search import Resident
+    gs = GpuSearch(0)
+    res = Resident(gs.ctx, _data(snps, 150, 201, 7 + snps))
+    assert gs.scan_digest(res, order, kernel=_lib.KERNEL_TENSOR) == \
+        gs.scan_digest(res, order, kernel=_lib.KERNEL_ELIDED_POPC)
+
+
+@pytest.mark.parametrize("order,snps,outputs", [(3, 150, 1), (3, 150, 7000), (3, 40, 7000), (4, 60, 3), (4, 60, 7000),
+                                                (4, 20, 7000)])
+def test_threshold_raised_in_the_kernel_keeps_the_list(order, snps, outputs):
+    """The list does not depend on when the device raises the threshold: few and many outputs, more
+    outputs than combinations, against the full-table kernel's chunked search; shards merged too."""
+    from fiuncho_gb300 import Distribution, GpuSearch, _lib
+    from fiuncho_gb300.search import Resident
+    gs = GpuSearch(0)
+    res = Resident(gs.ctx, _data(snps, 311, 290, 40 + snps))
+    gs.set_kernel(_lib.KERNEL_TENSOR)
+    d = Distribution(snps, order - 1)
+    a = gs.run(res, order, d, outputs)
+    parts = [r for s in range(3) for r in gs.run_shard(res, order, s, 3, outputs)]
+    gs.set_kernel(_lib.KERNEL_FULL)
+    b = gs.run(res, order, d, outputs)
+    assert [(r.combination, r.val) for r in a] == [(r.combination, r.val) for r in b]
+    if outputs < 100:
+        parts.sort(key=lambda r: (-r.val, r.combination))
+        assert [r.val for r in parts[:outputs]] == [r.val for r in b]
