@@ -236,12 +236,7 @@ int choose_tile(fiu_ctx* ctx, const fiu_resident* res, const ScanWork& w, int re
         if (!r->t3) {
             auto* plan = new (std::nothrow) T3Plan;
             if (!plan) return fail(ctx, FIU_ERR_NOMEM, "tensor plan");
-            cudaError_t e = tensor3_prepare(r->d, *plan, ctx->stream);
-            if (e != cudaSuccess) {
-                tensor3_release(*plan);
-                delete plan;
-                return cuda_fail(ctx, e, "tensor work items");
-            }
+            tensor3_prepare(r->d, *plan);
             r->t3 = plan;
         }
         // the core tables; the order-4 pair kernel makes its triples itself
@@ -324,6 +319,13 @@ int choose_tile(fiu_ctx* ctx, const fiu_resident* res, const ScanWork& w, int re
     return FIU_OK;
 }
 
+// A chunk's length on a context whose searches can be cancelled (the server's solo lanes).  The lanes'
+// kernels fill the GPU one at a time, and another scan's upload gets its small kernels in only between
+// them: at a quarter second a 28 ms search ran whole before anything else moved; at 2 to 4 ms two such
+// searches side by side still take 58 ms, and four scans submitted meanwhile are admitted in time to be
+// taken smallest first.
+constexpr double kLaneChunkSeconds = 0.003;
+
 // The search on a resident data set (ThreadedSearch::run semantics).
 int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu_distribution* dist,
                 unsigned outputs, int32_t* out_comb, float* out_vals, double* out_vals64, unsigned* out_count,
@@ -351,7 +353,7 @@ int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu
     const unsigned keep = outputs + std::max(32u, outputs / 8);
     const bool live = tensor && tensor_live(*res->t3, w);
     const size_t cap = std::max<size_t>(
-        {live ? 262144u : 65536u, (size_t)(live ? 64 : 16) * keep, (size_t)res->d.snps + keep});
+        {live ? 524288u : 65536u, (size_t)(live ? 128 : 16) * keep, (size_t)res->d.snps + keep});
     if ((rc = grow(ctx, ctx->cand, ctx->cand_cap, cap + 8192)) ||
         (rc = grow(ctx, ctx->tmp, ctx->tmp_cap, cap + 8192)) ||
         (rc = grow(ctx, ctx->mi64, ctx->mi64_cap, (size_t)keep)))
@@ -375,15 +377,17 @@ int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu
     // candidate buffer under that estimate (a chunk that overflows all the
     // same is re-run in smaller pieces), so a scan takes a few launches and
     // the same launches on every run.  On a context whose searches can be
-    // cancelled a chunk also stays under about a quarter second (measured per
-    // unit on the previous chunk), so that a cancellation takes effect soon.
+    // cancelled a chunk also stays near kLaneChunkSeconds (measured per unit on
+    // the previous chunk), so that a cancellation takes effect soon.
     long long chunk = std::max<long long>(1, (long long)(keep / std::max(1.0, per_unit)));
     double seen = 0, sec_per_unit = 0;
     long long m = units / n_shards * shard + std::min<long long>(shard, units % n_shards);
     const long long m_end = m + units / n_shards + (shard < units % n_shards ? 1 : 0);
-    // With a live threshold (the kernel raises it as candidates come) two launches cover the request
+    // With a live threshold (the kernel raises it as candidates come) a few launches cover the request
     // and the host waits once: the first takes enough units for a threshold to start from, and no
-    // more than a quarter of the candidate buffer holds, since every combination of it is one.  A
+    // more than a quarter of the candidate buffer holds, since every combination of it is one; in a
+    // large request the second is one unit per CTA pair (the first units may hold few combinations:
+    // the order-2 tiles on the diagonal), so that no launch starts all pairs on a weak threshold.  A
     // buffer that overflows all the same leaves the request to the loop below.
     if (live && !ctx->cancellable && m < m_end) {
         const long long few = std::max<long long>(1, (long long)(2.0 * keep / std::max(1.0, per_unit)));
@@ -401,12 +405,15 @@ int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu
         CK(launch_tensor3(w, *res->t3, m, m1, sink, nullptr, res->single, res->pairs, res->triples, t_status, s,
                           ctx->sms),
            "tensor kernel launch");
-        if (m1 < m_end) {
+        unsigned launches = 1;
+        sink.thr = 0;  // (from here on the kernel reads the live threshold; one exists)
+        for (long long a = m1; a < m_end; ++launches) {
+            const long long wave = ctx->sms / 2, b = launches == 1 && m_end - a > 16 * wave ? a + wave : m_end;
             CK(live_raise(sink, s), "threshold");
-            sink.thr = 0;  // (the kernel reads the live threshold; a threshold exists)
-            CK(launch_tensor3(w, *res->t3, m1, m_end, sink, nullptr, res->single, res->pairs, res->triples, t_status,
-                              s, ctx->sms),
+            CK(launch_tensor3(w, *res->t3, a, b, sink, nullptr, res->single, res->pairs, res->triples, t_status, s,
+                              ctx->sms),
                "tensor kernel launch");
+            a = b;
         }
         if (ctx->timing) CK(cudaEventRecord(ctx->ev1, s), "event");
         unsigned* kept = scratch;  // [0]: candidates at or above the last threshold
@@ -418,7 +425,7 @@ int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu
             float ms = 0;
             CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1), "event time");
             ctx->count_ms += ms;
-            ctx->count_launches += m1 < m_end ? 2 : 1;
+            ctx->count_launches += launches;
         }
         if (!ctx->pinned[1]) {
             std::swap(ctx->cand, ctx->tmp);
@@ -488,7 +495,7 @@ int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu
         m = m1;
         const double next = have < keep ? (double)(cap - have) / (4.0 * std::max(1.0, per_unit))
                                         : (double)cap / 4.0 * seen / ((double)keep * std::max(1.0, per_unit));
-        const double time_cap = ctx->cancellable ? 0.25 / std::max(sec_per_unit, 1e-12) : 4.0e18;
+        const double time_cap = ctx->cancellable ? kLaneChunkSeconds / std::max(sec_per_unit, 1e-12) : 4.0e18;
         chunk = (long long)std::max(1.0, std::min({next, time_cap, 4.0e18}));
     }
     if (tensor) {

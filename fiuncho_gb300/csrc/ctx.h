@@ -47,8 +47,8 @@ struct fiu_ctx {
     // its current chunk (FIU_ERR_CANCELLED)
     std::atomic<int> cancel{0};
     // searches on this context may be cancelled (the server's solo lanes):
-    // their chunks are also kept under about a quarter second, so a cancel
-    // takes effect soon.  Elsewhere the chunk schedule depends on the data only.
+    // their chunks are also kept to a few milliseconds, so a cancel
+    // takes effect soon and the lanes take turns.  Elsewhere the schedule depends on the data only.
     bool cancellable = false;
 };
 

@@ -178,11 +178,10 @@ cudaError_t launch_elided4p(const ScanWork& w, const long long* begin, long long
                             const CandSink& sink, uint32_t* dump, const uint32_t* single, const uint4* pairs,
                             const uint4* triples, cudaStream_t s, int sms);
 
-// tensor3.cu -- order-2 and order-3 core cells on tcgen05 (one-hot data, whole data set, one worker).
-// Device state of the tensor kernel for one data set: the e4m3 operand planes
-// (row 2*snp+g = "genotype of snp == g" per sample, cases then controls, each
-// class padded to a multiple of 128 samples), their TMA descriptors and the
-// work-item prefix sums.
+// tensor2x.cu, tensor3x.cu, tensor4x.cu (4-bit operands, CTA pairs) and tensor3.cu, tensor4.cu (per-class
+// e4m3 kernels of orders 3 and 4) -- core cells on tcgen05 (one-hot data, the whole data set or a layer of it).
+// Device state of the tensor kernels for one data set: operand planes, made on the first search of an
+// order, their TMA descriptors and the work-item prefix sums.
 // 4-bit operand layout of a data set (tensor_fp4.cuh, tensor3x.cu): e2m1 planes
 // for the operand that the MMA reads as it is, bit rows for the one its kernel
 // builds.
@@ -194,6 +193,8 @@ struct F4Plan {
     int nw_c = 0, nw_t = 0;     // 64-sample steps that hold samples, per class
     CUtensorMap map_b;          // planes, box 128 B x 120 rows, 128-byte swizzle
     CUtensorMap map_j, map_i;   // bit rows, boxes of 32 B x 64 and x 2 rows
+    uint8_t* ones = nullptr;    // order 2: planes of 1.0 where a genotype is, both operands
+    CUtensorMap map_a2, map_b2; // over them, boxes 128 B x 128 and x 120 rows
     // order 4: the cores of all triples and pairs as packed floats, cases + W controls, of (l, l + 1)
     // side by side; the entry of (.., k, l) is row_p[k] + l / 2, of (i, k, l) also + row_q[i]
     float* tri = nullptr;       // 16 floats an entry: (x, z, w) of the genotypes of i, k and l
@@ -205,8 +206,7 @@ struct T3Plan {
     std::mutex items_mu;  // guards the planes and item tables made on the first use of an order
     F4Plan f4;
     uint8_t* planes = nullptr;
-    int pack = 0;         // log2 of the control weight W when one accumulator holds both classes (else 0)
-    double item_combos = 0;  // combinations per work item, about 32 x L / 2
+    double item_combos = 0;  // combinations per work item
     int pitch = 0;        // bytes per plane row
     int k_cases = 0;      // padded case samples (= byte offset of the control region)
     bool pair3 = false;   // orders 3 and 4, classes that share an accumulator: items of the CTA-pair kernels
@@ -216,26 +216,20 @@ struct T3Plan {
     CUtensorMap map_l;    // box 128 B x 192 rows, 128-byte swizzle (l operand)
     CUtensorMap map_j;    // box 128 B x 64 rows, 128-byte swizzle (j rows of the (i,j) operand)
     CUtensorMap map_i;    // box 128 B x 2 rows, 128-byte swizzle (i rows)
-    // order 2: work items (64 i, 128 j) over i-tiles, or pair items (2 x 64 i, 128 j) of the
-    // CTA-pair kernel (pair2)
-    bool pair2 = false;
+    // order 2: work items (128 i, 120 j) of the pair kernel, first of each band
     long long* item2_begin = nullptr;
     long long total2 = 0;
     int n_itiles = 0;
     double item2_combos = 0;
-    CUtensorMap map_a2;   // box 128 B x 128 rows (i rows)
-    CUtensorMap map_b2;   // box 128 B x 256 rows (j rows)
     // order 4: work items (i, j, 32 k, up to 112 l) of the pair kernel, or (i, j, 16 k, 64 l) per class;
     // item4_begin[j] = first item of the pairs with second SNP j, item4_per[j] = items per such pair
     long long* item4_begin = nullptr;
     long long* item4_per = nullptr;
     long long total4 = 0;
     double item4_combos = 0;
+    CUtensorMap map_l4;   // box 128 B x 128 rows (l rows)
     CUtensorMap map_k4;   // box 128 B x 32 rows (k rows)
 };
-// log2 of the control weight W = 4^h when both classes fit one FP32 accumulator
-// (n_cases < W, n_cases + W * n_ctrls < 2^24), else 0.
-int tensor_pack(int n_cases, int n_ctrls);
 // Work units of a request on the tensor kernels (w's order and Distribution
 // layer; a layer's items must have been made by tensor3_layer), and the
 // combinations of an average unit.
@@ -249,7 +243,7 @@ bool tensor_live(const T3Plan& plan, const ScanWork& w);
 // planes ordered by SNP residue mod the layer's step, copied on stream s).
 bool tensor_layer_ok(const T3Plan& plan, const ScanWork& w);
 cudaError_t tensor3_layer(T3Plan& plan, const ScanWork& w, const uint4* pairs, cudaStream_t s, int sms);
-cudaError_t tensor3_prepare(const DevData& d, T3Plan& plan, cudaStream_t s);
+void tensor3_prepare(const DevData& d, T3Plan& plan);
 // The operand planes that searches of an order read and the whole data set's
 // work items at order 3 or 4, made on first use (thread-safe).
 cudaError_t tensor3_order_items(T3Plan& plan, const DevData& d, int order, const uint4* pairs, cudaStream_t s,

@@ -54,4 +54,15 @@ __device__ __forceinline__ void live_update(const CandSink& sink, int lane) {
     if (lane == 0 && thr > *(volatile long long*)sink.live) atomicMax(sink.live, thr);
 }
 
+// One lane's candidate: into the buffer and the histogram.
+__device__ __forceinline__ void live_append(const CandSink& sink, long long key, unsigned long long code) {
+    const unsigned idx = atomicAdd(sink.count, 1u);
+    if (idx < sink.cap) {
+        sink.buf[idx] = Cand{key, code};
+        if (sink.hist) atomicAdd(sink.hist + live_bin(key), 1u);
+    } else {
+        atomicOr(sink.overflow, 1u);
+    }
+}
+
 }  // namespace fiu

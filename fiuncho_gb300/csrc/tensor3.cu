@@ -57,8 +57,8 @@
 #include <mutex>
 
 #include "tensor3_eval.cuh"
+#include "tensor2x.h"
 #include "tensor3x.h"
-#include "tensor_fp4.cuh"
 
 namespace fiu {
 
@@ -473,711 +473,8 @@ __global__ void __launch_bounds__(kT3Threads, 1)
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
 }
 
-// ---------------------------------------------------------------------------
-// Order 2.  The 4 core cells of a pair (i, j) are plain dot products of two
-// plane rows, core[x][y] = sum_s a_ix(s) a_jy(s): a work item (64 i, 128 j)
-// is one GEMM D[(i,x), (j,y)] (M 128 x N 256) with both operands straight
-// from the operand planes by TMA -- no producer warps.  Both classes in one
-// accumulator when they pack (two alternating tensor-memory regions), else
-// cases in columns 0-255 and controls in 256-511 (the MMA then waits for the
-// epilogue between items).  4 stages of 48 KB; 8 epilogue warps.
-// Reference semantics: GenotypeTable::combine_and_popcnt for order 2
-// (src/base/gt_popcnt.cpp:4-35) over the pairs ThreadedSearch visits
-// (include/fiuncho/ThreadedSearch.h:157-180) with one worker.
-constexpr int kT2I = 64, kT2L = 128;                     // SNPs per tile
-constexpr int kT2M = 2 * kT2I, kT2N = 2 * kT2L;          // 128 x 256
-constexpr int kT2Stages = 4;
-constexpr int kT2SA = kT2M * kT3KB, kT2SB = kT2N * kT3KB;  // 16 KB, 32 KB
-constexpr int kT2Stage = kT2SA + kT2SB;                    // 48 KB
-constexpr int kT2Threads = 32 * (2 + kT3EpiWarps);         // 320
-constexpr size_t kT2Smem = 1024 + (size_t)kT2Stages * kT2Stage + (size_t)kT3EpiWarps * kT3Ebuf;
-constexpr uint32_t kT2Idesc = (1u << 4) | ((uint32_t)(kT2N >> 3) << 17) | ((uint32_t)(kT2M >> 4) << 24);
-static_assert(kT2Smem <= 227 * 1024 - 256, "order-2 tensor kernel shared memory");
-
-// Work items.  i-tiles a (i0 = 64 a) are grouped in bands of kT2Band; j-tiles
-// are global (j0 = 128 b).  Band r covers i-tiles [8 r, 8 r + 8) and j-tiles
-// b >= 4 r (the first j-tile holding a j > i of the band) and lists its items
-// j-tile by j-tile, i-tile fastest: the CTAs working at the same time share
-// a band's eight A tiles and each B tile, so the operands stream from HBM
-// about once per band instead of once per item (items left of the diagonal
-// are masked in the epilogue).  item_begin[r] = first item of band r.
-constexpr int kT2Band = 8;
-__device__ __forceinline__ void t2_decode(const long long* __restrict__ item_begin, int n_itiles, long long g, int& i0,
-                                          int& j0) {
-    const int n_bands = (n_itiles + kT2Band - 1) / kT2Band;
-    int lo = 0, hi = n_bands - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (item_begin[mid] <= g) lo = mid;
-        else hi = mid - 1;
-    }
-    const int ca = min(kT2Band, n_itiles - kT2Band * lo);  // i-tiles in the band
-    const long long idx = g - item_begin[lo];
-    const int b = kT2Band * kT2I / kT2L * lo + (int)(idx / ca);
-    i0 = kT2I * (kT2Band * lo + (int)(idx % ca));
-    j0 = kT2L * b;
-}
-
-// 8-byte slot of the order-2 transpose buffer holding (cases y0 | y1 << 16,
-// controls y0 | y1 << 16) of row (ii, x) and column group k; each half-warp
-// covers the 32 banks once for the row-wise writes (lanes (ii, x), fixed k)
-// and the pair-wise reads (lanes (ii, kh), fixed x, k = 4 kh + kk).
-__device__ __forceinline__ int t2_slot(int ii, int k, int x) {
-    return ((((ii >> 3) * 4 + (k & 3)) * 2 + (k >> 2)) * 16) + (((ii & 7) << 1) | (x ^ (k >> 2)));
-}
-
-// Distribution layers of order-2 scans: the owned prefixes are the SNPs
-// i = offset + step m, consecutive rows m of the operand planes ordered by
-// residue mod step (from row residue_row(offset)).  A layer tile is IT
-// consecutive owned i (positions p0 = IT a ..); tiles are grouped in bands of
-// BT (512 owned i), and a band lists its items j-tile by j-tile, tile fastest,
-// from the j-tile holding the band's first i + 1 (as the whole scan's bands:
-// the CTAs at work share a band's A tiles and each B tile in L2).
-// item_begin[r] = first item of band r.
-template <int IT, int BT>
-__device__ __forceinline__ void t2l_decode(const long long* __restrict__ item_begin, int n_tiles, const ScanWork& w,
-                                           long long g, int& p0, int& j0) {
-    const int n_bands = (n_tiles + BT - 1) / BT;
-    int lo = 0, hi = n_bands - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (item_begin[mid] <= g) lo = mid;
-        else hi = mid - 1;
-    }
-    const int ca = min(BT, n_tiles - BT * lo);  // tiles in the band
-    const long long idx = g - item_begin[lo];
-    const int i_first = w.dist_offset + w.dist_step * (IT * BT * lo);
-    p0 = IT * (BT * lo + (int)(idx % ca));
-    j0 = kT2L * ((i_first + 1) / kT2L + (int)(idx / ca));
-}
-
-// Evaluates pair (i, j) from its transpose chunks: exact 9-cell tables from the
-// cores and the single cores, the bounded single-precision prefilter, the exact
-// fixed-point key for survivors, warp-aggregated append (every lane calls it).
-__device__ __forceinline__ void t2_eval(const ScanWork& w, const CandSink& sink, float thr_f, uint32_t* dump,
-                                        const uint4& sjp, const uint32_t* ebuf, int ii, int k, int i, int j,
-                                        bool i_ok, const float (&si)[2][2], int lane) {
-    const DevData& d = w.d;
-    const int n = d.snps;
-    const uint32_t ncls[2] = {(uint32_t)d.n_cases, (uint32_t)d.n_ctrls};
-    const float ncf[2] = {(float)d.n_cases, (float)d.n_ctrls};
-    const float tiny = 9.5367431640625e-07f;  // 2^-20: x*lg2(x + tiny) = 0 at x = 0
-    const bool valid = i_ok && j < n && j > i;
-    float t[2][9];
-#pragma unroll
-    for (int x = 0; x < 2; ++x) {
-        const uint2 c2 = *reinterpret_cast<const uint2*>(ebuf + 2 * t2_slot(ii, k, x));
-        t[0][x * 3 + 0] = u2f(c2.x & 0xffffu);
-        t[0][x * 3 + 1] = u2f(c2.x >> 16);
-        t[1][x * 3 + 0] = u2f(c2.y & 0xffffu);
-        t[1][x * 3 + 1] = u2f(c2.y >> 16);
-    }
-    // single cores of j = jg + k, loaded by lane k of the warp for the column group
-    uint4 sj4;
-    sj4.x = __shfl_sync(0xffffffffu, sjp.x, k);
-    sj4.y = __shfl_sync(0xffffffffu, sjp.y, k);
-    sj4.z = __shfl_sync(0xffffffffu, sjp.z, k);
-    sj4.w = __shfl_sync(0xffffffffu, sjp.w, k);
-    const float sj[2][2] = {{u2f(sj4.x), u2f(sj4.y)}, {u2f(sj4.z), u2f(sj4.w)}};
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-#pragma unroll
-        for (int x = 0; x < 2; ++x) t[c][x * 3 + 2] = si[c][x] - t[c][x * 3] - t[c][x * 3 + 1];
-#pragma unroll
-        for (int y = 0; y < 2; ++y) t[c][6 + y] = sj[c][y] - t[c][y] - t[c][3 + y];
-        t[c][8] = ncf[c] - si[c][0] - si[c][1] - t[c][6] - t[c][7];
-    }
-    float kf = 0.f;
-#pragma unroll
-    for (int c = 0; c < 9; ++c) {
-        const float a = t[0][c], bb = t[1][c], s = a + bb;
-        kf = fmaf(a, t3_lg2(a + tiny), kf);
-        kf = fmaf(bb, t3_lg2(bb + tiny), kf);
-        kf = fmaf(-s, t3_lg2(s + tiny), kf);
-    }
-    const bool cand = valid && (dump != nullptr || sink.digest != nullptr || kf >= thr_f);
-    long long key = w.base_key;
-    bool pass = false;
-    unsigned long long dg = 0;
-    if (cand) {
-#pragma unroll
-        for (int c = 0; c < 9; ++c) {
-            const uint32_t a = min(f2u(fmaxf(t[0][c], 0.f)), ncls[0]);
-            const uint32_t bb = min(f2u(fmaxf(t[1][c], 0.f)), ncls[1]);
-            key += __ldg(d.ftab + a) + __ldg(d.ftab + bb) - __ldg(d.ftab + a + bb);
-        }
-        pass = key >= sink.thr;
-        if (dump) {
-            // owned prefix ordinal m of i: rank offset + m * step
-            uint32_t* o = dump + ((size_t)((i - w.dist_offset) / w.dist_step) * n + j) * 18;
-#pragma unroll
-            for (int c = 0; c < 9; ++c) {
-                o[c] = f2u(t[0][c]);
-                o[9 + c] = f2u(t[1][c]);
-            }
-        }
-        if (sink.digest) {
-            const int cmb[2] = {i, j};
-            dg = dg_begin(cmb, 2, n);
-#pragma unroll
-            for (int c = 0; c < 9; ++c) dg = dg_cell(dg, f2u(t[0][c]), f2u(t[1][c]));
-        }
-    }
-    if (sink.digest) dg_warp_add(sink.digest, dg);
-    if (sink.evaluated) {
-        const unsigned vmask = __ballot_sync(0xffffffffu, valid);
-        if (lane == 0 && vmask) atomicAdd(sink.evaluated, (unsigned long long)__popc(vmask));
-    }
-    const unsigned mask = __ballot_sync(0xffffffffu, pass);
-    if (mask) {
-        const int leader = __ffs(mask) - 1;
-        unsigned base = 0;
-        if (lane == leader) base = atomicAdd(sink.count, (unsigned)__popc(mask));
-        base = __shfl_sync(0xffffffffu, base, leader);
-        if (pass) {
-            const unsigned idx = base + __popc(mask & ((1u << lane) - 1u));
-            if (idx < sink.cap) {
-                const int cmb[2] = {i, j};
-                sink.buf[idx] = Cand{key, pack_code(cmb, 2, w.bits)};
-            } else {
-                atomicOr(sink.overflow, 1u);
-            }
-        }
-    }
-}
-
-struct T2Maps {
-    CUtensorMap a, b;
-};
-
-// LAYER: a Distribution layer (t2l_decode; maps.a covers the residue-ordered
-// planes, item_begin / n_itiles are the layer's tiles).
-template <bool LAYER>
-__global__ void __launch_bounds__(kT2Threads, 1)
-    tensor2_kernel(const __grid_constant__ T2Maps maps, ScanWork w, const long long* __restrict__ item_begin,
-                   int n_itiles, long long g0, long long g1, int k_cases, int pack, CandSink sink, float thr_f,
-                   uint32_t* dump, const uint32_t* __restrict__ single, int* status) {
-    extern __shared__ uint8_t smraw[];
-    __shared__ __align__(8) uint64_t full[kT2Stages], empty[kT2Stages];
-    __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2], done;
-    __shared__ uint32_t tmem_base;
-    __shared__ int abort_flag;
-    uint8_t* sm = (uint8_t*)(((uintptr_t)smraw + 1023) & ~(uintptr_t)1023);  // stages: A | B
-    uint32_t* ebuf_all = reinterpret_cast<uint32_t*>(sm + kT2Stages * kT2Stage);
-    volatile int* abort = &abort_flag;
-    const DevData& d = w.d;
-    const int n = d.snps;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int ks_c = k_cases / kT3KB;
-    const int ksteps = ks_c + (d.tw + 1) / 2;
-    const int nbuf = pack ? 2 : 1;  // accumulator regions that alternate between items
-
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
-                     "r"(512));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-    }
-    if (tid == 0) {
-        for (int s = 0; s < kT2Stages; ++s) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&full[s])));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&empty[s])));
-        }
-        for (int b = 0; b < 2; ++b) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&acc_full[b])));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&acc_empty[b])), "r"(kT3EpiWarps));
-        }
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&done)));
-        asm volatile("fence.mbarrier_init.release.cluster;");
-        abort_flag = 0;
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;");
-    const uint32_t tmem = tmem_base;
-    bool ok = true;
-
-    if (warp == 0) {
-        // ---------------------------------------------------------------- TMA producer
-        if (lane == 0) {
-            long long step = 0;
-            for (long long g = g0 + blockIdx.x; g < g1 && ok; g += gridDim.x) {
-                int i0, j0;  // LAYER: i0 = the tile's first row in the residue-ordered planes
-                if (LAYER) {
-                    int p0;
-                    t2l_decode<kT2I, 8>(item_begin, n_itiles, w, g, p0, j0);
-                    i0 = residue_row(w.dist_offset, w.dist_step, n) + p0;
-                } else {
-                    t2_decode(item_begin, n_itiles, g, i0, j0);
-                }
-                for (int ks = 0; ks < ksteps; ++ks) {
-                    const int s = (int)(step % kT2Stages);
-                    const long long u = step / kT2Stages;
-                    if (u > 0 && !t3_wait(smem_u32(&empty[s]), (uint32_t)((u - 1) & 1), abort)) {
-                        ok = false;
-                        break;
-                    }
-                    const int k0 = ks < ks_c ? ks * kT3KB : k_cases + (ks - ks_c) * kT3KB;
-                    uint8_t* st = sm + s * kT2Stage;
-                    const uint32_t bar = smem_u32(&full[s]);
-                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                                 "r"((uint32_t)kT2Stage)
-                                 : "memory");
-                    t3_tma(smem_u32(st), &maps.a, k0, 2 * i0, bar);
-                    t3_tma(smem_u32(st + kT2SA), &maps.b, k0, 2 * j0, bar);
-                    ++step;
-                }
-            }
-            for (int s = 0; s < kT2Stages; ++s) {
-                if (step <= s) continue;
-                const long long last = s + ((step - 1 - s) / kT2Stages) * kT2Stages;
-                if (!t3_drain(smem_u32(&full[s]), (uint32_t)((last / kT2Stages) & 1))) ok = false;
-            }
-        }
-    } else if (warp == 1) {
-        // ---------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
-            long long step = 0, item = 0;
-            for (long long g = g0 + blockIdx.x; g < g1 && ok; g += gridDim.x, ++item) {
-                const int buf = (int)(item % nbuf);
-                if (item >= nbuf &&
-                    !t3_wait(smem_u32(&acc_empty[buf]), (uint32_t)(((item / nbuf) - 1) & 1), abort)) {
-                    ok = false;
-                    break;
-                }
-                for (int ks = 0; ks < ksteps; ++ks, ++step) {
-                    const int s = (int)(step % kT2Stages);
-                    if (!t3_wait(smem_u32(&full[s]), (uint32_t)((step / kT2Stages) & 1), abort)) {
-                        ok = false;
-                        break;
-                    }
-                    asm volatile("tcgen05.fence::after_thread_sync;");
-                    const uint32_t sa = smem_u32(sm + s * kT2Stage), sb = sa + kT2SA;
-                    const int cls = ks >= ks_c;
-                    const uint32_t dcol = tmem + (uint32_t)(pack ? kT2N * buf : kT2N * cls);
-                    const bool first = pack ? ks == 0 : (ks == 0 || ks == ks_c);
-#pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) {
-                        const uint64_t ad = t3_desc(sa + 32 * kk), bd = t3_desc(sb + 32 * kk);
-                        const uint32_t acc = (first && kk == 0) ? 0u : 1u;
-                        asm volatile(
-                            "{.reg .pred p; setp.ne.b32 p, %4, 0;\n"
-                            "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;}\n" ::"r"(dcol),
-                            "l"(ad), "l"(bd), "r"(kT2Idesc), "r"(acc));
-                    }
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                        smem_u32(&empty[s])));
-                }
-                if (!ok) break;
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                    smem_u32(&acc_full[buf])));
-            }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                smem_u32(&done)));
-            if (!t3_drain(smem_u32(&done), 0)) ok = false;
-        }
-    } else {
-        // ---------------------------------------------------------------- epilogue
-        const int e = warp - 2;     // 0..7
-        const int q = warp & 3;     // tensor-memory lane quarter this warp may access
-        const int hh = e >> 2;      // column groups 2 cc + hh: j offsets 16 cc + 8 hh + [0, 8)
-        uint32_t* ebuf = ebuf_all + e * (kT3Ebuf / 4);
-        const uint32_t lane_base = tmem + ((uint32_t)(32 * q) << 16);
-        const uint32_t wmask = pack ? (1u << pack) - 1u : 0xffffffffu;
-        const int ii = lane >> 1, x = lane & 1, kh = lane & 1;  // row (ii, x); pairs k = 4 kh + kk
-        long long item = 0;
-        for (long long g = g0 + blockIdx.x; g < g1 && ok; g += gridDim.x, ++item) {
-            int i0, j0, istep = 1;
-            if (LAYER) {
-                int p0;
-                t2l_decode<kT2I, 8>(item_begin, n_itiles, w, g, p0, j0);
-                i0 = w.dist_offset + w.dist_step * p0;
-                istep = w.dist_step;
-            } else {
-                t2_decode(item_begin, n_itiles, g, i0, j0);
-            }
-            const int buf = (int)(item % nbuf);
-            const int i = i0 + istep * (16 * q + ii);
-            const bool i_ok = i < n;
-            float si[2][2];
-            {
-                uint4 a = make_uint4(0, 0, 0, 0);
-                if (i_ok) a = __ldg(reinterpret_cast<const uint4*>(single) + i);
-                si[0][0] = u2f(a.x);
-                si[0][1] = u2f(a.y);
-                si[1][0] = u2f(a.z);
-                si[1][1] = u2f(a.w);
-            }
-            if (!t3_wait(smem_u32(&acc_full[buf]), (uint32_t)((item / nbuf) & 1), abort)) {
-                ok = false;
-                break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;");
-#pragma unroll 1
-            for (int cc = 0; cc < 8; ++cc) {
-                // the two warps of a lane quarter interleave over the j range; a group without
-                // a valid pair for this warp (left of the diagonal, past the last SNP) is skipped
-                const int jg = j0 + 16 * cc + 8 * hh;
-                if (!__any_sync(0xffffffffu, i_ok && jg + 7 > i && jg < n)) {
-                    if (cc == 7) {
-                        asm volatile("tcgen05.fence::before_thread_sync;");
-                        __syncwarp();
-                        if (lane == 0)
-                            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[buf]))
-                                         : "memory");
-                    }
-                    continue;
-                }
-                // the group's 8 single cores of j: lane t loads j = jg + (t & 7) before the
-                // accumulator reads, so that its latency overlaps them
-                const int jl = jg + (lane & 7);
-                const uint4 sjp = jl < n ? __ldg(reinterpret_cast<const uint4*>(single) + jl) : make_uint4(0, 0, 0, 0);
-                {
-                    const uint32_t col = (uint32_t)((pack ? kT2N * buf : 0) + 32 * cc + 16 * hh);
-                    uint32_t v[16], vt[16];
-                    asm volatile(
-                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%"
-                        "15}, [%16];"
-                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-                          "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-                          "=r"(v[14]), "=r"(v[15])
-                        : "r"(lane_base + col));
-                    if (!pack)
-                        asm volatile(
-                            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%"
-                            "14,%15}, [%16];"
-                            : "=r"(vt[0]), "=r"(vt[1]), "=r"(vt[2]), "=r"(vt[3]), "=r"(vt[4]), "=r"(vt[5]),
-                              "=r"(vt[6]), "=r"(vt[7]), "=r"(vt[8]), "=r"(vt[9]), "=r"(vt[10]), "=r"(vt[11]),
-                              "=r"(vt[12]), "=r"(vt[13]), "=r"(vt[14]), "=r"(vt[15])
-                            : "r"(lane_base + (uint32_t)kT2N + col));
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (cc == 7) {  // last read of this item's accumulators
-                        asm volatile("tcgen05.fence::before_thread_sync;");
-                        __syncwarp();
-                        if (lane == 0)
-                            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[buf]))
-                                         : "memory");
-                    }
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        uint2 c2;
-                        if (pack) {
-                            const uint32_t u0 = __float2uint_rn(__uint_as_float(v[2 * k]));
-                            const uint32_t u1 = __float2uint_rn(__uint_as_float(v[2 * k + 1]));
-                            c2 = make_uint2((u0 & wmask) | (u1 & wmask) << 16, (u0 >> pack) | (u1 >> pack) << 16);
-                        } else {
-                            c2 = make_uint2(f2u(__uint_as_float(v[2 * k])) | f2u(__uint_as_float(v[2 * k + 1])) << 16,
-                                            f2u(__uint_as_float(vt[2 * k])) | f2u(__uint_as_float(vt[2 * k + 1])) << 16);
-                        }
-                        *reinterpret_cast<uint2*>(ebuf + 2 * t2_slot(ii, k, x)) = c2;
-                    }
-                }
-                __syncwarp();
-#pragma unroll 1
-                for (int kk = 0; kk < 4; ++kk) {
-                    const int k = 4 * kh + kk;
-                    t2_eval(w, sink, thr_f, dump, sjp, ebuf, ii, k, i, jg + k, i_ok, si, lane);
-                }
-                __syncwarp();
-            }
-        }
-    }
-    if (!ok) *abort = 1;
-    asm volatile("tcgen05.fence::before_thread_sync;");
-    __syncthreads();
-    if (tid == 0 && abort_flag) atomicOr(status, 1);
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
-}
-
-// ---------------------------------------------------------------------------
-// Order 2 on CTA pairs.  A cluster of two CTAs (the two SMs of a TPC) runs one
-// GEMM D[(i,x), (j,y)] of M 256 x N 256 per work item with
-// tcgen05.mma.cta_group::2: CTA r stages its own A tile (64 i x 2 rows, i-tile
-// 2p + r of the band) and half r of the B tile (64 j x 2 rows); CTA 0 issues
-// the MMAs, which read both CTAs' shared memory and leave each CTA's 128
-// accumulator rows in its own tensor memory.  Per SM a stage then moves 32
-// instead of 48 KB through shared memory (TMA writes and MMA operand reads of
-// B halve), which is what bounded the single-CTA kernel.
-// Handover: CTA 0's `full` barriers take one arrival with the transaction
-// bytes of both CTAs' copies (CTA 1's copies complete on them through the
-// .cta_group::2 TMA form); the MMA commits go to both CTAs' `empty`,
-// `acc_full` and `done`; both CTAs' epilogue warps arrive on CTA 0's
-// `acc_empty` (16 arrivals).  Every wait is bounded as in the other kernels;
-// both CTAs meet at a cluster barrier before tensor memory is released.
-constexpr int kT2xStages = 5;
-constexpr int kT2xSA = kT2M * kT3KB;        // 16 KB: this CTA's 64 i x 2 rows
-constexpr int kT2xSB = kT2M * kT3KB;        // 16 KB: this CTA's half of the 128 j x 2 rows
-constexpr int kT2xStage = kT2xSA + kT2xSB;  // 32 KB
-constexpr size_t kT2xSmem = 1024 + (size_t)kT2xStages * kT2xStage + (size_t)kT3EpiWarps * kT3Ebuf;
-constexpr uint32_t kT2xIdesc = (1u << 4) | ((uint32_t)(kT2N >> 3) << 17) | ((uint32_t)((2 * kT2M) >> 4) << 24);
-static_assert(kT2xSmem <= 227 * 1024 - 256, "paired order-2 tensor kernel shared memory");
-
-// Pair items: band r (i-tiles [8 r, 8 r + 8), j-tiles b >= 4 r) lists, j-tile by
-// j-tile, its i-tile pairs (2 p, 2 p + 1); i0 = first i of the pair.
-__device__ __forceinline__ void t2x_decode(const long long* __restrict__ item_begin, int n_itiles, long long g,
-                                           int& i0, int& j0) {
-    const int n_bands = (n_itiles + kT2Band - 1) / kT2Band;
-    int lo = 0, hi = n_bands - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (item_begin[mid] <= g) lo = mid;
-        else hi = mid - 1;
-    }
-    const int ca = min(kT2Band, n_itiles - kT2Band * lo);
-    const int cp = (ca + 1) >> 1;  // i-tile pairs in the band
-    const long long idx = g - item_begin[lo];
-    const int b = kT2Band * kT2I / kT2L * lo + (int)(idx / cp);
-    i0 = kT2I * (kT2Band * lo + 2 * (int)(idx % cp));
-    j0 = kT2L * b;
-}
-
-// LAYER: a Distribution layer (t2l_decode over tile pairs, as tensor2_kernel).
-template <bool LAYER>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kT2Threads, 1)
-    tensor2x_kernel(const __grid_constant__ T2Maps maps, ScanWork w, const long long* __restrict__ item_begin,
-                    int n_itiles, long long g0, long long g1, int k_cases, int pack, CandSink sink, float thr_f,
-                    uint32_t* dump, const uint32_t* __restrict__ single, int* status) {
-    extern __shared__ uint8_t smraw[];
-    __shared__ __align__(8) uint64_t full[kT2xStages], empty[kT2xStages];
-    __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2], done;
-    __shared__ uint32_t tmem_base;
-    __shared__ int abort_flag;
-    uint8_t* sm = (uint8_t*)(((uintptr_t)smraw + 1023) & ~(uintptr_t)1023);  // stages: A | B half
-    uint32_t* ebuf_all = reinterpret_cast<uint32_t*>(sm + kT2xStages * kT2xStage);
-    volatile int* abort = &abort_flag;
-    const DevData& d = w.d;
-    const int n = d.snps;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int ks_c = k_cases / kT3KB;
-    const int ksteps = ks_c + (d.tw + 1) / 2;
-    const int nbuf = pack ? 2 : 1;
-    const uint32_t rank = cluster_rank();  // 0 issues the MMAs
-    const long long cid = cluster_id(), ncl = cluster_count();
-
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
-                     "r"(512));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
-    }
-    if (tid == 0) {
-        for (int s = 0; s < kT2xStages; ++s) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&full[s])));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&empty[s])));
-        }
-        for (int b = 0; b < 2; ++b) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&acc_full[b])));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&acc_empty[b])),
-                         "r"(2 * kT3EpiWarps));
-        }
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&done)));
-        asm volatile("fence.mbarrier_init.release.cluster;");
-        abort_flag = 0;
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;");
-    __syncthreads();
-    cluster_sync_all();  // both CTAs' barriers exist before either signals the other
-    asm volatile("tcgen05.fence::after_thread_sync;");
-    const uint32_t tmem = tmem_base;
-    bool ok = true;
-
-    if (warp == 0) {
-        // ---------------------------------------------------------------- TMA producer (both CTAs)
-        if (lane == 0) {
-            long long step = 0;
-            for (long long g = g0 + cid; g < g1 && ok; g += ncl) {
-                int i0, j0;  // LAYER: i0 = the pair's first row in the residue-ordered planes
-                if (LAYER) {
-                    int p0;
-                    t2l_decode<2 * kT2I, 4>(item_begin, n_itiles, w, g, p0, j0);
-                    i0 = residue_row(w.dist_offset, w.dist_step, n) + p0;
-                } else {
-                    t2x_decode(item_begin, n_itiles, g, i0, j0);
-                }
-                for (int ks = 0; ks < ksteps; ++ks) {
-                    const int s = (int)(step % kT2xStages);
-                    const long long u = step / kT2xStages;
-                    if (u > 0 && !t3_wait_cl(smem_u32(&empty[s]), (uint32_t)((u - 1) & 1), abort)) {
-                        ok = false;
-                        break;
-                    }
-                    const int k0 = ks < ks_c ? ks * kT3KB : k_cases + (ks - ks_c) * kT3KB;
-                    uint8_t* st = sm + s * kT2xStage;
-                    const uint32_t bar = cluster_addr(smem_u32(&full[s]), 0);
-                    if (rank == 0)
-                        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&full[s])),
-                                     "r"((uint32_t)(2 * kT2xStage))
-                                     : "memory");
-                    t3_tma_pair(smem_u32(st), &maps.a, k0, 2 * (i0 + kT2I * (int)rank), bar);
-                    t3_tma_pair(smem_u32(st + kT2xSA), &maps.b, k0, 2 * j0 + kT2M * (int)rank, bar);
-                    ++step;
-                }
-            }
-            // copies in flight land before the pair is released: CTA 0 sees every copy of
-            // both CTAs complete on its `full` barriers, CTA 1 sees its stages consumed
-            for (int s = 0; s < kT2xStages; ++s) {
-                if (step <= s) continue;
-                const long long last = s + ((step - 1 - s) / kT2xStages) * kT2xStages;
-                const uint32_t par = (uint32_t)((last / kT2xStages) & 1);
-                if (!(rank == 0 ? t3_drain_cl(smem_u32(&full[s]), par) : t3_drain_cl(smem_u32(&empty[s]), par)))
-                    ok = false;
-            }
-        }
-    } else if (warp == 1) {
-        // ---------------------------------------------------------------- MMA issuer (CTA 0)
-        if (lane == 0 && rank == 0) {
-            long long step = 0, item = 0;
-            for (long long g = g0 + cid; g < g1 && ok; g += ncl, ++item) {
-                const int buf = (int)(item % nbuf);
-                if (item >= nbuf &&
-                    !t3_wait_cl(smem_u32(&acc_empty[buf]), (uint32_t)(((item / nbuf) - 1) & 1), abort)) {
-                    ok = false;
-                    break;
-                }
-                for (int ks = 0; ks < ksteps; ++ks, ++step) {
-                    const int s = (int)(step % kT2xStages);
-                    if (!t3_wait_cl(smem_u32(&full[s]), (uint32_t)((step / kT2xStages) & 1), abort)) {
-                        ok = false;
-                        break;
-                    }
-                    asm volatile("tcgen05.fence::after_thread_sync;");
-                    const uint32_t sa = smem_u32(sm + s * kT2xStage), sb = sa + kT2xSA;
-                    const int cls = ks >= ks_c;
-                    const uint32_t dcol = tmem + (uint32_t)(pack ? kT2N * buf : kT2N * cls);
-                    const bool first = pack ? ks == 0 : (ks == 0 || ks == ks_c);
-#pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) {
-                        const uint64_t ad = t3_desc(sa + 32 * kk), bd = t3_desc(sb + 32 * kk);
-                        const uint32_t acc = (first && kk == 0) ? 0u : 1u;
-                        asm volatile(
-                            "{.reg .pred p; setp.ne.b32 p, %4, 0;\n"
-                            "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;}\n" ::"r"(dcol),
-                            "l"(ad), "l"(bd), "r"(kT2xIdesc), "r"(acc));
-                    }
-                    commit_pair(smem_u32(&empty[s]));
-                }
-                if (!ok) break;
-                commit_pair(smem_u32(&acc_full[buf]));
-            }
-            commit_pair(smem_u32(&done));
-        }
-        // neither CTA releases shared or tensor memory before the pair's MMAs are
-        // done (CTA 1 waits once its own work is over, below: waiting here would
-        // span its whole launch, longer than the bound on a single wait)
-        if (lane == 0 && rank == 0 && !t3_drain_cl(smem_u32(&done), 0)) ok = false;
-    } else {
-        // ---------------------------------------------------------------- epilogue (both CTAs)
-        const int e = warp - 2;
-        const int q = warp & 3;
-        const int hh = e >> 2;
-        uint32_t* ebuf = ebuf_all + e * (kT3Ebuf / 4);
-        const uint32_t lane_base = tmem + ((uint32_t)(32 * q) << 16);
-        const uint32_t wmask = pack ? (1u << pack) - 1u : 0xffffffffu;
-        const int ii = lane >> 1, x = lane & 1, kh = lane & 1;
-        const uint32_t acc_empty0[2] = {cluster_addr(smem_u32(&acc_empty[0]), 0),
-                                        cluster_addr(smem_u32(&acc_empty[1]), 0)};
-        long long item = 0;
-        for (long long g = g0 + cid; g < g1 && ok; g += ncl, ++item) {
-            int i0, j0, istep = 1;
-            if (LAYER) {
-                int p0;
-                t2l_decode<2 * kT2I, 4>(item_begin, n_itiles, w, g, p0, j0);
-                i0 = w.dist_offset + w.dist_step * (p0 + kT2I * (int)rank);
-                istep = w.dist_step;
-            } else {
-                t2x_decode(item_begin, n_itiles, g, i0, j0);
-                i0 += kT2I * (int)rank;
-            }
-            const int buf = (int)(item % nbuf);
-            const int i = i0 + istep * (16 * q + ii);
-            const bool i_ok = i < n;
-            float si[2][2];
-            {
-                uint4 a = make_uint4(0, 0, 0, 0);
-                if (i_ok) a = __ldg(reinterpret_cast<const uint4*>(single) + i);
-                si[0][0] = u2f(a.x);
-                si[0][1] = u2f(a.y);
-                si[1][0] = u2f(a.z);
-                si[1][1] = u2f(a.w);
-            }
-            if (!t3_wait_cl(smem_u32(&acc_full[buf]), (uint32_t)((item / nbuf) & 1), abort)) {
-                ok = false;
-                break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;");
-#pragma unroll 1
-            for (int cc = 0; cc < 8; ++cc) {
-                const int jg = j0 + 16 * cc + 8 * hh;
-                if (!__any_sync(0xffffffffu, i_ok && jg + 7 > i && jg < n)) {
-                    if (cc == 7) {
-                        asm volatile("tcgen05.fence::before_thread_sync;");
-                        __syncwarp();
-                        if (lane == 0) arrive_cl(acc_empty0[buf]);
-                    }
-                    continue;
-                }
-                const int jl = jg + (lane & 7);
-                const uint4 sjp = jl < n ? __ldg(reinterpret_cast<const uint4*>(single) + jl) : make_uint4(0, 0, 0, 0);
-                {
-                    const uint32_t col = (uint32_t)((pack ? kT2N * buf : 0) + 32 * cc + 16 * hh);
-                    uint32_t v[16], vt[16];
-                    asm volatile(
-                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%"
-                        "15}, [%16];"
-                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-                          "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-                          "=r"(v[14]), "=r"(v[15])
-                        : "r"(lane_base + col));
-                    if (!pack)
-                        asm volatile(
-                            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%"
-                            "14,%15}, [%16];"
-                            : "=r"(vt[0]), "=r"(vt[1]), "=r"(vt[2]), "=r"(vt[3]), "=r"(vt[4]), "=r"(vt[5]),
-                              "=r"(vt[6]), "=r"(vt[7]), "=r"(vt[8]), "=r"(vt[9]), "=r"(vt[10]), "=r"(vt[11]),
-                              "=r"(vt[12]), "=r"(vt[13]), "=r"(vt[14]), "=r"(vt[15])
-                            : "r"(lane_base + (uint32_t)kT2N + col));
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (cc == 7) {
-                        asm volatile("tcgen05.fence::before_thread_sync;");
-                        __syncwarp();
-                        if (lane == 0) arrive_cl(acc_empty0[buf]);
-                    }
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        uint2 c2;
-                        if (pack) {
-                            const uint32_t u0 = __float2uint_rn(__uint_as_float(v[2 * k]));
-                            const uint32_t u1 = __float2uint_rn(__uint_as_float(v[2 * k + 1]));
-                            c2 = make_uint2((u0 & wmask) | (u1 & wmask) << 16, (u0 >> pack) | (u1 >> pack) << 16);
-                        } else {
-                            c2 = make_uint2(f2u(__uint_as_float(v[2 * k])) | f2u(__uint_as_float(v[2 * k + 1])) << 16,
-                                            f2u(__uint_as_float(vt[2 * k])) | f2u(__uint_as_float(vt[2 * k + 1])) << 16);
-                        }
-                        *reinterpret_cast<uint2*>(ebuf + 2 * t2_slot(ii, k, x)) = c2;
-                    }
-                }
-                __syncwarp();
-#pragma unroll 1
-                for (int kk = 0; kk < 4; ++kk) {
-                    const int k = 4 * kh + kk;
-                    t2_eval(w, sink, thr_f, dump, sjp, ebuf, ii, k, i, jg + k, i_ok, si, lane);
-                }
-                __syncwarp();
-            }
-        }
-    }
-    if (!ok) *abort = 1;
-    asm volatile("tcgen05.fence::before_thread_sync;");
-    __syncthreads();
-    // CTA 1: its epilogue has read the last accumulators, so the pair's final
-    // commit to this CTA's `done` lands soon; it must land before the CTA exits
-    if (rank == 1 && warp == 1 && lane == 0 && !t3_drain_cl(smem_u32(&done), 0)) *abort = 1;
-    cluster_sync_all();  // the other CTA is done with this CTA's shared and tensor memory
-    asm volatile("tcgen05.fence::after_thread_sync;");
-    if (tid == 0 && abort_flag) atomicOr(status, 1);
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
-}
-
 // Operand planes: one thread per 16 output bytes (16 samples of one row).
-__global__ void t3_planes_kernel(DevData d, uint8_t* planes, int pitch, int k_cases, uint32_t ctrl_byte) {
+__global__ void t3_planes_kernel(DevData d, uint8_t* planes, int pitch, int k_cases) {
     const long long chunks = (long long)pitch / 16;
     const long long total = 2ll * d.snps * chunks;
     const size_t per_snp = 3 * (size_t)(d.cw + d.tw);
@@ -1201,44 +498,9 @@ __global__ void t3_planes_kernel(DevData d, uint8_t* planes, int pitch, int k_ca
         uint32_t* pv = &v.x;
 #pragma unroll
         for (int qd = 0; qd < 4; ++qd)
-            pv[qd] = (((bits >> (4 * qd)) & 0xfu) * 0x00204081u & 0x01010101u) * (ctrl ? ctrl_byte : 0x38u);
+            pv[qd] = (((bits >> (4 * qd)) & 0xfu) * 0x00204081u & 0x01010101u) * 0x38u;
         *reinterpret_cast<uint4*>(planes + (size_t)row * pitch + o) = v;
     }
-}
-
-// Order-2 items (host): prefix sums over the bands of t2_decode; returns the
-// total and the number of i-tiles.
-static long long t2_items(int n, std::vector<long long>& item_begin, int& n_itiles) {
-    n_itiles = std::max(1, (n - 1 + kT2I - 1) / kT2I);
-    const int n_bands = (n_itiles + kT2Band - 1) / kT2Band;
-    const int nb = (n + kT2L - 1) / kT2L;  // global j-tiles
-    item_begin.assign((size_t)n_bands + 1, 0);
-    long long total = 0;
-    for (int r = 0; r < n_bands; ++r) {
-        item_begin[r] = total;
-        const int ca = std::min(kT2Band, n_itiles - kT2Band * r);
-        const int b0 = kT2Band * kT2I / kT2L * r;
-        if (nb > b0) total += (long long)ca * (nb - b0);
-    }
-    item_begin[n_bands] = total;
-    return total;
-}
-
-// Pair items of tensor2x_kernel (host): prefix sums over the bands of t2x_decode.
-static long long t2x_items(int n, std::vector<long long>& item_begin, int& n_itiles) {
-    n_itiles = std::max(1, (n - 1 + kT2I - 1) / kT2I);
-    const int n_bands = (n_itiles + kT2Band - 1) / kT2Band;
-    const int nb = (n + kT2L - 1) / kT2L;
-    item_begin.assign((size_t)n_bands + 1, 0);
-    long long total = 0;
-    for (int r = 0; r < n_bands; ++r) {
-        item_begin[r] = total;
-        const int ca = std::min(kT2Band, n_itiles - kT2Band * r);
-        const int b0 = kT2Band * kT2I / kT2L * r;
-        if (nb > b0) total += (long long)((ca + 1) / 2) * (nb - b0);
-    }
-    item_begin[n_bands] = total;
-    return total;
 }
 
 // Items per i of tensor3_kernel (host): prefix sums item_begin[0..n], item_begin[n] = total.
@@ -1285,18 +547,7 @@ static cudaError_t t3_map(CUtensorMap* m, uint8_t* base, int rows, int pitch, in
     return tensor_map(m, base, rows, pitch, kT3KB, box_rows, swizzle);
 }
 
-// One accumulator for both classes when some W = 4^h (h <= 8, so 2^h is an
-// e4m3 power of two) has n_cases < W and n_cases + W * n_ctrls < 2^24 (every
-// count exact in FP32).
-int tensor_pack(int n_cases, int n_ctrls) {
-    for (int h = 1; h <= 8; ++h) {
-        const long long W = 1ll << (2 * h);
-        if (W > n_cases && n_cases + W * (long long)n_ctrls < (1ll << 24)) return 2 * h;
-    }
-    return 0;
-}
-
-// e4m3 planes (every use but the order-3 pair kernel's).
+// e4m3 planes (the per-class kernels of orders 3 and 4).
 static cudaError_t e4m3_planes(T3Plan& plan, const DevData& d, cudaStream_t s) {
     if (plan.planes) return cudaSuccess;
     uint8_t* planes = nullptr;
@@ -1304,8 +555,7 @@ static cudaError_t e4m3_planes(T3Plan& plan, const DevData& d, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     const long long total = 2ll * d.snps * (plan.pitch / 16);
     const int grid = (int)std::min<long long>((total + 255) / 256, 4096);
-    const uint32_t ctrl_byte = plan.pack ? (uint32_t)((plan.pack / 2 + 7) << 3) : 0x38u;  // e4m3 2^h
-    t3_planes_kernel<<<grid, 256, 0, s>>>(d, planes, plan.pitch, plan.k_cases, ctrl_byte);
+    t3_planes_kernel<<<grid, 256, 0, s>>>(d, planes, plan.pitch, plan.k_cases);
     count_launch();
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -1313,29 +563,17 @@ static cudaError_t e4m3_planes(T3Plan& plan, const DevData& d, cudaStream_t s) {
     if (e == cudaSuccess) e = t3_map(&plan.map_l, planes, rows, plan.pitch, kT3N, true);
     if (e == cudaSuccess) e = t3_map(&plan.map_j, planes, rows, plan.pitch, 2 * kT3J, true);
     if (e == cudaSuccess) e = t3_map(&plan.map_i, planes, rows, plan.pitch, 2, true);
-    if (e == cudaSuccess) e = t3_map(&plan.map_a2, planes, rows, plan.pitch, kT2M, true);
-    if (e == cudaSuccess) e = t3_map(&plan.map_b2, planes, rows, plan.pitch, kT2N, true);
+    if (e == cudaSuccess) e = t3_map(&plan.map_l4, planes, rows, plan.pitch, 128, true);
     if (e != cudaSuccess) cudaFree(planes);
     else plan.planes = planes;
     return e;
 }
 
-cudaError_t tensor3_prepare(const DevData& d, T3Plan& plan, cudaStream_t) {
-    plan.pack = tensor_pack(d.n_cases, d.n_ctrls);
-    plan.f4.pack = f4_pack(d.n_cases, d.n_ctrls);
+void tensor3_prepare(const DevData& d, T3Plan& plan) {
+    f4_sizes(d, plan.f4);
     plan.pair3 = plan.f4.pack != 0;
     plan.k_cases = kT3KB * ((d.cw + 1) / 2);
     plan.pitch = plan.k_cases + kT3KB * ((d.tw + 1) / 2);
-    // order 2: CTA-pair items when the classes pack (per class the MMA waits for the epilogue between
-    // items, and the single-CTA kernel measured 2 % faster there)
-    std::vector<long long> ib2;
-    plan.pair2 = plan.pack != 0;
-    plan.total2 = plan.pair2 ? t2x_items(d.snps, ib2, plan.n_itiles) : t2_items(d.snps, ib2, plan.n_itiles);
-    plan.item2_combos = (double)d.snps * (d.snps - 1) / 2 / std::max(1ll, plan.total2);
-    cudaError_t e = cudaMalloc((void**)&plan.item2_begin, ib2.size() * sizeof(long long));
-    if (e == cudaSuccess)
-        e = cudaMemcpy(plan.item2_begin, ib2.data(), ib2.size() * sizeof(long long), cudaMemcpyHostToDevice);
-    return e;
 }
 
 // Copies a host item table to the device.
@@ -1364,8 +602,16 @@ static cudaError_t order3_items(T3Plan& plan, const DevData& d) {
 // layout and at order 4 the packed cores of the triples.
 static cudaError_t order_planes(T3Plan& plan, const DevData& d, int order, const uint4* pairs, cudaStream_t s,
                                 int sms) {
-    if (order == 2 || !plan.pair3) return e4m3_planes(plan, d, s);
     cudaError_t e = cudaSuccess;
+    if (order == 2) {
+        if (plan.f4.ones) return e;
+        e = f4_ones_planes(d, plan.f4, d.snps, 0, 1, plan.f4.ones, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e == cudaSuccess) e = f4_map_a2(&plan.f4.map_a2, plan.f4, plan.f4.ones, d.snps);
+        if (e == cudaSuccess) e = f4_map_b2(&plan.f4.map_b2, plan.f4, plan.f4.ones, d.snps);
+        return e;
+    }
+    if (!plan.pair3) return e4m3_planes(plan, d, s);
     if (!plan.f4.bits) {
         e = f4_prepare(d, plan.f4, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -1387,6 +633,12 @@ cudaError_t tensor3_order_items(T3Plan& plan, const DevData& d, int order, const
     std::lock_guard<std::mutex> g(plan.items_mu);
     cudaError_t e = order_planes(plan, d, order, pairs, s, sms);
     if (e == cudaSuccess && order == 3) e = order3_items(plan, d);
+    if (e == cudaSuccess && order == 2 && !plan.item2_begin) {
+        const std::vector<long long> ib = t2x_items(d.snps, d.snps - 1, 0, 1, plan.n_itiles);
+        plan.total2 = ib.back();
+        plan.item2_combos = (double)d.snps * (d.snps - 1) / 2 / std::max(1ll, plan.total2);
+        e = upload(plan.item2_begin, ib);
+    }
     if (e == cudaSuccess && order == 4 && !plan.item4_begin && d.snps >= 4) {
         std::vector<long long> per4;
         const std::vector<long long> ib4 = t4_item_table(d.snps, plan.pair3, per4);
@@ -1417,7 +669,8 @@ struct T3Layer {
     int n_tiles = 0;                  // order 2: tiles of owned i; order 4: listed pairs
     int4* pinfo = nullptr;            // order 4: (i, j, first owned k) of each listed pair
     CUtensorMap map_jr;               // order 3: 64 rows of the residue-ordered planes (pair kernel: bit rows)
-    CUtensorMap map_ar;               // order 2: box 128 B x 128 rows over the residue-ordered planes
+    uint8_t* planes = nullptr;        // order 2: the owned SNPs' planes
+    CUtensorMap map_ar;               // order 2: box 128 B x 128 rows over them
     CUtensorMap map_kr;               // order 4: 32 rows of the residue-ordered planes (pair kernel: bit rows)
 };
 struct T3Layers {
@@ -1470,12 +723,12 @@ cudaError_t tensor3_layer(T3Plan& plan, const ScanWork& w, const uint4* pairs, c
         std::lock_guard<std::mutex> gp(plan.items_mu);
         pe = order_planes(plan, w.d, w.order, pairs, s, sms);
     }
-    if (pe == cudaSuccess)
+    if (pe == cudaSuccess && w.order != 2)
         pe = px ? residue_copy(plan.layers->bits_by_residue, (const uint8_t*)plan.f4.bits, (size_t)8 * plan.f4.wpr,
                                w.d.snps, w.dist_step, s)
                 : residue_copy(plan.layers->by_residue, plan.planes, (size_t)2 * plan.pitch, w.d.snps, w.dist_step, s);
     if (pe != cudaSuccess) return pe;
-    uint8_t* perm = px ? nullptr : plan.layers->by_residue[w.dist_step];
+    uint8_t* perm = px || w.order == 2 ? nullptr : plan.layers->by_residue[w.dist_step];
     const int n = w.d.snps;
     const long long step = w.dist_step, offset = w.dist_offset;
     if (w.order == 4) {
@@ -1505,33 +758,20 @@ cudaError_t tensor3_layer(T3Plan& plan, const ScanWork& w, const uint4* pairs, c
         return cudaSuccess;
     }
     if (w.order == 2) {
-        // owned prefixes: SNPs i = offset + m step; tiles of IT consecutive owned i (a CTA pair's two
-        // i-tiles when the classes pack) in bands of BT (t2l_decode)
-        const int IT = plan.pack ? 2 * kT2I : kT2I, BT = plan.pack ? 4 : 8;
-        const long long count = offset < n ? (n - offset + step - 1) / step : 0;
-        const int tiles = (int)((count + IT - 1) / IT);
-        const int bands = (tiles + BT - 1) / BT;
-        const int nb = (n + kT2L - 1) / kT2L;
-        std::vector<long long> tb((size_t)bands + 1);
-        long long total = 0, combos = 0;
-        for (int r = 0; r < bands; ++r) {
-            tb[r] = total;
-            const long long i_first = offset + step * (long long)IT * BT * r;
-            const int ca = std::min(BT, tiles - BT * r);
-            total += (long long)ca * std::max(0ll, (long long)nb - (i_first + 1) / kT2L);
-        }
-        tb[bands] = total;
+        // owned prefixes: SNPs i = offset + m step, in planes of their own
+        const int count = offset < n ? (int)((n - offset + step - 1) / step) : 0;
+        long long combos = 0;
         for (long long i = offset; i < n; i += step) combos += n - 1 - i;
         T3Layer L;
-        L.total = total;
-        L.n_tiles = tiles;
-        L.item_combos = (double)combos / std::max(1ll, total);
-        cudaError_t e = t3_map(&L.map_ar, perm, 2 * n, plan.pitch, kT2M, true);
-        if (e == cudaSuccess) e = cudaMalloc((void**)&L.item_begin, tb.size() * sizeof(long long));
-        if (e == cudaSuccess)
-            e = cudaMemcpy(L.item_begin, tb.data(), tb.size() * sizeof(long long), cudaMemcpyHostToDevice);
+        const std::vector<long long> tb = t2x_items(n, count, offset, step, L.n_tiles);
+        L.total = tb.back();
+        L.item_combos = (double)combos / std::max(1ll, L.total);
+        cudaError_t e = f4_ones_planes(w.d, plan.f4, count, (int)offset, (int)step, L.planes, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e == cudaSuccess) e = f4_map_a2(&L.map_ar, plan.f4, L.planes, count);
+        if (e == cudaSuccess) e = upload(L.item_begin, tb);
         if (e != cudaSuccess) {
-            cudaFree(L.item_begin);
+            cudaFree(L.planes);
             return e;
         }
         plan.layers->by[key] = L;
@@ -1581,7 +821,7 @@ cudaError_t tensor3_layer(T3Plan& plan, const ScanWork& w, const uint4* pairs, c
     return cudaSuccess;
 }
 
-bool tensor_live(const T3Plan& plan, const ScanWork& w) { return w.order != 2 && plan.pair3; }
+bool tensor_live(const T3Plan& plan, const ScanWork& w) { return w.order == 2 || plan.pair3; }
 
 long long tensor_units(const T3Plan& plan, const ScanWork& w) {
     if (is_layer(w)) {
@@ -1605,6 +845,7 @@ void tensor3_release(T3Plan& plan) {
             cudaFree(kv.second.jl_begin);
             cudaFree(kv.second.jlist);
             cudaFree(kv.second.pinfo);
+            cudaFree(kv.second.planes);
         }
         for (auto& kv : plan.layers->by_residue) cudaFree(kv.second);
         for (auto& kv : plan.layers->bits_by_residue) cudaFree(kv.second);
@@ -1717,6 +958,14 @@ cudaError_t probe_lg2_error(unsigned max_c, double* max_abs_err, cudaStream_t s)
 cudaError_t launch_tensor3(const ScanWork& w, const T3Plan& plan, long long g0, long long g1, const CandSink& sink,
                            uint32_t* dump, const uint32_t* single, const uint4* pairs, const uint4* triples,
                            int* status, cudaStream_t s, int sms) {
+    if (w.order == 2) {
+        const T3Layer* L = is_layer(w) ? find_layer(plan, w) : nullptr;
+        if (is_layer(w) && (!L || !tensor_layer_ok(plan, w))) return cudaErrorInvalidValue;
+        const T2xRange r{L ? L->item_begin : plan.item2_begin, L ? L->n_tiles : plan.n_itiles,
+                         L ? &L->map_ar : &plan.f4.map_a2, &plan.f4.map_b2, L ? w.dist_offset : 0,
+                         L ? w.dist_step : 1};
+        return launch_tensor2x(w, plan.f4, r, g0, g1, sink, dump, single, status, s, sms);
+    }
     if (w.order == 4) {
         const T3Layer* L = is_layer(w) ? find_layer(plan, w) : nullptr;
         if (is_layer(w) && (!L || !tensor_layer_ok(plan, w))) return cudaErrorInvalidValue;
@@ -1725,7 +974,7 @@ cudaError_t launch_tensor3(const ScanWork& w, const T3Plan& plan, long long g0, 
                                  : T4xRange{plan.item4_begin, plan.item4_per, &plan.f4.map_k4};
             return launch_tensor4x(w, plan.f4, r, g0, g1, sink, dump, single, pairs, status, s, sms);
         }
-        return launch_tensor4(w, plan.map_a2, L ? L->map_kr : plan.map_k4, plan.map_i,
+        return launch_tensor4(w, plan.map_l4, L ? L->map_kr : plan.map_k4, plan.map_i,
                               L ? L->item_begin : plan.item4_begin, L ? nullptr : plan.item4_per, plan.k_cases, g0, g1,
                               sink, dump, single, pairs, triples, status, s, sms, L ? L->pinfo : nullptr,
                               L ? L->n_tiles : 0);
@@ -1736,15 +985,6 @@ cudaError_t launch_tensor3(const ScanWork& w, const T3Plan& plan, long long g0, 
                                              (int)kT3Smem);
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(tensor3_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kT3Smem);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(tensor2_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kT2Smem);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(tensor2_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kT2Smem);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(tensor2x_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)kT2xSmem);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(tensor2x_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kT2xSmem);
         return e;
     }();
     if (attr != cudaSuccess) return attr;
@@ -1754,35 +994,6 @@ cudaError_t launch_tensor3(const ScanWork& w, const T3Plan& plan, long long g0, 
     const double thr = ((double)sink.thr - (double)w.base_key) * scale - t3_margin(w.d.n_cases + w.d.n_ctrls);
     const float thr_f = (float)std::max(-3.0e38, std::min(3.0e38, thr));
     const unsigned grid = (unsigned)(items < sms ? items : sms);
-    if (w.order == 2) {
-        // a Distribution layer: A rows from the residue-ordered planes, the layer's tiles
-        const T3Layer* L = is_layer(w) ? find_layer(plan, w) : nullptr;
-        if (is_layer(w) && (!L || !tensor_layer_ok(plan, w))) return cudaErrorInvalidValue;
-        const long long* ib = L ? L->item_begin : plan.item2_begin;
-        const int nt = L ? L->n_tiles : plan.n_itiles;
-        if (plan.pair2) {
-            static const int max_clusters = pair_clusters(tensor2x_kernel<false>, kT2Threads, kT2xSmem);
-            const long long clusters = std::min<long long>(items, max_clusters > 0 ? max_clusters : sms / 2);
-            const unsigned grid2 = (unsigned)(2 * std::max(1ll, clusters));
-            const T2Maps maps2{L ? L->map_ar : plan.map_a2, plan.map_a2};  // both boxes 128 rows
-            if (L)
-                tensor2x_kernel<true><<<grid2, kT2Threads, kT2xSmem, s>>>(maps2, w, ib, nt, g0, g1, plan.k_cases,
-                                                                         plan.pack, sink, thr_f, dump, single, status);
-            else
-                tensor2x_kernel<false><<<grid2, kT2Threads, kT2xSmem, s>>>(maps2, w, ib, nt, g0, g1, plan.k_cases,
-                                                                          plan.pack, sink, thr_f, dump, single, status);
-        } else {
-            const T2Maps maps2{L ? L->map_ar : plan.map_a2, plan.map_b2};
-            if (L)
-                tensor2_kernel<true><<<grid, kT2Threads, kT2Smem, s>>>(maps2, w, ib, nt, g0, g1, plan.k_cases,
-                                                                       plan.pack, sink, thr_f, dump, single, status);
-            else
-                tensor2_kernel<false><<<grid, kT2Threads, kT2Smem, s>>>(maps2, w, ib, nt, g0, g1, plan.k_cases,
-                                                                        plan.pack, sink, thr_f, dump, single, status);
-        }
-        count_launch();
-        return cudaGetLastError();
-    }
     T3Maps maps{plan.map_l, plan.map_j, plan.map_i};
     if (plan.pair3) {
         const T3Layer* L = is_layer(w) ? find_layer(plan, w) : nullptr;

@@ -329,7 +329,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
         } else if (warp == 1) {
             // ---------------------------------------------------------------- MMA issuer (CTA 0)
             if (rank == 0 && elect_one()) {
-                ok = f4_pair_issue<kXAStages, kXStages, kXStage, kXN, kXColOne, kXColW>(
+                ok = f4_pair_issue<false, kXAStages, kXSA, kXStages, kXStage, kXN, kXColOne, kXColW>(
                     (g1 - g0 - cid + ncl - 1) / ncl, smem_u32(sma), smem_u32(sm), smem_u32(&full_a[0]),
                     smem_u32(&empty[0]), smem_u32(&acc_full[0]), smem_u32(&acc_empty[0]), tmem, nw_c, nw_t, abort,
                     [&](unsigned item) { return t3x_n(item_ng[item % kXMeta]); });
@@ -694,11 +694,15 @@ cudaError_t f4_bit_map(CUtensorMap* m, const F4Plan& f, const uint32_t* bits, in
     return tensor_map(m, bits, rows, 4 * f.wpr, kXBitRow, box_rows, false);
 }
 
-cudaError_t f4_prepare(const DevData& d, F4Plan& f, cudaStream_t s) {
+void f4_sizes(const DevData& d, F4Plan& f) {
+    f.pack = f4_pack(d.n_cases, d.n_ctrls);
     f.nw_c = (d.n_cases + 63) / 64;
     f.nw_t = (d.n_ctrls + 63) / 64;
-    const int wc = 8 * ((f.nw_c + 3) / 4), wt = 8 * ((f.nw_t + 3) / 4);
-    f.wpr = wc + wt;
+    f.wpr = 8 * ((f.nw_c + 3) / 4) + 8 * ((f.nw_t + 3) / 4);
+}
+
+cudaError_t f4_prepare(const DevData& d, F4Plan& f, cudaStream_t s) {
+    const int wc = 8 * ((f.nw_c + 3) / 4);
     f.rows = 16 * ((d.snps + 7) / 8);
     const size_t plane_bytes = (size_t)f.rows * f.wpr * 16;  // one allocation: planes, then bits
     cudaError_t e = cudaMalloc((void**)&f.planes, plane_bytes + (size_t)2 * d.snps * f.wpr * 4);
@@ -716,9 +720,10 @@ cudaError_t f4_prepare(const DevData& d, F4Plan& f, cudaStream_t s) {
 
 void f4_release(F4Plan& f) {
     cudaFree(f.planes);
+    cudaFree(f.ones);
     cudaFree(f.tri);
     cudaFree(f.row_p);
-    f.planes = nullptr;
+    f.planes = f.ones = nullptr;
     f.bits = nullptr;
     f.tri = f.pairf = nullptr;
     f.row_p = f.row_q = nullptr;

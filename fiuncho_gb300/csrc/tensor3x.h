@@ -15,6 +15,8 @@ constexpr int kPxG = 15;   // most groups of 8 l per item
 __host__ __device__ __forceinline__ int t3x_groups(int n, int jf) { return (n - ((jf + 1) & ~7) + 7) >> 3; }
 __host__ __device__ __forceinline__ int t3x_tiles(int n, int jf) { return (t3x_groups(n, jf) + kPxG - 1) / kPxG; }
 
+// Sizes of the 4-bit layout (host).
+void f4_sizes(const DevData& d, F4Plan& f);
 // Operand planes and bit rows of a data set (built once, on stream s).
 cudaError_t f4_prepare(const DevData& d, F4Plan& f, cudaStream_t s);
 void f4_release(F4Plan& f);

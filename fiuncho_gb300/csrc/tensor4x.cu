@@ -213,17 +213,6 @@ __device__ __forceinline__ void t4x_slices(const T4xCores<T>& v, TL&& tabl, TK&&
     }
 }
 
-__device__ __forceinline__ void t4x_append(const ScanWork& w, const CandSink& sink, const int (&cmb)[4],
-                                           long long key) {
-    const unsigned idx = atomicAdd(sink.count, 1u);
-    if (idx < sink.cap) {
-        sink.buf[idx] = Cand{key, pack_code(cmb, 4, w.bits)};
-        if (sink.hist) atomicAdd(sink.hist + live_bin(key), 1u);
-    } else {
-        atomicOr(sink.overflow, 1u);
-    }
-}
-
 // ALL: every combination takes the exact path (a search's first units, before a threshold; dumps and
 // digests).  Otherwise the bound comes first and the few combinations above it are evaluated from the
 // data set (warp_exact_key): the exact path's registers beside the bound's cost 20 % of the whole.
@@ -343,7 +332,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
         } else if (warp == 1) {
             // ---------------------------------------------------------------- MMA issuer (CTA 0)
             if (rank == 0 && elect_one()) {
-                ok = f4_pair_issue<kYAStages, kYStages, kYStage, kYN, kYColOne, kYColW>(
+                ok = f4_pair_issue<false, kYAStages, kYSA, kYStages, kYStage, kYN, kYColOne, kYColW>(
                     (g1 - g0 - cid + ncl - 1) / ncl, smem_u32(sma), smem_u32(sm), smem_u32(&full_a[0]),
                     smem_u32(&empty[0]), smem_u32(&acc_full[0]), smem_u32(&acc_empty[0]), tmem, nw_c, nw_t, abort,
                     [&](unsigned item) { return t4x_n(item_ng[item % kYMeta]); });
@@ -605,7 +594,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
                         const int cmb[4] = {it.i, it.j, __shfl_sync(0xffffffffu, k, src),
                                             __shfl_sync(0xffffffffu, l, src) + u};
                         const long long key = warp_exact_key<4>(&w.d, w.base_key, cmb[0], cmb[1], cmb[2], cmb[3]);
-                        if (lane == 0 && key >= thr) t4x_append(w, sink, cmb, key);
+                        if (lane == 0 && key >= thr) live_append(sink, key, pack_code(cmb, 4, w.bits));
                     }
                 } else {
 #pragma unroll 1
@@ -652,7 +641,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
                                 });
                         }
                         if (sink.digest) dg_warp_add(sink.digest, want && o ? dg_table(cmb, 4, n, o, 81) : 0ull);
-                        if (want && key >= thr) t4x_append(w, sink, cmb, key);
+                        if (want && key >= thr) live_append(sink, key, pack_code(cmb, 4, w.bits));
                     }
                     load(gi + 2);
                 }

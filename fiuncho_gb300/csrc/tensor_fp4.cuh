@@ -43,14 +43,16 @@ __device__ __forceinline__ void f4_mma(uint32_t d, uint64_t a, uint64_t b, uint3
 
 // The MMA issuer of a CTA-pair kernel (one elected thread of CTA 0): for each of
 // `items` items the GEMM of M 256 x n_of(item) columns over the class's 64-sample
-// steps.  A tiles come from a ring of kA stages of 16 KB at a0 (full0), B tiles
-// from a ring of kB stages of kBStage bytes at b0, released by empty0 (kB
+// steps.  A tiles come from a ring of kA stages of kAStage bytes at a0 (full0), B
+// tiles from a ring of kB stages of kBStage bytes at b0, released by empty0 (kB
 // barriers); accumulator regions of kRegion columns alternate by acc_full0 /
-// acc_empty0.  Returns false after a wait that gave up.  Its own time per stage
+// acc_empty0.  SPLIT (classes that do not share an accumulator): the cases of an
+// item, then its controls, are two GEMMs, each into a region of its own.
+// Returns false after a wait that gave up.  Its own time per stage
 // counts (about 230 cycles alone on an SM quarter, up to twice that beside other
 // warps, against 480 of MMA at N 240), so the loop holds what it must and decodes
 // no items.
-template <int kA, int kB, int kBStage, int kRegion, int kOne, int kW, class NOf>
+template <bool SPLIT, int kA, int kAStage, int kB, int kBStage, int kRegion, int kOne, int kW, class NOf>
 __device__ __forceinline__ bool f4_pair_issue(long long items, uint32_t a0, uint32_t b0, uint32_t full0,
                                               uint32_t empty0, uint32_t acc_full0, uint32_t acc_empty0, uint32_t tmem,
                                               int nw_c, int nw_t, volatile int* abort, NOf&& n_of) {
@@ -58,17 +60,17 @@ __device__ __forceinline__ bool f4_pair_issue(long long items, uint32_t a0, uint
     const uint32_t one = tmem + (uint32_t)kOne;
     uint32_t fbar = 0, ad = desc_a, par = 0;  // A stage: barrier offset, descriptor, parity
     uint32_t ebar = 0, bd = desc_b;           // B stage
-    for (unsigned item = 0; item < items; ++item) {
+    for (unsigned item = 0; item < (SPLIT ? 2 : 1) * items; ++item) {
         const unsigned buf = item & 1;
         if (item >= 2 && !t3_wait_cl(acc_empty0 + 8 * buf, ((item >> 1) - 1) & 1, abort)) return false;
         const uint32_t dcol = tmem + (uint32_t)(kRegion * buf);
         uint32_t acc = 0, idesc = 0;
-        for (int cls = 0; cls < 2; ++cls) {
-            const uint32_t sfb = tmem + (uint32_t)(cls ? kW : kOne);
+        for (int cls = SPLIT ? (int)buf : 0; cls < (SPLIT ? (int)buf + 1 : 2); ++cls) {
+            const uint32_t sfb = tmem + (uint32_t)(cls && !SPLIT ? kW : kOne);
             for (int left = cls ? nw_t : nw_c; left > 0; left -= 4) {
                 if (!t3_wait_cl(full0 + fbar, par, abort)) return false;  // both CTAs' A and B are in place
                 asm volatile("tcgen05.fence::after_thread_sync;");
-                if (!acc) idesc = f4_idesc(256, n_of(item));
+                if (!acc) idesc = f4_idesc(256, n_of(SPLIT ? item >> 1 : item));
                 auto mma = [&](int k) {
                     f4_mma<2>(dcol, (uint64_t)desc_hi << 32 | (ad + 2 * k), (uint64_t)desc_hi << 32 | (bd + 2 * k),
                               idesc, one, sfb, acc);
@@ -84,7 +86,7 @@ __device__ __forceinline__ bool f4_pair_issue(long long items, uint32_t a0, uint
                 }
                 commit_pair(empty0 + ebar);
                 fbar += 8;
-                ad += 16384 >> 4;
+                ad += kAStage >> 4;
                 if (fbar == 8 * kA) {
                     fbar = 0;
                     ad = desc_a;
@@ -132,6 +134,11 @@ __device__ __forceinline__ uint4 f4_expand_a(uint32_t i, uint32_t j) {
 __device__ __forceinline__ uint4 f4_expand_b(uint32_t w) {
     const uint32_t v = w >> 2;
     return make_uint4((w << 2) & 0x44444444u, w & 0x22222222u, v & 0x11111111u, v & 0x22222222u);
+}
+
+// 1.0 wherever a bit is set: planes that both operands of an MMA are read from.
+__device__ __forceinline__ uint4 f4_expand_ones(uint32_t w) {
+    return make_uint4((w << 1) & 0x22222222u, w & 0x22222222u, (w >> 1) & 0x22222222u, (w >> 2) & 0x22222222u);
 }
 
 // Row of SNP l, genotype z in the operand planes: SNPs in groups of 8, the
@@ -224,13 +231,16 @@ struct F4Bound {
         acc = f2_fma(b, f2_mul(b, f2_rcp(s)), acc);
     }
     // two cells with one reciprocal: (b1^2 s2 + b2^2 s1) / (s1 s2)
+    __device__ __forceinline__ void two(f2 b1, f2 s1, f2 b2, f2 s2) {
+        const f2 r = f2_rcp(f2_mul(s1, s2));
+        const f2 num = f2_fma(f2_mul(b1, b1), s2, f2_mul(f2_mul(b2, b2), s1));
+        acc = f2_fma(num, r, acc);
+    }
     __device__ __forceinline__ void two(f2 D1, f2 D2) {
         f2 b1, s1, b2, s2;
         split(D1, b1, s1);
         split(D2, b2, s2);
-        const f2 r = f2_rcp(f2_mul(s1, s2));
-        const f2 num = f2_fma(f2_mul(b1, b1), s2, f2_mul(f2_mul(b2, b2), s1));
-        acc = f2_fma(num, r, acc);
+        two(b1, s1, b2, s2);
     }
 };
 

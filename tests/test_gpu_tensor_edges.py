@@ -96,3 +96,38 @@ def test_threshold_raised_in_the_kernel_keeps_the_list(order, snps, outputs):
     if outputs < 100:
         parts.sort(key=lambda r: (-r.val, r.combination))
         assert [r.val for r in parts[:outputs]] == [r.val for r in b]
+
+
+EDGES_2 = [  # snps, cases, controls; the last four do not share an accumulator
+    (2, 1, 1), (8, 64, 65), (9, 63, 256), (65, 257, 129), (121, 65, 300), (129, 1023, 40), (241, 2047, 2049),
+    (2, 4100, 4100), (121, 9000, 9800), (130, 300, 65000), (250, 8000, 8000),
+]
+
+
+@pytest.mark.parametrize("snps,cases,ctrls", EDGES_2)
+def test_order2_tile_edges(oracle, snps, cases, ctrls):
+    _check(2, snps, cases, ctrls, oracle)
+
+
+@pytest.mark.parametrize("snps,step,offset", [(130, 2, 1), (263, 3, 0), (66, 67, 5), (260, 5, 4)])
+@pytest.mark.parametrize("cases,ctrls", [(130, 199), (4100, 4101)])
+def test_order2_layer_edges(oracle, snps, step, offset, cases, ctrls):
+    from fiuncho_gb300 import Distribution
+    _check(2, snps, cases, ctrls, oracle, Distribution(snps, 1, step, offset))
+
+
+@pytest.mark.parametrize("order,snps,cases,ctrls", [(2, 1900, 4100, 4100), (2, 2100, 300, 290)])
+def test_several_items_per_pair(order, snps, cases, ctrls):
+    """More items than CTA pairs, so that accumulators, stashes and tables are used again: every table and
+    the list against a kernel that shares no code path."""
+    from fiuncho_gb300 import Distribution, GpuSearch, _lib
+    from fiuncho_gb300.search import Resident
+    gs = GpuSearch(0)
+    res = Resident(gs.ctx, _data(snps, cases, ctrls, 3 * snps))
+    assert gs.scan_digest(res, order, kernel=_lib.KERNEL_TENSOR) == \
+        gs.scan_digest(res, order, kernel=_lib.KERNEL_ELIDED_HS)
+    lists = []
+    for kernel in (_lib.KERNEL_TENSOR, _lib.KERNEL_ELIDED_HS):
+        gs.set_kernel(kernel)
+        lists.append([(r.combination, r.val) for r in gs.run(res, order, Distribution(snps, order - 1), 1000)])
+    assert lists[0] == lists[1]
