@@ -239,9 +239,8 @@ int choose_tile(fiu_ctx* ctx, const fiu_resident* res, const ScanWork& w, int re
             tensor3_prepare(r->d, *plan);
             r->t3 = plan;
         }
-        // the core tables; the order-4 pair kernel makes its triples itself
-        const unsigned cores = w.order == 4 && r->t3->pair3 ? 3u : (unsigned)w.order;
-        int rc = choose_kernel(ctx, res, cores, FIU_KERNEL_ELIDED_HS, kernel);
+        // the single and pair cores (order 4 makes its triples itself)
+        int rc = choose_kernel(ctx, res, std::min(3u, (unsigned)w.order), FIU_KERNEL_ELIDED_HS, kernel);
         if (rc) return rc;
         if (!whole_data_set(res, w)) {
             cudaError_t e = tensor3_layer(*r->t3, w, res->pairs, ctx->stream, ctx->sms);
@@ -251,8 +250,8 @@ int choose_tile(fiu_ctx* ctx, const fiu_resident* res, const ScanWork& w, int re
             if (e != cudaSuccess) return cuda_fail(ctx, e, "tensor operands and work items");
         }
         kernel = FIU_KERNEL_TENSOR;
-        // GEMM width N: order 3 uses 256 with one accumulator for both classes, 192 with one per class
-        tp = (w.order != 3 || r->t3->pair3) ? 256 : 192;
+        // the tile class reported by fiu_last_tile: 192 names order 3 with one accumulator per class
+        tp = w.order != 3 || r->t3->f4.pack ? 256 : 192;
         return FIU_OK;
     }
     int rc = choose_kernel(ctx, res, (unsigned)w.order, requested_kernel, kernel);
@@ -351,9 +350,8 @@ int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu
     int* t_status = (int*)(ctx->ctl + 16);
     if (tensor) CK(cudaMemsetAsync(t_status, 0, sizeof(int), ctx->stream), "status reset");
     const unsigned keep = outputs + std::max(32u, outputs / 8);
-    const bool live = tensor && tensor_live(*res->t3, w);
     const size_t cap = std::max<size_t>(
-        {live ? 524288u : 65536u, (size_t)(live ? 128 : 16) * keep, (size_t)res->d.snps + keep});
+        {tensor ? 524288u : 65536u, (size_t)(tensor ? 128 : 16) * keep, (size_t)res->d.snps + keep});
     if ((rc = grow(ctx, ctx->cand, ctx->cand_cap, cap + 8192)) ||
         (rc = grow(ctx, ctx->tmp, ctx->tmp_cap, cap + 8192)) ||
         (rc = grow(ctx, ctx->mi64, ctx->mi64_cap, (size_t)keep)))
@@ -389,7 +387,7 @@ int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu
     // large request the second is one unit per CTA pair (the first units may hold few combinations:
     // the order-2 tiles on the diagonal), so that no launch starts all pairs on a weak threshold.  A
     // buffer that overflows all the same leaves the request to the loop below.
-    if (live && !ctx->cancellable && m < m_end) {
+    if (tensor && !ctx->cancellable && m < m_end) {
         const long long few = std::max<long long>(1, (long long)(2.0 * keep / std::max(1.0, per_unit)));
         const long long fit = (long long)((double)cap / 4 / std::max(1.0, per_unit));
         const long long m1 = std::min(m_end, m + std::max(few, std::min<long long>(fit, ctx->sms / 2)));
@@ -402,16 +400,14 @@ int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu
         sink.live = live_thr;
         sink.keep = keep;
         if (ctx->timing) CK(cudaEventRecord(ctx->ev0, s), "event");
-        CK(launch_tensor3(w, *res->t3, m, m1, sink, nullptr, res->single, res->pairs, res->triples, t_status, s,
-                          ctx->sms),
+        CK(launch_tensor3(w, *res->t3, m, m1, sink, nullptr, res->single, res->pairs, t_status, s, ctx->sms),
            "tensor kernel launch");
         unsigned launches = 1;
         sink.thr = 0;  // (from here on the kernel reads the live threshold; one exists)
         for (long long a = m1; a < m_end; ++launches) {
             const long long wave = ctx->sms / 2, b = launches == 1 && m_end - a > 16 * wave ? a + wave : m_end;
             CK(live_raise(sink, s), "threshold");
-            CK(launch_tensor3(w, *res->t3, a, b, sink, nullptr, res->single, res->pairs, res->triples, t_status, s,
-                              ctx->sms),
+            CK(launch_tensor3(w, *res->t3, a, b, sink, nullptr, res->single, res->pairs, t_status, s, ctx->sms),
                "tensor kernel launch");
             a = b;
         }
@@ -447,7 +443,7 @@ int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu
         memcpy(ctx->pinned + 2, &thr, sizeof(thr));
         CK(cudaMemcpyAsync(count, ctx->pinned, 4 * sizeof(unsigned), cudaMemcpyHostToDevice, s), "reset counters");
         CandSink sink{ctx->cand, count, overflow, (unsigned)cap, thr, ctx->timing ? ctx->evaluated : nullptr};
-        if (live) {
+        if (tensor) {
             CK(cudaMemsetAsync(hist, 0, kLiveBins * sizeof(unsigned), s), "reset counters");
             sink.hist = hist;
             sink.live = live_thr;
@@ -455,8 +451,7 @@ int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu
         }
         if (ctx->timing) CK(cudaEventRecord(ctx->ev0, s), "event");
         if (tensor)
-            CK(launch_tensor3(w, *res->t3, m, m1, sink, nullptr, res->single, res->pairs, res->triples, t_status, s,
-                              ctx->sms),
+            CK(launch_tensor3(w, *res->t3, m, m1, sink, nullptr, res->single, res->pairs, t_status, s, ctx->sms),
                "tensor kernel launch");
         else if (pair_major)
             CK(launch_elided4p(w, res->e4_begin, m, m1, sink, nullptr, res->single, res->pairs, res->triples, s,
@@ -982,7 +977,7 @@ int fiu_scan_tables(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const
         e = cudaMemsetAsync(ctx->ctl + 16, 0, sizeof(int), s);
         if (e == cudaSuccess)
             e = launch_tensor3(w, *res->t3, 0, tensor_units(*res->t3, w), sink, d, res->single, res->pairs,
-                               res->triples, (int*)(ctx->ctl + 16), s, ctx->sms);
+                               (int*)(ctx->ctl + 16), s, ctx->sms);
     } else if (e == cudaSuccess && e4_pair_major(kernel, res, w)) {
         if ((rc = ensure_e4_items(ctx, res))) {
             cudaFreeAsync(d, s);
@@ -1041,8 +1036,7 @@ int fiu_scan_digest(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const
                   d, sc, threads};
     if (e == cudaSuccess) {
         if (tensor)
-            e = launch_tensor3(w, *res->t3, 0, units, sink, nullptr, res->single, res->pairs, res->triples, t_status, s,
-                               ctx->sms);
+            e = launch_tensor3(w, *res->t3, 0, units, sink, nullptr, res->single, res->pairs, t_status, s, ctx->sms);
         else if (pair_major)
             e = launch_elided4p(w, res->e4_begin, 0, units, sink, nullptr, res->single, res->pairs, res->triples, s,
                                 ctx->sms);

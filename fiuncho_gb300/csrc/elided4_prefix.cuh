@@ -49,37 +49,7 @@ __device__ __forceinline__ void star_to_table(uint32_t* t) {
     for (int yz = 0; yz < 9; ++yz) t[18 + yz] -= t[yz] + t[9 + yz];
 }
 
-// Cell (x, y, z) of one class's triple word (8 uint16: [x][y][z]).
-__device__ __forceinline__ uint32_t tcell(const uint4& v, int x, int y, int z) {
-    const int q = x * 4 + y * 2 + z;
-    const uint32_t wv = (&v.x)[q >> 1];
-    return (q & 1) ? (wv >> 16) : (wv & 0xffffu);
-}
-
-// Value of pass PC (0 cases, 1 controls, 2 both classes summed) from a
-// per-class pair of values.
-// Sum of 27 floats, pairwise (every term takes part in at most 5 roundings).
-__device__ __forceinline__ float e4_sum27(const float* f) {
-    float a[14];
-#pragma unroll
-    for (int q = 0; q < 13; ++q) a[q] = f[2 * q] + f[2 * q + 1];
-    a[13] = f[26];
-    float b[7];
-#pragma unroll
-    for (int q = 0; q < 7; ++q) b[q] = a[2 * q] + a[2 * q + 1];
-    const float c0 = b[0] + b[1], c1 = b[2] + b[3], c2 = b[4] + b[5], c3 = b[6];
-    return (c0 + c1) + (c2 + c3);
-}
-
-template <int PC>
-__device__ __forceinline__ uint32_t by_pass(uint32_t a, uint32_t b) {
-    return PC == 0 ? a : PC == 1 ? b : a + b;
-}
-
 // Locations of the sub-combination cores of one combination (i, j, k, l).
-// Each pass loads what it reads itself, after a compiler memory barrier, so
-// that the loads of a pass are not hoisted above the previous one (fewer
-// registers held across the passes; the reloads hit L1).
 struct E4Src {
     const uint4* tij;  // triple (i,j,l): two words, cases then controls
     const uint4* tik;  // triple (i,k,l)
@@ -89,68 +59,6 @@ struct E4Src {
     const uint4* pkl;
     const uint4* sl;   // single l: [class][x]
 };
-
-// Sub-combination cores of one combination as read by one pass PC: the triple
-// words of the pass's class (ta: cases, or controls for PC 1; tb: controls for
-// PC 2, else zero) of (i,j,l), (i,k,l), (j,k,l), and the pair / single words.
-struct E4Words {
-    uint4 ta[3], tb[3];
-    uint4 pil, pjl, pkl, sl;
-};
-
-template <int PC>
-__device__ __forceinline__ E4Words e4_load(const E4Src& src) {
-    asm volatile("" ::: "memory");
-    E4Words wd;
-    const uint4* tp[3] = {src.tij, src.tik, src.tjk};
-#pragma unroll
-    for (int u = 0; u < 3; ++u) {
-        wd.ta[u] = __ldg(tp[u] + (PC == 1 ? 1 : 0));
-        wd.tb[u] = PC == 2 ? __ldg(tp[u] + 1) : make_uint4(0, 0, 0, 0);
-    }
-    wd.pil = __ldg(src.pil);
-    wd.pjl = __ldg(src.pjl);
-    wd.pkl = __ldg(src.pkl);
-    wd.sl = __ldg(src.sl);
-    return wd;
-}
-
-// One pass over the 81 cells: the slices l = 0, 1, 2, each an order-3
-// derivation from its star table (slice 2's is the prefix's star table,
-// pstar(q), minus slices 0 and 1: the derivation is linear); use(sw, t)
-// receives each slice's 27 cells t[(x*3+y)*3+z] (cell index
-// ((x*3+y)*3+z)*3 + sw).  The counted cores arrive packed:
-// cp[cls][r] = core (r, w=0) | core (r, w=1) << 16.
-template <int PC, class PStar, class Use>
-__device__ __forceinline__ void e4_slices_w(const uint32_t (&cp)[2][8], const E4Words& wd, const PStar& pstar,
-                                            Use&& use) {
-    auto tri = [&](int u, int x, int y, int z) {
-        return PC == 2 ? tcell(wd.ta[u], x, y, z) + tcell(wd.tb[u], x, y, z) : tcell(wd.ta[u], x, y, z);
-    };
-    auto pr = [&](const uint4& v, int x, int y) { return by_pass<PC>(pcore(v, 0, x, y), pcore(v, 1, x, y)); };
-    auto star = [&](int w, int q) -> uint32_t {
-        const int a = q / 9, b = (q / 3) % 3, z = q % 3;
-        if (a < 2 && b < 2 && z < 2) {
-            const int r = (a * 2 + b) * 2 + z;
-            return by_pass<PC>(w ? cp[0][r] >> 16 : cp[0][r] & 0xffffu, w ? cp[1][r] >> 16 : cp[1][r] & 0xffffu);
-        }
-        if (a < 2 && b < 2) return tri(0, a, b, w);
-        if (a < 2 && z < 2) return tri(1, a, z, w);
-        if (b < 2 && z < 2) return tri(2, b, z, w);
-        if (a < 2) return pr(wd.pil, a, w);
-        if (b < 2) return pr(wd.pjl, b, w);
-        if (z < 2) return pr(wd.pkl, z, w);
-        return by_pass<PC>(w ? wd.sl.y : wd.sl.x, w ? wd.sl.w : wd.sl.z);
-    };
-#pragma unroll
-    for (int sw = 0; sw < 3; ++sw) {
-        uint32_t t[27];
-#pragma unroll
-        for (int q = 0; q < 27; ++q) t[q] = sw < 2 ? star(sw, q) : pstar(q) - star(0, q) - star(1, q);
-        star_to_table(t);
-        use(sw, t);
-    }
-}
 
 // Both classes in one derivation, packed: a cell's case count in the low and
 // its control count in the high 16 bits of one word.  Every count lies below
@@ -203,96 +111,11 @@ __device__ __forceinline__ void e4_slices_packed(const uint32_t (&cp)[2][8], con
     }
 }
 
-// One slice's contribution to the key estimate, cell by cell, in units of
-// 2^-16 bits: the pairwise single-precision sum over its 27 packed cells of
-// g = a lg2 a + b lg2 b - (a+b) lg2 (a+b) (a cases, b controls; each g lies in
-// [-(a+b), 0]), rounded to 2^-16.  Each 16-bit half becomes the float 2^23 + c
-// by a byte permutation, minus 2^23.
-__device__ __forceinline__ long long e4_slice_estimate_packed(const uint32_t* t) {
-    const float tiny = 9.5367431640625e-07f;  // 2^-20: c*lg2(c + tiny) = 0 at c = 0
-    float g[27];
-#pragma unroll
-    for (int q = 0; q < 27; ++q) {
-        const float a = __uint_as_float(__byte_perm(t[q], 0x4B000000u, 0x7610)) - 8388608.0f;
-        const float b = __uint_as_float(__byte_perm(t[q], 0x4B000000u, 0x7632)) - 8388608.0f;
-        const float sab = a + b;
-        float la, lb, ls;
-        asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(la) : "f"(a + tiny));
-        asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(lb) : "f"(b + tiny));
-        asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(ls) : "f"(sab + tiny));
-        g[q] = fmaf(a, la, fmaf(b, lb, -sab * ls));
-    }
-    return __float2ll_rn(e4_sum27(g) * 65536.0f);
-}
-
-// The same with the words loaded from their locations (the loads of a pass are
-// not hoisted above the previous pass: fewer registers held across passes).
-template <int PC, class PStar, class Use>
-__device__ __forceinline__ void e4_slices(const uint32_t (&cp)[2][8], const E4Src& src, const PStar& pstar,
-                                          Use&& use) {
-    const E4Words wd = e4_load<PC>(src);
-    e4_slices_w<PC>(cp, wd, pstar, use);
-}
-
-// One pass of the exact key: the sum of T[cell] over the pass's 81 cells;
-// writes the cells to o[PC * 81 + ((x*3+y)*3+z)*3 + w] if o (cases, controls).
-template <int PC, class PStar>
-__device__ __forceinline__ long long e4_pass(const uint32_t (&cp)[2][8], const E4Src& src, const PStar& pstar,
-                                             const long long* __restrict__ ftab, uint32_t nc, uint32_t* o) {
-    long long part = 0;
-    e4_slices<PC>(cp, src, pstar, [&](int sw, const uint32_t* t) {
-        // derived cells of consistent one-hot data never exceed the class
-        // size; the clamp keeps any inconsistency inside the table
-#pragma unroll
-        for (int q = 0; q < 27; ++q) part += __ldg(ftab + min(t[q], nc));
-        if (PC < 2 && o) {
-#pragma unroll
-            for (int q = 0; q < 27; ++q) o[PC * 81 + q * 3 + sw] = t[q];
-        }
-    });
-    return part;
-}
-
 // Locations of the sub-combination cores of a prefix triple (i, j, k).
 struct E4Prefix {
     const uint4* tijk;             // triple (i,j,k): cases word, controls word
     const uint4 *pij, *pik, *pjk;  // pairs
     const uint4 *si, *sj, *sk;     // singles
-};
-
-// Star table of the prefix triple for pass PC, entry q; nc = the pass's class size.
-template <int PC>
-struct E4PrefixStar {
-    uint4 ta, tb, pij, pik, pjk, si, sj, sk;
-    uint32_t nc;
-    __device__ __forceinline__ E4PrefixStar(const E4Prefix& pre, uint32_t n) : nc(n) {
-        asm volatile("" ::: "memory");
-        ta = __ldg(pre.tijk + (PC == 1 ? 1 : 0));
-        tb = PC == 2 ? __ldg(pre.tijk + 1) : make_uint4(0, 0, 0, 0);
-        pij = __ldg(pre.pij);
-        pik = __ldg(pre.pik);
-        pjk = __ldg(pre.pjk);
-        si = __ldg(pre.si);
-        sj = __ldg(pre.sj);
-        sk = __ldg(pre.sk);
-    }
-    __device__ __forceinline__ uint32_t pr(const uint4& v, int x, int y) const {
-        return by_pass<PC>(pcore(v, 0, x, y), pcore(v, 1, x, y));
-    }
-    __device__ __forceinline__ uint32_t sg(const uint4& v, int x) const {
-        return by_pass<PC>(x ? v.y : v.x, x ? v.w : v.z);
-    }
-    __device__ __forceinline__ uint32_t operator()(int q) const {
-        const int a = q / 9, b = (q / 3) % 3, z = q % 3;
-        if (a < 2 && b < 2 && z < 2) return PC == 2 ? tcell(ta, a, b, z) + tcell(tb, a, b, z) : tcell(ta, a, b, z);
-        if (a < 2 && b < 2) return pr(pij, a, b);
-        if (a < 2 && z < 2) return pr(pik, a, z);
-        if (b < 2 && z < 2) return pr(pjk, b, z);
-        if (a < 2) return sg(si, a);
-        if (b < 2) return sg(sj, b);
-        if (z < 2) return sg(sk, z);
-        return nc;
-    }
 };
 
 // Packed star table of the prefix triple (i, j, k) (both classes), entry q,
@@ -353,10 +176,8 @@ __device__ __forceinline__ E4PrefixStarPacked e4_prefix_packed(const E4Prefix& p
 // The exact key of one combination (minus the base) from one packed
 // derivation of both classes: the sum over the 81 cells of
 // T[a] + T[b] - T[a + b] (a cases, b controls; each clamped to its class
-// size, so that an inconsistent input stays inside the table).  Equal to the
-// three passes e4_pass<0> + e4_pass<1> - e4_pass<2> on consistent one-hot
-// data; writes the tables to o (cases at o[q*3+sw], controls at
-// o[81+q*3+sw]) if o.
+// size, so that an inconsistent input stays inside the table); writes the
+// tables to o (cases at o[q*3+sw], controls at o[81+q*3+sw]) if o.
 template <class PS>
 __device__ __forceinline__ long long e4_exact_packed(const uint32_t (&cp)[2][8], const E4Both& wd, const PS& ps,
                                                      const long long* __restrict__ ftab, uint32_t n0, uint32_t n1,
@@ -377,14 +198,6 @@ __device__ __forceinline__ long long e4_exact_packed(const uint32_t (&cp)[2][8],
         }
     });
     return part;
-}
-
-// Exact pass with the prefix star table computed from the prefix's cores.
-template <int PC>
-__device__ __forceinline__ long long e4p_pass(const uint32_t (&cp)[2][8], const E4Src& src, const E4Prefix& pre,
-                                              const long long* __restrict__ ftab, uint32_t nc, uint32_t* o) {
-    const E4PrefixStar<PC> ps(pre, nc);
-    return e4_pass<PC>(cp, src, ps, ftab, nc, o);
 }
 
 // One prefix (owned ordinal m): the TP threads of group grp, one last SNP per

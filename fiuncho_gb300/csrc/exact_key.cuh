@@ -1,45 +1,80 @@
-// The exact fixed-point key of one combination, by one warp, from the data set
-// itself: lane c counts the cells c, c + 32, .. of the 3^K table (an AND and a
-// popcount a word).  For kernels that meet so few combinations above their bound
-// that keeping the tables' derivation beside the bound's would cost more.
+// The exact fixed-point key of one order-4 combination, by one warp, from the
+// data set itself, for a kernel that meets few combinations above its bound and
+// would pay more for keeping the tables' derivation beside the bound's.
+//
+// Bound by the latency of its loads: lanes are (genotype x of the first SNP,
+// word mod 8), so a step brings ten words a lane, all independent, from rows read
+// 64 bytes at a time, and the next step's are on their way while the 27 cells of
+// x are counted.  With a lane per cell instead (three of the 81 in turn, four
+// loads in flight) a key of 18 800 samples took 70 us.
 #pragma once
 
 #include "internal.h"
 
 namespace fiu {
 
-template <int K>
-__device__ __noinline__ long long warp_exact_key(const DevData* dp, long long base_key, int c0, int c1, int c2,
-                                                 int c3) {
+__device__ __noinline__ long long warp_exact_key4(const DevData* dp, long long base_key, int c0, int c1, int c2,
+                                                  int c3) {
     const DevData& d = *dp;
-    const int lane = threadIdx.x & 31;
-    constexpr int kCells = K == 4 ? 81 : 27;
+    const int lane = threadIdx.x & 31, x = lane >> 3, wl = lane & 7;  // x == 3: idle
     const size_t per_snp = 3 * (size_t)(d.cw + d.tw);
-    const int cmb[4] = {c0, c1, c2, c3};
-    long long key = 0;
-    for (int cell = lane; cell < kCells; cell += 32) {
-        const uint64_t* row[K];
-        uint32_t cnt[2];
+    uint32_t cnt[28];  // cells (y, z, g): cases | controls << 16, each at most 65535
 #pragma unroll
-        for (int cls = 0; cls < 2; ++cls) {
-            const int W = cls ? d.tw : d.cw;
-            int r = cell;
+    for (int c = 0; c < 28; ++c) cnt[c] = 0;
+#pragma unroll 1
+    for (int cls = 0; cls < 2; ++cls) {
+        const int W = x < 3 ? (cls ? d.tw : d.cw) : 0;
+        const size_t at = (cls ? 3 * (size_t)d.cw : 0) + wl;
+        const uint64_t* r0 = d.ref + (size_t)c0 * per_snp + at + (size_t)x * W;
+        const uint64_t* r1 = d.ref + (size_t)c1 * per_snp + at;
+        const uint64_t* r2 = d.ref + (size_t)c2 * per_snp + at;
+        const uint64_t* r3 = d.ref + (size_t)c3 * per_snp + at;
+        const uint32_t one = cls ? 1u << 16 : 1u;
+        uint64_t v[10];
+        auto load = [&](int w) {
+            v[0] = __ldg(r0 + w);
 #pragma unroll
-            for (int t = K - 1; t >= 0; --t) {  // first SNP most significant
-                row[t] = d.ref + (size_t)cmb[t] * per_snp + (cls ? 3 * (size_t)d.cw : 0) + (size_t)(r % 3) * W;
-                r /= 3;
+            for (int g = 0; g < 3; ++g) {
+                v[1 + g] = __ldg(r1 + g * W + w);
+                v[4 + g] = __ldg(r2 + g * W + w);
+                v[7 + g] = __ldg(r3 + g * W + w);
             }
-            uint32_t n = 0;
-#pragma unroll 4
-            for (int w = 0; w < W; ++w) {
-                uint64_t v = __ldg(row[0] + w);
+        };
+        if (wl < W) load(0);
+#pragma unroll 1
+        for (int w = 0; w + wl < W; w += 8) {
+            uint64_t u[10];
 #pragma unroll
-                for (int t = 1; t < K; ++t) v &= __ldg(row[t] + w);
-                n += (uint32_t)__popcll(v);
+            for (int e = 0; e < 10; ++e) u[e] = v[e];
+            if (w + 8 + wl < W) load(w + 8);
+#pragma unroll
+            for (int y = 0; y < 3; ++y) {
+                const uint64_t a = u[0] & u[1 + y];
+#pragma unroll
+                for (int z = 0; z < 3; ++z) {
+                    const uint64_t b = a & u[4 + z];
+#pragma unroll
+                    for (int g = 0; g < 3; ++g)
+                        cnt[9 * y + 3 * z + g] += (uint32_t)__popcll(b & u[7 + g]) * one;
+                }
             }
-            cnt[cls] = n;
         }
-        key += __ldg(d.ftab + cnt[0]) + __ldg(d.ftab + cnt[1]) - __ldg(d.ftab + cnt[0] + cnt[1]);
+    }
+    __syncwarp();
+    long long key = 0;
+#pragma unroll
+    for (int c = 0; c < 27; ++c) {  // over the eight lanes of an x; each then takes the cells wl, wl + 8, ..
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) cnt[c] += __shfl_xor_sync(0xffffffffu, cnt[c], o);
+    }
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        uint32_t v = 0;
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+            if (8 * s + c < 27 && wl == c) v = cnt[8 * s + c];
+        const uint32_t a = v & 0xffffu, b = v >> 16;
+        key += __ldg(d.ftab + a) + __ldg(d.ftab + b) - __ldg(d.ftab + a + b);  // 0 of an empty cell
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) key += __shfl_xor_sync(0xffffffffu, key, o);

@@ -178,8 +178,8 @@ cudaError_t launch_elided4p(const ScanWork& w, const long long* begin, long long
                             const CandSink& sink, uint32_t* dump, const uint32_t* single, const uint4* pairs,
                             const uint4* triples, cudaStream_t s, int sms);
 
-// tensor2x.cu, tensor3x.cu, tensor4x.cu (4-bit operands, CTA pairs) and tensor3.cu, tensor4.cu (per-class
-// e4m3 kernels of orders 3 and 4) -- core cells on tcgen05 (one-hot data, the whole data set or a layer of it).
+// tensor2x.cu, tensor3x.cu, tensor4x.cu (4-bit operands, CTA pairs) and tensor3.cu (their host side) -- core
+// cells on tcgen05 (one-hot data, the whole data set or a layer of it).
 // Device state of the tensor kernels for one data set: operand planes, made on the first search of an
 // order, their TMA descriptors and the work-item prefix sums.
 // 4-bit operand layout of a data set (tensor_fp4.cuh, tensor3x.cu): e2m1 planes
@@ -195,8 +195,8 @@ struct F4Plan {
     CUtensorMap map_j, map_i;   // bit rows, boxes of 32 B x 64 and x 2 rows
     uint8_t* ones = nullptr;    // order 2: planes of 1.0 where a genotype is, both operands
     CUtensorMap map_a2, map_b2; // over them, boxes 128 B x 128 and x 120 rows
-    // order 4: the cores of all triples and pairs as packed floats, cases + W controls, of (l, l + 1)
-    // side by side; the entry of (.., k, l) is row_p[k] + l / 2, of (i, k, l) also + row_q[i]
+    // order 4: the cores of all triples and pairs, for (l, l + 1): packed floats, cases + W controls, side by
+    // side, or (pack 0) words cases | controls << 16, those of l first; the entry of (.., k, l) is row_p[k] + l / 2, of (i, k, l) also + row_q[i]
     float* tri = nullptr;       // 16 floats an entry: (x, z, w) of the genotypes of i, k and l
     float* pairf = nullptr;     // 8 floats an entry: (z, w)
     int *row_p = nullptr, *row_q = nullptr;
@@ -205,42 +205,31 @@ struct F4Plan {
 struct T3Plan {
     std::mutex items_mu;  // guards the planes and item tables made on the first use of an order
     F4Plan f4;
-    uint8_t* planes = nullptr;
-    double item_combos = 0;  // combinations per work item
-    int pitch = 0;        // bytes per plane row
-    int k_cases = 0;      // padded case samples (= byte offset of the control region)
-    bool pair3 = false;   // orders 3 and 4, classes that share an accumulator: items of the CTA-pair kernels
-    struct T3Layers* layers = nullptr;  // order 3, packed: work items of Distribution layers (tensor3.cu)
+    double item_combos = 0;             // combinations per work item
+    struct T3Layers* layers = nullptr;  // work items of Distribution layers (tensor3.cu)
     long long* item_begin = nullptr;
     long long total = 0;  // work items
-    CUtensorMap map_l;    // box 128 B x 192 rows, 128-byte swizzle (l operand)
-    CUtensorMap map_j;    // box 128 B x 64 rows, 128-byte swizzle (j rows of the (i,j) operand)
-    CUtensorMap map_i;    // box 128 B x 2 rows, 128-byte swizzle (i rows)
     // order 2: work items (128 i, 120 j) of the pair kernel, first of each band
     long long* item2_begin = nullptr;
     long long total2 = 0;
     int n_itiles = 0;
     double item2_combos = 0;
-    // order 4: work items (i, j, 32 k, up to 112 l) of the pair kernel, or (i, j, 16 k, 64 l) per class;
+    // order 4: work items (i, j, 32 k, up to 112 l);
     // item4_begin[j] = first item of the pairs with second SNP j, item4_per[j] = items per such pair
     long long* item4_begin = nullptr;
     long long* item4_per = nullptr;
     long long total4 = 0;
     double item4_combos = 0;
-    CUtensorMap map_l4;   // box 128 B x 128 rows (l rows)
-    CUtensorMap map_k4;   // box 128 B x 32 rows (k rows)
 };
 // Work units of a request on the tensor kernels (w's order and Distribution
 // layer; a layer's items must have been made by tensor3_layer), and the
 // combinations of an average unit.
 long long tensor_units(const T3Plan& plan, const ScanWork& w);
 double tensor_item_combos(const T3Plan& plan, const ScanWork& w);
-// Whether the kernel that serves w takes a live threshold (CandSink::hist).
-bool tensor_live(const T3Plan& plan, const ScanWork& w);
-// Whether the tensor kernels serve the Distribution layer of w (order 3,
-// classes that pack, the layer of all SNPs), and the layer's work items,
-// made on first use (host enumeration of the owned prefixes; the operand
-// planes ordered by SNP residue mod the layer's step, copied on stream s).
+// Whether the tensor kernels serve the Distribution layer of w (the layer of
+// all SNPs), and the layer's work items, made on first use (host enumeration
+// of the owned prefixes; the bit rows ordered by SNP residue mod the layer's
+// step, copied on stream s).
 bool tensor_layer_ok(const T3Plan& plan, const ScanWork& w);
 cudaError_t tensor3_layer(T3Plan& plan, const ScanWork& w, const uint4* pairs, cudaStream_t s, int sms);
 void tensor3_prepare(const DevData& d, T3Plan& plan);
@@ -253,21 +242,13 @@ cudaError_t tensor_map(CUtensorMap* m, const void* base, int rows, int pitch, in
                        bool swizzle);
 void tensor3_release(T3Plan& plan);
 cudaError_t launch_tensor3(const ScanWork& w, const T3Plan& plan, long long g0, long long g1, const CandSink& sink,
-                           uint32_t* dump, const uint32_t* single, const uint4* pairs, const uint4* triples,
-                           int* status, cudaStream_t s, int sms);
-// tensor4.cu -- order 4 on tcgen05 (one-hot data, the whole data set or a Distribution layer of it).
-// Item tables of the pair kernel (pair) or the per-class kernel.
-std::vector<long long> t4_item_table(int n, bool pair, std::vector<long long>& per);
-long long t4_layer_items(int n, int step, long long offset, bool pair, std::vector<long long>& pbegin,
+                           uint32_t* dump, const uint32_t* single, const uint4* pairs, int* status, cudaStream_t s,
+                           int sms);
+// tensor4x.cu -- order 4 on tcgen05 (one-hot data, the whole data set or a Distribution layer of it).
+// Item tables of the whole data set, and of a layer (the listed pairs (i, j) with their first owned k).
+std::vector<long long> t4_item_table(int n, std::vector<long long>& per);
+long long t4_layer_items(int n, int step, long long offset, std::vector<long long>& pbegin,
                          std::vector<int4>& pinfo, long long& combos);
-// pinfo / n_pairs: a layer's pair tables (begin = their first items, per unused; map_k over the
-// residue-ordered planes), else nullptr
-cudaError_t launch_tensor4(const ScanWork& w, const CUtensorMap& map_l, const CUtensorMap& map_k,
-                           const CUtensorMap& map_i, const long long* begin, const long long* per, int k_cases,
-                           long long g0, long long g1,
-                           const CandSink& sink, uint32_t* dump, const uint32_t* single, const uint4* pairs,
-                           const uint4* triples, int* status, cudaStream_t s, int sms, const int4* pinfo = nullptr,
-                           int n_pairs = 0);
 // Largest absolute error of the kernel's single-precision log2 over all its inputs (counts <= max_c).
 cudaError_t probe_lg2_error(unsigned max_c, double* max_abs_err, cudaStream_t s);
 cudaError_t probe_wait_limit(unsigned limit_us, int arrive, int* completed, double* elapsed_ms, cudaStream_t s);

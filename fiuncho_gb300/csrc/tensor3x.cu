@@ -1,12 +1,15 @@
-// Order-3 contingency tables on CTA pairs with 4-bit operands (classes that
-// share one accumulator).
+// Order-3 contingency tables on CTA pairs with 4-bit operands.
 //
+// For one-hot data the 8 core cells of a combination (i, j, l) -- genotypes
+// x, y, z in {0, 1} -- are dot products over the samples of one class:
+//     core[x][y][z] = sum_s a_ix(s) a_jy(s) a_lz(s),
+// where a_gx(s) is 1 when sample s has genotype x at SNP g.
 // A cluster of two CTAs (the two SMs of a TPC) runs one GEMM per work item
 // (i, 64 j, up to 120 l):
 //     D[(j,x,y), (l,z)] = sum_s A[(j,x,y), s] B[(l,z), s]    (M 256, N <= 240)
 // with tcgen05.mma.cta_group::2.kind::mxf4, control samples weighted by W = 2^p
 // through the B scale, so an accumulator holds cases + W controls of one core
-// cell.  CTA r builds the A rows of its 32 j and stages half r of the l rows;
+// cell (classes too large to share one so: SPLIT, below).  CTA r builds the A rows of its 32 j and stages half r of the l rows;
 // CTA 0 issues the MMAs; each CTA's 128 accumulator rows end up in its own
 // tensor memory.  Two regions of 240 columns alternate between items, so the
 // next item's GEMM runs while the epilogue evaluates the last one; the other 32
@@ -31,14 +34,17 @@
 //
 // What bounds it (2 000 SNPs x 4 000/4 000, one launch over the whole scan):
 // 26.3 ms; without the evaluation 22.7, without the A build and the MMAs too
-// 22.3 -- the copies out of L2 (17 KB a stage and SM, 9.5 TB/s); the MMAs alone
-// are 18.6 (120 cycles per M 256 N 240 K 64).  Whole searches: 28.8 ms against
-// 74.7 with e4m3 operands (128-byte rows of 128 samples: twice the shared-memory
+// 22.3 (about 540 cycles a stage of 17 KB and SM: 9.5 TB/s out of L2); the MMAs
+// alone are 18.6 (120 cycles per M 256 N 240 K 64).  Whole searches: 27.7 ms
+// against 74.7 with e4m3 operands (128-byte rows of 128 samples: twice the shared-memory
 // and L2 traffic, 82 KB a stage with LSU and tensor wavefronts at 83 % of peak;
 // 81 logarithms a combination at 8 cycles a warp instruction and SM quarter where
 // the bound takes about 21 reciprocals and 215 arithmetic cycles; a transpose
 // through shared memory).  Tried on the way: A in tensor memory and B spread from
 // bits by warps (5 KB a stage from L2, N 192): 45 ms, bound by issue slots.
+//
+// SPLIT (500 SNPs x 9 000/9 800): 5.6 -> 2.3 ms against the e4m3 kernel, one CTA a
+// tile, that counted classes apart before; 610 cycles a stage.
 //
 // Reference semantics: GenotypeTable::combine_and_popcnt for order 3
 // (src/base/gt_popcnt.cpp:4-35) and MutualInformation::compute
@@ -59,11 +65,13 @@ constexpr int kXN = 2 * kXL;                        // columns of an accumulator
 constexpr int kXM = 4 * kXJ;                        // 128 accumulator rows per CTA
 constexpr int kXRow = kF4K / 2;                     // 128 bytes per operand row and stage
 constexpr int kXBitRow = kF4K / 8;                  // 32 bytes per bit row and stage
-// Copies land in a ring of their own, deeper than the A ring: the copies' latency
-// (about 3 000 cycles from one's issue to its stage's release) times the bytes in
-// flight sets the pace.  (One ring of six stages, A beside what it is built from:
-// 540 cycles a stage whatever the MMAs took.)
-constexpr int kXStages = 8, kXAStages = 4;
+// Copies land in a ring of their own, deeper than the A ring (one ring of six
+// stages, A beside what it is built from, kept the same pace: 27.1 against 26.9
+// ms).  SPLIT has its stash in the space of the stages it lacks.
+template <bool SPLIT>
+constexpr int kXStages = SPLIT ? 5 : 8;
+template <bool SPLIT>
+constexpr int kXAStages = SPLIT ? 3 : 4;
 constexpr int kXSA = kXM * kXRow;                   // 16 KB
 constexpr int kXSB = kXN / 2 * kXRow;               // 15 KB: this CTA's half of the l rows
 constexpr int kXSJ = 2 * kXJ * kXBitRow;            //  2 KB
@@ -77,13 +85,23 @@ constexpr int kXThreads = 32 * (4 + 2 * kXBuildWarps + kXEpiWarps);  // 640: cop
 // registers a thread: 96 at launch, then 56 / 56 / 152 (3 x 56 + 2 x 152 <= 5 x 96)
 constexpr int kXMeta = 16;                          // items in flight between the copies and the MMAs
 // an item's staged tables: (i, l) marginals, one column per l; per j of this CTA (i, j) cores and j
-// singles, each twice (both halves of a pair), and j; the threshold (key, estimate, bound)
-constexpr int kXTabL = 9 * kXL * 4, kXTabJ = 6 * kXJ * 8, kXTabT = kXTabL + kXTabJ + 4 * kXJ, kXTab = kXTabT + 16;
-constexpr size_t kXSmem = 1024 + (size_t)kXStages * kXStage + (size_t)kXAStages * kXSA + 2 * kXTab;
-static_assert(kXSmem <= 227 * 1024 - 512, "order-3 pair kernel shared memory");
+// singles, each twice (both halves of a pair), and j; the threshold (key, estimate, bound).  SPLIT:
+// cases and controls beside each other instead.
+template <bool SPLIT>
+constexpr int kXTabL = 9 * kXL * (SPLIT ? 8 : 4);
+constexpr int kXTabJ = 6 * kXJ * 8;
+template <bool SPLIT>
+constexpr int kXTabT = kXTabL<SPLIT> + kXTabJ + 4 * kXJ;
+template <bool SPLIT>
+constexpr int kXTab = kXTabT<SPLIT> + 16;
+constexpr int kXStash = kXEpiWarps * ((kPxG + 1) / 2) * 2 * 32 * 16;  // 64 KB: (warp, its group, x, lane), 8 counts
+template <bool SPLIT>
+constexpr size_t kXSmem = 1024 + (size_t)kXStages<SPLIT> * kXStage + (size_t)kXAStages<SPLIT> * kXSA +
+                          2 * kXTab<SPLIT> + (SPLIT ? kXStash : 0);
+static_assert(kXSmem<false> <= 227 * 1024 - 512 && kXSmem<true> <= 227 * 1024 - 512, "order-3 pair kernel shared memory");
 static_assert(kXSA % 1024 == 0 && kXSB % 1024 == 0, "operand tiles on swizzle atoms");
 static_assert(kXColW + 16 <= 512, "tensor memory columns");
-static_assert(kXStages < kXMeta, "an item has a stage at least");
+static_assert(kXStages<false> < kXMeta, "an item has a stage at least");
 
 // One item: (i, j0 ..), l-tile of ng groups of 8 from l0.  LIST (a Distribution
 // layer): p0 is the first listed j instead of j0.
@@ -140,14 +158,76 @@ __device__ __forceinline__ float t3x_pair(const uint4& v, int x, int y, float W)
     return t3x_pk(y ? c >> 16 : c & 0xffffu, y ? t >> 16 : t & 0xffffu, W);
 }
 
-// The rare path (lanes with want): from the 27 packed cells t[(x*3+y)*3+z] of
+// Both classes' counts of a pair core beside each other (SPLIT).
+__device__ __forceinline__ f2 t3x_pair_ab(const uint4& v, int x, int y) {
+    return f4_ab(x ? v.y : v.x, x ? v.w : v.z, y);
+}
+
+// Its inverse: cases | controls << 16.
+__device__ __forceinline__ uint32_t t3x_word(f2 v) {
+    float a, b;
+    f2_unpack(f2_add(v, f2_dup(8388608.0f)), a, b);
+    return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x5410);
+}
+
+// The 27 cells of a combination from its cores c (x, y, z), the (i, j) cores, the
+// marginal table il(x, z) of (i, l), the (j, l) cores and the j singles; T is one
+// value or two side by side.  use(e, q, cell): the e-th cell made, (x, y, z) at
+// q = (x*3+y)*3+z.
+__device__ __forceinline__ f2 t3x_less(f2 a, f2 b, f2 c) { return f2_sub(f2_sub(a, b), c); }
+__device__ __forceinline__ float t3x_less(float a, float b, float c) { return a - b - c; }
+template <class T, class IL, class Use>
+__device__ __forceinline__ void t3x_cells(const T (&c)[2][2][2], const T (&ij)[2][2], IL&& il, const T (&jl)[2][2],
+                                          const T (&sj)[2], Use&& use) {
+    T a[2][2][3], y2[2][3];  // cells (x, y, z); cells (2, y, z)
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int y = 0; y < 2; ++y) {
+            a[x][y][0] = c[x][y][0];
+            a[x][y][1] = c[x][y][1];
+            a[x][y][2] = t3x_less(ij[x][y], c[x][y][0], c[x][y][1]);
+#pragma unroll
+            for (int z = 0; z < 3; ++z) use(6 * x + 3 * y + z, 9 * x + 3 * y + z, a[x][y][z]);
+        }
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int z = 0; z < 3; ++z) use(12 + 3 * x + z, 9 * x + 6 + z, t3x_less(il(x, z), a[x][0][z], a[x][1][z]));
+#pragma unroll
+    for (int y = 0; y < 2; ++y) {
+        const T j2 = t3x_less(sj[y], jl[y][0], jl[y][1]);
+#pragma unroll
+        for (int z = 0; z < 3; ++z) {
+            y2[y][z] = t3x_less(z < 2 ? jl[y][z & 1] : j2, a[0][y][z], a[1][y][z]);
+            use(18 + 3 * y + z, 18 + 3 * y + z, y2[y][z]);
+        }
+    }
+#pragma unroll
+    for (int z = 0; z < 3; ++z) use(24 + z, 24 + z, t3x_less(il(2, z), y2[0][z], y2[1][z]));
+}
+
+// Counts of both classes of a cell: packed, or beside each other.
+__device__ __forceinline__ void t3x_counts(float t, int pack, uint32_t& a, uint32_t& b) {
+    const uint32_t u = __float2uint_rn(t);
+    a = u & ((1u << pack) - 1u);
+    b = u >> pack;
+}
+__device__ __forceinline__ void t3x_counts(f2 t, int, uint32_t& a, uint32_t& b) {
+    float x, y;
+    f2_unpack(t, x, y);
+    a = __float2uint_rn(x);
+    b = __float2uint_rn(y);
+}
+
+// The rare path (lanes with want): from the 27 cells t[(x*3+y)*3+z] of
 // combination (i, j, l), the bounded single-precision estimate of the key
 // (t3_margin), the exact fixed-point key for what passes it, and the
 // warp-aggregated append of candidates.  Warp-synchronous.
+template <class T>
 __device__ __forceinline__ void t3x_survivor(const ScanWork& w, const CandSink& sink, long long thr, float thr_f,
-                                             uint32_t* dump, const float (&t)[27], int pack, int i, int j, int l,
+                                             uint32_t* dump, const T (&t)[27], int pack, int i, int j, int l,
                                              bool want, int lane) {
-    const uint32_t mask = (1u << pack) - 1u;
     const int n = w.d.snps;
     bool cand = want;
     if (!dump && !sink.digest) {
@@ -155,8 +235,9 @@ __device__ __forceinline__ void t3x_survivor(const ScanWork& w, const CandSink& 
         float kf = 0.f;
 #pragma unroll
         for (int c = 0; c < 27; ++c) {
-            const uint32_t u = __float2uint_rn(t[c]);
-            const float a = u2f(u & mask), b = u2f(u >> pack), s = a + b;
+            uint32_t ua, ub;
+            t3x_counts(t[c], pack, ua, ub);
+            const float a = u2f(ua), b = u2f(ub), s = a + b;
             kf = fmaf(a, t3_lg2(a + tiny), kf);
             kf = fmaf(b, t3_lg2(b + tiny), kf);
             kf = fmaf(-s, t3_lg2(s + tiny), kf);
@@ -177,13 +258,15 @@ __device__ __forceinline__ void t3x_survivor(const ScanWork& w, const CandSink& 
         }
 #pragma unroll
         for (int c = 0; c < 27; ++c) {
-            const uint32_t u = __float2uint_rn(t[c]), a = min(u & mask, nc), b = min(u >> pack, nt);
+            uint32_t ua, ub;
+            t3x_counts(t[c], pack, ua, ub);
+            const uint32_t a = min(ua, nc), b = min(ub, nt);
             key += __ldg(w.d.ftab + a) + __ldg(w.d.ftab + b) - __ldg(w.d.ftab + a + b);
             if (o) {
-                o[c] = u & mask;
-                o[27 + c] = u >> pack;
+                o[c] = ua;
+                o[27 + c] = ub;
             }
-            if (sink.digest) dg = dg_cell(dg, u & mask, u >> pack);
+            if (sink.digest) dg = dg_cell(dg, ua, ub);
         }
     }
     if (sink.digest) dg_warp_add(sink.digest, dg);
@@ -213,7 +296,10 @@ __device__ __forceinline__ int t3x_n(int ng) { return 16 * max(ng, 4); }
 // store the cores of every triple (F4Plan::tri).
 enum { kXScan, kXLayer, kXCores };
 
-template <int MODE>
+// SPLIT: classes that do not share an accumulator: the cases of an item accumulate in one region and
+// its controls in the other; the epilogue packs the case counts to 16 bits in shared memory as soon as
+// their GEMM is done, so the next item's case GEMM runs while this item's controls are evaluated.
+template <int MODE, bool SPLIT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
     tensor3x_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_j,
                     const __grid_constant__ CUtensorMap map_i, const __grid_constant__ ScanWork w,
@@ -223,15 +309,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
                     const long long* __restrict__ jl_begin, const int* __restrict__ jlist, float* tri,
                     const int* __restrict__ row_p, const int* __restrict__ row_q) {
     constexpr bool LIST = MODE == kXLayer;
+    constexpr int kStages = kXStages<SPLIT>, kAStages = kXAStages<SPLIT>;
     extern __shared__ uint8_t smraw[];
-    __shared__ __align__(8) uint64_t full_t[kXStages], empty[kXStages], full_a[kXAStages];
+    __shared__ __align__(8) uint64_t full_t[kStages], empty[kStages], full_a[kAStages];
     __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2], tab_full[2], tab_empty[2], done;
     __shared__ uint32_t tmem_base;
     __shared__ int item_ng[kXMeta];  // groups of the items in flight, for the MMA issuer
     __shared__ int abort_flag;
     uint8_t* sm = (uint8_t*)(((uintptr_t)smraw + 1023) & ~(uintptr_t)1023);  // stages: B half | j | i; then the A tiles
-    uint8_t* sma = sm + kXStages * kXStage;
-    uint8_t* tabs = sma + kXAStages * kXSA;
+    uint8_t* sma = sm + kStages * kXStage;
+    uint8_t* tabs = sma + kAStages * kXSA;
+    uint4* stash = reinterpret_cast<uint4*>(tabs + 2 * kXTab<SPLIT>);
     volatile int* abort = &abort_flag;
     const int n = w.d.snps;
     const int tid = threadIdx.x, lane = tid & 31;
@@ -249,11 +337,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
         auto init = [](uint64_t* b, int count) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(count));
         };
-        for (int s = 0; s < kXStages; ++s) {
+        for (int s = 0; s < kStages; ++s) {
             init(&full_t[s], 1);
             init(&empty[s], 1);
         }
-        for (int s = 0; s < kXAStages; ++s) init(&full_a[s], 2 * kXBuildWarps);
+        for (int s = 0; s < kAStages; ++s) init(&full_a[s], 2 * kXBuildWarps);
         for (int b = 0; b < 2; ++b) {
             init(&acc_full[b], 1);
             init(&acc_empty[b], 2 * kXEpiWarps);
@@ -309,8 +397,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
                         t3_tma(st + kXSB, &map_j, kXBitRow * ks, 2 * jr, bar);
                         t3_tma(st + kXSB + kXSJ, &map_i, kXBitRow * ks, irow, bar);
                         t3_tma(st, &map_b, kXRow * ks, brow, bar);
-                        if (step < kXStages) ++step;
-                        if (++s == kXStages) {
+                        if (step < kStages) ++step;
+                        if (++s == kStages) {
                             s = 0;
                             par ^= 1;
                         }
@@ -329,7 +417,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
         } else if (warp == 1) {
             // ---------------------------------------------------------------- MMA issuer (CTA 0)
             if (rank == 0 && elect_one()) {
-                ok = f4_pair_issue<false, kXAStages, kXSA, kXStages, kXStage, kXN, kXColOne, kXColW>(
+                ok = f4_pair_issue<SPLIT, kAStages, kXSA, kStages, kXStage, kXN, kXColOne, kXColW>(
                     (g1 - g0 - cid + ncl - 1) / ncl, smem_u32(sma), smem_u32(sm), smem_u32(&full_a[0]),
                     smem_u32(&empty[0]), smem_u32(&acc_full[0]), smem_u32(&acc_empty[0]), tmem, nw_c, nw_t, abort,
                     [&](unsigned item) { return t3x_n(item_ng[item % kXMeta]); });
@@ -355,7 +443,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
                     ok = false;
                     break;
                 }
-                uint8_t* tab = tabs + buf * kXTab;
+                uint8_t* tab = tabs + buf * kXTab<SPLIT>;
                 const int i = it.i;
                 const uint4 s1 = __ldg(single4 + i);
                 // the threshold of this item (the pairs take turns at raising the live one)
@@ -365,17 +453,36 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
                     const long long thr = sink.hist ? *(volatile long long*)sink.live : sink.thr;
                     float est, bound;
                     live_tests(map, thr, est, bound);
-                    *reinterpret_cast<long long*>(tab + kXTabT) = thr;
-                    *reinterpret_cast<float2*>(tab + kXTabT + 8) = make_float2(est, bound);
+                    *reinterpret_cast<long long*>(tab + kXTabT<SPLIT>) = thr;
+                    *reinterpret_cast<float2*>(tab + kXTabT<SPLIT> + 8) = make_float2(est, bound);
                 }
-                float* tl = reinterpret_cast<float*>(tab);
                 for (int ll = t; ll < 8 * it.ng; ll += 64) {  // entries (x, z), x and z in {0, 1, any}
                     const int l = it.l0 + ll;
-                    float m[3][3];
-#pragma unroll
-                    for (int k = 0; k < 9; ++k) m[k / 3][k % 3] = 0.f;
+                    uint4 p = make_uint4(0, 0, 0, 0), sl = p;
                     if (l < n && l > i) {
-                        const uint4 p = __ldg(pairs + pair_index(i, l, n)), sl = __ldg(single4 + l);
+                        p = __ldg(pairs + pair_index(i, l, n));
+                        sl = __ldg(single4 + l);
+                    }
+                    if constexpr (SPLIT) {
+                        f2* tl = reinterpret_cast<f2*>(tab);
+                        f2 m[3][3];
+#pragma unroll
+                        for (int x = 0; x < 2; ++x) {
+#pragma unroll
+                            for (int z = 0; z < 2; ++z) m[x][z] = t3x_pair_ab(p, x, z);
+                            m[x][2] = t3x_less(f4_ab(x ? s1.y : s1.x, x ? s1.w : s1.z, 0), m[x][0], m[x][1]);
+                        }
+#pragma unroll
+                        for (int z = 0; z < 2; ++z)
+                            m[2][z] = t3x_less(f4_ab(z ? sl.y : sl.x, z ? sl.w : sl.z, 0), m[0][z], m[1][z]);
+                        m[2][2] = t3x_less(t3x_less(f2_pack((float)w.d.n_cases, (float)w.d.n_ctrls),
+                                                    f4_ab(s1.x, s1.z, 0), f4_ab(s1.y, s1.w, 0)),
+                                           m[2][0], m[2][1]);
+#pragma unroll
+                        for (int k = 0; k < 9; ++k) tl[k * kXL + ll] = m[k / 3][k % 3];
+                    } else {
+                        float* tl = reinterpret_cast<float*>(tab);
+                        float m[3][3];
 #pragma unroll
                         for (int x = 0; x < 2; ++x) {
 #pragma unroll
@@ -386,9 +493,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
                         for (int z = 0; z < 2; ++z)
                             m[2][z] = t3x_pk(z ? sl.y : sl.x, z ? sl.w : sl.z, W) - m[0][z] - m[1][z];
                         m[2][2] = ntot - t3x_pk(s1.x, s1.z, W) - t3x_pk(s1.y, s1.w, W) - m[2][0] - m[2][1];
-                    }
 #pragma unroll
-                    for (int k = 0; k < 9; ++k) tl[k * kXL + ll] = m[k / 3][k % 3];
+                        for (int k = 0; k < 9; ++k) tl[k * kXL + ll] = m[k / 3][k % 3];
+                    }
                 }
                 if (t < kXJ) {
                     int j = n;
@@ -403,14 +510,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
                         p = __ldg(pairs + pair_index(i, j, n));
                         sv = __ldg(single4 + j);
                     }
-                    float2* tj = reinterpret_cast<float2*>(tab + kXTabL);
+                    f2* tj = reinterpret_cast<f2*>(tab + kXTabL<SPLIT>);
 #pragma unroll
                     for (int k = 0; k < 6; ++k) {
-                        const float v = k < 4 ? t3x_pair(p, k >> 1, k & 1, W)
-                                              : t3x_pk(k & 1 ? sv.y : sv.x, k & 1 ? sv.w : sv.z, W);
-                        tj[k * kXJ + t] = make_float2(v, v);
+                        if constexpr (SPLIT)
+                            tj[k * kXJ + t] = k < 4 ? t3x_pair_ab(p, k >> 1, k & 1)
+                                                    : f4_ab(k & 1 ? sv.y : sv.x, k & 1 ? sv.w : sv.z, 0);
+                        else
+                            tj[k * kXJ + t] = f2_dup(k < 4 ? t3x_pair(p, k >> 1, k & 1, W)
+                                                           : t3x_pk(k & 1 ? sv.y : sv.x, k & 1 ? sv.w : sv.z, W));
                     }
-                    reinterpret_cast<int*>(tab + kXTabL + kXTabJ)[t] = j;
+                    reinterpret_cast<int*>(tab + kXTabL<SPLIT> + kXTabJ)[t] = j;
                 }
                 __syncwarp();
                 if (lane == 0)
@@ -427,7 +537,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
         const int jj = rg >> 1, y = rg & 1;
         const int dst0 = (8 * y + jj) * kXRow + ((c ^ jj) << 4);
         unsigned s = 0, par = 0, sa = 0;                  // copy stage, A stage
-        unsigned se = kXStages - kXAStages, pe = 1;       // the stage whose MMAs free this A stage
+        unsigned se = kStages - kAStages, pe = 1;       // the stage whose MMAs free this A stage
         bool mine = warp < 8;
         for (long long g = g0 + cid; g < g1 && ok; g += ncl) {
             for (int ks = 0; ks < ksteps; ++ks, mine = !mine) {
@@ -456,15 +566,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
                     __syncwarp();
                     if (lane == 0) arrive_cl(full0 + 8 * sa);
                 }
-                if (++s == kXStages) {
+                if (++s == kStages) {
                     s = 0;
                     par ^= 1;
                 }
-                if (++se == kXStages) {
+                if (++se == kStages) {
                     se = 0;
                     pe ^= 1;
                 }
-                if (++sa == kXAStages) sa = 0;
+                if (++sa == kAStages) sa = 0;
             }
         }
     } else {
@@ -474,35 +584,70 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
         const int jl = lane >> 2, lc = 2 * (lane & 3);  // this thread's j and its two l of a group
         const float W = (float)(1u << pack);
         const bool all = dump != nullptr || sink.digest != nullptr;  // every combination takes the exact path
+        uint4* mine = stash + (warp - 12) * ((kPxG + 1) / 2) * 64 + lane;  // written and read by this warp only
         unsigned item = 0;
         int wi = -1;
         for (long long g = g0 + cid; g < g1 && ok; g += ncl, ++item) {
             const T3xItem it = t3x_item<LIST>(item_begin, jl_begin, jlist, n, g, wi);
             const int i = it.i, l0 = it.l0, ng = it.ng;
             const unsigned buf = item & 1, ph = (item >> 1) & 1;
-            const uint8_t* tab = tabs + buf * kXTab;
+            const uint8_t* tab = tabs + buf * kXTab<SPLIT>;
+            const int gi0 = (hh + item) & 1;  // the odd group of an item goes to either warp in turn
+            // accumulators of one x: registers 4 z + 2 y (l) and + 1 (l + 1): lane block y, 8-column block z
+            auto ld = [&](int region, int x, int gi, uint32_t (&r)[8]) {
+                asm volatile(
+                    "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                    : "r"(tmem + ((uint32_t)(32 * q + 16 * x) << 16) + (uint32_t)(kXN * region + 16 * gi)));
+            };
+            if (SPLIT) {
+                // case counts -> 16 bits in shared memory (l | l + 1 << 16); their region is then free
+                if (!t3_wait_cl(smem_u32(&acc_full[0]), item & 1, abort)) {
+                    ok = false;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;");
+#pragma unroll 1
+                for (int gi = gi0; gi < ng; gi += 2) {
+                    uint32_t r[2][8];
+                    ld(0, 0, gi, r[0]);
+                    ld(0, 1, gi, r[1]);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) {
+                        uint32_t o[4];  // 2 z + y
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            o[k] = __byte_perm(__float_as_uint(__uint_as_float(r[x][2 * k]) + 8388608.0f),
+                                               __float_as_uint(__uint_as_float(r[x][2 * k + 1]) + 8388608.0f), 0x5410);
+                        mine[((gi >> 1) * 2 + x) * 32] = make_uint4(o[0], o[1], o[2], o[3]);
+                    }
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;");
+                __syncwarp();
+                if (lane == 0) arrive_cl(cluster_addr(smem_u32(&acc_empty[0]), 0));
+            }
             if (MODE != kXCores && !t3_wait(smem_u32(&tab_full[buf]), ph, abort)) {
                 ok = false;
                 break;
             }
             const int j = MODE == kXCores ? it.j0 + kXJ * (int)rank + 8 * q + jl
-                                          : reinterpret_cast<const int*>(tab + kXTabL + kXTabJ)[8 * q + jl];
+                                          : reinterpret_cast<const int*>(tab + kXTabL<SPLIT> + kXTabJ)[8 * q + jl];
             const bool j_ok = j < n;
-            const f2* tj = reinterpret_cast<const f2*>(tab + kXTabL) + 8 * q + jl;
+            const f2* tj = reinterpret_cast<const f2*>(tab + kXTabL<SPLIT>) + 8 * q + jl;
             const f2 ij[2][2] = {{tj[0], tj[kXJ]}, {tj[2 * kXJ], tj[3 * kXJ]}}, sj[2] = {tj[4 * kXJ], tj[5 * kXJ]};
-            const long long thr = *reinterpret_cast<const long long*>(tab + kXTabT);
-            const float thr_f = reinterpret_cast<const float*>(tab + kXTabT)[2];
-            const float thr_q = reinterpret_cast<const float*>(tab + kXTabT)[3];
+            const long long thr = *reinterpret_cast<const long long*>(tab + kXTabT<SPLIT>);
+            const float thr_f = reinterpret_cast<const float*>(tab + kXTabT<SPLIT>)[2];
+            const float thr_q = reinterpret_cast<const float*>(tab + kXTabT<SPLIT>)[3];
             const uint4* pj = j_ok ? pairs + pair_index(j, j + 1, n) - (j + 1) : pairs;  // + l: pair (j, l)
             const uint4 zero4 = make_uint4(0, 0, 0, 0);
-            const int gi0 = (hh + item) & 1;  // the odd group of an item goes to either warp in turn
             uint4 pa = zero4, pb = zero4;
             {
                 const int l = l0 + 8 * gi0 + lc;
                 if (MODE != kXCores && j_ok && gi0 < ng && l < n && l > j) pa = __ldg(pj + l);
                 if (MODE != kXCores && j_ok && gi0 < ng && l + 1 < n && l + 1 > j) pb = __ldg(pj + l + 1);
             }
-            if (!t3_wait_cl(smem_u32(&acc_full[buf]), ph, abort)) {
+            if (!t3_wait_cl(smem_u32(&acc_full[SPLIT ? 1 : buf]), SPLIT ? item & 1 : ph, abort)) {
                 ok = false;
                 break;
             }
@@ -522,19 +667,58 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
                 if (!(m0 | m1)) continue;
                 if (sink.evaluated && lane == 0)
                     atomicAdd(sink.evaluated, (unsigned long long)(__popc(m0) + __popc(m1)));
-                f2 c[2][2][2];  // [x][y][z], the two combinations side by side
-                {
-                    const uint32_t a0 = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(kXN * buf + 16 * gi);
-                    uint32_t r[2][8];
+                uint32_t r[2][8];
+                ld(SPLIT ? 1 : buf, 0, gi, r[0]);
+                ld(SPLIT ? 1 : buf, 1, gi, r[1]);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if constexpr (SPLIT) {
+                    // one combination at a time, both classes side by side
+#pragma unroll 1
+                    for (int u = 0; u < 2; ++u) {
+                        f2 c[2][2][2];
 #pragma unroll
-                    for (int x = 0; x < 2; ++x)
-                        asm volatile(
-                            "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                            : "=r"(r[x][0]), "=r"(r[x][1]), "=r"(r[x][2]), "=r"(r[x][3]), "=r"(r[x][4]),
-                              "=r"(r[x][5]), "=r"(r[x][6]), "=r"(r[x][7])
-                            : "r"(a0 + ((uint32_t)(16 * x) << 16)));
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    // registers 4 z + 2 y (l) and + 1 (l + 1): lane block y, 8-column block z
+                        for (int x = 0; x < 2; ++x) {
+                            const uint4 sv = mine[((gi >> 1) * 2 + x) * 32];
+#pragma unroll
+                            for (int y = 0; y < 2; ++y)
+#pragma unroll
+                                for (int z = 0; z < 2; ++z) {
+                                    const uint32_t o = (&sv.x)[2 * z + y];
+                                    c[x][y][z] = f2_pack(
+                                        __uint_as_float(__byte_perm(o, 0x4B000000u, u ? 0x7632 : 0x7610)) - 8388608.0f,
+                                        __uint_as_float(u ? r[x][4 * z + 2 * y + 1] : r[x][4 * z + 2 * y]));
+                                }
+                        }
+                        const bool valid = u ? v1 : v0;
+                        if constexpr (MODE == kXCores) {  // entries (x, y, z), cases | controls << 16: 32 bytes a triple
+                            if (valid) {
+                                uint4* o = reinterpret_cast<uint4*>(tri) +
+                                           4 * (size_t)(__ldg(row_q + i) + __ldg(row_p + j) + (l >> 1)) + 2 * u;
+#pragma unroll
+                                for (int x = 0; x < 2; ++x)
+                                    o[x] = make_uint4(t3x_word(c[x][0][0]), t3x_word(c[x][0][1]), t3x_word(c[x][1][0]),
+                                                      t3x_word(c[x][1][1]));
+                            }
+                        } else {
+                            const f2* tl = reinterpret_cast<const f2*>(tab) + 8 * gi + lc + u;
+                            auto il = [&](int x, int z) { return tl[(3 * x + z) * kXL]; };
+                            const uint4 cj = u ? cb : ca;
+                            f2 jl2[2][2];
+#pragma unroll
+                            for (int y = 0; y < 2; ++y)
+#pragma unroll
+                                for (int z = 0; z < 2; ++z) jl2[y][z] = t3x_pair_ab(cj, y, z);
+                            F4BoundAB bd;
+                            t3x_cells<f2>(c, ij, il, jl2, sj, [&](int, int, f2 cell) { bd.one(cell); });
+                            const bool want = valid && (all || bd.acc >= thr_q);
+                            if (!__any_sync(0xffffffffu, want)) continue;
+                            f2 t[27];
+                            t3x_cells<f2>(c, ij, il, jl2, sj, [&](int, int k, f2 cell) { t[k] = cell; });
+                            t3x_survivor(w, sink, thr, thr_f, dump, t, pack, i, j, l + u, want, lane);
+                        }
+                    }
+                } else {
+                    f2 c[2][2][2];  // [x][y][z], the two combinations side by side
 #pragma unroll
                     for (int x = 0; x < 2; ++x)
 #pragma unroll
@@ -543,101 +727,72 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
                             for (int z = 0; z < 2; ++z)
                                 c[x][y][z] = f2_pack(__uint_as_float(r[x][4 * z + 2 * y]),
                                                      __uint_as_float(r[x][4 * z + 2 * y + 1]));
-                }
-                if (MODE == kXCores) {  // entries (x, y, z) of l and l + 1 side by side, 64 bytes
-                    float4* o = reinterpret_cast<float4*>(tri) + 4 * (size_t)(__ldg(row_q + i) + __ldg(row_p + j) +
-                                                                               (l >> 1));
-                    if (v0 || v1) {
+                    if constexpr (MODE == kXCores) {  // entries (x, y, z) of l and l + 1 side by side, 64 bytes
+                        if (v0 || v1) {
+                            float4* o = reinterpret_cast<float4*>(tri) +
+                                        4 * (size_t)(__ldg(row_q + i) + __ldg(row_p + j) + (l >> 1));
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            float4 v;
-                            f2_unpack(c[k >> 1][k & 1][0], v.x, v.y);
-                            f2_unpack(c[k >> 1][k & 1][1], v.z, v.w);
-                            o[k] = v;
-                        }
-                    }
-                    continue;
-                }
-                const float* tl = reinterpret_cast<const float*>(tab) + 8 * gi + lc;
-                auto il = [&](int x, int z) { return *reinterpret_cast<const f2*>(tl + (3 * x + z) * kXL); };
-                F4Bound bd(pack);
-                f2 a[2][2][3], y2[2][3];  // cells (x, y, z); cells (2, y, z)
-#pragma unroll
-                for (int x = 0; x < 2; ++x)
-#pragma unroll
-                    for (int y = 0; y < 2; ++y) {
-                        a[x][y][0] = c[x][y][0];
-                        a[x][y][1] = c[x][y][1];
-                        a[x][y][2] = f2_sub(f2_sub(ij[x][y], c[x][y][0]), c[x][y][1]);
-                        bd.two(a[x][y][0], a[x][y][1]);
-                    }
-                bd.two(a[0][0][2], a[0][1][2]);
-                bd.two(a[1][0][2], a[1][1][2]);
-#pragma unroll
-                for (int x = 0; x < 2; ++x)
-#pragma unroll
-                    for (int z = 0; z < 3; ++z) bd.one(f2_sub(f2_sub(il(x, z), a[x][0][z]), a[x][1][z]));
-#pragma unroll
-                for (int y = 0; y < 2; ++y) {
-                    f2 jl3[3];
-#pragma unroll
-                    for (int z = 0; z < 2; ++z) jl3[z] = f2_pack(t3x_pair(ca, y, z, W), t3x_pair(cb, y, z, W));
-                    jl3[2] = f2_sub(f2_sub(sj[y], jl3[0]), jl3[1]);
-#pragma unroll
-                    for (int z = 0; z < 3; ++z) {
-                        y2[y][z] = f2_sub(f2_sub(jl3[z], a[0][y][z]), a[1][y][z]);
-                        bd.one(y2[y][z]);
-                    }
-                }
-#pragma unroll
-                for (int z = 0; z < 3; ++z) bd.one(f2_sub(f2_sub(il(2, z), y2[0][z]), y2[1][z]));
-                float b0, b1;
-                f2_unpack(bd.acc, b0, b1);
-                const bool w0 = v0 && (all || b0 >= thr_q), w1 = v1 && (all || b1 >= thr_q);
-                if (__any_sync(0xffffffffu, w0 || w1)) {
-#pragma unroll 1
-                    for (int u = 0; u < 2; ++u) {
-                        const bool want = u ? w1 : w0;
-                        if (!__any_sync(0xffffffffu, want)) continue;
-                        // the combination's cells again, one lane of each pair
-                        auto at = [&](f2 v) {
-                            float lo, hi;
-                            f2_unpack(v, lo, hi);
-                            return u ? hi : lo;
-                        };
-                        const uint4 cj = u ? cb : ca;
-                        float t[27];
-#pragma unroll
-                        for (int x = 0; x < 2; ++x)
-#pragma unroll
-                            for (int y = 0; y < 2; ++y) {
-                                t[9 * x + 3 * y] = at(c[x][y][0]);
-                                t[9 * x + 3 * y + 1] = at(c[x][y][1]);
-                                t[9 * x + 3 * y + 2] = at(ij[x][y]) - t[9 * x + 3 * y] - t[9 * x + 3 * y + 1];
+                            for (int k = 0; k < 4; ++k) {
+                                float4 t;
+                                f2_unpack(c[k >> 1][k & 1][0], t.x, t.y);
+                                f2_unpack(c[k >> 1][k & 1][1], t.z, t.w);
+                                o[k] = t;
                             }
-#pragma unroll
-                        for (int x = 0; x < 2; ++x)
-#pragma unroll
-                            for (int z = 0; z < 3; ++z)
-                                t[9 * x + 6 + z] = tl[(3 * x + z) * kXL + u] - t[9 * x + z] - t[9 * x + 3 + z];
-#pragma unroll
-                        for (int y = 0; y < 2; ++y) {
-                            const float z0 = t3x_pair(cj, y, 0, W), z1 = t3x_pair(cj, y, 1, W);
-                            t[18 + 3 * y] = z0 - t[3 * y] - t[9 + 3 * y];
-                            t[18 + 3 * y + 1] = z1 - t[3 * y + 1] - t[9 + 3 * y + 1];
-                            t[18 + 3 * y + 2] = at(sj[y]) - z0 - z1 - t[3 * y + 2] - t[9 + 3 * y + 2];
                         }
+                    } else {
+                        const float* tl = reinterpret_cast<const float*>(tab) + 8 * gi + lc;
+                        f2 jl2[2][2];
 #pragma unroll
-                        for (int z = 0; z < 3; ++z)
-                            t[24 + z] = tl[(6 + z) * kXL + u] - t[18 + z] - t[21 + z];
-                        t3x_survivor(w, sink, thr, thr_f, dump, t, pack, i, j, l + u, want, lane);
+                        for (int y = 0; y < 2; ++y)
+#pragma unroll
+                            for (int z = 0; z < 2; ++z) jl2[y][z] = f2_pack(t3x_pair(ca, y, z, W), t3x_pair(cb, y, z, W));
+                        F4Bound bd(pack);
+                        f2 prev = 0;
+                        t3x_cells<f2>(
+                            c, ij, [&](int x, int z) { return *reinterpret_cast<const f2*>(tl + (3 * x + z) * kXL); },
+                            jl2, sj, [&](int e, int, f2 cell) {  // the first twelve cells share reciprocals
+                                if (e >= 12) bd.one(cell);
+                                else if (e & 1) bd.two(prev, cell);
+                                else prev = cell;
+                            });
+                        float b0, b1;
+                        f2_unpack(bd.acc, b0, b1);
+                        const bool w0 = v0 && (all || b0 >= thr_q), w1 = v1 && (all || b1 >= thr_q);
+                        if (!__any_sync(0xffffffffu, w0 || w1)) continue;
+#pragma unroll 1
+                        for (int u = 0; u < 2; ++u) {
+                            const bool want = u ? w1 : w0;
+                            if (!__any_sync(0xffffffffu, want)) continue;
+                            // the combination's cells again, one lane of each pair
+                            auto at = [&](f2 v) {
+                                float lo, hi;
+                                f2_unpack(v, lo, hi);
+                                return u ? hi : lo;
+                            };
+                            const uint4 cj = u ? cb : ca;
+                            float c1[2][2][2], ij1[2][2], jl1[2][2], t[27];
+#pragma unroll
+                            for (int x = 0; x < 2; ++x)
+#pragma unroll
+                                for (int y = 0; y < 2; ++y) {
+                                    c1[x][y][0] = at(c[x][y][0]);
+                                    c1[x][y][1] = at(c[x][y][1]);
+                                    ij1[x][y] = at(ij[x][y]);
+                                    jl1[x][y] = t3x_pair(cj, x, y, W);
+                                }
+                            const float sj1[2] = {at(sj[0]), at(sj[1])};
+                            t3x_cells<float>(
+                                c1, ij1, [&](int x, int z) { return tl[(3 * x + z) * kXL + u]; }, jl1, sj1,
+                                [&](int, int k, float cell) { t[k] = cell; });
+                            t3x_survivor(w, sink, thr, thr_f, dump, t, pack, i, j, l + u, want, lane);
+                        }
                     }
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;");
             __syncwarp();
             if (lane == 0) {
-                arrive_cl(cluster_addr(smem_u32(&acc_empty[buf]), 0));
+                arrive_cl(cluster_addr(smem_u32(&acc_empty[SPLIT ? 1 : buf]), 0));
                 asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&tab_empty[buf])) : "memory");
             }
         }
@@ -739,20 +894,23 @@ std::vector<long long> t3x_items(int n) {
     return b;
 }
 
-// Pair cores packed as floats, entries (z, w) of (k, l) for l and l + 1 side by side (32 bytes).
-__global__ void f4_pairf_kernel(const uint4* __restrict__ pairs, float2* out, const int* __restrict__ row_p, int n,
+// Pair cores, entries (z, w) of (k, l) for l and l + 1 in 32 bytes: packed floats side by side, or (pack 0)
+// words cases | controls << 16, the four of l first.
+__global__ void f4_pairf_kernel(const uint4* __restrict__ pairs, uint32_t* out, const int* __restrict__ row_p, int n,
                                 int pack) {
     const float W = (float)(1u << pack);
     const int k = blockIdx.x;
     for (int m = ((k + 1) >> 1) + threadIdx.x; m < (n + 1) / 2; m += blockDim.x) {
-        float2* o = out + 4 * (size_t)(row_p[k] + m);
-        float v[2][4];
+        uint32_t* o = out + 8 * (size_t)(row_p[k] + m);
         for (int u = 0; u < 2; ++u) {
             const int l = 2 * m + u;
             const uint4 p = l > k && l < n ? __ldg(pairs + pair_index(k, l, n)) : make_uint4(0, 0, 0, 0);
-            for (int e = 0; e < 4; ++e) v[u][e] = t3x_pair(p, e >> 1, e & 1, W);
+            for (int e = 0; e < 4; ++e) {
+                const uint32_t c = e >> 1 ? p.y : p.x, t = e >> 1 ? p.w : p.z;
+                if (pack) o[2 * e + u] = __float_as_uint(t3x_pair(p, e >> 1, e & 1, W));
+                else o[4 * u + e] = e & 1 ? __byte_perm(c, t, 0x7632) : __byte_perm(c, t, 0x5410);
+            }
         }
-        for (int e = 0; e < 4; ++e) o[e] = make_float2(v[0][e], v[1][e]);
     }
 }
 
@@ -784,7 +942,7 @@ cudaError_t f4_triples(const DevData& d, F4Plan& f, const long long* item_begin,
         f.row_q = rows + n;
         f.tri = reinterpret_cast<float*>(tab);
         f.pairf = reinterpret_cast<float*>(tab + (size_t)B * 64);
-        f4_pairf_kernel<<<n, 128, 0, s>>>(pairs, reinterpret_cast<float2*>(f.pairf), f.row_p, n, f.pack);
+        f4_pairf_kernel<<<n, 128, 0, s>>>(pairs, reinterpret_cast<uint32_t*>(f.pairf), f.row_p, n, f.pack);
         count_launch();
         e = cudaGetLastError();
     }
@@ -813,29 +971,31 @@ cudaError_t f4_triples(const DevData& d, F4Plan& f, const long long* item_begin,
 cudaError_t launch_tensor3x(const ScanWork& w, const F4Plan& f, const T3xRange& r, long long g0, long long g1,
                             const CandSink& sink, uint32_t* dump, const uint32_t* single, const uint4* pairs,
                             double est_margin, int* status, cudaStream_t s, int sms, bool cores) {
-    using Fn = decltype(&tensor3x_kernel<kXScan>);
-    static const Fn fns[3] = {tensor3x_kernel<kXScan>, tensor3x_kernel<kXLayer>, tensor3x_kernel<kXCores>};
+    using Fn = decltype(&tensor3x_kernel<kXScan, false>);
+    static const Fn fns[6] = {tensor3x_kernel<kXScan, false>, tensor3x_kernel<kXLayer, false>,
+                              tensor3x_kernel<kXCores, false>, tensor3x_kernel<kXScan, true>,
+                              tensor3x_kernel<kXLayer, true>, tensor3x_kernel<kXCores, true>};
     // set once, by whichever host thread comes first (thread-safe static initialisation)
     static const cudaError_t attr = [] {
         cudaError_t e = cudaSuccess;
-        for (Fn fn : fns)
-            if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kXSmem);
+        for (int k = 0; k < 6 && e == cudaSuccess; ++k)
+            e = cudaFuncSetAttribute(fns[k], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)(k < 3 ? kXSmem<false> : kXSmem<true>));
         return e;
     }();
     if (attr != cudaSuccess) return attr;
     if (g1 <= g0) return cudaSuccess;
-    static const int max_clusters = pair_clusters(tensor3x_kernel<kXScan>, kXThreads, kXSmem);
+    static const int max_clusters = pair_clusters(tensor3x_kernel<kXScan, false>, kXThreads, kXSmem<false>);
     const long long clusters = std::min<long long>(g1 - g0, max_clusters > 0 ? max_clusters : sms / 2);
     const unsigned grid = (unsigned)(2 * std::max(1ll, clusters));
-    const Fn fn = fns[cores ? kXCores : r.jlist ? kXLayer : kXScan];
+    const Fn fn = fns[(cores ? kXCores : r.jlist ? kXLayer : kXScan) + (f.pack ? 0 : 3)];
     const double scale = 1.0 / (std::log(2.0) * 4294967296.0);
     LiveMap map{scale, -(double)w.base_key * scale - est_margin, 0, 0};
     f4_quadratic(w.d.n_cases, w.d.n_ctrls, 27, map.bound_k, map.bound_c);
     map.bound_k *= scale;
-    fn<<<grid, kXThreads, kXSmem, s>>>(f.map_b, *r.map_j, f.map_i, w, sink, r.item_begin, g0, g1, f.nw_c, f.nw_t,
-                                       f.pack, map, dump, single, pairs, status, r.jl_begin, r.jlist, f.tri,
-                                       f.row_p, f.row_q);
+    fn<<<grid, kXThreads, f.pack ? kXSmem<false> : kXSmem<true>, s>>>(
+        f.map_b, *r.map_j, f.map_i, w, sink, r.item_begin, g0, g1, f.nw_c, f.nw_t, f.pack, map, dump, single, pairs,
+        status, r.jl_begin, r.jlist, f.tri, f.row_p, f.row_q);
     count_launch();
     return cudaGetLastError();
 }

@@ -1,5 +1,4 @@
-// Order-4 contingency tables on CTA pairs with 4-bit operands (classes that
-// share one accumulator).
+// Order-4 contingency tables on CTA pairs with 4-bit operands.
 //
 // A cluster of two CTAs runs one GEMM per work item (i, j, 32 k, up to 112 l):
 //     D[(k,x,y,z), (l,w)] = sum_s A[(k,x,y,z), s] B[(l,w), s]    (M 256, N <= 224)
@@ -29,7 +28,9 @@
 // 558/1 012 66.2 -> 31.0 ms, against e4m3 operands, one CTA a tile, 243
 // logarithms a combination (1 944 cycles a warp and SM quarter; the bound takes 81
 // reciprocals and about 930 arithmetic cycles) and triples counted by POPC.
-// Without the evaluation the two take 26 and 13 ms.
+// Without the evaluation the two take 26 and 13 ms.  Classes that do not share an
+// accumulator (SPLIT): 100 SNPs x 9 000/9 800 6.7 -> 4.1 ms (2.3 of the kernel's
+// 3.1 ms without the evaluation).
 //
 // Reference semantics: GenotypeTable::combine_and_popcnt for order 4
 // (src/base/gt_popcnt.cpp:4-35) and MutualInformation::compute
@@ -37,6 +38,7 @@
 // visits (include/fiuncho/ThreadedSearch.h:157-180) with one worker.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "elided4_prefix.cuh"
 #include "exact_key.cuh"
@@ -52,12 +54,15 @@ constexpr int kYN = 2 * kYL;                        // columns of an accumulator
 constexpr int kYRow = kF4K / 2;                     // 128 bytes per operand row and stage
 constexpr int kYBitRow = kF4K / 8;                  // 32 bytes per bit row and stage
 constexpr int kYHalfG = 4;                          // items of at most 4 groups bring 64 l rows a CTA, others 112
-constexpr int kYStages = 8, kYAStages = 4;          // rings of the copies and of A, as in the order-3 kernel
+template <bool SPLIT>
+constexpr int kYStages = SPLIT ? 4 : 8;             // rings of the copies and of A, as in the order-3 kernel
+template <bool SPLIT>
+constexpr int kYAStages = SPLIT ? 3 : 4;
 constexpr int kYSA = 8 * kYK * kYRow;               // 16 KB
 constexpr int kYSB = kYN / 2 * kYRow;               // 14 KB: this CTA's half of the l rows
 constexpr int kYSK = 2 * kYK * kYBitRow;            //  1 KB
 constexpr int kYSI = 2 * kYBitRow;                  // 64 bytes of i, 64 of j (on 128-byte boundaries)
-constexpr int kYStage = (kYSB + kYSK + 256 + 1023) / 1024 * 1024;  // 16 KB
+constexpr int kYBits = kYSK + 256;                  // the bit rows of a stage, behind all stages' B tiles
 constexpr int kYColOne = 2 * kYN, kYColW = kYColOne + 16;
 // 640 threads: copies, MMAs and two staging warps; two groups of four builders
 // that take alternate stages; eight epilogue warps.  Registers a thread: 96 at
@@ -66,14 +71,21 @@ constexpr int kYBuildWarps = 4, kYEpiWarps = 8;
 constexpr int kYThreads = 32 * (4 + 2 * kYBuildWarps + kYEpiWarps);
 constexpr int kYMeta = 16;                          // items in flight between the copies and the MMAs
 // staged tables of an item: per l (ijl (x,y,w), il (x,w), jl (y,w), l (w); w = 0, 1, any), per k of
-// this CTA (ijk, ik, jk, k cores, each twice: both halves of a pair)
-// and the item's threshold (key, estimate, bound)
-constexpr int kYTabL = 27 * kYL * 4, kYTabK = 18 * kYK * 8, kYTab = kYTabL + kYTabK + 16;
-constexpr size_t kYSmem = 1024 + (size_t)kYStages * kYStage + (size_t)kYAStages * kYSA + 2 * kYTab;
-static_assert(kYSmem <= 227 * 1024 - 512, "order-4 pair kernel shared memory");
+// this CTA (ijk, ik, jk, k cores, each twice: both halves of a pair; SPLIT: cases and controls
+// beside each other, in both) and the item's threshold (key, estimate, bound)
+template <bool SPLIT>
+constexpr int kYTabL = 27 * kYL * (SPLIT ? 8 : 4);
+constexpr int kYTabK = 18 * kYK * 8;
+template <bool SPLIT>
+constexpr int kYTab = kYTabL<SPLIT> + kYTabK + 16;
+constexpr int kYStash = kYEpiWarps * ((kP4G + 1) / 2) * 4 * 32 * 16;  // 64 KB: (warp, its group, x, z, lane), 8 counts
+template <bool SPLIT>
+constexpr size_t kYSmem = 1024 + (size_t)kYStages<SPLIT> * (kYSB + kYBits) + (size_t)kYAStages<SPLIT> * kYSA +
+                          2 * kYTab<SPLIT> + (SPLIT ? kYStash : 0);
+static_assert(kYSmem<false> <= 227 * 1024 - 512 && kYSmem<true> <= 227 * 1024 - 512, "order-4 pair kernel shared memory");
 static_assert(kYSA % 1024 == 0 && kYSB % 1024 == 0, "operand tiles on swizzle atoms");
 static_assert(kYColW + 16 <= 512, "tensor memory columns");
-static_assert(kYStages < kYMeta, "an item has a stage at least");
+static_assert(kYStages<false> < kYMeta, "an item has a stage at least");
 
 // One item: (i, j, k0 ..), l-tile of ng groups of 16 from l0.
 struct T4xItem {
@@ -129,10 +141,22 @@ __device__ __forceinline__ T4xItem t4x_item(const long long* __restrict__ begin,
 // Columns the MMA of an item of ng groups multiplies (at least 64).
 __device__ __forceinline__ int t4x_n(int ng) { return 32 * max(ng, 2); }
 
-__device__ __forceinline__ float t4x_pk(uint32_t c, uint32_t t, float W) { return fmaf(W, u2f(t), u2f(c)); }
-__device__ __forceinline__ float t4x_pair(const uint4& v, int x, int y, float W) {
+// Counts of both classes: packed (float), or beside each other (f2).
+template <class T>
+__device__ __forceinline__ T t4x_pk(uint32_t c, uint32_t t, float W) {
+    if constexpr (sizeof(T) == 8) return f2_pack(u2f(c), u2f(t));
+    else return fmaf(W, u2f(t), u2f(c));
+}
+template <class T>
+__device__ __forceinline__ T t4x_pair(const uint4& v, int x, int y, float W) {
     const uint32_t c = x ? v.y : v.x, t = x ? v.w : v.z;
-    return t4x_pk(y ? c >> 16 : c & 0xffffu, y ? t >> 16 : t & 0xffffu, W);
+    return t4x_pk<T>(y ? c >> 16 : c & 0xffffu, y ? t >> 16 : t & 0xffffu, W);
+}
+// Core e of the triple whose pair-of-l entry is at row (F4Plan::tri).
+template <class T>
+__device__ __forceinline__ T t4x_tri(const float* row, int l, int e) {
+    if constexpr (sizeof(T) == 8) return f4_ab(__ldg(reinterpret_cast<const uint32_t*>(row) + 8 * (l & 1) + e));
+    else return __ldg(row + 2 * e + (l & 1));
 }
 
 // One 27-cell slice (one genotype of l) from its 8 cores c (x, y, z) and packed
@@ -215,8 +239,11 @@ __device__ __forceinline__ void t4x_slices(const T4xCores<T>& v, TL&& tabl, TK&&
 
 // ALL: every combination takes the exact path (a search's first units, before a threshold; dumps and
 // digests).  Otherwise the bound comes first and the few combinations above it are evaluated from the
-// data set (warp_exact_key): the exact path's registers beside the bound's cost 20 % of the whole.
-template <bool LAYER, bool ALL>
+// data set (warp_exact_key4): the exact path's registers beside the bound's cost 20 % of the whole.
+// SPLIT: classes that do not share an accumulator, as in the order-3 kernel: cases accumulate in one region
+// and go to shared memory as 16-bit counts, controls in the other; one combination at a time is evaluated
+// from both beside each other.
+template <bool LAYER, bool ALL, bool SPLIT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
     tensor4x_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_bh,
                     const __grid_constant__ CUtensorMap map_k,
@@ -228,15 +255,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
                     uint32_t* dump, const uint32_t* __restrict__ single, const uint4* __restrict__ pairs,
                     const float* __restrict__ tri, const float* __restrict__ pairf, const int* __restrict__ row_p,
                     const int* __restrict__ row_q, int* status) {
+    constexpr int kStages = kYStages<SPLIT>, kAStages = kYAStages<SPLIT>, kTab = kYTab<SPLIT>, kTabL = kYTabL<SPLIT>;
+    using Tab = std::conditional_t<SPLIT, f2, float>;
     extern __shared__ uint8_t smraw[];
-    __shared__ __align__(8) uint64_t full_t[kYStages], empty[kYStages], full_a[kYAStages];
+    __shared__ __align__(8) uint64_t full_t[kStages], empty[kStages], full_a[kAStages];
     __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2], tab_full[2], tab_empty[2], done;
     __shared__ uint32_t tmem_base;
     __shared__ int item_ng[kYMeta];  // groups of the items in flight, for the MMA issuer
     __shared__ int abort_flag;
-    uint8_t* sm = (uint8_t*)(((uintptr_t)smraw + 1023) & ~(uintptr_t)1023);  // stages: B half | k | i | j; then the A tiles
-    uint8_t* sma = sm + kYStages * kYStage;
-    uint8_t* tabs = sma + kYAStages * kYSA;
+    uint8_t* sm = (uint8_t*)(((uintptr_t)smraw + 1023) & ~(uintptr_t)1023);  // stages: B half; the A tiles; k | i | j
+    uint8_t* sma = sm + kStages * kYSB;
+    uint8_t* smk = sma + kAStages * kYSA;
+    uint8_t* tabs = smk + kStages * kYBits;
+    uint4* stash = reinterpret_cast<uint4*>(tabs + 2 * kTab);
     volatile int* abort = &abort_flag;
     const int n = w.d.snps, kstep = LAYER ? w.dist_step : 1;
     const int tid = threadIdx.x, lane = tid & 31;
@@ -254,11 +285,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
         auto init = [](uint64_t* b, int count) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(count));
         };
-        for (int s = 0; s < kYStages; ++s) {
+        for (int s = 0; s < kStages; ++s) {
             init(&full_t[s], 1);
             init(&empty[s], 1);
         }
-        for (int s = 0; s < kYAStages; ++s) init(&full_a[s], 2 * kYBuildWarps);
+        for (int s = 0; s < kAStages; ++s) init(&full_a[s], 2 * kYBuildWarps);
         for (int b = 0; b < 2; ++b) {
             init(&acc_full[b], 1);
             init(&acc_empty[b], 2 * kYEpiWarps);
@@ -302,8 +333,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
                             ok = false;
                             break;
                         }
-                        const uint32_t st = smem_u32(sm + s * kYStage), bar = smem_u32(&full_t[s]);
-                        const uint32_t sk = st + kYSB;
+                        const uint32_t st = smem_u32(sm + s * kYSB), bar = smem_u32(&full_t[s]);
+                        const uint32_t sk = smem_u32(smk + s * kYBits);
                         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
                                      "r"((uint32_t)((half ? 16 * kYHalfG * kYRow : kYSB) + kYSK + 2 * kYSI))
                                      : "memory");
@@ -311,8 +342,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
                         t3_tma(sk + kYSK, &map_i, kYBitRow * ks, irow, bar);
                         t3_tma(sk + kYSK + 128, &map_i, kYBitRow * ks, jrow, bar);
                         t3_tma(st, half ? &map_bh : &map_b, kYRow * ks, brow, bar);
-                        if (step < kYStages) ++step;
-                        if (++s == kYStages) {
+                        if (step < kStages) ++step;
+                        if (++s == kStages) {
                             s = 0;
                             par ^= 1;
                         }
@@ -332,7 +363,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
         } else if (warp == 1) {
             // ---------------------------------------------------------------- MMA issuer (CTA 0)
             if (rank == 0 && elect_one()) {
-                ok = f4_pair_issue<false, kYAStages, kYSA, kYStages, kYStage, kYN, kYColOne, kYColW>(
+                ok = f4_pair_issue<SPLIT, kAStages, kYSA, kStages, kYSB, kYN, kYColOne, kYColW>(
                     (g1 - g0 - cid + ncl - 1) / ncl, smem_u32(sma), smem_u32(sm), smem_u32(&full_a[0]),
                     smem_u32(&empty[0]), smem_u32(&acc_full[0]), smem_u32(&acc_empty[0]), tmem, nw_c, nw_t, abort,
                     [&](unsigned item) { return t4x_n(item_ng[item % kYMeta]); });
@@ -346,7 +377,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
             // ---------------------------------------------------------------- table staging (both CTAs)
             const int t = tid - 64;  // 0 .. 63
             const float W = (float)(1u << pack);
-            const float ntot = fmaf(W, (float)w.d.n_ctrls, (float)w.d.n_cases);
+            const Tab ntot = t4x_pk<Tab>(w.d.n_cases, w.d.n_ctrls, W);
             const uint4* single4 = reinterpret_cast<const uint4*>(single);
             unsigned item = 0;
             int at = -1;
@@ -364,73 +395,70 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
                     const long long thr = sink.hist ? *(volatile long long*)sink.live : sink.thr;
                     float est, bound;
                     live_tests(map, thr, est, bound);
-                    uint8_t* o = tabs + buf * kYTab + kYTabL + kYTabK;
+                    uint8_t* o = tabs + buf * kTab + kTabL + kYTabK;
                     *reinterpret_cast<long long*>(o) = thr;
                     *reinterpret_cast<float*>(o + 8) = bound;
                 }
-                float* tl = reinterpret_cast<float*>(tabs + buf * kYTab);
-                float2* tk = reinterpret_cast<float2*>(tabs + buf * kYTab + kYTabL);
+                Tab* tl = reinterpret_cast<Tab*>(tabs + buf * kTab);
+                f2* tk = reinterpret_cast<f2*>(tabs + buf * kTab + kTabL);
                 const int i = it.i, j = it.j;
                 const uint4 pij4 = __ldg(pairs + pair_index(i, j, n));
                 const uint4 si = __ldg(single4 + i), sj = __ldg(single4 + j);
                 const float* tij = tri + 16ll * (__ldg(row_q + i) + __ldg(row_p + j));
-                const float ci[2] = {t4x_pk(si.x, si.z, W), t4x_pk(si.y, si.w, W)};
-                const float cj[2] = {t4x_pk(sj.x, sj.z, W), t4x_pk(sj.y, sj.w, W)};
                 for (int ll = t; ll < 16 * it.ng; ll += 64) {
                     const int l = it.l0 + ll;
-                    float v[27];
-#pragma unroll
-                    for (int e = 0; e < 27; ++e) v[e] = 0.f;
+                    Tab* o = tl + ll;
                     if (l < n && l > j) {
-                        const float* e3 = tij + 16ll * (l >> 1) + (l & 1);
+                        const float* e3 = tij + 16ll * (l >> 1);
                         const uint4 pi = __ldg(pairs + pair_index(i, l, n)), pj = __ldg(pairs + pair_index(j, l, n));
                         const uint4 sl = __ldg(single4 + l);
+                        // w = 0, 1 and what is left of the marginal ("any" entries hold what is left after
+                        // genotypes 0 and 1, so the slice of genotype 2 reads its marginals as the others do)
+                        auto put = [&](int e, Tab a, Tab b, Tab all) {
+                            o[e * kYL] = a;
+                            o[(e + 1) * kYL] = b;
+                            o[(e + 2) * kYL] = t4x_less(all, a, b);
+                        };
 #pragma unroll
-                        for (int xy = 0; xy < 4; ++xy) {
-                            v[3 * xy] = __ldg(e3 + 4 * xy);
-                            v[3 * xy + 1] = __ldg(e3 + 4 * xy + 2);
-                            v[3 * xy + 2] = t4x_pair(pij4, xy >> 1, xy & 1, W) - v[3 * xy] - v[3 * xy + 1];
-                        }
+                        for (int xy = 0; xy < 4; ++xy)
+                            put(3 * xy, t4x_tri<Tab>(e3, l, 2 * xy), t4x_tri<Tab>(e3, l, 2 * xy + 1),
+                                t4x_pair<Tab>(pij4, xy >> 1, xy & 1, W));
 #pragma unroll
                         for (int x = 0; x < 2; ++x) {
-#pragma unroll
-                            for (int w2 = 0; w2 < 2; ++w2) {
-                                v[12 + 3 * x + w2] = t4x_pair(pi, x, w2, W);
-                                v[18 + 3 * x + w2] = t4x_pair(pj, x, w2, W);
-                            }
-                            v[14 + 3 * x] = ci[x] - v[12 + 3 * x] - v[13 + 3 * x];
-                            v[20 + 3 * x] = cj[x] - v[18 + 3 * x] - v[19 + 3 * x];
+                            put(12 + 3 * x, t4x_pair<Tab>(pi, x, 0, W), t4x_pair<Tab>(pi, x, 1, W),
+                                t4x_pk<Tab>(x ? si.y : si.x, x ? si.w : si.z, W));
+                            put(18 + 3 * x, t4x_pair<Tab>(pj, x, 0, W), t4x_pair<Tab>(pj, x, 1, W),
+                                t4x_pk<Tab>(x ? sj.y : sj.x, x ? sj.w : sj.z, W));
                         }
-                        v[24] = t4x_pk(sl.x, sl.z, W);
-                        v[25] = t4x_pk(sl.y, sl.w, W);
-                        // "any" entries hold what is left after genotypes 0 and 1, so the slice of
-                        // genotype 2 reads its marginals as the other slices do
-                        v[26] = ntot - v[24] - v[25];
-                    }
+                        put(24, t4x_pk<Tab>(sl.x, sl.z, W), t4x_pk<Tab>(sl.y, sl.w, W), ntot);
+                    } else {
 #pragma unroll
-                    for (int e = 0; e < 27; ++e) tl[e * kYL + ll] = v[e];
+                        for (int e = 0; e < 27; ++e) o[e * kYL] = 0;
+                    }
                 }
                 if (t < kYK) {
                     const int k = it.k0 + kstep * (kYK * (int)rank + t);
-                    float v[18];
-#pragma unroll
-                    for (int e = 0; e < 18; ++e) v[e] = 0.f;
+                    auto put = [&](int e, Tab v) {
+                        if constexpr (SPLIT) tk[e * kYK + t] = v;
+                        else tk[e * kYK + t] = f2_dup(v);
+                    };
                     if (k < n) {
-                        const float* e3 = tij + 16ll * (k >> 1) + (k & 1);
+                        const float* e3 = tij + 16ll * (k >> 1);
                         const uint4 pi = __ldg(pairs + pair_index(i, k, n)), pj = __ldg(pairs + pair_index(j, k, n));
                         const uint4 sk = __ldg(single4 + k);
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) v[e] = __ldg(e3 + 2 * e);
+                        for (int e = 0; e < 8; ++e) put(e, t4x_tri<Tab>(e3, k, e));
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
-                            v[8 + e] = t4x_pair(pi, e >> 1, e & 1, W);
-                            v[12 + e] = t4x_pair(pj, e >> 1, e & 1, W);
+                            put(8 + e, t4x_pair<Tab>(pi, e >> 1, e & 1, W));
+                            put(12 + e, t4x_pair<Tab>(pj, e >> 1, e & 1, W));
                         }
-                        v[16] = t4x_pk(sk.x, sk.z, W);
-                        v[17] = t4x_pk(sk.y, sk.w, W);
-                    }
+                        put(16, t4x_pk<Tab>(sk.x, sk.z, W));
+                        put(17, t4x_pk<Tab>(sk.y, sk.w, W));
+                    } else {
 #pragma unroll
-                    for (int e = 0; e < 18; ++e) tk[e * kYK + t] = make_float2(v[e], v[e]);
+                        for (int e = 0; e < 18; ++e) put(e, 0);
+                    }
                 }
                 __syncwarp();
                 if (lane == 0)
@@ -447,7 +475,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
         const int kk = rg >> 1, z = rg & 1, m0 = 32 * (kk >> 2) + 4 * z + (kk & 3);
         const int dst0 = m0 * kYRow + ((c ^ (m0 & 7)) << 4);
         unsigned s = 0, par = 0, sa = 0;                  // copy stage, A stage
-        unsigned se = kYStages - kYAStages, pe = 1;       // the stage whose MMAs free this A stage
+        unsigned se = kStages - kAStages, pe = 1;       // the stage whose MMAs free this A stage
         bool mine = warp < 8;
         for (long long g = g0 + cid; g < g1 && ok; g += ncl) {
             for (int ks = 0; ks < ksteps; ++ks, mine = !mine) {
@@ -456,7 +484,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
                         ok = false;
                         break;
                     }
-                    const uint32_t* sK = reinterpret_cast<const uint32_t*>(sm + s * kYStage + kYSB);
+                    const uint32_t* sK = reinterpret_cast<const uint32_t*>(smk + s * kYBits);
                     const uint32_t* sI = sK + kYSK / 4 + c;
                     const uint32_t k0 = sK[rg * 8 + c], k1 = sK[(rg + 16) * 8 + c];
                     const uint32_t i0 = sI[0], i1 = sI[8], j0 = sI[32], j1 = sI[40];
@@ -475,15 +503,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
                     __syncwarp();
                     if (lane == 0) arrive_cl(full0 + 8 * sa);
                 }
-                if (++s == kYStages) {
+                if (++s == kStages) {
                     s = 0;
                     par ^= 1;
                 }
-                if (++se == kYStages) {
+                if (++se == kStages) {
                     se = 0;
                     pe ^= 1;
                 }
-                if (++sa == kYAStages) sa = 0;
+                if (++sa == kAStages) sa = 0;
             }
         }
     } else {
@@ -492,6 +520,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
         const int q = warp & 3, hh = (warp - 12) >> 2;  // lane quarter (4 k); its two warps take alternate groups
         const int zb = lane >> 4, kk = 4 * q + ((lane >> 2) & 3), lc = 2 * (lane & 3);
         const uint32_t wmask = (1u << pack) - 1u;
+        uint4* mine = stash + (warp - 12) * ((kP4G + 1) / 2) * 128 + lane;  // written and read by this warp only
         unsigned item = 0;
         int at = -1;
         for (long long g = g0 + cid; g < g1 && ok; g += ncl, ++item) {
@@ -504,152 +533,281 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
             const uint4* tik = reinterpret_cast<const uint4*>(tri) + 4 * ((long long)__ldg(row_q + it.i) + rp);
             const uint4* tjk = reinterpret_cast<const uint4*>(tri) + 4 * ((long long)__ldg(row_q + it.j) + rp);
             const uint4* tkl = reinterpret_cast<const uint4*>(pairf) + 2 * (long long)rp;
-            if (!t3_wait(smem_u32(&tab_full[buf]), ph, abort) || !t3_wait_cl(smem_u32(&acc_full[buf]), ph, abort)) {
+            // accumulators of one x in group gi: 8 group + 4 w + 2 y (l) and + 1 (l + 1)
+            auto acc_ld = [&](int region, int x, int gi, uint32_t (&r)[16]) {
+                asm volatile(
+                    "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
+                    "[%16];"
+                    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                      "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
+                      "=r"(r[15])
+                    : "r"(tmem + ((uint32_t)(32 * q + 16 * x) << 16) + (uint32_t)(kYN * region + 32 * gi)));
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            };
+            // SPLIT: the same as 16-bit counts (l | l + 1 << 16), this lane's z first and then the other z,
+            // components 2 w + y
+            auto acc_counts = [&](int region, int x, int gi, uint4& own, uint4& other) {
+                uint32_t r[16], o[8];
+                acc_ld(region, x, gi, r);
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                    o[e] = __byte_perm(__float_as_uint(__uint_as_float(r[2 * e]) + 8388608.0f),
+                                       __float_as_uint(__uint_as_float(r[2 * e + 1]) + 8388608.0f), 0x5410);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    (&own.x)[e] = zb ? o[4 + e] : o[e];
+                    (&other.x)[e] = __shfl_xor_sync(0xffffffffu, zb ? o[e] : o[4 + e], 16);
+                }
+            };
+            if (SPLIT) {
+                // case counts to shared memory; their region is then free
+                if (!t3_wait_cl(smem_u32(&acc_full[0]), item & 1, abort)) {
+                    ok = false;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;");
+#pragma unroll 1
+                for (int gi = hh; gi < it.ng; gi += 2)
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) {
+                        uint4 o[2];
+                        acc_counts(0, x, gi, o[0], o[1]);
+                        mine[(2 * (gi & ~1) + 2 * x) * 32] = o[0];
+                        mine[(2 * (gi & ~1) + 2 * x + 1) * 32] = o[1];
+                    }
+                asm volatile("tcgen05.fence::before_thread_sync;");
+                __syncwarp();
+                if (lane == 0) arrive_cl(cluster_addr(smem_u32(&acc_empty[0]), 0));
+            }
+            if (!t3_wait(smem_u32(&tab_full[buf]), ph, abort) ||
+                !t3_wait_cl(smem_u32(&acc_full[SPLIT ? 1 : buf]), SPLIT ? item & 1 : ph, abort)) {
                 ok = false;
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;");
-            const float* tabl0 = reinterpret_cast<const float*>(tabs + buf * kYTab);
-            const f2* tabk0 = reinterpret_cast<const f2*>(tabs + buf * kYTab + kYTabL) + kk;
-            const long long thr = *reinterpret_cast<const long long*>(tabs + buf * kYTab + kYTabL + kYTabK);
-            const float thr_q = *reinterpret_cast<const float*>(tabs + buf * kYTab + kYTabL + kYTabK + 8);
-            // (i,k,l), (j,k,l) and (k,l) of group gi: 16 bytes hold one (x, z) and both w
-            T4xCores<f2> v;
-            auto load = [&](int gi) {
-                const int l = it.l0 + 16 * gi + 8 * zb + lc, m = l >> 1;
-                const bool any = gi < it.ng && k_ok && l < n && l + 1 > k;
-                auto ld = [&](const uint4* p, f2 (&o)[2]) {
-                    uint4 x = make_uint4(0, 0, 0, 0);
-                    if (any) x = __ldg(p);
-                    o[0] = f2_pack(__uint_as_float(x.x), __uint_as_float(x.y));
-                    o[1] = f2_pack(__uint_as_float(x.z), __uint_as_float(x.w));
-                };
-#pragma unroll
-                for (int x = 0; x < 2; ++x)
+            const Tab* tabl0 = reinterpret_cast<const Tab*>(tabs + buf * kTab);
+            const f2* tabk0 = reinterpret_cast<const f2*>(tabs + buf * kTab + kTabL) + kk;
+            const long long thr = *reinterpret_cast<const long long*>(tabs + buf * kTab + kTabL + kYTabK);
+            const float thr_q = *reinterpret_cast<const float*>(tabs + buf * kTab + kTabL + kYTabK + 8);
+            // per-k entries: the index's last bit is z
+            auto tabk = [&](int e) { return tabk0[(e ^ zb) * kYK]; };
+            auto exact_append = [&](int src, int u, int lu) {  // a survivor of lane src
+                const int cmb[4] = {it.i, it.j, __shfl_sync(0xffffffffu, k, src), __shfl_sync(0xffffffffu, lu, src) + u};
+                const long long key = warp_exact_key4(&w.d, w.base_key, cmb[0], cmb[1], cmb[2], cmb[3]);
+                if (lane == 0 && key >= thr) live_append(sink, key, pack_code(cmb, 4, w.bits));
+            };
+            // the exact path of combination (i, j, k, lu), whose slices walk(use) makes: use(w, cell index,
+            // cases, controls)
+            auto every = [&](int lu, bool want, auto&& walk) {
+                const int cmb[4] = {it.i, it.j, k, lu};
+                long long key = w.base_key;
+                uint32_t* o = nullptr;
+                if (want) {
+                    // owned prefix ordinal of (i, j, k): rank offset + m * step
+                    if (dump)
+                        o = dump + ((size_t)((triple_index(it.i, it.j, k, n) - w.dist_offset) / w.dist_step) * n +
+                                    cmb[3]) * 162;
+                    const unsigned gt = blockIdx.x * blockDim.x + threadIdx.x;
+                    if (sink.digest && gt < sink.dscratch_threads) o = sink.dscratch + (size_t)gt * 162;
+                    const uint32_t nc = (uint32_t)w.d.n_cases, nt = (uint32_t)w.d.n_ctrls;
+                    walk([&](int sw, int c, uint32_t ua, uint32_t ub) {
+                        const uint32_t a = min(ua, nc), b = min(ub, nt);
+                        key += __ldg(w.d.ftab + a) + __ldg(w.d.ftab + b) - __ldg(w.d.ftab + a + b);
+                        if (o) {
+                            const int z = c % 3, zt = z < 2 ? z ^ zb : 2;
+                            o[(c - z + zt) * 3 + sw] = a;
+                            o[81 + (c - z + zt) * 3 + sw] = b;
+                        }
+                    });
+                }
+                if (sink.digest) dg_warp_add(sink.digest, want && o ? dg_table(cmb, 4, n, o, 81) : 0ull);
+                if (want && key >= thr) live_append(sink, key, pack_code(cmb, 4, w.bits));
+            };
+            if constexpr (SPLIT) {
+                // (i,k,l), (j,k,l) and (k,l) of combination u of group gi: words of w = 0, 1
+                uint2 ik[2][2], jk[2][2], kl[2];
+                auto load = [&](int gi, int u) {
+                    const int l = it.l0 + 16 * gi + 8 * zb + lc + u;
+                    const bool any = gi < it.ng && k_ok && l < n && l > k;
+                    auto ld = [&](const uint4* p, int e, uint2& o) {
+                        o = make_uint2(0, 0);
+                        if (any) o = __ldg(reinterpret_cast<const uint2*>(p) + e);
+                    };
 #pragma unroll
                     for (int z = 0; z < 2; ++z) {
-                        ld(tik + 4 * m + 2 * x + (z ^ zb), v.ik[x][z]);
-                        ld(tjk + 4 * m + 2 * x + (z ^ zb), v.jk[x][z]);
-                    }
 #pragma unroll
-                for (int z = 0; z < 2; ++z) ld(tkl + 2 * m + (z ^ zb), v.kl[z]);
-            };
-            load(hh);
-#pragma unroll 1
-            for (int gi = hh; gi < it.ng; gi += 2) {
-                const int ll = 16 * gi + 8 * zb + lc, l = it.l0 + ll;
-                const bool v0 = k_ok && l < n && l > k, v1 = k_ok && l + 1 < n && l + 1 > k;
-                const unsigned m0 = __ballot_sync(0xffffffffu, v0), m1 = __ballot_sync(0xffffffffu, v1);
-                if (!(m0 | m1)) {
-                    load(gi + 2);
-                    continue;
-                }
-                if (sink.evaluated && lane == 0)
-                    atomicAdd(sink.evaluated, (unsigned long long)(__popc(m0) + __popc(m1)));
-#pragma unroll
-                for (int x = 0; x < 2; ++x) {
-                    uint32_t r[16];  // 8 group + 4 w + 2 y (l) and + 1 (l + 1)
-                    asm volatile(
-                        "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
-                        "[%16];"
-                        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-                          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-                          "=r"(r[14]), "=r"(r[15])
-                        : "r"(tmem + ((uint32_t)(32 * q + 16 * x) << 16) + (uint32_t)(kYN * buf + 32 * gi)));
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                    for (int y = 0; y < 2; ++y)
-#pragma unroll
-                        for (int w2 = 0; w2 < 2; ++w2) {
-                            const int e = 4 * w2 + 2 * y;
-                            const uint32_t o0 = zb ? r[8 + e] : r[e], o1 = zb ? r[9 + e] : r[1 + e];
-                            const uint32_t s0 = zb ? r[e] : r[8 + e], s1 = zb ? r[1 + e] : r[9 + e];
-                            const uint32_t p0 = __shfl_xor_sync(0xffffffffu, s0, 16);
-                            const uint32_t p1 = __shfl_xor_sync(0xffffffffu, s1, 16);
-                            v.c[x][y][0][w2] = f2_pack(__uint_as_float(o0), __uint_as_float(o1));
-                            v.c[x][y][1][w2] = f2_pack(__uint_as_float(p0), __uint_as_float(p1));
+                        for (int x = 0; x < 2; ++x) {
+                            ld(tik, 4 * l + 2 * x + (z ^ zb), ik[x][z]);
+                            ld(tjk, 4 * l + 2 * x + (z ^ zb), jk[x][z]);
                         }
-                }
-                const float* tl = tabl0 + ll;
-                // per-k entries: the index's last bit is z
-                auto tabk = [&](int e) { return tabk0[(e ^ zb) * kYK]; };
-                if constexpr (!ALL) {
-                    F4Bound4 bd(pack, quart);
-                    t4x_slices<f2>(
-                        v, [&](int e) { return *reinterpret_cast<const f2*>(tl + e * kYL); }, tabk,
-                        [&](int sw, int c, f2 cell) {
-                            // the last slice has read the triples: the next group's are on their way
-                            // while its cells are summed
-                            if (sw == 2 && c == 0) load(gi + 2);
-                            bd.one(cell);
-                        });
-                    float b0, b1;
-                    f2_unpack(bd.acc, b0, b1);
-                    unsigned s0 = __ballot_sync(0xffffffffu, v0 && b0 >= thr_q);
-                    unsigned s1 = __ballot_sync(0xffffffffu, v1 && b1 >= thr_q);
-                    while (s0 | s1) {
-                        const int u = s0 ? 0 : 1, src = __ffs(u ? s1 : s0) - 1;
-                        if (u) s1 &= s1 - 1;
-                        else s0 &= s0 - 1;
-                        const int cmb[4] = {it.i, it.j, __shfl_sync(0xffffffffu, k, src),
-                                            __shfl_sync(0xffffffffu, l, src) + u};
-                        const long long key = warp_exact_key<4>(&w.d, w.base_key, cmb[0], cmb[1], cmb[2], cmb[3]);
-                        if (lane == 0 && key >= thr) live_append(sink, key, pack_code(cmb, 4, w.bits));
+                        ld(tkl, 2 * l + (z ^ zb), kl[z]);
                     }
-                } else {
+                };
+                load(hh, 0);
+#pragma unroll 1
+                for (int gi = hh; gi < it.ng; gi += 2) {
+                    const int ll = 16 * gi + 8 * zb + lc, l = it.l0 + ll;
+                    const bool v0 = k_ok && l < n && l > k, v1 = k_ok && l + 1 < n && l + 1 > k;
+                    const unsigned m0 = __ballot_sync(0xffffffffu, v0), m1 = __ballot_sync(0xffffffffu, v1);
+                    if (!(m0 | m1)) {
+                        load(gi + 2, 0);
+                        continue;
+                    }
+                    if (sink.evaluated && lane == 0)
+                        atomicAdd(sink.evaluated, (unsigned long long)(__popc(m0) + __popc(m1)));
+                    uint4 t[2][2];  // control counts (x, z)
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) acc_counts(1, x, gi, t[x][0], t[x][1]);
 #pragma unroll 1
                     for (int u = 0; u < 2; ++u) {
+                        T4xCores<f2> v;
+#pragma unroll
+                        for (int x = 0; x < 2; ++x)
+#pragma unroll
+                            for (int z = 0; z < 2; ++z) {
+                                const uint4 c = mine[(2 * (gi & ~1) + 2 * x + z) * 32];
+#pragma unroll
+                                for (int e = 0; e < 4; ++e)
+                                    v.c[x][e & 1][z][e >> 1] = f4_ab((&c.x)[e], (&t[x][z].x)[e], u);
+                                v.ik[x][z][0] = f4_ab(ik[x][z].x);
+                                v.ik[x][z][1] = f4_ab(ik[x][z].y);
+                                v.jk[x][z][0] = f4_ab(jk[x][z].x);
+                                v.jk[x][z][1] = f4_ab(jk[x][z].y);
+                            }
+#pragma unroll
+                        for (int z = 0; z < 2; ++z) {
+                            v.kl[z][0] = f4_ab(kl[z].x);
+                            v.kl[z][1] = f4_ab(kl[z].y);
+                        }
+                        load(u ? gi + 2 : gi, u ^ 1);  // the next one's, on their way while this one is evaluated
+                        const Tab* tl = tabl0 + ll + u;
+                        auto tabl = [&](int e) { return tl[e * kYL]; };
                         const bool want = u ? v1 : v0;
-                        auto at1 = [&](f2 a) {
-                            float lo, hi;
-                            f2_unpack(a, lo, hi);
-                            return u ? hi : lo;
-                        };
-                        T4xCores<float> s;
-#pragma unroll
-                        for (int e = 0; e < 16; ++e)
-                            s.c[e >> 3][(e >> 2) & 1][(e >> 1) & 1][e & 1] = at1(v.c[e >> 3][(e >> 2) & 1][(e >> 1) & 1][e & 1]);
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) {
-                            s.ik[e >> 2][(e >> 1) & 1][e & 1] = at1(v.ik[e >> 2][(e >> 1) & 1][e & 1]);
-                            s.jk[e >> 2][(e >> 1) & 1][e & 1] = at1(v.jk[e >> 2][(e >> 1) & 1][e & 1]);
-                        }
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) s.kl[e >> 1][e & 1] = at1(v.kl[e >> 1][e & 1]);
-                        const int cmb[4] = {it.i, it.j, k, l + u};
-                        long long key = w.base_key;
-                        uint32_t* o = nullptr;
-                        if (want) {
-                            // owned prefix ordinal of (i, j, k): rank offset + m * step
-                            if (dump)
-                                o = dump + ((size_t)((triple_index(it.i, it.j, k, n) - w.dist_offset) / w.dist_step) * n +
-                                            cmb[3]) * 162;
-                            const unsigned gt = blockIdx.x * blockDim.x + threadIdx.x;
-                            if (sink.digest && gt < sink.dscratch_threads) o = sink.dscratch + (size_t)gt * 162;
-                            const uint32_t nc = (uint32_t)w.d.n_cases, nt = (uint32_t)w.d.n_ctrls;
-                            t4x_slices<float>(
-                                s, [&](int e) { return tl[e * kYL + u]; }, [&](int e) { return at1(tabk(e)); },
-                                [&](int sw, int c, float cell) {
-                                    const uint32_t cu = __float2uint_rn(cell);
-                                    const uint32_t a = min(cu & wmask, nc), b = min(cu >> pack, nt);
-                                    key += __ldg(w.d.ftab + a) + __ldg(w.d.ftab + b) - __ldg(w.d.ftab + a + b);
-                                    if (o) {
-                                        const int z = c % 3, zt = z < 2 ? z ^ zb : 2;
-                                        o[(c - z + zt) * 3 + sw] = a;
-                                        o[81 + (c - z + zt) * 3 + sw] = b;
-                                    }
+                        if constexpr (!ALL) {
+                            F4Bound4AB bd(quart);
+                            t4x_slices<f2>(v, tabl, tabk, [&](int, int, f2 cell) { bd.one(cell); });
+                            unsigned sv = __ballot_sync(0xffffffffu, want && bd.acc >= thr_q);
+                            for (; sv; sv &= sv - 1) exact_append(__ffs(sv) - 1, u, l);
+                        } else {
+                            every(l + u, want, [&](auto&& use) {
+                                t4x_slices<f2>(v, tabl, tabk, [&](int sw, int c, f2 cell) {
+                                    float a, b;
+                                    f2_unpack(cell, a, b);
+                                    use(sw, c, __float2uint_rn(a), __float2uint_rn(b));
                                 });
+                            });
                         }
-                        if (sink.digest) dg_warp_add(sink.digest, want && o ? dg_table(cmb, 4, n, o, 81) : 0ull);
-                        if (want && key >= thr) live_append(sink, key, pack_code(cmb, 4, w.bits));
                     }
-                    load(gi + 2);
+                }
+            } else {
+                // (i,k,l), (j,k,l) and (k,l) of group gi: 16 bytes hold one (x, z) and both w
+                T4xCores<f2> v;
+                auto load = [&](int gi) {
+                    const int l = it.l0 + 16 * gi + 8 * zb + lc, m = l >> 1;
+                    const bool any = gi < it.ng && k_ok && l < n && l + 1 > k;
+                    auto ld = [&](const uint4* p, f2 (&o)[2]) {
+                        uint4 x = make_uint4(0, 0, 0, 0);
+                        if (any) x = __ldg(p);
+                        o[0] = f2_pack(__uint_as_float(x.x), __uint_as_float(x.y));
+                        o[1] = f2_pack(__uint_as_float(x.z), __uint_as_float(x.w));
+                    };
+#pragma unroll
+                    for (int x = 0; x < 2; ++x)
+#pragma unroll
+                        for (int z = 0; z < 2; ++z) {
+                            ld(tik + 4 * m + 2 * x + (z ^ zb), v.ik[x][z]);
+                            ld(tjk + 4 * m + 2 * x + (z ^ zb), v.jk[x][z]);
+                        }
+#pragma unroll
+                    for (int z = 0; z < 2; ++z) ld(tkl + 2 * m + (z ^ zb), v.kl[z]);
+                };
+                load(hh);
+#pragma unroll 1
+                for (int gi = hh; gi < it.ng; gi += 2) {
+                    const int ll = 16 * gi + 8 * zb + lc, l = it.l0 + ll;
+                    const bool v0 = k_ok && l < n && l > k, v1 = k_ok && l + 1 < n && l + 1 > k;
+                    const unsigned m0 = __ballot_sync(0xffffffffu, v0), m1 = __ballot_sync(0xffffffffu, v1);
+                    if (!(m0 | m1)) {
+                        load(gi + 2);
+                        continue;
+                    }
+                    if (sink.evaluated && lane == 0)
+                        atomicAdd(sink.evaluated, (unsigned long long)(__popc(m0) + __popc(m1)));
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) {
+                        uint32_t r[16];
+                        acc_ld(buf, x, gi, r);
+#pragma unroll
+                        for (int y = 0; y < 2; ++y)
+#pragma unroll
+                            for (int w2 = 0; w2 < 2; ++w2) {
+                                const int e = 4 * w2 + 2 * y;
+                                const uint32_t o0 = zb ? r[8 + e] : r[e], o1 = zb ? r[9 + e] : r[1 + e];
+                                const uint32_t s0 = zb ? r[e] : r[8 + e], s1 = zb ? r[1 + e] : r[9 + e];
+                                const uint32_t p0 = __shfl_xor_sync(0xffffffffu, s0, 16);
+                                const uint32_t p1 = __shfl_xor_sync(0xffffffffu, s1, 16);
+                                v.c[x][y][0][w2] = f2_pack(__uint_as_float(o0), __uint_as_float(o1));
+                                v.c[x][y][1][w2] = f2_pack(__uint_as_float(p0), __uint_as_float(p1));
+                            }
+                    }
+                    const float* tl = tabl0 + ll;
+                    if constexpr (!ALL) {
+                        F4Bound4 bd(pack, quart);
+                        t4x_slices<f2>(
+                            v, [&](int e) { return *reinterpret_cast<const f2*>(tl + e * kYL); }, tabk,
+                            [&](int sw, int c, f2 cell) {
+                                // the last slice has read the triples: the next group's are on their way
+                                // while its cells are summed
+                                if (sw == 2 && c == 0) load(gi + 2);
+                                bd.one(cell);
+                            });
+                        float b0, b1;
+                        f2_unpack(bd.acc, b0, b1);
+                        unsigned s0 = __ballot_sync(0xffffffffu, v0 && b0 >= thr_q);
+                        unsigned s1 = __ballot_sync(0xffffffffu, v1 && b1 >= thr_q);
+                        while (s0 | s1) {
+                            const int u = s0 ? 0 : 1, src = __ffs(u ? s1 : s0) - 1;
+                            if (u) s1 &= s1 - 1;
+                            else s0 &= s0 - 1;
+                            exact_append(src, u, l);
+                        }
+                    } else {
+#pragma unroll 1
+                        for (int u = 0; u < 2; ++u) {
+                            const bool want = u ? v1 : v0;
+                            auto at1 = [&](f2 a) {
+                                float lo, hi;
+                                f2_unpack(a, lo, hi);
+                                return u ? hi : lo;
+                            };
+                            T4xCores<float> s;
+#pragma unroll
+                            for (int e = 0; e < 16; ++e)
+                                s.c[e >> 3][(e >> 2) & 1][(e >> 1) & 1][e & 1] = at1(v.c[e >> 3][(e >> 2) & 1][(e >> 1) & 1][e & 1]);
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) {
+                                s.ik[e >> 2][(e >> 1) & 1][e & 1] = at1(v.ik[e >> 2][(e >> 1) & 1][e & 1]);
+                                s.jk[e >> 2][(e >> 1) & 1][e & 1] = at1(v.jk[e >> 2][(e >> 1) & 1][e & 1]);
+                            }
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) s.kl[e >> 1][e & 1] = at1(v.kl[e >> 1][e & 1]);
+                            every(l + u, want, [&](auto&& use) {
+                                t4x_slices<float>(
+                                    s, [&](int e) { return tl[e * kYL + u]; }, [&](int e) { return at1(tabk(e)); },
+                                    [&](int sw, int c, float cell) {
+                                        const uint32_t cu = __float2uint_rn(cell);
+                                        use(sw, c, cu & wmask, cu >> pack);
+                                    });
+                            });
+                        }
+                        load(gi + 2);
+                    }
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;");
             __syncwarp();
             if (lane == 0) {
-                arrive_cl(cluster_addr(smem_u32(&acc_empty[buf]), 0));
+                arrive_cl(cluster_addr(smem_u32(&acc_empty[SPLIT ? 1 : buf]), 0));
                 asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&tab_empty[buf])) : "memory");
             }
         }
@@ -666,6 +824,43 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
 }
 
+std::vector<long long> t4_item_table(int n, std::vector<long long>& per) {
+    std::vector<long long> begin((size_t)n + 1, 0);
+    per.assign((size_t)std::max(n, 1), 0);
+    for (int j = 0; j < n; ++j) {
+        for (int k0 = j + 1; k0 <= n - 2; k0 += kP4K) per[j] += t4x_tiles(n, k0);
+        begin[j + 1] = begin[j] + (long long)j * per[j];
+    }
+    return begin;
+}
+
+// Pair tables of a Distribution layer of an order-4 scan (host): the listed pairs (i, j) with at
+// least one item, their first owned k and first item.  Returns the items; combos = combinations.
+long long t4_layer_items(int n, int step, long long offset, std::vector<long long>& pbegin,
+                         std::vector<int4>& pinfo, long long& combos) {
+    pbegin.clear();
+    pinfo.clear();
+    combos = 0;
+    long long total = 0;
+    for (int i = 0; i + 3 < n; ++i)
+        for (int j = i + 1; j + 2 < n; ++j) {
+            const long long base = triple_index(i, j, j + 1, n), cnt = n - 1 - j;  // ranks base .. base + cnt - 1
+            long long t = std::max(0ll, offset - base);
+            t += ((offset - base - t) % step + step) % step;  // first t with base + t = offset (mod step)
+            if (t >= cnt) continue;
+            const int kf = j + 1 + (int)t;
+            long long items = 0;
+            for (long long k = kf; k <= n - 2; k += (long long)kP4K * step) items += t4x_tiles(n, (int)k);
+            for (long long k = kf; k < n; k += step) combos += n - 1 - k;
+            if (items == 0) continue;
+            pbegin.push_back(total);
+            pinfo.push_back(make_int4(i, j, kf, 0));
+            total += items;
+        }
+    pbegin.push_back(total);
+    return total;
+}
+
 cudaError_t f4_order4_maps(F4Plan& f, int snps) {
     cudaError_t e = tensor_map(&f.map_b4, f.planes, f.rows, 16 * f.wpr, kYRow, kYN / 2, true);
     if (e == cudaSuccess) e = tensor_map(&f.map_b4h, f.planes, f.rows, 16 * f.wpr, kYRow, 16 * kYHalfG, true);
@@ -677,20 +872,23 @@ cudaError_t launch_tensor4x(const ScanWork& w, const F4Plan& f, const T4xRange& 
                             const CandSink& sink, uint32_t* dump, const uint32_t* single, const uint4* pairs,
                             int* status, cudaStream_t s, int sms) {
     if (!f.tri || !pairs || !single || !r.begin || (!r.per && !r.pinfo)) return cudaErrorInvalidValue;
-    using Fn = decltype(&tensor4x_kernel<false, false>);
-    static const Fn fns[4] = {tensor4x_kernel<false, false>, tensor4x_kernel<true, false>, tensor4x_kernel<false, true>,
-                              tensor4x_kernel<true, true>};
+    using Fn = decltype(&tensor4x_kernel<false, false, false>);
+    // bits of the index: layer, all, split
+    static const Fn fns[8] = {tensor4x_kernel<false, false, false>, tensor4x_kernel<true, false, false>,
+                              tensor4x_kernel<false, true, false>,  tensor4x_kernel<true, true, false>,
+                              tensor4x_kernel<false, false, true>,  tensor4x_kernel<true, false, true>,
+                              tensor4x_kernel<false, true, true>,   tensor4x_kernel<true, true, true>};
     // set once, by whichever host thread comes first (thread-safe static initialisation)
     static const cudaError_t attr = [] {
         cudaError_t e = cudaSuccess;
-        for (Fn fn : fns)
-            if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kYSmem);
+        for (int k = 0; k < 8 && e == cudaSuccess; ++k)
+            e = cudaFuncSetAttribute(fns[k], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)(k < 4 ? kYSmem<false> : kYSmem<true>));
         return e;
     }();
     if (attr != cudaSuccess) return attr;
     if (g1 <= g0) return cudaSuccess;
-    static const int max_clusters = pair_clusters(tensor4x_kernel<false, false>, kYThreads, kYSmem);
+    static const int max_clusters = pair_clusters(tensor4x_kernel<false, false, false>, kYThreads, kYSmem<false>);
     const long long clusters = std::min<long long>(g1 - g0, max_clusters > 0 ? max_clusters : sms / 2);
     const unsigned grid = (unsigned)(2 * std::max(1ll, clusters));
     const double scale = 1.0 / (std::log(2.0) * 4294967296.0);
@@ -698,9 +896,9 @@ cudaError_t launch_tensor4x(const ScanWork& w, const F4Plan& f, const T4xRange& 
     const F4Quartic quart = f4_quartic(w.d.n_cases, w.d.n_ctrls, 81, map.bound_k, map.bound_c);
     map.bound_k *= scale;
     const bool all = dump || sink.digest || sink.thr == (long long)0x8000000000000000ull;
-    fns[2 * all + (r.pinfo != nullptr)]<<<grid, kYThreads, kYSmem, s>>>(
-        f.map_b4, f.map_b4h, *r.map_k, f.map_i, w, sink, r.begin, r.per, r.pinfo, r.n_pairs, g0, g1, f.nw_c, f.nw_t, f.pack, map,
-        quart, dump, single, pairs, f.tri, f.pairf, f.row_p, f.row_q, status);
+    fns[4 * !f.pack + 2 * all + (r.pinfo != nullptr)]<<<grid, kYThreads, f.pack ? kYSmem<false> : kYSmem<true>, s>>>(
+        f.map_b4, f.map_b4h, *r.map_k, f.map_i, w, sink, r.begin, r.per, r.pinfo, r.n_pairs, g0, g1, f.nw_c, f.nw_t,
+        f.pack, map, quart, dump, single, pairs, f.tri, f.pairf, f.row_p, f.row_q, status);
     count_launch();
     return cudaGetLastError();
 }

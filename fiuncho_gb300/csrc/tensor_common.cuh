@@ -1,6 +1,6 @@
-// Device helpers shared by the tcgen05 kernels (tensor3.cu: orders 2 and 3,
-// tensor4.cu: order 4): bounded mbarrier waits, TMA copies, shared-memory
-// matrix descriptors, exact integer <-> float views and the fast log2.
+// Device helpers shared by the tcgen05 kernels (tensor2x.cu, tensor3x.cu,
+// tensor4x.cu): bounded mbarrier waits, TMA copies, shared-memory matrix
+// descriptors, the exact float of an integer and the fast log2.
 #pragma once
 
 #include <cudaTypedefs.h>
@@ -9,7 +9,6 @@
 
 namespace fiu {
 
-constexpr int kT3KB = 128;                                // samples (= e4m3 bytes) per pipeline stage
 constexpr unsigned long long kT3LimitNs = 2000000000ull;  // 2 s per wait
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -138,10 +137,6 @@ __device__ __forceinline__ uint64_t t3_desc(uint32_t saddr) {
 
 __device__ __forceinline__ float u2f(uint32_t v) {  // exact for v < 2^23
     return __uint_as_float(0x4B000000u | v) - 8388608.0f;
-}
-
-__device__ __forceinline__ uint32_t f2u(float f) {  // f an exact integer in [0, 2^23)
-    return __float_as_uint(f + 8388608.0f) & 0x7FFFFFu;
 }
 
 // Row (SNP position) of SNP j in the operand planes ordered by residue mod

@@ -244,6 +244,30 @@ struct F4Bound {
     }
 };
 
+// Both classes' counts beside each other, from 16-bit halves of the words c and t.
+__device__ __forceinline__ f2 f4_ab(uint32_t c, uint32_t t, int hi) {
+    const uint32_t sel = hi ? 0x7632 : 0x7610;
+    return f2_add(f2_pack(__uint_as_float(__byte_perm(c, 0x4B000000u, sel)),
+                          __uint_as_float(__byte_perm(t, 0x4B000000u, sel))),
+                  f2_dup(-8388608.0f));
+}
+// The same of a word cases | controls << 16.
+__device__ __forceinline__ f2 f4_ab(uint32_t w) {
+    return f2_add(f2_pack(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7610)),
+                          __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7632))),
+                  f2_dup(-8388608.0f));
+}
+// The quadratic bound with the cases and controls of one combination's cells side by side.
+struct F4BoundAB {
+    float acc = 0.f;
+    __device__ __forceinline__ void one(f2 ab) {
+        float a, b, r;
+        f2_unpack(ab, a, b);
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"((a + b) + 9.5367431640625e-07f));
+        acc = fmaf(b, b * r, acc);
+    }
+};
+
 // A closer bound, for tables of many cells (order 4, where the quadratic one
 // leaves a third of the warps a survivor).  g(p) = D(p||q) / (p-q)^2 is an
 // average of D''(q + u (p-q)) = 1 / (ln2 t (1-t)) over u, which is convex, so g
@@ -268,6 +292,18 @@ struct F4Bound4 : F4Bound {
         split(D, b, s);
         const f2 pr = f2_mul(b, f2_rcp(s));
         acc = f2_fma(f2_mul(b, pr), f2_fma(pr, f2_fma(pr, a4, a3), a2), acc);
+    }
+};
+struct F4Bound4AB {
+    F4Quartic k;
+    float acc = 0.f;
+    __device__ __forceinline__ explicit F4Bound4AB(const F4Quartic& q) : k(q) {}
+    __device__ __forceinline__ void one(f2 ab) {
+        float a, b, r;
+        f2_unpack(ab, a, b);
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"((a + b) + 9.5367431640625e-07f));
+        const float pr = b * r;
+        acc = fmaf(b * pr, fmaf(pr, fmaf(pr, k.a4, k.a3), k.a2), acc);
     }
 };
 // The quartic bound's coefficients and test (as f4_quadratic).

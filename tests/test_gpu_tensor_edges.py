@@ -66,6 +66,29 @@ def test_order4_layer_edges(oracle, snps, step, offset):
     _check(4, snps, 130, 199, oracle, Distribution(snps, 3, step, offset))
 
 
+SPLIT = [  # classes that do not share an accumulator: order, snps, cases, controls
+    (3, 3, 4100, 4100), (3, 65, 9000, 9800), (3, 66, 4097, 4160), (3, 121, 300, 65000), (3, 130, 16384, 5000),
+    (4, 4, 4100, 4100), (4, 33, 4097, 4160), (4, 36, 9000, 9800), (4, 19, 300, 65000),
+]
+
+
+@pytest.mark.parametrize("order,snps,cases,ctrls", SPLIT)
+def test_split_classes_tile_edges(oracle, order, snps, cases, ctrls):
+    from fiuncho_gb300 import GpuSearch, _lib
+    from fiuncho_gb300.search import Resident
+    ds = _data(snps, cases, ctrls, 1000 * order + snps)
+    gs = GpuSearch(0)
+    res = Resident(gs.ctx, ds)
+    assert gs.scan_digest(res, order, kernel=_lib.KERNEL_TENSOR) == \
+        oracle.table_digest(ds.data, snps, ds.cases_words, ds.ctrls_words, order, dist=(snps, 1, 0))
+
+
+@pytest.mark.parametrize("order,snps,step,offset", [(3, 70, 2, 1), (3, 135, 3, 0), (4, 37, 3, 0), (4, 20, 2, 1)])
+def test_split_classes_layer_edges(oracle, order, snps, step, offset):
+    from fiuncho_gb300 import Distribution
+    _check(order, snps, 4100, 4101, oracle, Distribution(snps, order - 1, step, offset))
+
+
 @pytest.mark.parametrize("snps,order", [(130, 4), (260, 3)])
 def test_wide_tiles_against_the_reduced_work_kernel(snps, order):
     """Full column tiles (112 and 120 SNPs): digests of two kernels that share no code path."""
@@ -116,7 +139,8 @@ def test_order2_layer_edges(oracle, snps, step, offset, cases, ctrls):
     _check(2, snps, cases, ctrls, oracle, Distribution(snps, 1, step, offset))
 
 
-@pytest.mark.parametrize("order,snps,cases,ctrls", [(2, 1900, 4100, 4100), (2, 2100, 300, 290)])
+@pytest.mark.parametrize("order,snps,cases,ctrls", [(2, 1900, 4100, 4100), (2, 2100, 300, 290),
+                                                    (3, 300, 4097, 4100), (4, 130, 4097, 4100)])
 def test_several_items_per_pair(order, snps, cases, ctrls):
     """More items than CTA pairs, so that accumulators, stashes and tables are used again: every table and
     the list against a kernel that shares no code path."""
