@@ -251,12 +251,13 @@ cudaError_t launch_select_scans(const ScanDesc* scans, ScanState* states, int n_
     return cudaGetLastError();
 }
 
-// FP64 re-score: one warp per kept candidate slot of every scan.
-__global__ void rescore_scans_kernel(const ScanDesc* __restrict__ scans, const ScanState* __restrict__ states,
-                                     const unsigned* __restrict__ slot_begin, int n_scans, unsigned total_slots) {
-    const unsigned q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (q >= total_slots) return;
+// FP64 re-score: one CTA per kept candidate slot of every scan.
+__global__ void __launch_bounds__(kScoreThreads) rescore_scans_kernel(const ScanDesc* __restrict__ scans,
+                                                                      const ScanState* __restrict__ states,
+                                                                      const unsigned* __restrict__ slot_begin,
+                                                                      int n_scans) {
+    __shared__ ScoreShared sh;
+    const unsigned q = blockIdx.x;
     int lo = 0, hi = n_scans - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
@@ -269,9 +270,8 @@ __global__ void rescore_scans_kernel(const ScanDesc* __restrict__ scans, const S
     const Cand c = sd.cand[i];
     int comb[kMaxOrder];
     unpack_code(c.code, sd.w.order, sd.w.bits, comb);
-    double mi = 0.0;
-    combo_tables(sd.w.d, sd.w.order, comb, lane, nullptr, nullptr, &mi);
-    if (lane == 0) sd.scored[i] = ScoredRec{mi, c.code, c.key};
+    const double mi = block_mi(sd.w.d, sd.w.order, comb, sh);
+    if (threadIdx.x == 0) sd.scored[i] = ScoredRec{mi, c.code, c.key};
 }
 
 struct RecBetter {
@@ -311,8 +311,7 @@ cudaError_t launch_finish_scans(const ScanDesc* scans, ScanState* states, const 
     if (n_scans <= 0) return cudaSuccess;
     if (!g_finish_attr) return cudaErrorInvalidConfiguration;
     if (total_slots) {
-        rescore_scans_kernel<<<(unsigned)(((size_t)total_slots * 32 + 255) / 256), 256, 0, s>>>(
-            scans, states, slot_begin, n_scans, total_slots);
+        rescore_scans_kernel<<<total_slots, kScoreThreads, 0, s>>>(scans, states, slot_begin, n_scans);
         count_launch();
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;

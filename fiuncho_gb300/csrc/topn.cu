@@ -160,16 +160,15 @@ cudaError_t live_compact(const CandSink& sink, Cand* out, unsigned* out_count, c
     return cudaGetLastError();
 }
 
-__global__ void rescore_kernel(DevData d, int K, int bits, const Cand* __restrict__ cands, unsigned n,
-                               Scored* __restrict__ out) {
-    const unsigned warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (warp >= n) return;
+__global__ void __launch_bounds__(kScoreThreads) rescore_kernel(DevData d, int K, int bits,
+                                                                const Cand* __restrict__ cands,
+                                                                Scored* __restrict__ out) {
+    __shared__ ScoreShared sh;
+    const Cand cand = cands[blockIdx.x];
     int c[kMaxOrder];
-    unpack_code(cands[warp].code, K, bits, c);
-    double mi = 0.0;
-    combo_tables(d, K, c, lane, nullptr, nullptr, &mi);
-    if (lane == 0) out[warp] = Scored{mi, cands[warp].code, cands[warp].key};
+    unpack_code(cand.code, K, bits, c);
+    const double mi = block_mi(d, K, c, sh);
+    if (threadIdx.x == 0) out[blockIdx.x] = Scored{mi, cand.code, cand.key};
 }
 
 __global__ void unscore_kernel(const Scored* __restrict__ in, unsigned n, Cand* __restrict__ cands,
@@ -189,7 +188,7 @@ cudaError_t rescore_sort(const DevData& d, int order, int bits, Cand* cands, uns
     Scored* sc = nullptr;
     cudaError_t e = cudaMallocAsync((void**)&sc, (size_t)n * sizeof(Scored), s);
     if (e != cudaSuccess) return e;
-    rescore_kernel<<<(n * 32 + 255) / 256, 256, 0, s>>>(d, order, bits, cands, n, sc);
+    rescore_kernel<<<n, kScoreThreads, 0, s>>>(d, order, bits, cands, sc);
     count_launch();
     if ((e = cudaGetLastError()) == cudaSuccess)
         e = sort_small<Scored, ScoredBetter>(sc, n, Scored{-1.0e300, ~0ull, 0}, s);
