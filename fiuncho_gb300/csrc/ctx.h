@@ -59,6 +59,7 @@ struct fiu_resident {
     long long* ftab = nullptr;
     long long ftab_max = 0;
     int one_hot = 0;
+    int disjoint = 0;  // no sample has two genotypes at an SNP, and none past a class's last is set
     int device = 0;
     uint32_t* single = nullptr;  // single-SNP cores (elided kernels)
     uint4* pairs = nullptr;      // pair cores (elided order-3 and order-4 kernels)

@@ -178,7 +178,7 @@ cudaError_t launch_elided4p(const ScanWork& w, const long long* begin, long long
                             const CandSink& sink, uint32_t* dump, const uint32_t* single, const uint4* pairs,
                             const uint4* triples, cudaStream_t s, int sms);
 
-// tensor2x.cu, tensor3x.cu, tensor4x.cu (4-bit operands, CTA pairs) and tensor3.cu (their host side) -- core
+// tensor2x.cu, tensor3x.cu, tensor3m.cu, tensor4x.cu (4-bit operands, CTA pairs) and tensor3.cu (their host side) -- core
 // cells on tcgen05 (one-hot data, the whole data set or a layer of it).
 // Device state of the tensor kernels for one data set: operand planes, made on the first search of an
 // order, their TMA descriptors and the work-item prefix sums.
@@ -207,6 +207,7 @@ struct T3Plan {
     F4Plan f4;
     double item_combos = 0;             // combinations per work item
     struct T3Layers* layers = nullptr;  // work items of Distribution layers (tensor3.cu)
+    bool missing = false;               // data with missing calls: order 3 alone, three genotypes a SNP (tensor3m.cu)
     long long* item_begin = nullptr;
     long long total = 0;  // work items
     // order 2: work items (128 i, 120 j) of the pair kernel, first of each band

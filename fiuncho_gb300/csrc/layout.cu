@@ -30,7 +30,8 @@ cudaError_t launch_transpose(const uint64_t* ref, uint64_t* tr, int snps, int ro
 // per-class popcount; this asks for the stronger exact form): for every SNP and
 // class the three rows are pairwise disjoint and their union is exactly the
 // bit set of the class's samples (full words, then the right-aligned partial
-// word, then zero padding).  Sets *bad on any violation.
+// word, then zero padding).  Sets bit 0 of *bad on any violation and bit 1 if rows
+// share a sample or a bit past the class is set.
 __global__ void onehot_kernel(const uint64_t* __restrict__ ref, int snps, int cw, int tw, int n_cases, int n_ctrls,
                               int* bad) {
     const size_t per_snp = 3 * (size_t)(cw + tw);
@@ -47,7 +48,12 @@ __global__ void onehot_kernel(const uint64_t* __restrict__ ref, int snps, int cw
         const uint64_t r0 = base[w], r1 = base[W + w], r2 = base[2 * W + w];
         const int full = n / 64, rem = n % 64;
         const uint64_t want = w < full ? ~0ull : (w == full && rem ? ((1ull << rem) - 1) : 0ull);
-        if (((r0 & r1) | (r0 & r2) | (r1 & r2)) != 0 || (r0 | r1 | r2) != want) atomicOr(bad, 1);
+        const bool shared = ((r0 & r1) | (r0 & r2) | (r1 & r2) | ((r0 | r1 | r2) & ~want)) != 0;
+        // (one atomic for all but the first such words: data with missing calls has millions)
+        if ((shared || (r0 | r1 | r2) != want) && (*(volatile int*)bad & 3) != 3) {
+            const int flags = shared ? 3 : 1;
+            if ((*(volatile int*)bad & flags) != flags) atomicOr(bad, flags);
+        }
     }
 }
 

@@ -16,7 +16,7 @@
 #include <mutex>
 
 #include "tensor2x.h"
-#include "tensor3x.h"
+#include "tensor3m.h"
 #include "tensor_common.cuh"
 
 namespace fiu {
@@ -64,7 +64,7 @@ static cudaError_t upload(long long*& out, const std::vector<long long>& v) {
 // Order-3 items of the whole data set.
 static cudaError_t order3_items(T3Plan& plan, const DevData& d) {
     if (plan.item_begin) return cudaSuccess;
-    const std::vector<long long> ib = t3x_items(d.snps);
+    const std::vector<long long> ib = plan.missing ? t3m_items(d.snps) : t3x_items(d.snps);
     plan.total = ib.back();
     const double n = d.snps;
     plan.item_combos = n * (n - 1) * (n - 2) / 6.0 / std::max(1ll, plan.total);
@@ -85,7 +85,7 @@ static cudaError_t order_planes(T3Plan& plan, const DevData& d, int order, const
         return e;
     }
     if (!plan.f4.bits) {
-        e = f4_prepare(d, plan.f4, s);
+        e = f4_prepare(d, plan.f4, plan.missing ? 3 : 2, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) f4_release(plan.f4);
     }
@@ -429,10 +429,11 @@ cudaError_t launch_tensor3(const ScanWork& w, const T3Plan& plan, long long g0, 
                              : T4xRange{plan.item4_begin, plan.item4_per, &plan.f4.map_k4};
         return launch_tensor4x(w, plan.f4, r, g0, g1, sink, dump, single, pairs, status, s, sms);
     }
+    const double margin = t3_margin(w.d.n_cases + w.d.n_ctrls);
+    if (plan.missing) return launch_tensor3m(w, plan.f4, plan.item_begin, g0, g1, sink, margin, status, s, sms);
     const T3xRange r = L ? T3xRange{L->item_begin, &L->map_jr, L->jl_begin, L->jlist}
                          : T3xRange{plan.item_begin, &plan.f4.map_j};
-    return launch_tensor3x(w, plan.f4, r, g0, g1, sink, dump, single, pairs, t3_margin(w.d.n_cases + w.d.n_ctrls),
-                           status, s, sms);
+    return launch_tensor3x(w, plan.f4, r, g0, g1, sink, dump, single, pairs, margin, status, s, sms);
 }
 
 }  // namespace fiu

@@ -54,7 +54,7 @@
 #include <cmath>
 
 #include "live.cuh"
-#include "tensor3x.h"
+#include "tensor3m.h"
 #include "tensor_fp4.cuh"
 
 namespace fiu {
@@ -810,10 +810,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
 }
 
 // ---------------------------------------------------------------------------
-// Operand layout of a data set, 32 samples of an SNP's genotype row g (0, 1) per thread: the bit
-// rows 2 snp + g hold the class's words of the reference layout, cases then controls, each class
+// Operand layout of a data set, 32 samples of an SNP's genotype row g < G per thread: the bit
+// rows G snp + g hold the class's words of the reference layout, cases then controls, each class
 // padded to a multiple of 256 samples; the planes hold the same bits spread to e2m1 in rows
-// f4_row(snp, g), SNPs past the last one zero.
+// 8 G (snp / 8) + 8 g + snp % 8, SNPs past the last one zero.
+template <int G>
 __global__ void f4_layout_kernel(DevData d, uint32_t* bits, uint4* planes, int wpr, int wc, int nc32, int nt32,
                                  int rows) {
     const size_t per_snp = 3 * (size_t)(d.cw + d.tw);
@@ -821,7 +822,7 @@ __global__ void f4_layout_kernel(DevData d, uint32_t* bits, uint4* planes, int w
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
          e += (long long)gridDim.x * blockDim.x) {
         const int row = (int)(e / wpr), o = (int)(e - (long long)row * wpr);
-        const int snp = 8 * (row >> 4) + (row & 7), g = (row >> 3) & 1;
+        const int snp = 8 * (row / (8 * G)) + (row & 7), g = (row >> 3) % G;
         const bool ctrl = o >= wc;
         const int k = ctrl ? o - wc : o;
         uint32_t v = 0;
@@ -831,7 +832,7 @@ __global__ void f4_layout_kernel(DevData d, uint32_t* bits, uint4* planes, int w
                                             (size_t)g * (ctrl ? d.tw : d.cw) + (k >> 1));
                 v = (uint32_t)(word >> (32 * (k & 1)));
             }
-            bits[((size_t)2 * snp + g) * wpr + o] = v;
+            bits[((size_t)G * snp + g) * wpr + o] = v;
         }
         planes[e] = f4_expand_b(v);
     }
@@ -856,18 +857,20 @@ void f4_sizes(const DevData& d, F4Plan& f) {
     f.wpr = 8 * ((f.nw_c + 3) / 4) + 8 * ((f.nw_t + 3) / 4);
 }
 
-cudaError_t f4_prepare(const DevData& d, F4Plan& f, cudaStream_t s) {
+cudaError_t f4_prepare(const DevData& d, F4Plan& f, int genotypes, cudaStream_t s) {
     const int wc = 8 * ((f.nw_c + 3) / 4);
-    f.rows = 16 * ((d.snps + 7) / 8);
+    f.rows = 8 * genotypes * ((d.snps + 7) / 8);
     const size_t plane_bytes = (size_t)f.rows * f.wpr * 16;  // one allocation: planes, then bits
-    cudaError_t e = cudaMalloc((void**)&f.planes, plane_bytes + (size_t)2 * d.snps * f.wpr * 4);
+    cudaError_t e = cudaMalloc((void**)&f.planes, plane_bytes + (size_t)genotypes * d.snps * f.wpr * 4);
     if (e != cudaSuccess) return e;
     f.bits = reinterpret_cast<uint32_t*>(f.planes + plane_bytes);
     const long long total = (long long)f.rows * f.wpr;
-    f4_layout_kernel<<<(unsigned)std::min<long long>((total + 255) / 256, 8192), 256, 0, s>>>(
+    const unsigned grid = (unsigned)std::min<long long>((total + 255) / 256, 8192);
+    (genotypes == 2 ? f4_layout_kernel<2> : f4_layout_kernel<3>)<<<grid, 256, 0, s>>>(
         d, f.bits, reinterpret_cast<uint4*>(f.planes), f.wpr, wc, 2 * f.nw_c, 2 * f.nw_t, f.rows);
     count_launch();
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (genotypes == 3) return f4_missing_maps(f, d.snps);
     if ((e = tensor_map(&f.map_b, f.planes, f.rows, 16 * f.wpr, kXRow, kXN / 2, true)) != cudaSuccess) return e;
     if ((e = f4_bit_map(&f.map_j, f, f.bits, 2 * d.snps, 2 * kXJ)) != cudaSuccess) return e;
     return f4_bit_map(&f.map_i, f, f.bits, 2 * d.snps, 2);

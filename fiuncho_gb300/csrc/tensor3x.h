@@ -17,8 +17,9 @@ __host__ __device__ __forceinline__ int t3x_tiles(int n, int jf) { return (t3x_g
 
 // Sizes of the 4-bit layout (host).
 void f4_sizes(const DevData& d, F4Plan& f);
-// Operand planes and bit rows of a data set (built once, on stream s).
-cudaError_t f4_prepare(const DevData& d, F4Plan& f, cudaStream_t s);
+// Operand planes and bit rows of a data set (built once, on stream s), of 2 genotypes a SNP or of 3 (data
+// with missing calls).
+cudaError_t f4_prepare(const DevData& d, F4Plan& f, int genotypes, cudaStream_t s);
 void f4_release(F4Plan& f);
 cudaError_t f4_bit_map(CUtensorMap* m, const F4Plan& f, const uint32_t* bits, int rows, int box_rows);
 // log2 of the control weight W when cases + W controls fit one FP32

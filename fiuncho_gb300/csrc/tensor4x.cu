@@ -239,7 +239,7 @@ __device__ __forceinline__ void t4x_slices(const T4xCores<T>& v, TL&& tabl, TK&&
 
 // ALL: every combination takes the exact path (a search's first units, before a threshold; dumps and
 // digests).  Otherwise the bound comes first and the few combinations above it are evaluated from the
-// data set (warp_exact_key4): the exact path's registers beside the bound's cost 20 % of the whole.
+// data set (warp_exact_key): the exact path's registers beside the bound's cost 20 % of the whole.
 // SPLIT: classes that do not share an accumulator, as in the order-3 kernel: cases accumulate in one region
 // and go to shared memory as 16-bit counts, controls in the other; one combination at a time is evaluated
 // from both beside each other.
@@ -593,7 +593,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
             auto tabk = [&](int e) { return tabk0[(e ^ zb) * kYK]; };
             auto exact_append = [&](int src, int u, int lu) {  // a survivor of lane src
                 const int cmb[4] = {it.i, it.j, __shfl_sync(0xffffffffu, k, src), __shfl_sync(0xffffffffu, lu, src) + u};
-                const long long key = warp_exact_key4(&w.d, w.base_key, cmb[0], cmb[1], cmb[2], cmb[3]);
+                const long long key = warp_exact_key<4>(&w.d, w.base_key, cmb[0], cmb[1], cmb[2], cmb[3]);
                 if (lane == 0 && key >= thr) live_append(sink, key, pack_code(cmb, 4, w.bits));
             };
             // the exact path of combination (i, j, k, lu), whose slices walk(use) makes: use(w, cell index,

@@ -155,3 +155,57 @@ def test_several_items_per_pair(order, snps, cases, ctrls):
         gs.set_kernel(kernel)
         lists.append([(r.combination, r.val) for r in gs.run(res, order, Distribution(snps, order - 1), 1000)])
     assert lists[0] == lists[1]
+
+
+MISSING_3 = [  # snps, cases, controls, missing rate
+    (32, 1, 1, 0.3), (33, 64, 65, 0.2), (41, 63, 256, 0.05), (65, 257, 129, 0.01), (66, 100, 300, 0.1),
+    (97, 512, 40, 0.03), (130, 1023, 1025, 0.002), (177, 2047, 2049, 0.02), (121, 100, 4000, 0.5),
+]
+
+
+@pytest.mark.parametrize("snps,cases,ctrls,rate", MISSING_3)
+def test_order3_missing_calls(snps, cases, ctrls, rate):
+    """Data with missing calls: the list, for few outputs (a tight threshold) and for many, of the kernel that
+    counts all 27 cells on the tensor cores against the full-table kernel's, and its shards'."""
+    import numpy as np
+    from fiuncho_gb300 import Dataset, Distribution, GpuSearch, _lib
+    from fiuncho_gb300.search import Resident
+    full = _data(snps, cases, ctrls, 5 * snps)
+    rng = np.random.default_rng(snps)
+    rows = full.data.copy().reshape(snps, -1)
+    for at, words in ((0, full.cases_words), (3 * full.cases_words, full.ctrls_words)):
+        called = np.packbits(rng.random((snps, 64 * words)) >= rate, axis=1, bitorder="little").view(np.uint64)
+        for g in range(3):
+            rows[:, at + g * words:at + (g + 1) * words] &= called
+    ds = Dataset(cases, ctrls, snps, full.cases_words, full.ctrls_words, rows.reshape(-1))
+    gs = GpuSearch(0)
+    res = Resident(gs.ctx, ds)
+    d = Distribution(snps, 2)
+    for outputs in (3, 40, 3000):
+        gs.set_kernel(_lib.KERNEL_AUTO)
+        a = gs.run(res, 3, d, outputs)
+        assert gs.last_tile()[0] == _lib.KERNEL_TENSOR
+        parts = [r for s in range(3) for r in gs.run_shard(res, 3, s, 3, outputs)]
+        gs.set_kernel(_lib.KERNEL_FULL)
+        b = gs.run(res, 3, d, outputs)
+        assert [(r.combination, r.val) for r in a] == [(r.combination, r.val) for r in b]
+        parts.sort(key=lambda r: (-r.val, r.combination))
+        assert [r.val for r in parts[:outputs]] == [r.val for r in b]
+
+
+def test_order3_rows_that_share_samples_keep_the_full_tables():
+    """Rows that are not genotypes (a sample in two of them, bits past the class) stay with the full-table
+    kernel, which takes any data."""
+    import numpy as np
+    from fiuncho_gb300 import Dataset, Distribution, GpuSearch, _lib
+    full = _data(40, 100, 90, 3)
+    gs = GpuSearch(0)
+    for change in ("shared", "past"):
+        rows = full.data.copy().reshape(40, -1)
+        if change == "shared":
+            rows[7, 0] |= np.uint64(1)
+            rows[7, full.cases_words] |= np.uint64(1)
+        else:
+            rows[7, full.cases_words - 1] |= np.uint64(1) << np.uint64(63)
+        gs.run(Dataset(100, 90, 40, full.cases_words, full.ctrls_words, rows.reshape(-1)), 3, Distribution(40, 2), 5)
+        assert gs.last_tile()[0] == _lib.KERNEL_FULL
