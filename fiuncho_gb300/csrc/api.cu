@@ -382,8 +382,6 @@ int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu
     const bool tensor = kernel == FIU_KERNEL_TENSOR;
     const bool pair_major = e4_pair_major(kernel, res, w);
     const long long units = tensor ? tensor_units(*res->t3, w) : pair_major ? res->e4_items : w.n_prefixes;
-    int* t_status = (int*)(ctx->ctl + 16);
-    if (tensor) CK(cudaMemsetAsync(t_status, 0, sizeof(int), ctx->stream), "status reset");
     const unsigned keep = outputs + std::max(32u, outputs / 8);
     const size_t cap = std::max<size_t>(
         {tensor ? 524288u : 65536u, (size_t)(tensor ? 128 : 16) * keep, (size_t)res->d.snps + keep});
@@ -392,11 +390,24 @@ int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu
         (rc = grow(ctx, ctx->mi64, ctx->mi64_cap, (size_t)keep)))
         return rc;
     cudaStream_t s = ctx->stream;
+    // counters, reset and read together (kCtl words): candidates, overflow, live threshold, candidates at or
+    // above the last threshold, status of the tensor kernels
     unsigned* count = ctx->ctl;
     unsigned* overflow = ctx->ctl + 1;
-    unsigned* scratch = ctx->ctl + 4;
-    unsigned* hist = ctx->ctl + 512;
     long long* live_thr = (long long*)(ctx->ctl + 2);
+    unsigned* kept = ctx->ctl + 4;
+    int* t_status = (int*)(ctx->ctl + 5);
+    constexpr size_t kCtl = 6 * sizeof(unsigned);
+    unsigned* scratch = ctx->ctl + 8;
+    unsigned* hist = ctx->ctl + 512;
+    auto reset = [&](unsigned held, long long thr) {
+        ctx->pinned[0] = held;
+        ctx->pinned[1] = ctx->pinned[4] = ctx->pinned[5] = 0;
+        memcpy(ctx->pinned + 2, &thr, sizeof(thr));
+        return cudaMemcpyAsync(count, ctx->pinned, kCtl, cudaMemcpyHostToDevice, s);
+    };
+    bool sorted = false;  // the held candidates are in order
+    bool waited_out = false;  // a tensor kernel gave up a wait
     long long thr = (long long)0x8000000000000000ull;
     unsigned have = 0;
     const double per_prefix = (double)binom(w.dist_n, order) / std::max<double>(1.0, (double)binom(w.dist_n, order - 1));
@@ -426,9 +437,7 @@ int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu
         const long long few = std::max<long long>(1, (long long)(2.0 * keep / std::max(1.0, per_unit)));
         const long long fit = (long long)((double)cap / 4 / std::max(1.0, per_unit));
         const long long m1 = std::min(m_end, m + std::max(few, std::min<long long>(fit, ctx->sms / 2)));
-        ctx->pinned[0] = ctx->pinned[1] = 0;
-        memcpy(ctx->pinned + 2, &thr, sizeof(thr));
-        CK(cudaMemcpyAsync(count, ctx->pinned, 4 * sizeof(unsigned), cudaMemcpyHostToDevice, s), "reset counters");
+        CK(reset(0, thr), "reset counters");
         CK(cudaMemsetAsync(hist, 0, kLiveBins * sizeof(unsigned), s), "reset counters");
         CandSink sink{ctx->cand, count, overflow, (unsigned)cap, thr, ctx->timing ? ctx->evaluated : nullptr};
         sink.hist = hist;
@@ -447,10 +456,8 @@ int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu
             a = b;
         }
         if (ctx->timing) CK(cudaEventRecord(ctx->ev1, s), "event");
-        unsigned* kept = scratch;  // [0]: candidates at or above the last threshold
-        CK(cudaMemsetAsync(kept, 0, sizeof(unsigned), s), "reset counters");
         CK(live_compact(sink, ctx->tmp, kept, s), "candidate selection");
-        CK(cudaMemcpyAsync(ctx->pinned, count, 5 * sizeof(unsigned), cudaMemcpyDeviceToHost, s), "read counters");
+        CK(cudaMemcpyAsync(ctx->pinned, count, kCtl, cudaMemcpyDeviceToHost, s), "read counters");
         CK(cudaStreamSynchronize(s), "count kernel");
         if (ctx->timing) {
             float ms = 0;
@@ -458,6 +465,7 @@ int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu
             ctx->count_ms += ms;
             ctx->count_launches += launches;
         }
+        waited_out = ctx->pinned[5] != 0;
         if (!ctx->pinned[1]) {
             std::swap(ctx->cand, ctx->tmp);
             std::swap(ctx->cand_cap, ctx->tmp_cap);
@@ -465,6 +473,7 @@ int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu
             if (have > keep) {
                 CK(select_top(ctx->cand, have, keep, ctx->tmp, scratch, s), "top-N selection");
                 have = keep;
+                sorted = true;
             }
             m = m_end;
         }
@@ -473,10 +482,7 @@ int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu
         if (ctx->cancel.load(std::memory_order_relaxed)) return fail(ctx, FIU_ERR_CANCELLED, "search cancelled");
         const long long m1 = std::min(m_end, m + chunk);
         const auto t_chunk = std::chrono::steady_clock::now();
-        ctx->pinned[0] = have;
-        ctx->pinned[1] = 0;
-        memcpy(ctx->pinned + 2, &thr, sizeof(thr));
-        CK(cudaMemcpyAsync(count, ctx->pinned, 4 * sizeof(unsigned), cudaMemcpyHostToDevice, s), "reset counters");
+        CK(reset(have, thr), "reset counters");
         CandSink sink{ctx->cand, count, overflow, (unsigned)cap, thr, ctx->timing ? ctx->evaluated : nullptr};
         if (tensor) {
             CK(cudaMemsetAsync(hist, 0, kLiveBins * sizeof(unsigned), s), "reset counters");
@@ -495,8 +501,9 @@ int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu
         else
             CK(launch_kernel(kernel, tp, res, w, m, m1, sink, nullptr, s, ctx->sms), "count kernel launch");
         if (ctx->timing) CK(cudaEventRecord(ctx->ev1, s), "event");
-        CK(cudaMemcpyAsync(ctx->pinned, count, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, s), "read counters");
+        CK(cudaMemcpyAsync(ctx->pinned, count, kCtl, cudaMemcpyDeviceToHost, s), "read counters");
         CK(cudaStreamSynchronize(s), "count kernel");
+        waited_out = waited_out || ctx->pinned[5] != 0;
         sec_per_unit = std::chrono::duration<double>(std::chrono::steady_clock::now() - t_chunk).count() /
                        (double)(m1 - m);
         if (ctx->timing) {
@@ -519,8 +526,10 @@ int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu
             CK(cudaStreamSynchronize(s), "top-N selection");
             thr = last.key;
             have = keep;
+            sorted = true;
         } else {
             have = M;
+            sorted = false;
         }
         m = m1;
         const double next = have < keep ? (double)(cap - have) / (4.0 * std::max(1.0, per_unit))
@@ -528,21 +537,22 @@ int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu
         const double time_cap = ctx->cancellable ? kLaneChunkSeconds / std::max(sec_per_unit, 1e-12) : 4.0e18;
         chunk = (long long)std::max(1.0, std::min({next, time_cap, 4.0e18}));
     }
-    if (tensor) {
-        int st = 0;
-        CK(cudaMemcpyAsync(&st, t_status, sizeof(int), cudaMemcpyDeviceToHost, s), "status");
-        CK(cudaStreamSynchronize(s), "status");
-        if (st) return fail(ctx, FIU_ERR_TIMEOUT, "tensor kernel: a tensor-memory wait ran past its limit");
-    }
-    // Final order of the kept set, then FP64 re-score of every kept candidate.
-    CK(select_top(ctx->cand, have, keep, ctx->tmp, scratch, s), "top-N selection");
+    if (waited_out) return fail(ctx, FIU_ERR_TIMEOUT, "tensor kernel: a tensor-memory wait ran past its limit");
+    // Final order of the kept set, then FP64 re-score of every kept candidate.  (Its scratch is the candidates'
+    // second buffer: allocated from the stream's pool on each call it cost 150 us.)
+    if (!sorted) CK(select_top(ctx->cand, have, keep, ctx->tmp, scratch, s), "top-N selection");
     const unsigned n = std::min(have, keep);
-    CK(rescore_sort(w.d, (int)order, w.bits, ctx->cand, n, ctx->mi64, s), "FP64 rescore");
+    CK(rescore_sort(w.d, (int)order, w.bits, ctx->cand, n, ctx->mi64, ctx->tmp, s), "FP64 rescore");
     const unsigned nout = std::min(n, outputs);
-    std::vector<Cand> hc(nout);
-    std::vector<double> hv(nout);
-    CK(cudaMemcpyAsync(hc.data(), ctx->cand, nout * sizeof(Cand), cudaMemcpyDeviceToHost, s), "results");
-    CK(cudaMemcpyAsync(hv.data(), ctx->mi64, nout * sizeof(double), cudaMemcpyDeviceToHost, s), "results");
+    std::vector<Cand> pageable;
+    Cand* hc = reinterpret_cast<Cand*>(ctx->pinned + kPinnedWords);
+    if (nout > kPinnedResults) {
+        pageable.resize(nout + (nout + 1) / 2);
+        hc = pageable.data();
+    }
+    double* hv = reinterpret_cast<double*>(hc + nout);
+    CK(cudaMemcpyAsync(hc, ctx->cand, nout * sizeof(Cand), cudaMemcpyDeviceToHost, s), "results");
+    CK(cudaMemcpyAsync(hv, ctx->mi64, nout * sizeof(double), cudaMemcpyDeviceToHost, s), "results");
     CK(cudaStreamSynchronize(s), "results");
     for (unsigned i = 0; i < nout; ++i) {
         int c[kMaxOrder];
@@ -640,7 +650,8 @@ int fiu_create(int device, fiu_ctx** out) {
         cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
         cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaMalloc((void**)&ctx->ctl, (512 + kLiveBins) * sizeof(unsigned)) != cudaSuccess ||
-        cudaMallocHost((void**)&ctx->pinned, 16 * sizeof(unsigned)) != cudaSuccess) {
+        cudaMallocHost((void**)&ctx->pinned, kPinnedWords * sizeof(unsigned) + kPinnedResults * (sizeof(Cand) + 8)) !=
+            cudaSuccess) {
         fiu_destroy(ctx);
         return FIU_ERR_CUDA;
     }

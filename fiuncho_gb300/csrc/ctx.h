@@ -10,6 +10,10 @@
 #include "../../include/fiuncho_gpu.h"
 #include "internal.h"
 
+namespace fiu {
+constexpr size_t kPinnedWords = 16, kPinnedResults = 1024;
+}
+
 struct fiu_ctx {
     int device = 0;
     int sms = 0;
@@ -21,10 +25,10 @@ struct fiu_ctx {
     size_t cand_cap = 0;
     fiu::Cand* tmp = nullptr;   // select_top working space
     size_t tmp_cap = 0;
-    unsigned* ctl = nullptr;  // [0] count, [1] overflow, [2..] select scratch (262)
+    unsigned* ctl = nullptr;  // [0..5] counters of a search, [8..] select scratch (262), [512..] key histogram
     double* mi64 = nullptr;
     size_t mi64_cap = 0;
-    unsigned* pinned = nullptr;  // host mirror of ctl[0..1]
+    unsigned* pinned = nullptr;  // host mirror of the first words of ctl (kPinnedWords), then up to kPinnedResults results
     // optional timing of the counting kernels (CUDA events on `stream`)
     bool timing = false;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;

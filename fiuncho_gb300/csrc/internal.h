@@ -276,7 +276,8 @@ cudaError_t live_compact(const CandSink& sink, Cand* out, unsigned* out_count, c
 cudaError_t select_top(Cand* buf, unsigned M, unsigned keep, Cand* tmp, unsigned* scratch, cudaStream_t s);
 // FP64 MI of candidates (recomputing their full tables), then sorts
 // (mi64 desc, code asc) in place; out_mi64[i] matches cands[i] after the sort.
-cudaError_t rescore_sort(const DevData& d, int order, int bits, Cand* cands, unsigned n, double* mi64,
+// tmp: scratch of at least 2 n entries.
+cudaError_t rescore_sort(const DevData& d, int order, int bits, Cand* cands, unsigned n, double* mi64, Cand* tmp,
                          cudaStream_t s);
 cudaError_t launch_tables(const DevData& d, int order, const int* combos, size_t count, uint32_t* cases_out,
                           uint32_t* ctrls_out, double* mi64, cudaStream_t s);

@@ -180,25 +180,21 @@ __global__ void unscore_kernel(const Scored* __restrict__ in, unsigned n, Cand* 
     }
 }
 
-cudaError_t rescore_sort(const DevData& d, int order, int bits, Cand* cands, unsigned n, double* mi64,
+cudaError_t rescore_sort(const DevData& d, int order, int bits, Cand* cands, unsigned n, double* mi64, Cand* tmp,
                          cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     if (n > kSortCap) return cudaErrorInvalidValue;
-    // Scored scratch lives in the mi64 buffer's companion: allocate transiently.
-    Scored* sc = nullptr;
-    cudaError_t e = cudaMallocAsync((void**)&sc, (size_t)n * sizeof(Scored), s);
-    if (e != cudaSuccess) return e;
+    Scored* sc = reinterpret_cast<Scored*>(tmp);
     rescore_kernel<<<n, kScoreThreads, 0, s>>>(d, order, bits, cands, sc);
     count_launch();
-    if ((e = cudaGetLastError()) == cudaSuccess)
-        e = sort_small<Scored, ScoredBetter>(sc, n, Scored{-1.0e300, ~0ull, 0}, s);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = sort_small<Scored, ScoredBetter>(sc, n, Scored{-1.0e300, ~0ull, 0}, s);
     if (e == cudaSuccess) {
         unscore_kernel<<<(n + 255) / 256, 256, 0, s>>>(sc, n, cands, mi64);
         count_launch();
         e = cudaGetLastError();
     }
-    cudaError_t e2 = cudaFreeAsync(sc, s);
-    return e != cudaSuccess ? e : e2;
+    return e;
 }
 
 __global__ void tables_kernel(DevData d, int K, const int* __restrict__ combos, size_t count,
