@@ -24,13 +24,17 @@
 // others get the exact fixed-point key, so the kept set is the one of the exact
 // key.
 //
-// Measured (whole searches): 300 SNPs x 4 000/4 000 81.9 -> 37.0 ms, 300 x
-// 558/1 012 66.2 -> 31.0 ms, against e4m3 operands, one CTA a tile, 243
-// logarithms a combination (1 944 cycles a warp and SM quarter; the bound takes 81
-// reciprocals and about 930 arithmetic cycles) and triples counted by POPC.
-// Without the evaluation the two take 26 and 13 ms.  Classes that do not share an
-// accumulator (SPLIT): 100 SNPs x 9 000/9 800 6.7 -> 4.1 ms (2.3 of the kernel's
-// 3.1 ms without the evaluation).
+// Measured (whole searches): 300 SNPs x 4 000/4 000 81.9 -> 34.3 ms, 300 x
+// 558/1 012 60.0 -> 29.4 ms, against e4m3 operands, one CTA a tile, 243
+// logarithms a combination (1 944 cycles a warp and SM quarter) and triples
+// counted by POPC.  Without the evaluation the two take 26 and 13 ms; the
+// evaluation of 64 combinations by a warp is 2 240 cycles of bound (81 x 2
+// reciprocals 800, splitting the classes 650) and about 700 of derivation and takes
+// 5 400 beside the builders, with two warps a quarter to hide latencies.  Tried:
+// three warps a quarter on one combination at a time (104 registers) 40 ms; the
+// slices in a loop (a third of the code) 32.8; three cells at a time through the
+// bound 29.5.  Classes that do not share an accumulator (SPLIT): 100 SNPs x
+// 9 000/9 800 6.7 -> 3.1 ms.
 //
 // Reference semantics: GenotypeTable::combine_and_popcnt for order 4
 // (src/base/gt_popcnt.cpp:4-35) and MutualInformation::compute
@@ -137,6 +141,13 @@ __device__ __forceinline__ T4xItem t4x_item(const long long* __restrict__ begin,
         q -= nl;
     }
 }
+
+// Every other item of a walker is turned over: CTA r has the k of half 1 - r, in
+// blocks of 4 from the last to the first (position kk holds k kk ^ 12), since in a
+// tile on the diagonal the first k have the most l above them and an SM quarter
+// keeps its block: with all items one way up the fullest quarter had 1.14 (300
+// SNPs) to 1.43 (100) times the mean.
+__device__ __forceinline__ int t4x_flip(unsigned item) { return item & 1 ? 12 : 0; }
 
 // Columns the MMA of an item of ng groups multiplies (at least 64).
 __device__ __forceinline__ int t4x_n(int ng) { return 32 * max(ng, 2); }
@@ -323,7 +334,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
                 for (long long g = g0 + cid; g < g1 && ok; g += ncl) {
                     // this CTA's first k row (in a layer the owned k are consecutive residue-ordered rows;
                     // rows past the last owned one are loaded too and ignored by the epilogue)
-                    const int krow = 2 * ((LAYER ? residue_row(it.k0, kstep, n) : it.k0) + kYK * (int)rank);
+                    const int krow =
+                        2 * ((LAYER ? residue_row(it.k0, kstep, n) : it.k0) + kYK * ((int)rank ^ (int)(item & 1)));
                     const int brow = 2 * it.l0 + t4x_n(it.ng) / 2 * (int)rank, irow = 2 * it.i, jrow = 2 * it.j;
                     const bool half = it.ng <= kYHalfG;
                     item_ng[item++ % kYMeta] = it.ng;
@@ -437,7 +449,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
                     }
                 }
                 if (t < kYK) {
-                    const int k = it.k0 + kstep * (kYK * (int)rank + t);
+                    const int k = it.k0 + kstep * (kYK * ((int)rank ^ (int)(item & 1)) + t);
                     auto put = [&](int e, Tab v) {
                         if constexpr (SPLIT) tk[e * kYK + t] = v;
                         else tk[e * kYK + t] = f2_dup(v);
@@ -471,13 +483,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
         // thread: 16-byte chunk c (32 samples) of the k rows rg and rg + 16 of every second stage
         const int t = (tid - 128) & (32 * kYBuildWarps - 1), c = t & 7, rg = t >> 3;
         const uint32_t full0 = cluster_addr(smem_u32(&full_a[0]), 0);
-        // A row (kk / 4, x, y, z, kk % 4) of staged row (kk, z) = rg + 16 u: u + 1 is 64 rows on
+        // A row (kk / 4, x, y, z, kk % 4) of staged row (kk, z) = rg + 16 u: u + 1 is 64 rows on (back when turned over)
         const int kk = rg >> 1, z = rg & 1, m0 = 32 * (kk >> 2) + 4 * z + (kk & 3);
         const int dst0 = m0 * kYRow + ((c ^ (m0 & 7)) << 4);
         unsigned s = 0, par = 0, sa = 0;                  // copy stage, A stage
         unsigned se = kStages - kAStages, pe = 1;       // the stage whose MMAs free this A stage
         bool mine = warp < 8;
-        for (long long g = g0 + cid; g < g1 && ok; g += ncl) {
+        int turn = 0;  // an item turned over: block b is block 3 - b
+        for (long long g = g0 + cid; g < g1 && ok; g += ncl, turn ^= 96 * kYRow) {
             for (int ks = 0; ks < ksteps; ++ks, mine = !mine) {
                 if (mine) {
                     if (!t3_wait(smem_u32(&full_t[s]), par, abort)) {
@@ -492,12 +505,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
                         ok = false;
                         break;
                     }
-                    uint8_t* dst = sma + sa * kYSA + dst0;
+                    uint8_t *dst = sma + sa * kYSA + (dst0 ^ turn), *dst2 = sma + sa * kYSA + (dst0 ^ turn ^ 64 * kYRow);
 #pragma unroll
                     for (int xy = 0; xy < 4; ++xy) {
                         const uint32_t ij = (xy & 2 ? i1 : i0) & (xy & 1 ? j1 : j0);
                         *reinterpret_cast<uint4*>(dst + 8 * xy * kYRow) = f4_expand_a(ij, k0);
-                        *reinterpret_cast<uint4*>(dst + (64 + 8 * xy) * kYRow) = f4_expand_a(ij, k1);
+                        *reinterpret_cast<uint4*>(dst2 + 8 * xy * kYRow) = f4_expand_a(ij, k1);
                     }
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     __syncwarp();
@@ -518,7 +531,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
         asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");
         // ---------------------------------------------------------------- epilogue (both CTAs)
         const int q = warp & 3, hh = (warp - 12) >> 2;  // lane quarter (4 k); its two warps take alternate groups
-        const int zb = lane >> 4, kk = 4 * q + ((lane >> 2) & 3), lc = 2 * (lane & 3);
+        const int zb = lane >> 4, kk0 = 4 * q + ((lane >> 2) & 3), lc = 2 * (lane & 3);
         const uint32_t wmask = (1u << pack) - 1u;
         uint4* mine = stash + (warp - 12) * ((kP4G + 1) / 2) * 128 + lane;  // written and read by this warp only
         unsigned item = 0;
@@ -526,7 +539,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
         for (long long g = g0 + cid; g < g1 && ok; g += ncl, ++item) {
             const T4xItem it = t4x_item<LAYER>(begin, per, pinfo, n_pairs, n, kstep, g, at);
             const unsigned buf = item & 1, ph = (item >> 1) & 1;
-            const int k = it.k0 + kstep * (kYK * (int)rank + kk);
+            const int gi0 = (hh + item) & 1;  // the odd group of an item goes to either warp in turn
+            const int kk = kk0 ^ t4x_flip(item), k = it.k0 + kstep * (kYK * ((int)rank ^ (int)(item & 1)) + kk);
             const bool k_ok = k < n;
             // entries of the rows (i, k), (j, k) and k, in units of 16 bytes
             const int rp = k_ok ? __ldg(row_p + k) : 0;
@@ -567,7 +581,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;");
 #pragma unroll 1
-                for (int gi = hh; gi < it.ng; gi += 2)
+                for (int gi = gi0; gi < it.ng; gi += 2)
 #pragma unroll
                     for (int x = 0; x < 2; ++x) {
                         uint4 o[2];
@@ -643,9 +657,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
                         ld(tkl, 2 * l + (z ^ zb), kl[z]);
                     }
                 };
-                load(hh, 0);
+                load(gi0, 0);
 #pragma unroll 1
-                for (int gi = hh; gi < it.ng; gi += 2) {
+                for (int gi = gi0; gi < it.ng; gi += 2) {
                     const int ll = 16 * gi + 8 * zb + lc, l = it.l0 + ll;
                     const bool v0 = k_ok && l < n && l > k, v1 = k_ok && l + 1 < n && l + 1 > k;
                     const unsigned m0 = __ballot_sync(0xffffffffu, v0), m1 = __ballot_sync(0xffffffffu, v1);
@@ -721,9 +735,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
 #pragma unroll
                     for (int z = 0; z < 2; ++z) ld(tkl + 2 * m + (z ^ zb), v.kl[z]);
                 };
-                load(hh);
+                load(gi0);
 #pragma unroll 1
-                for (int gi = hh; gi < it.ng; gi += 2) {
+                for (int gi = gi0; gi < it.ng; gi += 2) {
                     const int ll = 16 * gi + 8 * zb + lc, l = it.l0 + ll;
                     const bool v0 = k_ok && l < n && l > k, v1 = k_ok && l + 1 < n && l + 1 > k;
                     const unsigned m0 = __ballot_sync(0xffffffffu, v0), m1 = __ballot_sync(0xffffffffu, v1);
