@@ -11,7 +11,7 @@ with the data set resident in HBM; ``e2e`` is the same metric through the
 public host-buffer call (``fiu_search``: pinned host data set -> device ->
 search -> results to host, all inside the timed region).  ``roofline`` is the
 roofline of the dominant (counting) kernel: for the tcgen05 kernel the tensor
-bound (2^k multiply-adds per combination and sample, e4m3 peak = 2 x the
+bound (2^k multiply-adds per combination and sample, 4-bit peak = 4 x the
 measured dense bf16 rate); for the CUDA-core kernels the HBM bound, with
 ``int_roofline`` their integer (AND+POPC) roofline against a peak measured
 live on this GPU.
@@ -321,14 +321,14 @@ def run_gpu(args, spec):
         pass
     if kernel_id == _lib.KERNEL_TENSOR:
         # 2^k core cells per combination, each a dot product over the samples of its class:
-        # 2^k multiply-adds (2 * 2^k flops) per combination and sample, e4m3 operands.
+        # 2^k multiply-adds (2 * 2^k flops) per combination and sample, e2m1 operands.
         flops_per_launch = kcombos.value * 2 * 2 ** k * spec.samples / max(1, klaunch.value)
         tc_achieved = flops_per_launch / avg_launch_s / 1e12 if avg_launch_s > 0 else 0.0
-        tc_peak = 2.0 * peaks.get("bf16_tflops", 1900.0)
+        tc_peak = 4.0 * peaks.get("bf16_tflops", 1900.0)
         roofline = {"bound": "tensor", "achieved": tc_achieved, "peak": tc_peak, "unit": "TFLOP/s",
                     "frac": tc_achieved / tc_peak, "traffic": traffic,
                     "flops_per_combination_sample": 2 * 2 ** k,
-                    "peak_source": "2 x measured dense bf16 (%s; e4m3 dense rate = 2 x bf16), of measured"
+                    "peak_source": "4 x measured dense bf16 (%s; 4-bit dense rate = 4 x bf16), of measured"
                                    % ("MEASURED_PEAKS.json" if "bf16_tflops" in peaks else "fallback 1.9 PF"),
                     "hbm": {"achieved": hbm_achieved, "peak": hbm_peak, "unit": "GB/s",
                             "frac": hbm_achieved / hbm_peak}}
@@ -346,9 +346,9 @@ def run_gpu(args, spec):
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": ws, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": 1e3 * my_time / args.steps, "step_ms": [round(x, 3) for x in step_ms],
         "higher_is_better": True, "scaling": "strong",  # the one scan's work units split over the ranks
-        "vs_baseline": None, "dtype": "e4m3", "data": "synthetic",
-        "arithmetic": "one-hot data: e4m3 0/1 operands on the tensor cores with FP32 accumulation (exact integer "
-                      "counts below 2^24), derived cells in int32, MI keys in int64 fixed point, the kept candidates "
+        "vs_baseline": None, "dtype": "e2m1", "data": "synthetic",
+        "arithmetic": "one-hot data: e2m1 operands (products of two samples are 0 or 1) on the tensor cores with FP32 "
+                      "accumulation (exact integer counts below 2^24), derived cells exact in FP32, MI keys in int64 fixed point, the kept candidates "
                       "re-scored in FP64; other data: uint64 AND + POPC",
         "config": {"workload": args.workload, "snps": spec.snps, "cases": spec.cases, "ctrls": spec.ctrls,
                    "order": spec.order, "outputs": spec.outputs, "combinations": total_combos,

@@ -242,14 +242,13 @@ static int missing_plan(fiu_ctx* ctx, const fiu_resident* res) {
     return cuda_fail(ctx, e, "tensor operands and work items");
 }
 
-// Below this many samples an order-4 scan is faster on the CUDA-core
-// pair-major kernel: the tensor kernel's per-combination epilogue then
-// outweighs the counting it saves (measured at 150 SNPs, pair-major vs
-// tensor: 1 060 samples 7.1 vs 6.2 ms, 1 800 samples 8.9 vs 6.3 ms, 4 000
-// samples 14.8 vs 7.0 ms, 14 900 samples 44.8 vs 16.9 ms; the pair-major
-// time falls with the samples, the tensor kernel's hardly below 6 ms).
-// Forcing FIU_KERNEL_TENSOR still uses it.
-constexpr int kT4MinSamples = 1024;
+// Order-4 scans of fewer samples and SNPs keep the CUDA-core pair-major kernel unless FIU_KERNEL_TENSOR is
+// forced.  In a search of its own the tensor kernel is the faster one at every size measured from 30 SNPs
+// (pair-major vs tensor, resident data: 30 SNPs x 200 samples 0.54 vs 0.24 ms, 100 x 300 1.24 vs 1.00, 150 x
+// 200 3.3 vs 2.9, 150 x 900 4.8 vs 2.9, 300 x 900 65 vs 28), so there the SNPs decide alone; scans that
+// share rounds with others (batched and served ones) go by the samples, since a round takes many small
+// scans at once and the tensor kernel one.
+constexpr int kT4MinSamples = 1024, kT4MinSnps = 32;
 
 int choose_tile(fiu_ctx* ctx, const fiu_resident* res, const ScanWork& w, int requested_kernel, int& kernel, int& tp,
                 bool allow_tensor) {
@@ -369,7 +368,9 @@ int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu
     if (outputs == 0 || w.n_prefixes == 0) return FIU_OK;
     CK(cudaSetDevice(ctx->device), "cudaSetDevice");
     int tp = 256;
-    const int requested = kernel ? kernel : ctx->kernel;
+    int requested = kernel ? kernel : ctx->kernel;
+    if (requested == FIU_KERNEL_AUTO && order == 4 && res->d.snps >= kT4MinSnps && tensor_ok(res, w))
+        requested = FIU_KERNEL_TENSOR;
     const bool missing = requested == FIU_KERNEL_AUTO && missing_ok(res, w);
     if (missing && (rc = missing_plan(ctx, res)) == FIU_OK) {
         kernel = FIU_KERNEL_TENSOR;

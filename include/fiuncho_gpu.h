@@ -45,7 +45,9 @@ extern "C" {
 #define FIU_KERNEL_ELIDED_POPC 2 /* one-hot data, orders 2-4: 2^order cells + exact marginals, POPC
                                     (order 4 over the whole data set: pair-major schedule) */
 #define FIU_KERNEL_ELIDED_HS 3   /* as 2, Harley-Seal carry-save counting on the ALU pipe */
-#define FIU_KERNEL_TENSOR 4      /* one-hot data, order 2, 3 or 4, whole data set: core cells on tcgen05 (e4m3, FP32 accumulate) */
+#define FIU_KERNEL_TENSOR 4      /* one-hot data, order 2, 3 or 4, whole data set: core cells on tcgen05 (4-bit
+                                    operands, FP32 accumulate).  FIU_KERNEL_AUTO also takes it for order-3 searches
+                                    of the whole data set where samples lack calls */
 #define FIU_MAX_OUTPUTS 7000  /* largest top-N supported */
 
 typedef struct fiu_ctx fiu_ctx;           /* one per device per host thread */
