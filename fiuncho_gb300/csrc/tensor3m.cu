@@ -21,7 +21,7 @@
 // Bound by the pace of the stages, as the complete-data kernel (its cost is three
 // GEMMs where that one takes one, on tiles of 80 l instead of 120); the
 // evaluation (81 logarithms a combination) takes 18 000 cycles an item.  400 SNPs x
-// 4 000/4 000: 26.2 -> 2.3 ms against the full-table kernel (27 AND, POPC and ADD a
+// 4 000/4 000: 28.2 -> 1.9 ms a search (kernels 1.7) against the full-table kernel (27 AND, POPC and ADD a
 // word of a combination, 16 POPC a cycle and SM).
 //
 // Reference semantics: GenotypeTable::combine_and_popcnt for order 3

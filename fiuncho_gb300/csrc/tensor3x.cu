@@ -34,8 +34,8 @@
 //
 // What bounds it (2 000 SNPs x 4 000/4 000, one launch over the whole scan):
 // 26.3 ms; without the evaluation 22.7, without the A build and the MMAs too
-// 22.3 (about 540 cycles a stage of 17 KB and SM: 9.5 TB/s out of L2); the MMAs
-// alone are 18.6 (120 cycles per M 256 N 240 K 64).  Whole searches: 27.7 ms
+// 22.3 (about 540 cycles a stage; neither fewer bytes nor other copies a stage
+// changed it); the MMAs alone are 18.6 (120 cycles per M 256 N 240 K 64).  Whole searches: 27.7 ms
 // against 74.7 with e4m3 operands (128-byte rows of 128 samples: twice the shared-memory
 // and L2 traffic, 82 KB a stage with LSU and tensor wavefronts at 83 % of peak;
 // 81 logarithms a combination at 8 cycles a warp instruction and SM quarter where
@@ -43,7 +43,7 @@
 // through shared memory).  Tried on the way: A in tensor memory and B spread from
 // bits by warps (5 KB a stage from L2, N 192): 45 ms, bound by issue slots.
 //
-// SPLIT (500 SNPs x 9 000/9 800): 5.6 -> 2.3 ms against the e4m3 kernel, one CTA a
+// SPLIT (500 SNPs x 9 000/9 800): 5.6 -> 1.9 ms a search (kernels 1.6) against the e4m3 kernel, one CTA a
 // tile, that counted classes apart before; 610 cycles a stage.
 //
 // Reference semantics: GenotypeTable::combine_and_popcnt for order 3

@@ -27,7 +27,7 @@
 // Measured (whole searches): 300 SNPs x 4 000/4 000 81.9 -> 34.3 ms, 300 x
 // 558/1 012 60.0 -> 29.4 ms, against e4m3 operands, one CTA a tile, 243
 // logarithms a combination (1 944 cycles a warp and SM quarter) and triples
-// counted by POPC.  Without the evaluation the two take 26 and 13 ms; the
+// counted by POPC.  Without the evaluation the two take 22 and 13 ms; the
 // evaluation of 64 combinations by a warp is 2 240 cycles of bound (81 x 2
 // reciprocals 800, splitting the classes 650) and about 700 of derivation and takes
 // 5 400 beside the builders, with two warps a quarter to hide latencies.  Tried:
