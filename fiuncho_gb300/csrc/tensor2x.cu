@@ -48,11 +48,16 @@ constexpr int kZSA = 2 * kZI * kZRow;               // 16 KB
 constexpr int kZSB = kZN / 2 * kZRow;               // 15 KB
 constexpr int kZStage = kZSA + kZSB;                // 31 KB
 constexpr int kZColOne = 2 * kZN, kZColW = kZColOne + 16;
-constexpr int kZEpiWarps = 8;
-constexpr int kZThreads = 32 * (4 + kZEpiWarps);    // copies, MMAs, two staging warps; epilogue
+// Epilogue warps: three an SM quarter hide latencies better than two where the evaluation binds
+// (counting kernels of 12 001 SNPs x 3 999 samples 0.714 -> 0.688 ms, of 1 000 x 4 000 0.117 -> 0.099);
+// SPLIT holds both classes' cells (166 registers).
+template <bool SPLIT>
+constexpr int kZEpiWarps = SPLIT ? 8 : 12;
+template <bool SPLIT>
+constexpr int kZThreads = 32 * (4 + kZEpiWarps<SPLIT>);  // copies, MMAs, two staging warps; epilogue
 // staged per item: single cores of the j (packed, or cases then controls), the threshold (key, bound)
 constexpr int kZTabT = 4 * kP2J * 4, kZTab = kZTabT + 16;
-constexpr int kZStash = kZEpiWarps * ((kZG + 1) / 2) * 2 * 32 * 16;  // 64 KB: (warp, its group, lane block, lane), 8 counts
+constexpr int kZStash = kZEpiWarps<true> * ((kZG + 1) / 2) * 2 * 32 * 16;  // 64 KB: (warp, its group, lane block, lane), 8 counts
 template <bool SPLIT>
 constexpr int kZStages = SPLIT ? 5 : 7;
 template <bool SPLIT>
@@ -92,7 +97,7 @@ __device__ __forceinline__ void t2x_cells(const f2 (&c)[2][2], const f2 (&si)[3]
 
 // SPLIT: one accumulator region per class.
 template <bool SPLIT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kZThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kZThreads<SPLIT>, 1)
     tensor2x_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const __grid_constant__ ScanWork w, const __grid_constant__ CandSink sink,
                     const long long* __restrict__ begin, int tiles, int first, int istep, long long g0, long long g1,
@@ -130,9 +135,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kZThreads, 1)
         }
         for (int b = 0; b < 2; ++b) {
             init(&acc_full[b], 1);
-            init(&acc_empty[b], 2 * kZEpiWarps);
+            init(&acc_empty[b], 2 * kZEpiWarps<SPLIT>);
             init(&tab_full[b], 2);
-            init(&tab_empty[b], kZEpiWarps);
+            init(&tab_empty[b], kZEpiWarps<SPLIT>);
         }
         init(&done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;");
@@ -243,7 +248,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kZThreads, 1)
         }
     } else {
         // ---------------------------------------------------------------- epilogue (both CTAs)
-        const int q = warp & 3, hh = (warp - 4) >> 2;  // lane quarter (16 i); its two warps take alternate groups
+        const int q = warp & 3, hh = (warp - 4) >> 2;  // lane quarter (16 i); its warps take groups in turn
+        constexpr unsigned kShare = kZEpiWarps<SPLIT> / 4;
         const int il = lane >> 2, lc = 2 * (lane & 3);  // this thread's i of a block of 8, its two j of a group
         const float W = (float)(1u << pack);
         const uint32_t wmask = (1u << pack) - 1u;
@@ -256,7 +262,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kZThreads, 1)
             int p0, j0;
             t2x_item(begin, tiles, first, istep, g, p0, j0);
             const unsigned buf = item & 1, ph = (item >> 1) & 1;
-            const unsigned gi0 = (hh + item) & 1;  // the odd group of an item goes to either warp in turn
+            const unsigned gi0 = (hh + item) % kShare;  // the odd group of an item goes to each warp in turn
             // this thread's i and their single cores (0, 1, what is left), packed or per class
             int iv[2];
             f2 si[2][SPLIT ? 2 : 1][3];
@@ -294,7 +300,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kZThreads, 1)
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;");
 #pragma unroll 1
-                for (unsigned gi = gi0; gi < kZG; gi += 2) {
+                for (unsigned gi = gi0; gi < kZG; gi += kShare) {
                     uint32_t r[2][8];
                     ld(0, 0, gi, r[0]);
                     ld(0, 1, gi, r[1]);
@@ -323,7 +329,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kZThreads, 1)
             const long long thr = *reinterpret_cast<const long long*>(tabs + buf * kZTab + kZTabT);
             const float thr_q = *reinterpret_cast<const float*>(tabs + buf * kZTab + kZTabT + 8);
 #pragma unroll 1
-            for (unsigned gi = gi0; gi < kZG; gi += 2) {
+            for (unsigned gi = gi0; gi < kZG; gi += kShare) {
                 const int ll = 8 * gi + lc, j = j0 + ll;
                 bool v[2][2];
                 unsigned vm = 0, count = 0;
@@ -523,18 +529,18 @@ cudaError_t launch_tensor2x(const ScanWork& w, const F4Plan& f, const T2xRange& 
     }();
     if (attr != cudaSuccess) return attr;
     if (g1 <= g0) return cudaSuccess;
-    static const int max_clusters = pair_clusters(tensor2x_kernel<false>, kZThreads, kZSmem<false>);
+    static const int max_clusters = pair_clusters(tensor2x_kernel<false>, kZThreads<false>, kZSmem<false>);
     const long long clusters = std::min<long long>(g1 - g0, max_clusters > 0 ? max_clusters : sms / 2);
     const unsigned grid = (unsigned)(2 * std::max(1ll, clusters));
     LiveMap map{0, 0, 0, 0};
     f4_quadratic(w.d.n_cases, w.d.n_ctrls, 9, map.bound_k, map.bound_c);
     map.bound_k /= std::log(2.0) * 4294967296.0;
     if (f.pack)
-        tensor2x_kernel<false><<<grid, kZThreads, kZSmem<false>, s>>>(*r.map_a, *r.map_b, w, sink, r.item_begin, r.tiles,
+        tensor2x_kernel<false><<<grid, kZThreads<false>, kZSmem<false>, s>>>(*r.map_a, *r.map_b, w, sink, r.item_begin, r.tiles,
                                                                       r.first, r.step, g0, g1, f.nw_c, f.nw_t, f.pack,
                                                                       map, dump, single, status);
     else
-        tensor2x_kernel<true><<<grid, kZThreads, kZSmem<true>, s>>>(*r.map_a, *r.map_b, w, sink, r.item_begin, r.tiles,
+        tensor2x_kernel<true><<<grid, kZThreads<true>, kZSmem<true>, s>>>(*r.map_a, *r.map_b, w, sink, r.item_begin, r.tiles,
                                                                     r.first, r.step, g0, g1, f.nw_c, f.nw_t, 1, map,
                                                                     dump, single, status);
     count_launch();
