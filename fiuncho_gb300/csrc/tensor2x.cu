@@ -26,7 +26,7 @@
 // Bound by the MMAs at many samples (40 000 SNPs x 8 000/8 000: 41.6 -> 14.3 ms a
 // search against e4m3 operands and one accumulator region per class, 94 % of 4 x
 // the measured bf16 rate) and by the evaluation below about 8 000 samples (12 001
-// SNPs x 3 999: 2.24 -> 0.82 ms).
+// SNPs x 3 999: 2.25 -> 0.77 ms).
 //
 // Reference semantics: GenotypeTable::combine_and_popcnt for order 2
 // (src/base/gt_popcnt.cpp:4-35) over the pairs ThreadedSearch visits

@@ -230,7 +230,7 @@ __device__ __forceinline__ void t3x_survivor(const ScanWork& w, const CandSink& 
                                              bool want, int lane) {
     const int n = w.d.snps;
     bool cand = want;
-    if (!dump && !sink.digest) {
+    if (!dump && !sink.digest && thr != (long long)0x8000000000000000ull) {
         const float tiny = 9.5367431640625e-07f;  // 2^-20: x*lg2(x + tiny) = 0 at x = 0
         float kf = 0.f;
 #pragma unroll
