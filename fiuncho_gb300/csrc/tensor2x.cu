@@ -78,7 +78,7 @@ __device__ __forceinline__ void t2x_item(const long long* __restrict__ begin, in
     const int ca = min(kP2Band, tiles - kP2Band * lo);  // tiles in the band
     const unsigned idx = (unsigned)(g - __ldg(begin + lo)), b = idx / ca;
     p0 = kP2I * (kP2Band * lo + (int)(idx - b * ca));
-    j0 = kP2J * ((first + step * (kP2I * kP2Band * lo) + 1) / kP2J + (int)b);
+    j0 = kP2J * ((layer_snp(first, step, kP2I * kP2Band * lo) + 1) / kP2J + (int)b);
 }
 
 // 9 cells of both classes (or packed) from cores c (x, y), singles of i (si: 0, 1, any left) and of j.
@@ -268,7 +268,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kZThreads<SPLIT>, 1)
             f2 si[2][SPLIT ? 2 : 1][3];
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
-                iv[u] = first + istep * (p0 + kZI * (int)rank + 16 * q + 8 * u + il);
+                iv[u] = layer_snp(first, istep, p0 + kZI * (int)rank + 16 * q + 8 * u + il);
                 const uint4 v = iv[u] < n ? __ldg(reinterpret_cast<const uint4*>(single) + iv[u]) : make_uint4(0, 0, 0, 0);
                 const float a0 = u2f(v.x), a1 = u2f(v.y), b0 = u2f(v.z), b1 = u2f(v.w);
                 const float ar = (float)nc - a0 - a1, br = (float)nt - b0 - b1;

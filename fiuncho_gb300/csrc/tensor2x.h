@@ -27,7 +27,7 @@ struct T2xRange {
     const long long* item_begin;  // first item of each band
     int tiles;
     const CUtensorMap *map_a, *map_b;
-    int first, step;              // owned i = first + step m
+    int first, step;              // owned i = first + step m (layer_step's)
 };
 cudaError_t launch_tensor2x(const ScanWork& w, const F4Plan& f, const T2xRange& r, long long g0, long long g1,
                             const CandSink& sink, uint32_t* dump, const uint32_t* single, int* status, cudaStream_t s,

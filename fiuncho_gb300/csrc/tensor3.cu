@@ -147,26 +147,38 @@ struct T3Layer {
 struct T3Layers {
     std::mutex mu;
     std::map<std::tuple<int, int, int>, T3Layer> by;  // (order, step, offset)
-    std::map<int, uint8_t*> bits_by_residue;  // residue-ordered bit rows (orders 3 and 4), per step
+    std::map<int, uint8_t*> bits_by_residue;  // residue-ordered bit rows (orders 3 and 4), per layer_step
 };
 
-// The rows of every SNP (row_bytes each, SNP-major in src) ordered by residue mod step, made on first use.
-static cudaError_t residue_copy(std::map<int, uint8_t*>& by, const uint8_t* src, size_t row_bytes, int n, int step,
-                                cudaStream_t s) {
+// Bit rows (2 an SNP, wpr words each) ordered by residue, 16 bytes a thread.
+__global__ void residue_rows_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, int n, int step,
+                                    int per_snp) {
+    const long long total = (long long)n * per_snp;
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
+         e += (long long)gridDim.x * blockDim.x) {
+        const int row = (int)(e / per_snp), o = (int)(e - (long long)row * per_snp);
+        dst[e] = __ldg(src + (long long)residue_snp(row, step, n) * per_snp + o);
+    }
+}
+
+// The bit rows ordered by residue mod step (layer_step's), made on first use.  (A kernel: a copy with
+// the step as its pitch is refused from 2 GB on, which a step of a few hundred thousand SNPs reaches.)
+static cudaError_t residue_copy(std::map<int, uint8_t*>& by, const F4Plan& f, int n, int step, cudaStream_t s) {
     if (by.count(step)) return cudaSuccess;
+    const int per_snp = f.wpr / 2;  // 2 rows of wpr words; wpr is a multiple of 8
     uint8_t* perm = nullptr;
-    cudaError_t e = cudaMalloc((void**)&perm, (size_t)n * row_bytes);
-    // residue class r holds SNPs r + step m, m < ceil((n - r) / step)
-    for (int r = 0; r < step && r < n && e == cudaSuccess; ++r)
-        e = cudaMemcpy2DAsync(perm + (size_t)residue_row(r, step, n) * row_bytes, row_bytes,
-                              src + (size_t)r * row_bytes, (size_t)step * row_bytes, row_bytes,
-                              (size_t)((n - r + step - 1) / step), cudaMemcpyDeviceToDevice, s);
+    cudaError_t e = cudaMalloc((void**)&perm, (size_t)n * per_snp * 16);
+    if (e != cudaSuccess) return e;
+    const long long total = (long long)n * per_snp;
+    residue_rows_kernel<<<(unsigned)std::min<long long>((total + 255) / 256, 8192), 256, 0, s>>>(
+        reinterpret_cast<const uint4*>(f.bits), reinterpret_cast<uint4*>(perm), n, step, per_snp);
+    count_launch();
+    e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) cudaFree(perm);
     else by[step] = perm;
     return e;
 }
-
 
 static bool is_layer(const ScanWork& w) { return w.dist_step != 1 || w.dist_offset != 0; }
 
@@ -193,10 +205,9 @@ cudaError_t tensor3_layer(T3Plan& plan, const ScanWork& w, const uint4* pairs, c
         pe = order_planes(plan, w.d, w.order, pairs, s, sms);
     }
     if (pe == cudaSuccess && w.order != 2)
-        pe = residue_copy(plan.layers->bits_by_residue, (const uint8_t*)plan.f4.bits, (size_t)8 * plan.f4.wpr,
-                          w.d.snps, w.dist_step, s);
+        pe = residue_copy(plan.layers->bits_by_residue, plan.f4, w.d.snps, layer_step(w.dist_step, w.d.snps), s);
     if (pe != cudaSuccess) return pe;
-    const int n = w.d.snps;
+    const int n = w.d.snps, pstep = layer_step(w.dist_step, n);
     const long long step = w.dist_step, offset = w.dist_offset;
     if (w.order == 4) {
         std::vector<long long> pb;
@@ -207,7 +218,7 @@ cudaError_t tensor3_layer(T3Plan& plan, const ScanWork& w, const uint4* pairs, c
         L.total = total;
         L.n_tiles = (int)pi.size();
         L.item_combos = (double)combos / std::max(1ll, total);
-        cudaError_t e = f4_bit_map(&L.map_kr, plan.f4, (const uint32_t*)plan.layers->bits_by_residue[w.dist_step],
+        cudaError_t e = f4_bit_map(&L.map_kr, plan.f4, (const uint32_t*)plan.layers->bits_by_residue[pstep],
                                    2 * n, 32);
         if (e == cudaSuccess) e = cudaMalloc((void**)&L.item_begin, pb.size() * sizeof(long long));
         if (e == cudaSuccess) e = cudaMalloc((void**)&L.pinfo, std::max<size_t>(1, pi.size()) * sizeof(int4));
@@ -265,7 +276,7 @@ cudaError_t tensor3_layer(T3Plan& plan, const ScanWork& w, const uint4* pairs, c
     T3Layer L;
     L.total = total;
     L.item_combos = (double)combos / std::max(1ll, total);
-    cudaError_t e = f4_bit_map(&L.map_jr, plan.f4, (const uint32_t*)plan.layers->bits_by_residue[w.dist_step], 2 * n,
+    cudaError_t e = f4_bit_map(&L.map_jr, plan.f4, (const uint32_t*)plan.layers->bits_by_residue[pstep], 2 * n,
                                kPxJ);
     if (e == cudaSuccess) e = cudaMalloc((void**)&L.item_begin, ib.size() * sizeof(long long));
     if (e == cudaSuccess) e = cudaMalloc((void**)&L.jl_begin, jb.size() * sizeof(long long));
@@ -421,7 +432,7 @@ cudaError_t launch_tensor3(const ScanWork& w, const T3Plan& plan, long long g0, 
     if (w.order == 2) {
         const T2xRange r{L ? L->item_begin : plan.item2_begin, L ? L->n_tiles : plan.n_itiles,
                          L ? &L->map_ar : &plan.f4.map_a2, &plan.f4.map_b2, L ? w.dist_offset : 0,
-                         L ? w.dist_step : 1};
+                         L ? layer_step(w.dist_step, w.d.snps) : 1};
         return launch_tensor2x(w, plan.f4, r, g0, g1, sink, dump, single, status, s, sms);
     }
     if (w.order == 4) {

@@ -380,7 +380,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kXThreads, 1)
                         // 32 listed j are consecutive residue-ordered rows from the first one (rows past the
                         // end of i's list are loaded too and ignored by the epilogue)
                         const long long p = it.p0 + kXJ * (int)rank;
-                        jr = p < __ldg(jl_begin + it.i + 1) ? residue_row(__ldg(jlist + p), w.dist_step, n) : 0;
+                        jr = p < __ldg(jl_begin + it.i + 1) ? residue_row(__ldg(jlist + p), layer_step(w.dist_step, n), n) : 0;
                     }
                     const int brow = 2 * it.l0 + t3x_n(it.ng) / 2 * (int)rank, irow = 2 * it.i;
                     item_ng[item++ % kXMeta] = it.ng;

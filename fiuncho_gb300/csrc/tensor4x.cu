@@ -280,7 +280,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
     uint8_t* tabs = smk + kStages * kYBits;
     uint4* stash = reinterpret_cast<uint4*>(tabs + 2 * kTab);
     volatile int* abort = &abort_flag;
-    const int n = w.d.snps, kstep = LAYER ? w.dist_step : 1;
+    const int n = w.d.snps, kstep = LAYER ? layer_step(w.dist_step, w.d.snps) : 1;
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // warp-uniform for the compiler too
     const int ksteps = ((nw_c + 3) >> 2) + ((nw_t + 3) >> 2);  // stages of 256 samples
@@ -449,7 +449,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
                     }
                 }
                 if (t < kYK) {
-                    const int k = it.k0 + kstep * (kYK * ((int)rank ^ (int)(item & 1)) + t);
+                    const int k = layer_snp(it.k0, kstep, kYK * ((int)rank ^ (int)(item & 1)) + t);
                     auto put = [&](int e, Tab v) {
                         if constexpr (SPLIT) tk[e * kYK + t] = v;
                         else tk[e * kYK + t] = f2_dup(v);
@@ -540,7 +540,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
             const T4xItem it = t4x_item<LAYER>(begin, per, pinfo, n_pairs, n, kstep, g, at);
             const unsigned buf = item & 1, ph = (item >> 1) & 1;
             const int gi0 = (hh + item) & 1;  // the odd group of an item goes to either warp in turn
-            const int kk = kk0 ^ t4x_flip(item), k = it.k0 + kstep * (kYK * ((int)rank ^ (int)(item & 1)) + kk);
+            const int kk = kk0 ^ t4x_flip(item), k = layer_snp(it.k0, kstep, kYK * ((int)rank ^ (int)(item & 1)) + kk);
             const bool k_ok = k < n;
             // entries of the rows (i, k), (j, k) and k, in units of 16 bytes
             const int rp = k_ok ? __ldg(row_p + k) : 0;

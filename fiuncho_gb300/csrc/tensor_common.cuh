@@ -6,6 +6,7 @@
 #include <cudaTypedefs.h>
 
 #include "elided_prefix.cuh"
+#include "layer_pos.h"
 
 namespace fiu {
 
@@ -137,14 +138,6 @@ __device__ __forceinline__ uint64_t t3_desc(uint32_t saddr) {
 
 __device__ __forceinline__ float u2f(uint32_t v) {  // exact for v < 2^23
     return __uint_as_float(0x4B000000u | v) - 8388608.0f;
-}
-
-// Row (SNP position) of SNP j in the operand planes ordered by residue mod
-// step (SNPs r, r + step, .. for r = 0, 1, ..; residue r holds
-// n / step + (r < n % step) SNPs).
-__host__ __device__ __forceinline__ int residue_row(int j, int step, int n) {
-    const int r = j % step;
-    return r * (n / step) + min(r, n % step) + j / step;
 }
 
 __device__ __forceinline__ float t3_lg2(float x) {

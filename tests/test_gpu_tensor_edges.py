@@ -209,3 +209,26 @@ def test_order3_rows_that_share_samples_keep_the_full_tables():
             rows[7, full.cases_words - 1] |= np.uint64(1) << np.uint64(63)
         gs.run(Dataset(100, 90, 40, full.cases_words, full.ctrls_words, rows.reshape(-1)), 3, Distribution(40, 2), 5)
         assert gs.last_tile()[0] == _lib.KERNEL_FULL
+
+
+@pytest.mark.parametrize("order,snps,step,offset", [
+    (2, 130, 16_900_001, 0), (2, 260, 2 ** 28, 129), (2, 66, 2 ** 31 - 1, 5), (3, 70, 2 ** 28, 3),
+    (3, 66, 2 ** 31 - 1, 64), (4, 40, 70_000_001, 0), (4, 37, 2 ** 28, 40), (4, 36, 2 ** 31 - 1, 7)])
+def test_layers_of_steps_past_32_bit_positions(oracle, order, snps, step, offset):
+    """A step so large that a tile's later positions would leave 32 bits owns one prefix, the one of rank
+    `offset`: its tables and its list."""
+    import math
+    from fiuncho_gb300 import Distribution, GpuSearch, _lib
+    from fiuncho_gb300.search import Resident
+    ds = _data(snps, 300, 311, 90 + snps)
+    gs = GpuSearch(0)
+    res = Resident(gs.ctx, ds)
+    d = Distribution(snps, order - 1, step, offset)
+    digest, count = gs.scan_digest(res, order, d, kernel=_lib.KERNEL_TENSOR)
+    assert (digest, count) == oracle.table_digest(ds.data, snps, ds.cases_words, ds.ctrls_words, order,
+                                                  dist=(snps, math.comb(snps, order - 1), offset))
+    lists = []
+    for kernel in (_lib.KERNEL_AUTO, _lib.KERNEL_FULL):
+        gs.set_kernel(kernel)
+        lists.append([(r.combination, r.val) for r in gs.run(res, order, d, 25)])
+    assert lists[0] == lists[1] and len(lists[0]) == min(25, count)
