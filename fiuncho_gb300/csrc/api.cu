@@ -12,6 +12,7 @@
 
 #include "../../include/fiuncho_gpu.h"
 #include "ctx.h"
+#include "layer_pos.h"
 #include "tensor3x.h"
 #include "digest.cuh"
 
@@ -312,7 +313,7 @@ int choose_tile(fiu_ctx* ctx, const fiu_resident* res, const ScanWork& w, int re
     ScanWork sw = w;
     const long long want = (long long)ctx->sms * 16;
     const long long stride = std::max<long long>(1, w.n_prefixes / want);
-    sw.dist_step = w.dist_step * (int)std::min<long long>(stride, 1 << 20);
+    sw.dist_step = sample_step(w.dist_step, stride);
     sw.n_prefixes = (w.n_prefixes - 1) / stride + 1;
     const CandSink none{ctx->cand, ctx->ctl + 8, ctx->ctl + 9, 0, (long long)0x7fffffffffffffffll, nullptr};
     cudaEvent_t e0 = nullptr, e1 = nullptr;

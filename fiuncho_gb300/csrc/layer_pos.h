@@ -37,4 +37,11 @@ FIU_POS int residue_snp(int row, int step, int n) {
     return row < in ? row / (q + 1) + step * (row % (q + 1)) : more + (row - in) / q + step * ((row - in) % q);
 }
 
+// The step of a sample of a scan's prefixes, every stride-th one of those owned (stride >= 1): the most
+// whole strides that a step holds (a sample that then ends early is still one of owned prefixes).
+FIU_POS int sample_step(int step, long long stride) {
+    const long long most = INT_MAX / step;
+    return step * (int)(stride < most ? stride : most);
+}
+
 }  // namespace fiu

@@ -17,11 +17,14 @@ def pos(tmp_path_factory):
         '#include "layer_pos.h"\nextern "C" {\n'
         "int owned(int first, int step, int n, int m) { return fiu::layer_snp(first, fiu::layer_step(step, n), m); }\n"
         "int row(int j, int step, int n) { return fiu::residue_row(j, fiu::layer_step(step, n), n); }\n"
-        "int snp(int r, int step, int n) { return fiu::residue_snp(r, fiu::layer_step(step, n), n); }\n}\n")
+        "int snp(int r, int step, int n) { return fiu::residue_snp(r, fiu::layer_step(step, n), n); }\n"
+        "int sample(int step, long long stride) { return fiu::sample_step(step, stride); }\n}\n")
     so = str(d / "pos.so")
     subprocess.run(["g++", "-std=c++17", "-O1", "-fwrapv", "-shared", "-fPIC", "-I",
                     os.path.join(ROOT, "fiuncho_gb300", "csrc"), str(d / "pos.cpp"), "-o", so], check=True)
-    return ctypes.CDLL(so)
+    lib = ctypes.CDLL(so)
+    lib.sample.argtypes = [ctypes.c_int, ctypes.c_longlong]
+    return lib
 
 
 @pytest.mark.parametrize("n", [2, 40, 1150, 2 ** 21 - 1])
@@ -40,3 +43,10 @@ def test_residue_order(pos, n, step):
     order = [j for r in range(min(step, n)) for j in range(r, n, step)]
     assert [pos.snp(r, step, n) for r in range(n)] == order
     assert [pos.row(j, step, n) for j in order] == list(range(n))
+
+
+@pytest.mark.parametrize("step,stride", [(1, 1), (1, 10 ** 10), (7, 1000), (2 ** 21, 1078), (2 ** 30, 3), (INT_MAX, 2)])
+def test_sample_of_prefixes(pos, step, stride):
+    got = pos.sample(step, stride)
+    assert step <= got <= min(step * stride, INT_MAX) and got % step == 0
+    assert step * stride > INT_MAX or got == step * stride
