@@ -221,6 +221,10 @@ static bool tensor_ok(const fiu_resident* res, const ScanWork& w) {
 // host work (tensor vs full-table kernel, host data: 10 SNPs x 200 0.61 vs 0.61 ms, 30 x 500 0.63 vs 0.67,
 // 45 x 900 0.65 vs 0.80, 200 x 8 000 1.2 vs 5.7; resident 400 x 8 000 2.0 vs 25, 1 000 x 1 000 6.5 vs 61).
 constexpr int kMissingMinSnps = 32;
+// Batched and served scans below this many combinations x samples stay in the rounds, which take many of them at
+// once (batches of 24, rounds vs tensor kernel on the lanes: 32 SNPs x 900 samples 1.06 vs 1.69 ms, 60 x 900 1.56
+// vs 1.80, 100 x 900 2.98 vs 3.29 [1.5e8 each]; 60 x 8 000 4.14 vs 2.00 [2.7e8], 200 x 900 16.0 vs 4.9).
+constexpr double kMissingRoundsWork = 2e8;
 static bool missing_ok(const fiu_resident* res, const ScanWork& w) {
     return !res->one_hot && res->disjoint && w.order == 3 && res->d.snps >= kMissingMinSnps && whole_data_set(res, w) && res->d.n_cases >= 1 &&
            res->d.n_ctrls >= 1 && res->d.n_cases <= 65535 && res->d.n_ctrls <= 65535 && res->d.snps < (1 << 21) &&
@@ -252,11 +256,21 @@ static int missing_plan(fiu_ctx* ctx, const fiu_resident* res) {
 constexpr int kT4MinSamples = 1024, kT4MinSnps = 32;
 
 int choose_tile(fiu_ctx* ctx, const fiu_resident* res, const ScanWork& w, int requested_kernel, int& kernel, int& tp,
-                bool allow_tensor) {
-    const bool auto_tensor = allow_tensor && tensor_ok(res, w) &&
-                             (w.order != 4 || res->d.n_cases + res->d.n_ctrls >= kT4MinSamples);
+                Use use) {
+    if (requested_kernel == FIU_KERNEL_AUTO && use != Use::kTables && missing_ok(res, w) &&
+        (use != Use::kShared ||
+         (double)binom(w.dist_n, 3) * (res->d.n_cases + res->d.n_ctrls) >= kMissingRoundsWork)) {
+        const int rc = missing_plan(ctx, res);
+        if (rc == FIU_OK) {
+            kernel = FIU_KERNEL_TENSOR;
+            tp = 256;
+            return FIU_OK;
+        }
+        if (use == Use::kShard) return rc;  // (not the full tables: other shards are cut by this kernel's units)
+    }
+    const bool auto_tensor = tensor_ok(res, w) && (w.order != 4 || res->d.n_cases + res->d.n_ctrls >= kT4MinSamples);
     if (requested_kernel == FIU_KERNEL_TENSOR || (requested_kernel == FIU_KERNEL_AUTO && auto_tensor)) {
-        if (!allow_tensor || !tensor_ok(res, w))
+        if (!tensor_ok(res, w))
             return fail(ctx, FIU_ERR_UNSUPPORTED,
                         "the tensor-core kernels need one-hot data, order 2, 3 or 4 and the whole data set on one "
                         "worker");
@@ -372,16 +386,10 @@ int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu
     int requested = kernel ? kernel : ctx->kernel;
     if (requested == FIU_KERNEL_AUTO && order == 4 && res->d.snps >= kT4MinSnps && tensor_ok(res, w))
         requested = FIU_KERNEL_TENSOR;
-    const bool missing = requested == FIU_KERNEL_AUTO && missing_ok(res, w);
-    if (missing && (rc = missing_plan(ctx, res)) == FIU_OK) {
-        kernel = FIU_KERNEL_TENSOR;
-    } else {
-        if (missing && n_shards > 1) return rc;  // (shards are cut by work units: all have to take one path)
-        if ((rc = choose_tile(ctx, res, w, requested, kernel, tp, true))) return rc;
-    }
+    if ((rc = choose_tile(ctx, res, w, requested, kernel, tp, n_shards > 1 ? Use::kShard : Use::kSearch))) return rc;
     ctx->last_kernel = kernel;
     ctx->last_tp = tp;
-    const bool tensor = kernel == FIU_KERNEL_TENSOR;
+    const bool tensor = kernel == FIU_KERNEL_TENSOR, missing = tensor && res->t3->missing;
     const bool pair_major = e4_pair_major(kernel, res, w);
     const long long units = tensor ? tensor_units(*res->t3, w) : pair_major ? res->e4_items : w.n_prefixes;
     const unsigned keep = outputs + std::max(32u, outputs / 8);
@@ -1020,7 +1028,7 @@ int fiu_scan_tables(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const
     int tp = (kernel >> 8) & 0x1ff;
     kernel &= 0xff;
     if (kernel == FIU_KERNEL_TENSOR) {
-        if ((rc = choose_tile(ctx, res, w, kernel, kernel, tp, true))) return rc;
+        if ((rc = choose_tile(ctx, res, w, kernel, kernel, tp, Use::kTables))) return rc;
     } else {
         if ((rc = choose_kernel(ctx, res, order, kernel, kernel))) return rc;
         if (tp != 32 && tp != 64 && tp != 128 && tp != 256) tp = heuristic_tp(kernel, w);
@@ -1072,7 +1080,7 @@ int fiu_scan_digest(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const
     if (w.n_prefixes == 0) return FIU_OK;
     CK(cudaSetDevice(ctx->device), "cudaSetDevice");
     int tp = 256;
-    if ((rc = choose_tile(ctx, res, w, kernel ? kernel : ctx->kernel, kernel, tp, true))) return rc;
+    if ((rc = choose_tile(ctx, res, w, kernel ? kernel : ctx->kernel, kernel, tp, Use::kTables))) return rc;
     if (kernel == FIU_KERNEL_FULL && order > 4)
         return fail(ctx, FIU_ERR_UNSUPPORTED, "the full-table kernel's digest covers orders 2-4");
     const bool tensor = kernel == FIU_KERNEL_TENSOR;

@@ -93,11 +93,20 @@ int grow_host(fiu_ctx* ctx, size_t need);
 int make_work(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu_distribution* dist,
               unsigned outputs, ScanWork& w);
 int choose_kernel(fiu_ctx* ctx, const fiu_resident* res, unsigned order, int requested, int& kernel);
+// What a kernel is chosen for.  A shard is a range of the serving kernel's work
+// units, so every caller that searches shards has to get the same kernel for the
+// same data set: the choice for kShard depends on nothing else.
+enum class Use {
+    kTables,  // tables or digests: kernels that have a table path
+    kSearch,  // a search on its own
+    kShard,   // a shard of one
+    kShared,  // a search that could progress in rounds with others (batched, served)
+};
 // Picks the counting kernel variant and l-tile width (threads per prefix) of a
 // request: measured on a strided sample of its prefixes (cached per shape
 // bucket) when autotuning is on and the request is large, else a heuristic.
 int choose_tile(fiu_ctx* ctx, const fiu_resident* res, const ScanWork& w, int requested_kernel, int& kernel, int& tp,
-                bool allow_tensor = false);
+                Use use);
 bool e4_pair_major(int kernel, const fiu_resident* res, const ScanWork& w);
 cudaError_t launch_kernel(int kernel, int tp, const fiu_resident* res, const ScanWork& w, long long m0, long long m1,
                           const CandSink& sink, uint32_t* dump, cudaStream_t s, int sms);

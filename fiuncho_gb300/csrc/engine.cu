@@ -5,7 +5,7 @@
 // whose candidate buffer overflowed is re-run alone on the single-scan path
 // (whose chunking adapts on the host), so results never depend on batching.
 // Scans served by the tensor-core kernels (one-hot order 2, 3 or 4 over the whole
-// data set) or by the pair-major order-4 kernel (one-hot, whole data set) are
+// data set; order 3 with missing calls, unless small) or by the pair-major order-4 kernel (one-hot, whole data set) are
 // not split into rounds: each runs on the single-scan path, as in a loop of
 // single calls, but on one of two helper lanes (a context with its own stream
 // and scratch) concurrently with the rounds and with the other lane, and the
@@ -74,7 +74,7 @@ extern "C" int fiu_search_batch(fiu_ctx* ctx, fiu_scan* scans, unsigned n_scans,
         }
         if (sc.outputs == 0 || w.n_prefixes == 0) continue;
         int kind = 0, tp = 256;
-        if ((rc = choose_tile(ctx, sc.res, w, ctx->kernel, kind, tp, true))) {
+        if ((rc = choose_tile(ctx, sc.res, w, ctx->kernel, kind, tp, ns > 1 ? Use::kShard : Use::kShared))) {
             sc.status = rc;
             continue;
         }

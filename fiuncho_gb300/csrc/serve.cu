@@ -13,8 +13,8 @@
 // scans that arrived meanwhile are admitted before the next round.
 //
 // Scans that run best alone -- those served by the tensor-core kernels
-// (one-hot orders 2-4) or the pair-major order-4 kernel, full-table scans
-// above order 4, and any scan admitted while every slot is taken -- go to the
+// (one-hot orders 2-4; order 3 with missing calls, unless small) or the
+// pair-major order-4 kernel, full-table scans above order 4, and any scan admitted while every slot is taken -- go to the
 // solo lanes: kSoloLanes worker threads, each with its own context and
 // stream, take them from one FIFO and run each through the single-scan path.
 // The lanes run concurrently with one another and with the rounds, so the
@@ -199,7 +199,8 @@ bool admit(fiu_server* sv, ServeScan* s) {
         s->cursor = P / N * s->shard + std::min<long long>(s->shard, P % N);
         s->m_end = s->cursor + P / N + ((long long)s->shard < P % N ? 1 : 0);
     }
-    if ((rc = choose_tile(ctx, s->res, s->w, ctx->kernel, s->kind, s->tp, true))) {
+    if ((rc = choose_tile(ctx, s->res, s->w, ctx->kernel, s->kind, s->tp,
+                          s->n_shards > 1 ? Use::kShard : Use::kShared))) {
         finish(sv, s, rc);
         return false;
     }

@@ -47,7 +47,8 @@ extern "C" {
 #define FIU_KERNEL_ELIDED_HS 3   /* as 2, Harley-Seal carry-save counting on the ALU pipe */
 #define FIU_KERNEL_TENSOR 4      /* one-hot data, order 2, 3 or 4, whole data set: core cells on tcgen05 (4-bit
                                     operands, FP32 accumulate).  FIU_KERNEL_AUTO also takes it for order-3 searches
-                                    of the whole data set where samples lack calls */
+                                    of the whole data set where samples lack calls (from 32 SNPs; small
+                                    ones in batches and the server progress in rounds) */
 #define FIU_MAX_OUTPUTS 7000  /* largest top-N supported */
 
 typedef struct fiu_ctx fiu_ctx;           /* one per device per host thread */

@@ -116,3 +116,34 @@ def test_batch_rejects_shard_of_a_layer(batch_setup):
     res, order, dist, outputs = reqs[3]  # a Distribution(..., 3, 1) layer
     with pytest.raises(FiunchoError):
         gs.run_batch([(res, order, dist, outputs, 0, 2)])
+
+
+def _missing_data(seed, snps, n_case, n_ctrl, copies=False):
+    """Genotypes with 2 % missing calls; copies: every SNP the same (all combinations tie)."""
+    from fiuncho_gb300 import Dataset
+    rng = np.random.default_rng(seed)
+    geno = rng.integers(0, 3, (snps, n_case + n_ctrl)).astype(np.uint8)
+    geno[rng.random(geno.shape) < 0.02] = 3
+    if copies:
+        geno[:] = geno[0]
+    return Dataset.from_genotypes(geno, np.r_[np.ones(n_case, np.uint8), np.zeros(n_ctrl, np.uint8)])
+
+
+@pytest.mark.parametrize("use_graph", [True, False])
+@pytest.mark.parametrize("copies", [False, True])
+def test_batch_shards_of_missing_calls(copies, use_graph):
+    """Order-3 shards of data with missing calls are cut alike by the batch and by run_shard (also where all
+    combinations tie, more than a round's candidate buffer holds), and merge to the whole scan's list."""
+    from fiuncho_gb300 import Distribution, GpuSearch, Resident
+    gs = GpuSearch(0)
+    res = Resident(gs.ctx, _missing_data(77, 90, 700, 650, copies))
+    dist = Distribution(90, 2)
+    whole, wv = gs.run(res, 3, dist, 40, with_fp64=True)
+    (got, gv), = gs.run_batch([(res, 3, dist, 40)], use_graph=use_graph)
+    assert [x.combination for x in got] == [x.combination for x in whole] and np.array_equal(gv, wv)
+    merged = []
+    for r, (rs, v) in enumerate(gs.run_batch([(res, 3, dist, 40, r, 5) for r in range(5)], use_graph=use_graph)):
+        want, sv = gs.run_shard(res, 3, r, 5, 40, with_fp64=True)
+        assert [x.combination for x in rs] == [x.combination for x in want] and np.array_equal(v, sv)
+        merged += zip(-v, (x.combination for x in rs))
+    assert [c for _, c in sorted(merged)[:40]] == [x.combination for x in whole]

@@ -211,3 +211,24 @@ def test_server_shortest_first():
         assert st["completed"] == 6 and st["failed"] == 0
     finally:
         srv.close()
+
+
+@pytest.mark.parametrize("copies", [False, True])
+def test_server_shards_of_missing_calls(copies):
+    """Order-3 shards of data with missing calls are cut by the server as by run_shard, also where all
+    combinations tie (more than a round's candidate buffer holds)."""
+    from fiuncho_gb300 import Dataset, GpuSearch, Server
+    rng = np.random.default_rng(80)
+    geno = rng.integers(0, 3, (90, 1350)).astype(np.uint8)
+    geno[rng.random(geno.shape) < 0.02] = 3
+    if copies:
+        geno[:] = geno[0]
+    ds = Dataset.from_genotypes(geno, np.r_[np.ones(700, np.uint8), np.zeros(650, np.uint8)])
+    gs = GpuSearch(0)
+    srv = Server(0)
+    try:
+        tickets = [srv.submit(ds, 3, 40, r, 5) for r in range(5)]
+        for r, t in enumerate(tickets):
+            _same(srv.result(t), gs.run_shard(ds, 3, r, 5, 40, with_fp64=True))
+    finally:
+        srv.close()
