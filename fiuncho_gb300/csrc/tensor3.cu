@@ -78,16 +78,31 @@ static cudaError_t order_planes(T3Plan& plan, const DevData& d, int order, const
     cudaError_t e = cudaSuccess;
     if (order == 2) {
         if (plan.f4.ones) return e;
-        e = f4_ones_planes(d, plan.f4, d.snps, 0, 1, plan.f4.ones, s);
+        uint8_t* ones = nullptr;
+        e = f4_ones_planes(d, plan.f4, d.snps, 0, 1, ones, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e == cudaSuccess) e = f4_map_a2(&plan.f4.map_a2, plan.f4, plan.f4.ones, d.snps);
-        if (e == cudaSuccess) e = f4_map_b2(&plan.f4.map_b2, plan.f4, plan.f4.ones, d.snps);
+        if (e == cudaSuccess) e = f4_map_a2(&plan.f4.map_a2, plan.f4, ones, d.snps);
+        if (e == cudaSuccess) e = f4_map_b2(&plan.f4.map_b2, plan.f4, ones, d.snps);
+        if (e == cudaSuccess) plan.f4.ones = ones;  // (what is named here is complete)
+        else cudaFree(ones);
         return e;
     }
     if (!plan.f4.bits) {
-        e = f4_prepare(d, plan.f4, plan.missing ? 3 : 2, s);
+        // made apart: searches of order 2 may be reading what the plan holds
+        F4Plan made = plan.f4;
+        e = f4_prepare(d, made, plan.missing ? 3 : 2, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) f4_release(plan.f4);
+        if (e != cudaSuccess) {
+            cudaFree(made.planes);
+            return e;
+        }
+        plan.f4.map_b = made.map_b;
+        plan.f4.map_j = made.map_j;
+        plan.f4.map_i = made.map_i;
+        plan.f4.map_b4h = made.map_b4h;
+        plan.f4.rows = made.rows;
+        plan.f4.planes = made.planes;
+        plan.f4.bits = made.bits;
     }
     if (e == cudaSuccess && order == 4 && !plan.f4.tri) {
         e = order3_items(plan, d);
@@ -114,12 +129,11 @@ cudaError_t tensor3_order_items(T3Plan& plan, const DevData& d, int order, const
     if (e == cudaSuccess && order == 4 && !plan.item4_begin && d.snps >= 4) {
         std::vector<long long> per4;
         const std::vector<long long> ib4 = t4_item_table(d.snps, per4);
-        e = upload(plan.item4_per, per4);
-        if (e != cudaSuccess) return e;
         plan.total4 = ib4.back();
         const double n = d.snps;
         plan.item4_combos = n * (n - 1) * (n - 2) * (n - 3) / 24.0 / std::max(1ll, plan.total4);
-        e = upload(plan.item4_begin, ib4);
+        if (!plan.item4_per) e = upload(plan.item4_per, per4);
+        if (e == cudaSuccess) e = upload(plan.item4_begin, ib4);
     }
     return e;
 }
