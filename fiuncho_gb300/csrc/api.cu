@@ -130,13 +130,25 @@ int choose_kernel(fiu_ctx* ctx, const fiu_resident* res_c, unsigned order, int r
     const bool need_pairs = order >= 3 && !res->pairs, need_triples = order == 4 && !res->triples;
     if (!res->single || need_pairs || need_triples) {
         const long long np = (long long)res->d.snps * (res->d.snps - 1) / 2;
+        // (the data set names a table once it is complete: a later search takes what is named for made)
+        uint32_t* single = res->single;
+        uint4 *pairs = res->pairs, *triples = res->triples;
         cudaError_t e = cudaSuccess;
-        if (!res->single) e = cudaMalloc((void**)&res->single, (size_t)res->d.snps * 4 * sizeof(uint32_t));
-        if (e == cudaSuccess && need_pairs && np > 0) e = cudaMalloc((void**)&res->pairs, (size_t)np * sizeof(uint4));
-        if (e == cudaSuccess) e = build_cores(res->d, res->single, need_pairs ? res->pairs : nullptr, ctx->sms, ctx->stream);
-        if (e == cudaSuccess && need_triples) e = cudaMalloc((void**)&res->triples, triples_bytes(res->d.snps));
-        if (e == cudaSuccess && need_triples) e = build_triples(res->d, res->triples, ctx->sms, ctx->stream);
+        if (!single) e = cudaMalloc((void**)&single, (size_t)res->d.snps * 4 * sizeof(uint32_t));
+        if (e == cudaSuccess && need_pairs && np > 0) e = cudaMalloc((void**)&pairs, (size_t)np * sizeof(uint4));
+        if (e == cudaSuccess) e = build_cores(res->d, single, need_pairs ? pairs : nullptr, ctx->sms, ctx->stream);
+        if (e == cudaSuccess && need_triples) e = cudaMalloc((void**)&triples, triples_bytes(res->d.snps));
+        if (e == cudaSuccess && need_triples) e = build_triples(res->d, triples, ctx->sms, ctx->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+        if (e != cudaSuccess) {
+            if (single != res->single) cudaFree(single);
+            if (pairs != res->pairs) cudaFree(pairs);
+            if (triples != res->triples) cudaFree(triples);
+        } else {
+            res->single = single;
+            res->pairs = pairs;
+            res->triples = triples;
+        }
         if (e != cudaSuccess) return cuda_fail(ctx, e, "core tables");
     }
     return FIU_OK;

@@ -129,8 +129,26 @@ static void layers() {
     CHECK(live.empty());
 }
 
+static void core_tables() {
+    fiu_ctx ctx;
+    ctx.sms = 152;
+    fiu_resident r;
+    r.d = kData;
+    r.one_hot = 1;
+    int kernel = 0;
+    each_failure([&] { return choose_kernel(&ctx, &r, 2, FIU_KERNEL_ELIDED_HS, kernel); }, [&] { CHECK(!r.single); });
+    uint32_t* single = r.single;
+    CHECK(live.count(single) && !r.pairs);
+    each_failure([&] { return choose_kernel(&ctx, &r, 4, FIU_KERNEL_ELIDED_POPC, kernel); },
+                 [&] { CHECK(r.single == single && live.count(single) && !r.pairs && !r.triples); });
+    CHECK(r.single == single && live.count(r.pairs) && live.count(r.triples) && live.size() == 3);
+    for (void* p : {(void*)r.single, (void*)r.pairs, (void*)r.triples}) __wrap_cudaFree(p);
+    CHECK(live.empty());
+}
+
 int main() {
     whole_scans();
     layers();
+    core_tables();
     std::printf("ok\n");
 }
