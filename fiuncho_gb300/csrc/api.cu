@@ -233,10 +233,18 @@ static bool tensor_ok(const fiu_resident* res, const ScanWork& w) {
 // host work (tensor vs full-table kernel, host data: 10 SNPs x 200 0.61 vs 0.61 ms, 30 x 500 0.63 vs 0.67,
 // 45 x 900 0.65 vs 0.80, 200 x 8 000 1.2 vs 5.7; resident 400 x 8 000 2.0 vs 25, 1 000 x 1 000 6.5 vs 61).
 constexpr int kMissingMinSnps = 32;
-// Batched and served scans below this many combinations x samples stay in the rounds, which take many of them at
-// once (batches of 24, rounds vs tensor kernel on the lanes: 32 SNPs x 900 samples 1.06 vs 1.69 ms, 60 x 900 1.56
-// vs 1.80, 100 x 900 2.98 vs 3.29 [1.5e8 each]; 60 x 8 000 4.14 vs 2.00 [2.7e8], 200 x 900 16.0 vs 4.9).
-constexpr double kMissingRoundsWork = 2e8;
+// Of the scans that rounds could take and a tensor kernel too (order 3 with missing calls, order-4 layers of few
+// samples), batches and the server leave those below this many combinations x samples to the rounds, which take
+// many of them at once (rounds vs tensor kernel on the lanes; missing calls, batches of 24: 32 SNPs x 900 samples
+// 1.06 vs 1.69 ms, 60 x 900 1.56 vs 1.80, 100 x 900 [1.5e8 each] 2.98 vs 3.29, 60 x 8 000 [2.7e8] 4.14 vs 2.00,
+// 200 x 900 16.0 vs 4.9; layers, 24 of 60 x 300 step 4 [3.7e7] 4.7 vs 6.2, 24 of 60 x 900 step 2 [2.2e8] 8.9 vs
+// 6.9, 12 of 100 x 900 step 4 11.4 vs 7.3).
+constexpr double kRoundsWork = 2e8;
+static bool in_rounds(Use use, const ScanWork& w) {
+    return use == Use::kShared && (double)binom(w.dist_n, w.order) / std::max(1, w.dist_step) *
+                                          ((double)w.d.n_cases + w.d.n_ctrls) <
+                                      kRoundsWork;
+}
 static bool missing_ok(const fiu_resident* res, const ScanWork& w) {
     return !res->one_hot && res->disjoint && w.order == 3 && res->d.snps >= kMissingMinSnps && whole_data_set(res, w) && res->d.n_cases >= 1 &&
            res->d.n_ctrls >= 1 && res->d.n_cases <= 65535 && res->d.n_ctrls <= 65535 && res->d.snps < (1 << 21) &&
@@ -259,19 +267,17 @@ static int missing_plan(fiu_ctx* ctx, const fiu_resident* res) {
     return cuda_fail(ctx, e, "tensor operands and work items");
 }
 
-// Order-4 scans of fewer samples and SNPs keep the CUDA-core pair-major kernel unless FIU_KERNEL_TENSOR is
-// forced.  In a search of its own the tensor kernel is the faster one at every size measured from 30 SNPs
-// (pair-major vs tensor, resident data: 30 SNPs x 200 samples 0.54 vs 0.24 ms, 100 x 300 1.24 vs 1.00, 150 x
-// 200 3.3 vs 2.9, 150 x 900 4.8 vs 2.9, 300 x 900 65 vs 28), so there the SNPs decide alone; scans that
-// share rounds with others (batched and served ones) go by the samples, since a round takes many small
-// scans at once and the tensor kernel one.
+// Order-4 scans of fewer SNPs and samples than these keep the CUDA-core kernels (pair-major for the whole data
+// set) unless FIU_KERNEL_TENSOR is forced: the tensor kernel is the faster one at every size measured from 30
+// SNPs (pair-major vs tensor, resident data: 30 SNPs x 200 samples 0.54 vs 0.24 ms, 100 x 300 1.24 vs 1.00, 150 x
+// 200 3.3 vs 2.9, 150 x 900 4.8 vs 2.9, 300 x 900 65 vs 28).  For the whole data set both run alone in batches and
+// on the server too, so the rule is one for all of them; small layers of few samples stay in the rounds.
 constexpr int kT4MinSamples = 1024, kT4MinSnps = 32;
 
 int choose_tile(fiu_ctx* ctx, const fiu_resident* res, const ScanWork& w, int requested_kernel, int& kernel, int& tp,
                 Use use) {
     if (requested_kernel == FIU_KERNEL_AUTO && use != Use::kTables && missing_ok(res, w) &&
-        (use != Use::kShared ||
-         (double)binom(w.dist_n, 3) * (res->d.n_cases + res->d.n_ctrls) >= kMissingRoundsWork)) {
+        !in_rounds(use, w)) {
         const int rc = missing_plan(ctx, res);
         if (rc == FIU_OK) {
             kernel = FIU_KERNEL_TENSOR;
@@ -280,7 +286,9 @@ int choose_tile(fiu_ctx* ctx, const fiu_resident* res, const ScanWork& w, int re
         }
         if (use == Use::kShard) return rc;  // (not the full tables: other shards are cut by this kernel's units)
     }
-    const bool auto_tensor = tensor_ok(res, w) && (w.order != 4 || res->d.n_cases + res->d.n_ctrls >= kT4MinSamples);
+    const bool auto_tensor = tensor_ok(res, w) && (w.order != 4 || res->d.n_cases + res->d.n_ctrls >= kT4MinSamples ||
+                                                   (res->d.snps >= kT4MinSnps &&
+                                                    (whole_data_set(res, w) || !in_rounds(use, w))));
     if (requested_kernel == FIU_KERNEL_TENSOR || (requested_kernel == FIU_KERNEL_AUTO && auto_tensor)) {
         if (!tensor_ok(res, w))
             return fail(ctx, FIU_ERR_UNSUPPORTED,
@@ -395,10 +403,9 @@ int search_impl(fiu_ctx* ctx, const fiu_resident* res, unsigned order, const fiu
     if (outputs == 0 || w.n_prefixes == 0) return FIU_OK;
     CK(cudaSetDevice(ctx->device), "cudaSetDevice");
     int tp = 256;
-    int requested = kernel ? kernel : ctx->kernel;
-    if (requested == FIU_KERNEL_AUTO && order == 4 && res->d.snps >= kT4MinSnps && tensor_ok(res, w))
-        requested = FIU_KERNEL_TENSOR;
-    if ((rc = choose_tile(ctx, res, w, requested, kernel, tp, n_shards > 1 ? Use::kShard : Use::kSearch))) return rc;
+    if ((rc = choose_tile(ctx, res, w, kernel ? kernel : ctx->kernel, kernel, tp,
+                          n_shards > 1 ? Use::kShard : Use::kSearch)))
+        return rc;
     ctx->last_kernel = kernel;
     ctx->last_tp = tp;
     const bool tensor = kernel == FIU_KERNEL_TENSOR, missing = tensor && res->t3->missing;

@@ -245,6 +245,8 @@ void tensor3_release(T3Plan& plan);
 cudaError_t launch_tensor3(const ScanWork& w, const T3Plan& plan, long long g0, long long g1, const CandSink& sink,
                            uint32_t* dump, const uint32_t* single, const uint4* pairs, int* status, cudaStream_t s,
                            int sms);
+// Bytes of order 4's cores (F4Plan::tri and pairf), more than triples_bytes.
+size_t f4_triples_bytes(int snps);
 // tensor4x.cu -- order 4 on tcgen05 (one-hot data, the whole data set or a Distribution layer of it).
 // Item tables of the whole data set, and of a layer (the listed pairs (i, j) with their first owned k).
 std::vector<long long> t4_item_table(int n, std::vector<long long>& per);

@@ -78,12 +78,11 @@ size_t footprint(const ServeScan& s) {
     const size_t snps = s.host.snps, W = s.host.cases_words + s.host.ctrls_words;
     size_t b = 2 * snps * 3 * W * 8 + (64 * W + 1) * 8 + snps * 16;  // data set, transposed copy, c ln c table
     if (s.order >= 3) b += snps * (snps - 1) / 2 * 16;                     // pair cores
-    if (s.order == 4) b += (size_t)binom((long long)snps, 3) * 32;         // triple cores
+    if (s.order == 4) b += f4_triples_bytes((int)snps);                    // triple cores and pair cores once more
     // operand planes of the tensor-core kernels and their bit rows, up to 3 rows per SNP, each class padded to
-    // 256 samples; at order 4 the pair cores again
+    // 256 samples
     const size_t cw = s.host.cases_words, tw = s.host.ctrls_words;
     b += 3 * snps * 160 * ((cw + 3) / 4 + (tw + 3) / 4);
-    if (s.order == 4) b += snps * snps / 2 * 16;
     const size_t keep = s.outputs + std::max(32u, s.outputs / 8);
     b += std::max<size_t>({32768, 16 * keep, snps + keep}) * sizeof(Cand) + keep * sizeof(ScoredRec) +
          (size_t)s.outputs * (4 * s.order + 12) + 4096;

@@ -917,28 +917,51 @@ __global__ void f4_pairf_kernel(const uint4* __restrict__ pairs, uint32_t* out, 
     }
 }
 
+// Rows of l pairs, row k from l = k + 1 rounded down to even: row_p (n), row_q (n), where F4Plan has them, and
+// the entries of the pairs and of the triples.
+struct F4Rows {
+    std::vector<int> p;
+    long long pairs = 0, triples = 0;
+};
+static F4Rows f4_rows(int n) {
+    F4Rows r;
+    r.p.resize((size_t)2 * n + 1);  // and the launch's status
+    std::vector<long long> P((size_t)n + 1);
+    for (int k = 0; k < n; ++k) {
+        P[k] = r.pairs;
+        r.p[k] = (int)(r.pairs - ((k + 1) >> 1));
+        r.pairs += ((n + 1) >> 1) - ((k + 1) >> 1);
+    }
+    P[n] = r.pairs;
+    for (int i = 0; i < n; ++i) {
+        r.p[n + i] = (int)(r.triples - P[i + 1]);
+        r.triples += P[n] - P[i + 1];
+    }
+    return r;
+}
+
+size_t f4_triples_bytes(int snps) {
+    // row k has ceil(n / 2) - floor((k + 1) / 2) entries, and a triple's (i, k) one of row k for every i < k
+    const unsigned long long n = snps, h = (n + 1) / 2;
+    unsigned long long pairs = 0, triples = 0;
+    if (n > 4096) return (size_t)std::min(5.34 * n * n * n, 4e18);  // (larger than any device)
+    for (unsigned long long k = 0; k < n; ++k) {
+        pairs += h - (k + 1) / 2;
+        triples += k * (h - (k + 1) / 2);
+    }
+    return (size_t)triples * 64 + (size_t)pairs * 32;
+}
+
 cudaError_t f4_triples(const DevData& d, F4Plan& f, const long long* item_begin, long long items, const uint4* pairs,
                        cudaStream_t s, int sms) {
     const int n = d.snps;
-    // rows of l pairs: row k starts at l = k + 1 rounded down to even
-    std::vector<int> p((size_t)2 * n + 1);  // and the launch's status
-    long long at = 0;
-    std::vector<long long> P((size_t)n + 1);
-    for (int k = 0; k < n; ++k) {
-        P[k] = at;
-        p[k] = (int)(at - ((k + 1) >> 1));
-        at += ((n + 1) >> 1) - ((k + 1) >> 1);
-    }
-    P[n] = at;
-    long long B = 0;
-    for (int i = 0; i < n; ++i) {
-        p[n + i] = (int)(B - P[i + 1]);
-        B += P[n] - P[i + 1];
-    }
+    const F4Rows r4 = f4_rows(n);
+    const std::vector<int>& p = r4.p;
+    const long long B = r4.triples;
     int* rows = nullptr;
     char* tab = nullptr;  // triples, then pairs
     cudaError_t e = cudaMalloc((void**)&rows, p.size() * sizeof(int));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&tab, (size_t)B * 64 + (size_t)P[n] * 32);
+    if (e == cudaSuccess) e = cudaMalloc((void**)&tab, f4_triples_bytes(n));
     if (e == cudaSuccess) e = cudaMemcpyAsync(rows, p.data(), p.size() * sizeof(int), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) {
         f.row_p = rows;

@@ -232,3 +232,23 @@ def test_server_shards_of_missing_calls(copies):
             _same(srv.result(t), gs.run_shard(ds, 3, r, 5, 40, with_fp64=True))
     finally:
         srv.close()
+
+
+def test_server_order4_holds_what_it_counts():
+    """An order-4 scan of few samples holds the device memory that the budget counts for it: one table of
+    triple cores (0.67 GB here), not one for each kernel that could serve it."""
+    import torch
+    from fiuncho_gb300 import Server
+    srv = Server(0)
+    try:
+        srv.result(srv.submit(_ds(81, 60, 450, 450), 4, 10))  # the lanes' own buffers
+        srv.result(srv.submit(_ds(82, 60, 450, 450), 4, 10))
+        free0 = low = torch.cuda.mem_get_info()[0]
+        ticket = srv.submit(_ds(83, 500, 450, 450), 4, 10)
+        while srv.result(ticket, 1) is None:
+            low = min(low, torch.cuda.mem_get_info()[0])
+        peak = srv.stats()["peak_bytes"]
+        # 64 MB: the second lane's candidate buffers and the allocator's 2 MB steps
+        assert 0.5 * peak < free0 - low < peak + (64 << 20)
+    finally:
+        srv.close()

@@ -232,3 +232,19 @@ def test_layers_of_steps_past_32_bit_positions(oracle, order, snps, step, offset
         gs.set_kernel(kernel)
         lists.append([(r.combination, r.val) for r in gs.run(res, order, d, 25)])
     assert lists[0] == lists[1] and len(lists[0]) == min(25, count)
+
+
+@pytest.mark.parametrize("snps,cases,ctrls,kernel", [(31, 300, 300, 2), (32, 300, 300, 4), (31, 600, 424, 4)])
+def test_order4_choice_is_one_for_searches_batches_and_digests(snps, cases, ctrls, kernel):
+    """The automatic order-4 kernel from 32 SNPs or 1 024 samples, below and above; a batch's lanes and the
+    digest's own choice give what a search alone gives."""
+    from fiuncho_gb300 import Distribution, GpuSearch, _lib
+    from fiuncho_gb300.search import Resident
+    gs = GpuSearch(0)
+    res = Resident(gs.ctx, _data(snps, cases, ctrls, 60 + snps))
+    d = Distribution(snps, 3)
+    alone = gs.run(res, 4, d, 30)
+    assert gs.last_tile()[0] == kernel
+    (batched, _), = gs.run_batch([(res, 4, d, 30)])
+    assert [(r.combination, r.val) for r in batched] == [(r.combination, r.val) for r in alone]
+    assert gs.scan_digest(res, 4) == gs.scan_digest(res, 4, kernel=_lib.KERNEL_FULL)
