@@ -20,12 +20,17 @@
 // triples (i,k,l), (j,k,l) and the pair (k,l) come as packed floats of (l, l + 1)
 // side by side (F4Plan::tri, pairf; the triples are made by the order-3 pair
 // kernel, whose accumulators they are).  The quartic bound (F4Bound4) rejects
-// nearly all combinations (300 SNPs x 558/1 012: 5 500 of 3.3e8 pass it); the
-// others get the exact fixed-point key, so the kept set is the one of the exact
-// key.
+// nearly all combinations of classes that are near in size (300 SNPs x 558/1 012:
+// 5 500 of 3.3e8 pass it) and fewer the more one outweighs the other (0.2 % pass at
+// 1 000/4 000, 9 % at 800/8 000, 73 % at 1 000/20 000); a group that has some left
+// takes their logarithm estimate, whose error bound is proven (t4x_estimate), and what
+// passes that gets the exact fixed-point key, so the kept set is the one of the
+// exact key.  150 SNPs, exact keys right after the bound -> with the estimate
+// between: 1 000/4 000 6.0 -> 4.8 ms, 800/8 000 53 -> 7.2, 1 000/20 000 643 -> 16
+// (e4m3 kernel with the estimate for all: 7.3, 10.5 and 22).
 //
-// Measured (whole searches): 300 SNPs x 4 000/4 000 81.9 -> 34.3 ms, 300 x
-// 558/1 012 60.0 -> 29.4 ms, against e4m3 operands, one CTA a tile, 243
+// Measured (whole searches): 300 SNPs x 4 000/4 000 81.9 -> 33.6 ms, 300 x
+// 558/1 012 60.0 -> 28.5 ms, against e4m3 operands, one CTA a tile, 243
 // logarithms a combination (1 944 cycles a warp and SM quarter) and triples
 // counted by POPC.  Without the evaluation the two take 22 and 13 ms; the
 // evaluation of 64 combinations by a warp is 2 240 cycles of bound (81 x 2
@@ -34,7 +39,7 @@
 // three warps a quarter on one combination at a time (104 registers) 40 ms; the
 // slices in a loop (a third of the code) 32.8; three cells at a time through the
 // bound 29.5.  Classes that do not share an accumulator (SPLIT): 100 SNPs x
-// 9 000/9 800 6.7 -> 3.1 ms.
+// 9 000/9 800 6.7 -> 2.9 ms.
 //
 // Reference semantics: GenotypeTable::combine_and_popcnt for order 4
 // (src/base/gt_popcnt.cpp:4-35) and MutualInformation::compute
@@ -248,9 +253,67 @@ __device__ __forceinline__ void t4x_slices(const T4xCores<T>& v, TL&& tabl, TK&&
     }
 }
 
+// The key estimate, in bits, of the combinations in v: of the two side by side, or (SPLIT) of one, in both
+// halves.  It is within t4x_margin of the exact key: a cell's three terms a lg a + b lg b - s lg s are added up
+// first (at most s in magnitude), so that the running sum stays below the samples.  For the groups in which a
+// combination passes the quartic bound; out of line, with the cores through local memory, since its
+// registers beside the bound's would slow every group down.  Bound by its 486 logarithms (3 888 cycles a warp and
+// SM quarter), against 10 to 70 us for each exact key that it saves.
+template <bool SPLIT>
+__device__ __noinline__ f2 t4x_estimate(const T4xCores<f2>* v, const std::conditional_t<SPLIT, f2, float>* tl,
+                                        const f2* tabk0, int zb, int pack) {
+    const f2 tiny = f2_dup(9.5367431640625e-07f);  // 2^-20: x lg2(x + tiny) = 0 at x = 0
+    const f2 inv_w = f2_dup(__uint_as_float((uint32_t)(127 - pack) << 23)), neg_w = f2_dup(-(float)(1 << pack));
+    const f2 m23 = f2_dup(8388608.0f), neg_m23 = f2_dup(-8388608.0f);
+    f2 kf = 0;
+    t4x_slices<f2>(
+        *v,
+        [&](int e) {
+            if constexpr (SPLIT) return tl[e * kYL];
+            else return *reinterpret_cast<const f2*>(tl + e * kYL);
+        },
+        [&](int e) { return tabk0[(e ^ zb) * kYK]; },
+        [&](int, int, f2 cell) {
+            if constexpr (SPLIT) {
+                float a, b, k, unused;
+                f2_unpack(cell, a, b);
+                f2_unpack(kf, k, unused);
+                const float t2 = 9.5367431640625e-07f, s = a + b;
+                k += fmaf(-s, t3_lg2(s + t2), fmaf(b, t3_lg2(b + t2), a * t3_lg2(a + t2)));
+                kf = f2_dup(k);
+            } else {
+                auto lg = [](f2 x) {
+                    float lo, hi;
+                    f2_unpack(x, lo, hi);
+                    return f2_pack(t3_lg2(lo), t3_lg2(hi));
+                };
+                const f2 b = f2_add(f2_fma_rz(cell, inv_w, m23), neg_m23), a = f2_fma(neg_w, b, cell), s = f2_add(a, b);
+                const f2 ab = f2_fma(b, lg(f2_add(b, tiny)), f2_mul(a, lg(f2_add(a, tiny))));
+                kf = f2_add(kf, f2_sub(ab, f2_mul(s, lg(f2_add(s, tiny)))));
+            }
+        });
+    return kf;
+}
+
+// Bound (in bits) on |t4x_estimate - exact key / (ln2 * 2^32)|, N samples: each sample lies in one of the 81
+// cells, so sum s over the cells is N and sum s lg2 s <= N lg2 N.  A cell's products and sums round at most 5
+// times by 2^-24 of at most s lg2 s; lg2.approx is within 2^-18 of log2 on every input the kernel can see (checked
+// exhaustively by fiu_probe_lg2_error), which moves a cell by at most 2 s 2^-18; the x + 2^-20 shift moves each
+// of the 243 products by at most 2^-20 / ln 2 and its rounding each logarithm by at most 2^-24 / ln 2; the
+// running sum, below N, rounds 81 times; the integer table rounds each of the 243 exact terms by 1/2 of 2^-32
+// nats.  Doubled.  (0.3 bits at 8 000 samples, 4.9 at 130 000.)
+static double t4x_margin(int n_samples) {
+    const double N = n_samples, lgN = std::log2(std::max(2.0, N)), l2 = std::log(2.0);
+    const double u = std::ldexp(1.0, -24), e20 = std::ldexp(1.0, -20), e_lg2 = std::ldexp(1.0, -18);
+    const double err = 5 * u * N * lgN + 2 * N * e_lg2 + 243 * e20 / l2 + 2 * N * u / l2 + 82 * u * N +
+                       243 * 0.5 / (l2 * 4294967296.0);
+    return 2 * err + 1e-3;
+}
+
 // ALL: every combination takes the exact path (a search's first units, before a threshold; dumps and
-// digests).  Otherwise the bound comes first and the few combinations above it are evaluated from the
-// data set (warp_exact_key): the exact path's registers beside the bound's cost 20 % of the whole.
+// digests).  Otherwise the bound comes first, a group with combinations above it gets their estimates
+// (t4x_estimate), and the few that pass those are evaluated from the data set (warp_exact_key): the exact
+// path's registers beside the bound's cost 20 % of the whole.
 // SPLIT: classes that do not share an accumulator, as in the order-3 kernel: cases accumulate in one region
 // and go to shared memory as 16-bit counts, controls in the other; one combination at a time is evaluated
 // from both beside each other.
@@ -409,7 +472,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
                     live_tests(map, thr, est, bound);
                     uint8_t* o = tabs + buf * kTab + kTabL + kYTabK;
                     *reinterpret_cast<long long*>(o) = thr;
-                    *reinterpret_cast<float*>(o + 8) = bound;
+                    *reinterpret_cast<float2*>(o + 8) = make_float2(bound, est);
                 }
                 Tab* tl = reinterpret_cast<Tab*>(tabs + buf * kTab);
                 f2* tk = reinterpret_cast<f2*>(tabs + buf * kTab + kTabL);
@@ -603,6 +666,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
             const f2* tabk0 = reinterpret_cast<const f2*>(tabs + buf * kTab + kTabL) + kk;
             const long long thr = *reinterpret_cast<const long long*>(tabs + buf * kTab + kTabL + kYTabK);
             const float thr_q = *reinterpret_cast<const float*>(tabs + buf * kTab + kTabL + kYTabK + 8);
+            auto thr_f = [&] { return reinterpret_cast<const float*>(tabs + buf * kTab + kTabL + kYTabK)[3]; };
             // per-k entries: the index's last bit is z
             auto tabk = [&](int e) { return tabk0[(e ^ zb) * kYK]; };
             auto exact_append = [&](int src, int u, int lu) {  // a survivor of lane src
@@ -674,25 +738,28 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
                     for (int x = 0; x < 2; ++x) acc_counts(1, x, gi, t[x][0], t[x][1]);
 #pragma unroll 1
                     for (int u = 0; u < 2; ++u) {
-                        T4xCores<f2> v;
+                        auto cores = [&](T4xCores<f2>& v) {  // of combination u, whose triples and pair are in ik, jk, kl
 #pragma unroll
-                        for (int x = 0; x < 2; ++x)
+                            for (int x = 0; x < 2; ++x)
+#pragma unroll
+                                for (int z = 0; z < 2; ++z) {
+                                    const uint4 c = mine[(2 * (gi & ~1) + 2 * x + z) * 32];
+#pragma unroll
+                                    for (int e = 0; e < 4; ++e)
+                                        v.c[x][e & 1][z][e >> 1] = f4_ab((&c.x)[e], (&t[x][z].x)[e], u);
+                                    v.ik[x][z][0] = f4_ab(ik[x][z].x);
+                                    v.ik[x][z][1] = f4_ab(ik[x][z].y);
+                                    v.jk[x][z][0] = f4_ab(jk[x][z].x);
+                                    v.jk[x][z][1] = f4_ab(jk[x][z].y);
+                                }
 #pragma unroll
                             for (int z = 0; z < 2; ++z) {
-                                const uint4 c = mine[(2 * (gi & ~1) + 2 * x + z) * 32];
-#pragma unroll
-                                for (int e = 0; e < 4; ++e)
-                                    v.c[x][e & 1][z][e >> 1] = f4_ab((&c.x)[e], (&t[x][z].x)[e], u);
-                                v.ik[x][z][0] = f4_ab(ik[x][z].x);
-                                v.ik[x][z][1] = f4_ab(ik[x][z].y);
-                                v.jk[x][z][0] = f4_ab(jk[x][z].x);
-                                v.jk[x][z][1] = f4_ab(jk[x][z].y);
+                                v.kl[z][0] = f4_ab(kl[z].x);
+                                v.kl[z][1] = f4_ab(kl[z].y);
                             }
-#pragma unroll
-                        for (int z = 0; z < 2; ++z) {
-                            v.kl[z][0] = f4_ab(kl[z].x);
-                            v.kl[z][1] = f4_ab(kl[z].y);
-                        }
+                        };
+                        T4xCores<f2> v;
+                        cores(v);
                         load(u ? gi + 2 : gi, u ^ 1);  // the next one's, on their way while this one is evaluated
                         const Tab* tl = tabl0 + ll + u;
                         auto tabl = [&](int e) { return tl[e * kYL]; };
@@ -701,7 +768,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
                             F4Bound4AB bd(quart);
                             t4x_slices<f2>(v, tabl, tabk, [&](int, int, f2 cell) { bd.one(cell); });
                             unsigned sv = __ballot_sync(0xffffffffu, want && bd.acc >= thr_q);
-                            for (; sv; sv &= sv - 1) exact_append(__ffs(sv) - 1, u, l);
+                            if (sv) {
+                                load(gi, u);  // (the next one's triples have taken the place of this one's)
+                                T4xCores<f2> again;
+                                cores(again);
+                                float est, unused;
+                                f2_unpack(t4x_estimate<true>(&again, tl, tabk0, zb, pack), est, unused);
+                                sv &= __ballot_sync(0xffffffffu, est >= thr_f());
+                                for (; sv; sv &= sv - 1) exact_append(__ffs(sv) - 1, u, l);
+                                load(u ? gi + 2 : gi, u ^ 1);
+                            }
                         } else {
                             every(l + u, want, [&](auto&& use) {
                                 t4x_slices<f2>(v, tabl, tabk, [&](int sw, int c, f2 cell) {
@@ -779,11 +855,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
                         f2_unpack(bd.acc, b0, b1);
                         unsigned s0 = __ballot_sync(0xffffffffu, v0 && b0 >= thr_q);
                         unsigned s1 = __ballot_sync(0xffffffffu, v1 && b1 >= thr_q);
-                        while (s0 | s1) {
-                            const int u = s0 ? 0 : 1, src = __ffs(u ? s1 : s0) - 1;
-                            if (u) s1 &= s1 - 1;
-                            else s0 &= s0 - 1;
-                            exact_append(src, u, l);
+                        if (s0 | s1) {
+                            load(gi);  // (the next group's triples have taken the place of this one's)
+                            const T4xCores<f2> again = v;
+                            f2_unpack(t4x_estimate<false>(&again, tl, tabk0, zb, pack), b0, b1);
+                            s0 &= __ballot_sync(0xffffffffu, b0 >= thr_f());
+                            s1 &= __ballot_sync(0xffffffffu, b1 >= thr_f());
+                            while (s0 | s1) {
+                                const int u = s0 ? 0 : 1, src = __ffs(u ? s1 : s0) - 1;
+                                if (u) s1 &= s1 - 1;
+                                else s0 &= s0 - 1;
+                                exact_append(src, u, l);
+                            }
+                            load(gi + 2);
                         }
                     } else {
 #pragma unroll 1
@@ -906,7 +990,7 @@ cudaError_t launch_tensor4x(const ScanWork& w, const F4Plan& f, const T4xRange& 
     const long long clusters = std::min<long long>(g1 - g0, max_clusters > 0 ? max_clusters : sms / 2);
     const unsigned grid = (unsigned)(2 * std::max(1ll, clusters));
     const double scale = 1.0 / (std::log(2.0) * 4294967296.0);
-    LiveMap map{0, 0, 0, 0};
+    LiveMap map{scale, -(double)w.base_key * scale - t4x_margin(w.d.n_cases + w.d.n_ctrls), 0, 0};
     const F4Quartic quart = f4_quartic(w.d.n_cases, w.d.n_ctrls, 81, map.bound_k, map.bound_c);
     map.bound_k *= scale;
     const bool all = dump || sink.digest || sink.thr == (long long)0x8000000000000000ull;

@@ -248,3 +248,42 @@ def test_order4_choice_is_one_for_searches_batches_and_digests(snps, cases, ctrl
     (batched, _), = gs.run_batch([(res, 4, d, 30)])
     assert [(r.combination, r.val) for r in batched] == [(r.combination, r.val) for r in alone]
     assert gs.scan_digest(res, 4) == gs.scan_digest(res, 4, kernel=_lib.KERNEL_FULL)
+
+
+@pytest.mark.parametrize("snps,cases,ctrls,step", [
+    (60, 30, 900, 1), (60, 900, 30, 1), (50, 200, 7800, 1), (50, 7800, 200, 1), (45, 1000, 20000, 1),
+    (45, 20000, 1000, 1), (40, 600, 60000, 1), (40, 60000, 600, 1), (60, 100, 3000, 3), (45, 1000, 20000, 2)])
+def test_order4_uneven_classes(snps, cases, ctrls, step):
+    """Classes of which one is many times the other: the bound rejects little there, and the estimate that
+    follows it decides what gets an exact key.  Few outputs (a tight threshold) and many, against the
+    full-table kernel."""
+    from fiuncho_gb300 import Distribution, GpuSearch, _lib
+    from fiuncho_gb300.search import Resident
+    gs = GpuSearch(0)
+    res = Resident(gs.ctx, _data(snps, cases, ctrls, 70 + snps))
+    d = Distribution(snps, 3, step, step - 1)
+    for outputs in (10, 3000):
+        gs.set_kernel(_lib.KERNEL_TENSOR)
+        a = gs.run(res, 4, d, outputs)
+        gs.set_kernel(_lib.KERNEL_FULL)
+        b = gs.run(res, 4, d, outputs)
+        assert [(r.combination, r.val) for r in a] == [(r.combination, r.val) for r in b]
+
+
+def test_order4_uneven_classes_cost_no_exact_key_each():
+    """100 SNPs x 1 000 cases and 20 000 controls, where seven combinations in ten pass the bound, within five
+    times the time of even classes (with an exact key for each of them 150 SNPs took 643 ms, now 16)."""
+    import time
+    from fiuncho_gb300 import Distribution, GpuSearch
+    from fiuncho_gb300.search import Resident
+    gs = GpuSearch(0)
+    best = []
+    for cases, ctrls in ((10500, 10500), (1000, 20000)):
+        res = Resident(gs.ctx, _data(100, cases, ctrls, 71))
+        times = []
+        for _ in range(4):
+            t = time.perf_counter()
+            gs.run(res, 4, Distribution(100, 3), 50)
+            times.append(time.perf_counter() - t)
+        best.append(min(times))
+    assert best[1] < 5 * best[0], best
