@@ -295,6 +295,31 @@ __device__ __noinline__ f2 t4x_estimate(const T4xCores<f2>* v, const std::condit
     return kf;
 }
 
+// SPLIT: the exact key (without the base) of the combination in v, a lane each, from its cells, for groups with
+// several left (no threshold yet, or many that tie with it): one a warp from the data set (warp_exact_key) takes
+// 10 to 70 us at these classes' samples.  Bound by its gathers from the c ln c table.  100 copies of one SNP x
+// 18 000 samples, all combinations tied: 1 920 -> 90 ms (e4m3 kernel 724); a layer of 100 SNPs, step 7, 7 000
+// outputs 12.5 -> 8.7.  Classes that share an accumulator stay with warp_exact_key, which is short there: with this
+// beside it their kernel's code came out 6 % slower (300 SNPs x 558/1 012 28.5 -> 30.4 ms; all tied, 100 x
+// 2 000, 232 -> 58, e4m3 407).
+__device__ __noinline__ long long t4x_key(const T4xCores<f2>* v, const f2* tl, const f2* tabk0, int zb,
+                                          const DevData* d) {
+    const uint32_t nc = (uint32_t)d->n_cases, nt = (uint32_t)d->n_ctrls;
+    const long long* ftab = d->ftab;
+    long long key = 0;
+    t4x_slices<f2>(
+        *v, [&](int e) { return tl[e * kYL]; }, [&](int e) { return tabk0[(e ^ zb) * kYK]; },
+        [&](int, int, f2 cell) {
+            float x, y;
+            f2_unpack(cell, x, y);
+            // (a lane without a combination holds anything: clamped)
+            const uint32_t a = min(__float2uint_rn(x), nc), b = min(__float2uint_rn(y), nt);
+            key += __ldg(ftab + a) + __ldg(ftab + b) - __ldg(ftab + a + b);
+        });
+    return key;
+}
+constexpr int kYGroupKeys = 4;  // combinations left of a group from which t4x_key makes all their keys
+
 // Bound (in bits) on |t4x_estimate - exact key / (ln2 * 2^32)|, N samples: each sample lies in one of the 81
 // cells, so sum s over the cells is N and sum s lg2 s <= N lg2 N.  A cell's products and sums round at most 5
 // times by 2^-24 of at most s lg2 s; lg2.approx is within 2^-18 of log2 on every input the kernel can see (checked
@@ -775,6 +800,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
                                 float est, unused;
                                 f2_unpack(t4x_estimate<true>(&again, tl, tabk0, zb, pack), est, unused);
                                 sv &= __ballot_sync(0xffffffffu, est >= thr_f());
+                                if (__popc(sv) >= kYGroupKeys) {
+                                    const int cmb[4] = {it.i, it.j, k, l + u};
+                                    const long long key = t4x_key(&again, tl, tabk0, zb, &w.d) + w.base_key;
+                                    if ((sv >> lane & 1) && key >= thr) live_append(sink, key, pack_code(cmb, 4, w.bits));
+                                    sv = 0;
+                                }
                                 for (; sv; sv &= sv - 1) exact_append(__ffs(sv) - 1, u, l);
                                 load(u ? gi + 2 : gi, u ^ 1);
                             }

@@ -287,3 +287,25 @@ def test_order4_uneven_classes_cost_no_exact_key_each():
             times.append(time.perf_counter() - t)
         best.append(min(times))
     assert best[1] < 5 * best[0], best
+
+
+@pytest.mark.parametrize("cases,ctrls", [(300, 311), (4100, 4101), (9000, 9800)])
+@pytest.mark.parametrize("copies", [1, 8, 40])
+def test_order4_many_keys_in_a_group(cases, ctrls, copies):
+    """Groups of which several combinations reach the threshold -- SNPs that are copies of one another, and a
+    layer whose first launch holds fewer combinations than are kept -- take all their keys at once: the
+    lists against the full-table kernel's."""
+    from fiuncho_gb300 import Dataset, Distribution, GpuSearch, _lib
+    from fiuncho_gb300.search import Resident
+    ds = _data(40, cases, ctrls, 72)
+    rows = ds.data.copy().reshape(40, -1)
+    rows[:copies] = rows[0]
+    gs = GpuSearch(0)
+    res = Resident(gs.ctx, Dataset(cases, ctrls, 40, ds.cases_words, ds.ctrls_words, rows.reshape(-1)))
+    for step, outputs in ((1, 10), (1, 5000), (3, 7000)):
+        d = Distribution(40, 3, step, step - 1)
+        gs.set_kernel(_lib.KERNEL_TENSOR)
+        a = gs.run(res, 4, d, outputs)
+        gs.set_kernel(_lib.KERNEL_FULL)
+        b = gs.run(res, 4, d, outputs)
+        assert [(r.combination, r.val) for r in a] == [(r.combination, r.val) for r in b]
