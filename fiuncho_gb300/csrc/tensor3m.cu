@@ -389,7 +389,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kMThreads, 1)
                         if (u) s1 &= s1 - 1;
                         else s0 &= s0 - 1;
                         const int cmb[3] = {it.i, __shfl_sync(0xffffffffu, j, src), __shfl_sync(0xffffffffu, l, src) + u};
-                        const long long ke = warp_exact_key<3>(&w.d, w.base_key, cmb[0], cmb[1], cmb[2], 0);
+                        const long long ke = warp_exact_key<3>(&w.d, w.base_key, cmb[0], cmb[1], cmb[2], 0, sink.overflow);
                         if (lane == 0 && ke >= thr) live_append(sink, ke, pack_code(cmb, 3, w.bits));
                     }
                 }

@@ -696,7 +696,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kYThreads, 1)
             auto tabk = [&](int e) { return tabk0[(e ^ zb) * kYK]; };
             auto exact_append = [&](int src, int u, int lu) {  // a survivor of lane src
                 const int cmb[4] = {it.i, it.j, __shfl_sync(0xffffffffu, k, src), __shfl_sync(0xffffffffu, lu, src) + u};
-                const long long key = warp_exact_key<4>(&w.d, w.base_key, cmb[0], cmb[1], cmb[2], cmb[3]);
+                const long long key = warp_exact_key<4>(&w.d, w.base_key, cmb[0], cmb[1], cmb[2], cmb[3], sink.overflow);
                 if (lane == 0 && key >= thr) live_append(sink, key, pack_code(cmb, 4, w.bits));
             };
             // the exact path of combination (i, j, k, lu), whose slices walk(use) makes: use(w, cell index,

@@ -309,3 +309,18 @@ def test_order4_many_keys_in_a_group(cases, ctrls, copies):
         gs.set_kernel(_lib.KERNEL_FULL)
         b = gs.run(res, 4, d, outputs)
         assert [(r.combination, r.val) for r in a] == [(r.combination, r.val) for r in b]
+
+
+@pytest.mark.parametrize("cases,ctrls", [(300, 311), (4100, 4101)])
+def test_order4_more_ties_than_the_buffer_holds(cases, ctrls):
+    """916 895 combinations of equal value: the launch overflows its candidate buffer and is made again in
+    pieces; the list is the first combinations'."""
+    import itertools
+    from fiuncho_gb300 import Dataset, Distribution, GpuSearch
+    ds = _data(70, cases, ctrls, 73)
+    rows = ds.data.copy().reshape(70, -1)
+    rows[:] = rows[0]
+    gs = GpuSearch(0)
+    got = gs.run(Dataset(cases, ctrls, 70, ds.cases_words, ds.ctrls_words, rows.reshape(-1)), 4, Distribution(70, 3), 40)
+    assert gs.last_tile()[0] == 4
+    assert [tuple(r.combination) for r in got] == list(itertools.islice(itertools.combinations(range(70), 4), 40))
