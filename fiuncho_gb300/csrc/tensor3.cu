@@ -17,6 +17,7 @@
 
 #include "tensor2x.h"
 #include "tensor3m.h"
+#include "tensor_bounds.h"
 #include "tensor_common.cuh"
 
 namespace fiu {
@@ -346,22 +347,6 @@ void tensor3_release(T3Plan& plan) {
     plan.item2_begin = nullptr;
     plan.item4_begin = nullptr;
     plan.item4_per = nullptr;
-}
-
-// Bound on |single-precision estimate - exact key / (ln2 * 2^32)| over the 81
-// terms of one combination: with N the number of samples every partial sum is
-// at most 2 N lg2 N (81 roundings of at most 2^-24 of it), lg2.approx is
-// within 2^-18 of log2 on every input the kernel can see (measured worst case
-// 1.93e-6, checked exhaustively against FP64 by fiu_probe_lg2_error), the
-// x + 2^-20 shift moves each term by at most 2^-20 / ln 2 (counts below 16)
-// or one rounding of the count, and the integer table rounds each term by
-// 1/2.  Doubled.
-static double t3_margin(int n_samples) {
-    const double N = n_samples, lgN = std::log2(std::max(2.0, N)), B = 2 * N * lgN;
-    const double u = std::ldexp(1.0, -24), e20 = std::ldexp(1.0, -20), e_lg2 = std::ldexp(1.0, -18);
-    const double err = 81 * u * B + 2 * N * (18 * u + e_lg2) + 81 * e20 / std::log(2.0) +
-                       2 * N * std::ldexp(1.0, -23) / std::log(2.0) + 81 * 0.5 / (std::log(2.0) * 4294967296.0);
-    return 2 * err + 1e-3;
 }
 
 // Self-check of the bounded mbarrier wait the tensor kernels use: one thread

@@ -320,21 +320,6 @@ __device__ __noinline__ long long t4x_key(const T4xCores<f2>* v, const f2* tl, c
 }
 constexpr int kYGroupKeys = 4;  // combinations left of a group from which t4x_key makes all their keys
 
-// Bound (in bits) on |t4x_estimate - exact key / (ln2 * 2^32)|, N samples: each sample lies in one of the 81
-// cells, so sum s over the cells is N and sum s lg2 s <= N lg2 N.  A cell's products and sums round at most 5
-// times by 2^-24 of at most s lg2 s; lg2.approx is within 2^-18 of log2 on every input the kernel can see (checked
-// exhaustively by fiu_probe_lg2_error), which moves a cell by at most 2 s 2^-18; the x + 2^-20 shift moves each
-// of the 243 products by at most 2^-20 / ln 2 and its rounding each logarithm by at most 2^-24 / ln 2; the
-// running sum, below N, rounds 81 times; the integer table rounds each of the 243 exact terms by 1/2 of 2^-32
-// nats.  Doubled.  (0.3 bits at 8 000 samples, 4.9 at 130 000.)
-static double t4x_margin(int n_samples) {
-    const double N = n_samples, lgN = std::log2(std::max(2.0, N)), l2 = std::log(2.0);
-    const double u = std::ldexp(1.0, -24), e20 = std::ldexp(1.0, -20), e_lg2 = std::ldexp(1.0, -18);
-    const double err = 5 * u * N * lgN + 2 * N * e_lg2 + 243 * e20 / l2 + 2 * N * u / l2 + 82 * u * N +
-                       243 * 0.5 / (l2 * 4294967296.0);
-    return 2 * err + 1e-3;
-}
-
 // ALL: every combination takes the exact path (a search's first units, before a threshold; dumps and
 // digests).  Otherwise the bound comes first, a group with combinations above it gets their estimates
 // (t4x_estimate), and the few that pass those are evaluated from the data set (warp_exact_key): the exact

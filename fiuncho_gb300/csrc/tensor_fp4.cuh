@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "tensor_bounds.h"
 #include "tensor_common.cuh"
 
 namespace fiu {
@@ -193,20 +194,10 @@ __device__ __forceinline__ f2 f2_rcp(f2 v) {
     return f2_pack(a, b);
 }
 
-// ---- the quadratic bound on the mutual information ----------------------------
-// With q the control fraction, D(p||q) the binary relative entropy in bits and
-// s, b the size and the controls of a cell, N MI = sum over the cells of
-// s D(b/s || q).  D(p||q) <= c (p - q)^2 on [0, 1] for
-//     c = max(1 / (2 ln2 q (1-q)), -lg(1-q) / q^2, -lg(q) / (1-q)^2):
-// f(p) = D(p||q) - c (p-q)^2 has f(q) = f'(q) = 0 and
-// f'' = 1 / (ln2 p (1-p)) - 2c, which is <= 0 on an interval around q (first
-// term of the maximum) and > 0 beyond it, so f falls from 0 up to where the
-// interval ends and lies below its chord to the end point (second and third
-// terms) after that.  As the sizes add up to N and the controls to n_ctrls,
-//     N MI <= c (sum b^2 / s - n_ctrls^2 / N)      [bits],
-// one reciprocal a cell instead of three logarithms.  For q = 1/2 the bound is
-// at most 4 / (2 / ln2) = 1.39 times the value, so nearly every combination
-// falls below a top-N threshold and its logarithms are never taken.
+// ---- the quadratic bound on the mutual information (tensor_bounds.h) -------------
+// One reciprocal a cell instead of three logarithms.  For q = 1/2 the bound is at
+// most 4 / (2 / ln2) = 1.39 times the value, so nearly every combination falls
+// below a top-N threshold and its logarithms are never taken.
 //
 // Cells arrive packed, D = cases + W controls (exact in FP32): controls =
 // floor(D / W) by a fused multiply-add that rounds toward zero at 2^23.
@@ -268,18 +259,8 @@ struct F4BoundAB {
     }
 };
 
-// A closer bound, for tables of many cells (order 4, where the quadratic one
-// leaves a third of the warps a survivor).  g(p) = D(p||q) / (p-q)^2 is an
-// average of D''(q + u (p-q)) = 1 / (ln2 t (1-t)) over u, which is convex, so g
-// is convex in p and lies below its chord L(p) = g(0) + (g(1) - g(0)) p.  It lies
-// below Q(p) = L(p) - k p (1-p) as well, k the least (L - g) / (p (1-p)) (which
-// grows without limit towards both ends).  So D <= (p-q)^2 Q(p), exact at p = 0,
-// p = 1 and where k is taken.  Summed over the cells with p = b/s the powers
-// below the second give constants:
-//     N MI <= a0 N + a1 n_ctrls + sum b p (a2 + a3 p + a4 p^2).
-struct F4Quartic {
-    float a2, a3, a4;
-};
+// A closer bound (tensor_bounds.h), for tables of many cells: at order 4 the
+// quadratic one leaves a third of the warps a survivor.
 struct F4Bound4 : F4Bound {
     f2 a2, a3, a4;
     __device__ __forceinline__ F4Bound4(int p, const F4Quartic& k) : F4Bound(p) {
@@ -306,43 +287,6 @@ struct F4Bound4AB {
         acc = fmaf(b * pr, fmaf(pr, fmaf(pr, k.a4, k.a3), k.a2), acc);
     }
 };
-// The quartic bound's coefficients and test (as f4_quadratic).
-// Slack: a term of magnitude at most b (|a2| + |a3| + |a4|) carries at most 12
-// roundings of 2^-24, the sum `cells` more; doubled.
-inline F4Quartic f4_quartic(int n_cases, int n_ctrls, int cells, double& bound_k, double& bound_c) {
-    const double N = (double)n_cases + n_ctrls, q = n_ctrls / N, r = 1 - q, l2 = std::log(2.0);
-    const double L0 = -std::log2(r) / (q * q), L1 = -std::log2(q) / (r * r);
-    double k = 1e300;  // the least on a grid, lowered by 0.1 %: between grid points the ratio moves less
-    for (int i = 1; i < 1024; ++i) {
-        const double p = i / 1024.0, d = p - q;
-        const double g = std::fabs(d) < 1e-4 ? 1 / (2 * l2 * q * r)
-                                             : (p * std::log2(p / q) + (1 - p) * std::log2((1 - p) / r)) / (d * d);
-        k = std::min(k, (L0 + (L1 - L0) * p - g) / (p * (1 - p)));
-    }
-    k = std::max(0.0, k * 0.999 - 1e-4);
-    const double A = L0, B = L1 - L0 - k, C = k;
-    const double a4 = C, a3 = B - 2 * q * C, a2 = A - 2 * q * B + q * q * C, a1 = q * q * B - 2 * q * A, a0 = q * q * A;
-    const double S = std::fabs(a2) + std::fabs(a3) + std::fabs(a4), u = std::ldexp(1.0, -24);
-    const double slack = 2 * n_ctrls * S * (12 + 3 + cells) * u + 1e-3;  // 3: the coefficients' own rounding
-    bound_k = 1 - 1e-9;
-    bound_c = -a0 * N - a1 * n_ctrls - slack;
-    return F4Quartic{(float)a2, (float)a3, (float)a4};
-}
-
-// The quadratic bound's test (host): a combination whose N MI reaches thr_bits has
-// sum b^2 / s >= bound_k * thr_bits + bound_c.  Slack: each of `cells` terms, at
-// most b <= n_ctrls, carries at most 12 roundings or approximations of 2^-22 and
-// the sum `cells` more of 2^-24 of the total n_ctrls; the 2^-20 shift lowers a term
-// by at most 2^-20 of it.  Doubled.
-inline void f4_quadratic(int n_cases, int n_ctrls, int cells, double& bound_k, double& bound_c) {
-    const double N = (double)n_cases + n_ctrls, q = n_ctrls / N;
-    const double lg_q = std::log2(q), lg_1q = std::log2(1 - q);
-    const double c = std::max({1 / (2 * std::log(2.0) * q * (1 - q)), -lg_1q / (q * q), -lg_q / ((1 - q) * (1 - q))});
-    const double u = std::ldexp(1.0, -24);
-    bound_k = (1 - 1e-9) / c;
-    bound_c = q * n_ctrls * (1 - 1e-9) - (2 * n_ctrls * (12 * 4 * u + 16 * u + cells * u) + 1e-3);
-}
-
 // A threshold key as the kernels' tests, rounded down (device).
 __device__ __forceinline__ void live_tests(const LiveMap& m, long long thr, float& est, float& bound) {
     est = __double2float_rd(fma((double)thr, m.est_k, m.est_c));
