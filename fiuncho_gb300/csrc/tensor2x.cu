@@ -20,8 +20,9 @@
 // fixed-point key, so the kept set is the one of the exact key.
 //
 // Items are listed in bands of 512 i, j-tile by j-tile: the pairs at work share a
-// band's i rows and each j tile in L2 (40 000 SNPs x 16 000 samples: planes of 640
-// MB, read about once per band).
+// band's i rows and, in part, each j tile in L2.  40 000 SNPs x 16 000 samples: planes
+// of 640 MB, of which the 79 bands need the j above their first i, 25 GB in all; the
+// largest launch reads 67 GB (5.0 TB/s), 2.7 times that.
 //
 // Bound by the MMAs at many samples (40 000 SNPs x 8 000/8 000: 41.6 -> 14.3 ms a
 // search against e4m3 operands and one accumulator region per class, 94 % of 4 x

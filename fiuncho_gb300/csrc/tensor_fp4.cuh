@@ -27,19 +27,12 @@ __host__ __device__ constexpr uint32_t f4_idesc(int M, int N) {
     return (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | (1u << 23) | ((uint32_t)(M >> 4) << 24);
 }
 
-template <int CG>
 __device__ __forceinline__ void f4_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t sfa, uint32_t sfb,
                                        uint32_t acc) {
-    if (CG == 1)
-        asm volatile(
-            "{.reg .pred p; setp.ne.b32 p, %6, 0;\n"
-            "tcgen05.mma.cta_group::1.kind::mxf4.block_scale.block32 [%0], %1, %2, %3, [%4], [%5], p;}\n" ::"r"(d),
-            "l"(a), "l"(b), "r"(idesc), "r"(sfa), "r"(sfb), "r"(acc));
-    else
-        asm volatile(
-            "{.reg .pred p; setp.ne.b32 p, %6, 0;\n"
-            "tcgen05.mma.cta_group::2.kind::mxf4.block_scale.block32 [%0], %1, %2, %3, [%4], [%5], p;}\n" ::"r"(d),
-            "l"(a), "l"(b), "r"(idesc), "r"(sfa), "r"(sfb), "r"(acc));
+    asm volatile(
+        "{.reg .pred p; setp.ne.b32 p, %6, 0;\n"
+        "tcgen05.mma.cta_group::2.kind::mxf4.block_scale.block32 [%0], %1, %2, %3, [%4], [%5], p;}\n" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"(sfa), "r"(sfb), "r"(acc));
 }
 
 // The MMA issuer of a CTA-pair kernel (one elected thread of CTA 0): for each of
@@ -73,8 +66,8 @@ __device__ __forceinline__ bool f4_pair_issue(long long items, uint32_t a0, uint
                 asm volatile("tcgen05.fence::after_thread_sync;");
                 if (!acc) idesc = f4_idesc(256, n_of(SPLIT ? item >> 1 : item));
                 auto mma = [&](int k) {
-                    f4_mma<2>(dcol, (uint64_t)desc_hi << 32 | (ad + 2 * k), (uint64_t)desc_hi << 32 | (bd + 2 * k),
-                              idesc, one, sfb, acc);
+                    f4_mma(dcol, (uint64_t)desc_hi << 32 | (ad + 2 * k), (uint64_t)desc_hi << 32 | (bd + 2 * k), idesc,
+                           one, sfb, acc);
                     acc = 1;
                 };
                 mma(0);
