@@ -322,7 +322,8 @@ int fiu_scan_tables(fiu_ctx *ctx, const fiu_resident *res, unsigned order, const
  * (src/base/gt_popcnt.cpp:4-35) gives for every combination ThreadedSearch
  * visits (include/fiuncho/ThreadedSearch.h:157-180) without storing the tables.
  * The kernel `kernel` (FIU_KERNEL_*, FIU_KERNEL_AUTO = the search's own
- * choice; orders <= 4 for FIU_KERNEL_FULL) evaluates every combination of
+ * choice, for data with missing calls the full tables; orders <= 4 for
+ * FIU_KERNEL_FULL) evaluates every combination of
  * `distribution` (NULL = the whole data set) and
  *   *digest = sum over the combinations c (mod 2^64) of h(c), where
  *   v = c[0] snps^(order-1) + ... + c[order-1]   (uint64, wrapping),

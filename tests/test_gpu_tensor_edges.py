@@ -324,3 +324,31 @@ def test_order4_more_ties_than_the_buffer_holds(cases, ctrls):
     got = gs.run(Dataset(cases, ctrls, 70, ds.cases_words, ds.ctrls_words, rows.reshape(-1)), 4, Distribution(70, 3), 40)
     assert gs.last_tile()[0] == 4
     assert [tuple(r.combination) for r in got] == list(itertools.islice(itertools.combinations(range(70), 4), 40))
+
+
+@pytest.mark.parametrize("i,j,l", [(0, 1, 2), (0, 63, 71), (3, 40, 41), (5, 70, 71), (7, 36, 69), (69, 70, 71)])
+def test_order3_missing_calls_every_cell(i, j, l):
+    """A combination whose association lies in one of its 27 cells, for every cell as the kernel for data with
+    missing calls counts them (places at the edges of its tiles and halves): the best combinations (it and
+    those that share two of its SNPs) against the full-table kernel's."""
+    import itertools
+    import numpy as np
+    from fiuncho_gb300 import Dataset, Distribution, GpuSearch, _lib
+    gs = GpuSearch(0)
+    rng = np.random.default_rng(100 * i + j)
+    base = rng.integers(0, 3, (72, 590)).astype(np.uint8)
+    base[rng.random(base.shape) < 0.05] = 3
+    is_case = np.arange(590) < 300
+    for cell in itertools.product(range(3), repeat=3):
+        geno = base.copy()
+        rows = geno[[i, j, l]]
+        rows[:, rng.choice(300, 50, replace=False)] = np.array(cell, np.uint8)[:, None]
+        hit = (rows == np.array(cell, np.uint8)[:, None]).all(0) & ~is_case
+        rows[rng.integers(0, 3), hit] = 3  # no control has it
+        geno[[i, j, l]] = rows
+        ds, lists = Dataset.from_genotypes(geno, is_case), []
+        for kernel in (_lib.KERNEL_AUTO, _lib.KERNEL_FULL):
+            gs.set_kernel(kernel)
+            lists.append([(tuple(r.combination), r.val) for r in gs.run(ds, 3, Distribution(72, 2), 100)])
+            assert gs.last_tile()[0] == (kernel or _lib.KERNEL_TENSOR)
+        assert lists[0] == lists[1] and (i, j, l) in [c for c, _ in lists[0]], cell
