@@ -298,7 +298,7 @@ __device__ __noinline__ f2 t4x_estimate(const T4xCores<f2>* v, const std::condit
 // SPLIT: the exact key (without the base) of the combination in v, a lane each, from its cells, for groups with
 // several left (no threshold yet, or many that tie with it): one a warp from the data set (warp_exact_key) takes
 // 10 to 70 us at these classes' samples.  Bound by its gathers from the c ln c table.  100 copies of one SNP x
-// 18 000 samples, all combinations tied: 1 920 -> 90 ms (e4m3 kernel 724); a layer of 100 SNPs, step 7, 7 000
+// 18 000 samples, all combinations tied: 1 920 -> 72 ms (e4m3 kernel 724); a layer of 100 SNPs, step 7, 7 000
 // outputs 12.5 -> 8.7.  Classes that share an accumulator stay with warp_exact_key, which is short there: with this
 // beside it their kernel's code came out 6 % slower (300 SNPs x 558/1 012 28.5 -> 30.4 ms; all tied, 100 x
 // 2 000, 232 -> 58, e4m3 407).
