@@ -127,6 +127,7 @@ int choose_kernel(fiu_ctx* ctx, const fiu_resident* res_c, unsigned order, int r
     if (!elided_ok)
         return fail(ctx, FIU_ERR_UNSUPPORTED,
                     "elided kernels need one-hot data, order 2, 3 or 4 (at most 1 150 SNPs), classes <= 65535");
+    std::lock_guard<std::mutex> g(res->mu);
     const bool need_pairs = order >= 3 && !res->pairs, need_triples = order == 4 && !res->triples;
     if (!res->single || need_pairs || need_triples) {
         const long long np = (long long)res->d.snps * (res->d.snps - 1) / 2;
@@ -199,6 +200,7 @@ bool e4_pair_major(int kernel, const fiu_resident* res, const ScanWork& w) {
 // Work-item table of the pair-major order-4 schedule, built once per data set.
 static int ensure_e4_items(fiu_ctx* ctx, const fiu_resident* res_c) {
     fiu_resident* res = const_cast<fiu_resident*>(res_c);
+    std::lock_guard<std::mutex> g(res->mu);
     if (res->e4_begin) return FIU_OK;
     const std::vector<long long> b = e4p_item_begin(res->d.snps);
     long long* d = nullptr;
@@ -208,8 +210,8 @@ static int ensure_e4_items(fiu_ctx* ctx, const fiu_resident* res_c) {
         cudaFree(d);
         return cuda_fail(ctx, e, "work-item table");
     }
-    res->e4_begin = d;
     res->e4_items = b.back();
+    res->e4_begin = d;
     return FIU_OK;
 }
 
@@ -251,17 +253,23 @@ static bool missing_ok(const fiu_resident* res, const ScanWork& w) {
            res->d.n_ctrls <= 65535 && res->d.snps < (1 << 21) && f4_pack(res->d.n_cases, res->d.n_ctrls) != 0;
 }
 
-// Its operands and work items, made on the first such search.
-static int missing_plan(fiu_ctx* ctx, const fiu_resident* res) {
+// A data set's plan of the tensor kernels, made on the first search that takes them.
+static int tensor_plan(fiu_ctx* ctx, const fiu_resident* res) {
     fiu_resident* r = const_cast<fiu_resident*>(res);
-    if (!r->t3) {
-        auto* plan = new (std::nothrow) T3Plan;
-        if (!plan) return fail(ctx, FIU_ERR_NOMEM, "tensor plan");
-        tensor3_prepare(r->d, *plan);
-        plan->missing = true;
-        r->t3 = plan;
-    }
-    const cudaError_t e = tensor3_order_items(*r->t3, r->d, 3, nullptr, ctx->stream, ctx->sms);
+    std::lock_guard<std::mutex> g(r->mu);
+    if (r->t3) return FIU_OK;
+    auto* plan = new (std::nothrow) T3Plan;
+    if (!plan) return fail(ctx, FIU_ERR_NOMEM, "tensor plan");
+    tensor3_prepare(r->d, *plan);
+    plan->missing = !r->one_hot;
+    r->t3 = plan;
+    return FIU_OK;
+}
+
+// The operands and work items of data with missing calls, made on the first such search.
+static int missing_plan(fiu_ctx* ctx, const fiu_resident* res) {
+    if (const int rc = tensor_plan(ctx, res)) return rc;
+    const cudaError_t e = tensor3_order_items(*res->t3, res->d, 3, nullptr, ctx->stream, ctx->sms);
     if (e == cudaSuccess) return FIU_OK;
     cudaGetLastError();
     return cuda_fail(ctx, e, "tensor operands and work items");
@@ -294,26 +302,21 @@ int choose_tile(fiu_ctx* ctx, const fiu_resident* res, const ScanWork& w, int re
             return fail(ctx, FIU_ERR_UNSUPPORTED,
                         "the tensor-core kernels need one-hot data, order 2, 3 or 4 and the whole data set on one "
                         "worker");
-        fiu_resident* r = const_cast<fiu_resident*>(res);
-        if (!r->t3) {
-            auto* plan = new (std::nothrow) T3Plan;
-            if (!plan) return fail(ctx, FIU_ERR_NOMEM, "tensor plan");
-            tensor3_prepare(r->d, *plan);
-            r->t3 = plan;
-        }
+        int rc = tensor_plan(ctx, res);
+        if (rc) return rc;
         // the single and pair cores (order 4 makes its triples itself)
-        int rc = choose_kernel(ctx, res, std::min(3u, (unsigned)w.order), FIU_KERNEL_ELIDED_HS, kernel);
+        rc = choose_kernel(ctx, res, std::min(3u, (unsigned)w.order), FIU_KERNEL_ELIDED_HS, kernel);
         if (rc) return rc;
         if (!whole_data_set(res, w)) {
-            cudaError_t e = tensor3_layer(*r->t3, w, res->pairs, ctx->stream, ctx->sms);
+            cudaError_t e = tensor3_layer(*res->t3, w, res->pairs, ctx->stream, ctx->sms);
             if (e != cudaSuccess) return cuda_fail(ctx, e, "tensor work items of a distribution layer");
         } else {
-            cudaError_t e = tensor3_order_items(*r->t3, r->d, w.order, res->pairs, ctx->stream, ctx->sms);
+            cudaError_t e = tensor3_order_items(*res->t3, res->d, w.order, res->pairs, ctx->stream, ctx->sms);
             if (e != cudaSuccess) return cuda_fail(ctx, e, "tensor operands and work items");
         }
         kernel = FIU_KERNEL_TENSOR;
         // the tile class reported by fiu_last_tile: 192 names order 3 with one accumulator per class
-        tp = w.order != 3 || r->t3->f4.pack ? 256 : 192;
+        tp = w.order != 3 || res->t3->f4.pack ? 256 : 192;
         return FIU_OK;
     }
     int rc = choose_kernel(ctx, res, (unsigned)w.order, requested_kernel, kernel);

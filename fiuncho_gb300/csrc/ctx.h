@@ -4,6 +4,7 @@
 
 #include <atomic>
 #include <map>
+#include <mutex>
 #include <string>
 #include <utility>
 
@@ -65,6 +66,7 @@ struct fiu_resident {
     int one_hot = 0;
     int disjoint = 0;  // no sample has two genotypes at an SNP, and none past a class's last is set
     int device = 0;
+    std::mutex mu;  // guards the making, on first use, of what follows: several contexts may search a data set at once
     uint32_t* single = nullptr;  // single-SNP cores (elided kernels)
     uint4* pairs = nullptr;      // pair cores (elided order-3 and order-4 kernels)
     uint4* triples = nullptr;    // triple cores (elided order-4 kernel)

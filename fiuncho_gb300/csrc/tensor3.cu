@@ -210,7 +210,10 @@ static const T3Layer* find_layer(const T3Plan& plan, const ScanWork& w) {
 
 cudaError_t tensor3_layer(T3Plan& plan, const ScanWork& w, const uint4* pairs, cudaStream_t s, int sms) {
     if (!tensor_layer_ok(plan, w)) return cudaErrorInvalidValue;
-    if (!plan.layers) plan.layers = new T3Layers;
+    {
+        std::lock_guard<std::mutex> gp(plan.items_mu);
+        if (!plan.layers) plan.layers = new T3Layers;
+    }
     std::lock_guard<std::mutex> g(plan.layers->mu);
     const auto key = std::make_tuple(w.order, w.dist_step, w.dist_offset);
     if (plan.layers->by.count(key)) return cudaSuccess;

@@ -2,19 +2,23 @@
 // wrapped (-Wl,--wrap) by a fake that keeps "device" memory on the host, launches nothing and fails the
 // k-th call on demand.  For every k: what another search may be reading stays, nothing that was begun
 // is taken for made, a second try completes, and at the end nothing is left allocated.
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <set>
+#include <thread>
 #include <vector>
 
 #include "ctx.h"
 #include "tensor3x.h"
 
 static std::set<void*> live;
-static long calls = 0, fail_at = 0, launches = 0, maps = 0;
+static std::mutex fake_mu;  // (the last scenario has several threads)
+static std::atomic<long> calls{0}, fail_at{0}, launches{0}, maps{0};
 static bool failing() { return ++calls == fail_at; }
-#define CHECK(c) do { if (!(c)) { std::printf("%s:%d: %s (fail_at %ld)\n", __FILE__, __LINE__, #c, fail_at); std::exit(1); } } while (0)
+#define CHECK(c) do { if (!(c)) { std::printf("%s:%d: %s (fail_at %ld)\n", __FILE__, __LINE__, #c, fail_at.load()); std::exit(1); } } while (0)
 
 static CUresult encode(CUtensorMap* m, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                        const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -27,12 +31,15 @@ static CUresult encode(CUtensorMap* m, CUtensorMapDataType, cuuint32_t, void*, c
 extern "C" {
 cudaError_t __wrap_cudaMalloc(void** p, size_t n) {
     if (failing()) return cudaErrorMemoryAllocation;
+    std::this_thread::yield();
+    std::lock_guard<std::mutex> g(fake_mu);
     *p = std::calloc(1, n ? n : 1);
     live.insert(*p);
     return cudaSuccess;
 }
 cudaError_t __wrap_cudaFree(void* p) {
     if (!p) return cudaSuccess;
+    std::lock_guard<std::mutex> g(fake_mu);
     CHECK(live.erase(p) == 1);
     std::free(p);
     return cudaSuccess;
@@ -146,9 +153,41 @@ static void core_tables() {
     CHECK(live.empty());
 }
 
+// Several contexts make the tables, plan and layer of one data set at once: each is made once.
+static void at_once() {
+    for (int round = 0; round < 200; ++round) {
+        fiu_resident r;
+        r.d = kData;
+        r.one_hot = 1;
+        std::vector<std::thread> threads;
+        std::vector<int> rc(4, -1);
+        for (int t = 0; t < 4; ++t)
+            threads.emplace_back([&, t] {
+                fiu_ctx ctx;
+                ctx.sms = 152;
+                ScanWork w{};
+                w.d = kData;
+                w.order = 2 + t % 3;
+                w.dist_n = kData.snps;
+                w.dist_step = t == 3 ? 3 : 1;
+                int kernel = 0, tp = 0;
+                rc[t] = choose_tile(&ctx, &r, w, FIU_KERNEL_AUTO, kernel, tp, Use::kSearch);
+            });
+        for (std::thread& t : threads) t.join();
+        for (int e : rc) CHECK(e == FIU_OK);
+        CHECK(r.single && r.pairs && r.t3);
+        tensor3_release(*r.t3);
+        delete r.t3;
+        __wrap_cudaFree(r.single);
+        __wrap_cudaFree(r.pairs);
+        CHECK(live.empty());
+    }
+}
+
 int main() {
     whole_scans();
     layers();
     core_tables();
+    at_once();
     std::printf("ok\n");
 }
