@@ -300,8 +300,7 @@ __device__ __noinline__ f2 t4x_estimate(const T4xCores<f2>* v, const std::condit
 // 10 to 70 us at these classes' samples.  Bound by its gathers from the c ln c table.  100 copies of one SNP x
 // 18 000 samples, all combinations tied: 1 920 -> 72 ms (e4m3 kernel 724); a layer of 100 SNPs, step 7, 7 000
 // outputs 12.5 -> 8.7.  Classes that share an accumulator stay with warp_exact_key, which is short there: with this
-// beside it their kernel's code came out 6 % slower (300 SNPs x 558/1 012 28.5 -> 30.4 ms; all tied, 100 x
-// 2 000, 232 -> 58, e4m3 407).
+// beside it their kernel's code came out 6 % slower (300 SNPs x 558/1 012 28.5 -> 30.4 ms).
 __device__ __noinline__ long long t4x_key(const T4xCores<f2>* v, const f2* tl, const f2* tabk0, int zb,
                                           const DevData* d) {
     const uint32_t nc = (uint32_t)d->n_cases, nt = (uint32_t)d->n_ctrls;
